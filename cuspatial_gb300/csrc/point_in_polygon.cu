@@ -15,18 +15,18 @@
 // float64 instruction) and the float32 filter decides each polygon, as in the
 // quadtree join.
 //
-// Pairwise form: every polygon is used once, so no index is built; a group
-// of G lanes (1, 4, 8 or 32, from the mean polygon size) walks the polygon's
-// edges in parallel and combines the edge results (on-edge OR, crossing
+// Pairwise form: every polygon is used once, so no index is built; a warp
+// walks the vertices of up to 32 consecutive polygons as one run, one vertex
+// per lane, and combines the edge results per ring (on-edge OR, crossing
 // parity XOR), which equals the reference's sequential walk wherever its
 // skipped vertices are exact repeats (polygon_index.cuh, points 1 and 2);
 // polygons where that can fail (non-finite or sub-2^-1019 coordinates) are
-// walked sequentially by the group's first lane.  With float64 input and the
-// filtered method each vertex is moved into the point's frame in float32
-// (one float64 subtraction per coordinate) and an edge falls back to the
-// reference's float64 expression only where the error bound below cannot
-// decide it.
+// walked sequentially by one lane.  With float64 input and the filtered
+// method each vertex is moved into the point's frame in float32 on the
+// integer and float32 pipes, and an edge takes the reference's float64
+// expression only where the error bound below cannot decide it.
 #include "common.cuh"
+#include "f32_split.cuh"
 #include "pip_test.cuh"
 #include "polygon_index.cuh"
 
@@ -200,137 +200,254 @@ __device__ inline bool tiny_bits(double a)
 }
 __device__ inline bool tiny_bits(float a) { return ((__float_as_uint(a) >> 23) & 0xFFu) <= 3u; }
 
-template <int G, typename V>
-__device__ inline V group_up(unsigned gmask, V v)
-{
-  if constexpr (G == 1)
-    return v;
-  else
-    return __shfl_up_sync(gmask, v, 1, G);
-}
-template <int G, typename V>
-__device__ inline V group_last(unsigned gmask, V v)
-{
-  if constexpr (G == 1)
-    return v;
-  else
-    return __shfl_sync(gmask, v, G - 1, G);
-}
-
-// Pairwise form: a group of G lanes per (point i, polygon i).  Lane g takes
-// the vertices v0 + c + g of each ring; the edge ending at vertex v starts at
-// v - 1 (the ring's last vertex for v0), passed from the neighbouring lane.
+// Pairwise form: a warp takes `per_warp` consecutive (point, polygon) pairs.
+// Their polygons' vertices are one contiguous run, which the warp walks 32
+// vertices at a time, one per lane, whatever the sizes of the rings in it: no
+// lane waits for a larger polygon, and every load is coalesced.  The rings
+// come 32 at a time, one per lane (vertex range, its point's offset parts,
+// its closing vertex); a vertex finds its ring by counting ring starts, and
+// the chunk's toggles and on-edge hits go back to the rings as ballots.
 //
-// Filtered (float64 input): a = fl32(v_a - p), b = fl32(v_b - p) with one
-// rounding each (|error| <= u32 M, M = max |a|, |b|).  The reference compares
-// lhs = (px - ax)(by - ay) with rhs = (bx - ax)(py - ay), whose difference is
-// a_y b_x - a_x b_y; cr = fma(a_y, b_x, -a_x b_y) is within 7 u32 M^2 of it,
-// the float64 roundings of lhs and rhs add 12 u64 M^2 and the 4-ULP collinear
-// band 2^-49 M^2, all below eb = 2^-17 M^2 (+ 2^-120 for float32 underflow).
-// The y-flags (ay > py) are the signs of a_y and b_y, exact unless zero; the
-// x-range (min(ax, bx) <= px <= max(ax, bx)) is excluded when a_x and b_x
-// have the same non-zero sign.  Anything else goes to the float64 edge test.
-template <typename T, int G, bool Filtered>
-__global__ void __launch_bounds__(kPointsBlock)
+// Filtered (float64 input): a vertex coordinate minus the point's is taken
+// from the float32 parts of both (f32_split.cuh):
+//   f = (hi_v - hi_p) + (lo_v - lo_p),  |f - (v - p)| <= 2^-23 |f| + 2^-44 (|v| + |p|)
+// (three float32 roundings and the parts left out).  Per edge, with
+// m = max |f| of its two ends on an axis and p's coordinate there,
+//   t = 2^-20 m + 2^-41 |p| + 2^-60
+// is more than 4 times that error (|v| <= |p| + 1.01 m).
+//   * Both y offsets beyond t_y: the y-flags (ay > py) are their signs.
+//   * Same flags: the edge cannot toggle, and can be on the point only if it
+//     is within 2^-48 |rise| of py (it is not: t_y >= 2^-21 |rise|) or exactly
+//     vertical at px; with one x offset beyond t_x it is not vertical there.
+//   * Flags differ and both x offsets beyond t_x on one side: px is outside
+//     the edge's x-range, so it is not on the edge, and the reference's
+//     comparison of lhs = (px - ax)(by - ay) with rhs = (bx - ax)(py - ay) has
+//     |px - ax| >= |bx - ax| + t_x on the right of both (or a sign that
+//     decides) and |by - ay| >= |py - ay| + t_y, far beyond its roundings:
+//     toggles exactly when px is left of the edge.
+//   * Flags differ otherwise: cr = a_y b_x - a_x b_y in float32 against
+//     eb = 2 (t_x (|a_y| + |b_y|) + t_y (|a_x| + |b_x|)), above the offsets'
+//     errors, float32's roundings (2^-23 of each product) and float64's.
+// Anything else, and any vertex with a coordinate that does not split (zero,
+// below 2^-100, 2^100 and above, non-finite), takes the reference's float64
+// edge test, which also finds the polygons that need the sequential walk
+// (non-finite or sub-2^-1019 coordinates): its skip rule can differ only
+// where a coordinate is below 2^-1019.
+//
+// 1M pairs of 4..400 vertices (9.4e7 vertices, 1.56 GB): 3.37 ms with a
+// float64 subtraction and conversion per coordinate (float64 pipe 83% busy)
+// and 8 lanes per polygon, 0.61 ms this way (2.5 TB/s; bound by instruction
+// issue and the vertex loads: without the next chunk's loads in flight 1.18).
+// Five resident blocks of 256 measured fastest: 0.99 / 0.71 / 0.64 / 0.61 ms
+// with 2 / 3 / 4 / 5.  Exact float64: 7.8 -> 2.9 ms, float32 1.36 -> 0.50.
+template <typename T, bool Filtered>
+__global__ void __launch_bounds__(kPointsBlock, 5)
   pairwise_pip_kernel(T const* __restrict__ x, T const* __restrict__ y, size_t n,
                       uint32_t const* __restrict__ po, uint32_t const* __restrict__ ro,
-                      T const* __restrict__ vx, T const* __restrict__ vy,
+                      T const* __restrict__ vx, T const* __restrict__ vy, uint32_t per_warp,
                       uint8_t* __restrict__ out, unsigned long long* __restrict__ refined)
 {
-  static_assert(G == 1 || G == 4 || G == 8 || G == 32, "group width");
-  int const lane       = threadIdx.x & 31;
-  int const g          = lane & (G - 1);
-  unsigned const gmask = G == 32 ? 0xFFFFFFFFu : (((1u << G) - 1u) << (lane & ~(G - 1)));
-  size_t const per_warp = 32 / G;
-  size_t const warp     = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
-  size_t const nwarps   = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
-  uint32_t nref         = 0;
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  // what a lane keeps of a vertex: its float32 offset, or the vertex itself
+  using V                 = typename std::conditional<Filtered, float, T>::type;
+  unsigned const lane     = threadIdx.x & 31;
+  unsigned const le       = kAll >> (31u - lane);  // this lane and those below
+  size_t const warp       = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
+  size_t const nwarps     = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
+  uint32_t nref           = 0;
   for (size_t base = warp * per_warp; base < n; base += nwarps * per_warp) {
-    size_t const i = base + static_cast<size_t>(lane / G);
-    if (i >= n) continue;  // uniform over the group
-    T const px    = x[i];
-    T const py    = y[i];
-    bool on       = false;
-    bool within   = false;
-    bool literal  = !(isfinite(px) && isfinite(py));
+    uint32_t const np = n - base < per_warp ? static_cast<uint32_t>(n - base) : per_warp;
+    // lane p: pair base + p
+    bool const have_p = lane < np;
+    size_t const i    = base + (have_p ? lane : np - 1);
+    T const px = x[i], py = y[i];
     uint32_t const r0 = po[i], r1 = po[i + 1];
-    for (uint32_t r = r0; r < r1 && !literal; ++r) {
-      uint32_t const v0 = ro[r], v1 = ro[r + 1];
-      if (v1 <= v0) continue;
-      // the edge into v0 starts at the ring's last vertex
-      T cx = T{0}, cy = T{0};
-      float cfx = 0.0f, cfy = 0.0f;
-      if (g == 0) {
-        cx = vx[v1 - 1];
-        cy = vy[v1 - 1];
-        if constexpr (Filtered) {
-          cfx = static_cast<float>(cx - px);
-          cfy = static_cast<float>(cy - py);
-        }
-      }
-      for (uint32_t c = v0; c < v1; c += G) {
-        uint32_t const v = c + static_cast<uint32_t>(g);
-        bool const own   = v < v1;
-        T const ax       = own ? vx[v] : T{0};
-        T const ay       = own ? vy[v] : T{0};
-        float fax = 0.0f, fay = 0.0f;
-        if constexpr (Filtered) {
-          fax = static_cast<float>(ax - px);
-          fay = static_cast<float>(ay - py);
-        }
-        T bx = group_up<G>(gmask, ax), by = group_up<G>(gmask, ay);
-        float fbx = group_up<G>(gmask, fax), fby = group_up<G>(gmask, fay);
-        if (g == 0) {
-          bx  = cx;
-          by  = cy;
-          fbx = cfx;
-          fby = cfy;
-        }
-        // the next chunk's first edge starts at this chunk's last vertex
-        cx  = group_last<G>(gmask, ax);
-        cy  = group_last<G>(gmask, ay);
-        cfx = group_last<G>(gmask, fax);
-        cfy = group_last<G>(gmask, fay);
-        if (!own) continue;
-        bool const ex = same_bits(ax, bx), ey = same_bits(ay, by);
-        if (!(isfinite(ax) && isfinite(ay)) ||
-            ((ex || (tiny_bits(ax) && tiny_bits(bx))) &&
-             (ey || (tiny_bits(ay) && tiny_bits(by))) && !(ex && ey))) {
-          literal = true;  // the reference's skip rule needs the sequential walk
-          continue;
-        }
-        if (ex && ey) continue;  // repeated vertex: skipped, b kept
-        int ee = -1;
-        if constexpr (Filtered) {
-          float const m = fmaxf(fmaxf(fabsf(fax), fabsf(fay)), fmaxf(fabsf(fbx), fabsf(fby)));
-          if (m < 1.152921504606847e18f) {  // 2^60: M^2 finite
-            float const eb  = __fmaf_rn(7.62939453125e-06f * m, m, 7.52316384526264e-37f);
-            float const cr  = __fmaf_rn(fay, fbx, -(fax * fby));
-            bool const y1   = fay > 0.0f;
-            bool const y0   = fby > 0.0f;
-            bool const xout = (fax > 0.0f && fbx > 0.0f) || (fax < 0.0f && fbx < 0.0f);
-            bool const undecided =
-              fay == 0.0f || fby == 0.0f || (fabsf(cr) <= eb && (y1 != y0 || !xout));
-            if (!undecided) ee = (y1 != y0 && ((cr < 0.0f) != y1)) ? 1 : 0;
-          }
-          if (ee < 0) ++nref;
-        }
-        if (ee < 0) ee = exact_edge<T>(px, py, ax, ay, bx, by);
-        if (ee == 2) on = true;
-        if (ee == 1) within = !within;
-      }
-      if constexpr (G > 1) literal = __any_sync(gmask, literal);
+    bool literal = !(isfinite(px) && isfinite(py));
+    bool on = false, within = false;
+    F32Pair fx{0.0f, 0.0f}, fy{0.0f, 0.0f};
+    if constexpr (Filtered) {
+      // a point coordinate of 0 is its own parts; others that do not split
+      // make every edge undecided
+      float const nan = __int_as_float(0x7FC00000);
+      if (px != T{0}) fx = splits_f32(px) ? split_f32(px) : F32Pair{nan, nan};
+      if (py != T{0}) fy = splits_f32(py) ? split_f32(py) : F32Pair{nan, nan};
     }
-    if constexpr (G > 1) {
+    uint32_t const rb = __shfl_sync(kAll, r0, 0);
+    uint32_t const re = __shfl_sync(kAll, r1, static_cast<int>(np - 1));
+    for (uint32_t rr = rb; rr < re; rr += 32) {
+      // lane j: ring rr + j, vertices [s, e)
+      uint32_t const nr = re - rr < 32u ? re - rr : 32u;
+      uint32_t const r  = rr + (lane < nr ? lane : nr - 1u);
+      uint32_t const e  = ro[r + 1];
+      uint32_t const s  = lane < nr ? ro[r] : e;
+      // the pair holding the ring: the first whose rings end beyond it
+      uint32_t pl = 0;
 #pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) {
-        on     = on | static_cast<bool>(__shfl_xor_sync(gmask, static_cast<int>(on), o, G));
-        within = within != static_cast<bool>(__shfl_xor_sync(gmask, static_cast<int>(within), o, G));
-        literal =
-          literal | static_cast<bool>(__shfl_xor_sync(gmask, static_cast<int>(literal), o, G));
+      for (int step = 16; step > 0; step >>= 1) {
+        uint32_t const v = __shfl_sync(kAll, r1, static_cast<int>(pl) + step - 1);
+        if (v <= r && pl + step < np) pl += step;
       }
+      F32Pair qx{}, qy{};
+      T rpx{}, rpy{};
+      if constexpr (Filtered) {
+        qx = F32Pair{__shfl_sync(kAll, fx.hi, pl), __shfl_sync(kAll, fx.lo, pl)};
+        qy = F32Pair{__shfl_sync(kAll, fy.hi, pl), __shfl_sync(kAll, fy.lo, pl)};
+      } else {
+        rpx = __shfl_sync(kAll, px, pl);
+        rpy = __shfl_sync(kAll, py, pl);
+      }
+      // the vertex, or its offset from the point with parts (ox, oy): NaN
+      // where the vertex does not split
+      auto keep = [](T ax, T ay, F32Pair const& ox, F32Pair const& oy, V& fa, V& fb) {
+        if constexpr (Filtered) {
+          F32Pair const a = split_f32(ax), b = split_f32(ay);
+          bool const ok   = splits_f32(ax) && splits_f32(ay);
+          float const nan = __int_as_float(0x7FC00000);
+          fa              = ok ? (a.hi - ox.hi) + (a.lo - ox.lo) : nan;
+          fb              = ok ? (b.hi - oy.hi) + (b.lo - oy.lo) : nan;
+        } else {
+          fa = ax;
+          fb = ay;
+        }
+      };
+      // the edge into a ring's first vertex starts at its last
+      V zx{}, zy{};
+      if (e > s) keep(vx[e - 1], vy[e - 1], qx, qy, zx, zy);
+      bool rpar = false, ron = false, rlit = false;
+      uint32_t const vb   = __shfl_sync(kAll, s, 0);
+      uint32_t const ve   = __shfl_sync(kAll, e, static_cast<int>(nr - 1));
+      bool const empties  = __any_sync(kAll, lane < nr && e <= s);
+      uint32_t before     = 0;  // rings that start before the chunk
+      V cx{}, cy{};                // the vertex before the chunk
+      // the next chunk's vertices are loaded while this one's are tested
+      T nx = vb + lane < ve ? vx[vb + lane] : T{1};
+      T ny = vb + lane < ve ? vy[vb + lane] : T{1};
+      for (uint32_t c = vb; c < ve; c += 32) {
+        uint32_t const v = c + lane;
+        bool const own   = v < ve;
+        T const ax = nx, ay = ny;
+        bool const more = ve - c > 32u && v + 32u < ve;
+        nx              = more ? vx[v + 32u] : T{1};
+        ny              = more ? vy[v + 32u] : T{1};
+        // the vertex's ring
+        uint32_t const d   = s - c;
+        unsigned const beg = __reduce_or_sync(kAll, (d < 32u && e > s) ? 1u << d : 0u);
+        int k              = static_cast<int>(before + __popc(beg & le)) - 1;
+        if (empties) {
+          k = 0;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1) {
+            uint32_t const q = __shfl_sync(kAll, e, k + step - 1);
+            if (q <= v && k + step < 32) k += step;
+          }
+        }
+        before += __popc(beg);
+        bool und = own, tog = false, hit = false, lit = false;
+        F32Pair ox{}, oy{};
+        if constexpr (Filtered) {
+          ox = F32Pair{__shfl_sync(kAll, qx.hi, k), __shfl_sync(kAll, qx.lo, k)};
+          oy = F32Pair{__shfl_sync(kAll, qy.hi, k), __shfl_sync(kAll, qy.lo, k)};
+        }
+        V fax, fay;
+        keep(ax, ay, ox, oy, fax, fay);
+        V fbx = __shfl_up_sync(kAll, fax, 1), fby = __shfl_up_sync(kAll, fay, 1);
+        if (lane == 0) {
+          fbx = cx;
+          fby = cy;
+        }
+        V const wx = __shfl_sync(kAll, zx, k), wy = __shfl_sync(kAll, zy, k);
+        if ((beg >> lane) & 1u) {
+          fbx = wx;
+          fby = wy;
+        }
+        cx = __shfl_sync(kAll, fax, 31);
+        cy = __shfl_sync(kAll, fay, 31);
+        if constexpr (Filtered) {
+          float const tx = __fmaf_rn(9.5367431640625e-07f, fmaxf(fabsf(fax), fabsf(fbx)),
+                                     __fmaf_rn(4.547473508864641e-13f, fabsf(ox.hi),
+                                               8.673617379884035e-19f));
+          float const ty = __fmaf_rn(9.5367431640625e-07f, fmaxf(fabsf(fay), fabsf(fby)),
+                                     __fmaf_rn(4.547473508864641e-13f, fabsf(oy.hi),
+                                               8.673617379884035e-19f));
+          if (own && fabsf(fay) > ty && fabsf(fby) > ty) {
+            bool const y1 = fay > 0.0f, y0 = fby > 0.0f;
+            if (y1 == y0) {
+              und = !(fabsf(fax) > tx || fabsf(fbx) > tx);
+            } else if (fabsf(fax) > tx && fabsf(fbx) > tx && (fax > 0.0f) == (fbx > 0.0f)) {
+              tog = fax > 0.0f;
+              und = false;
+            } else {
+              float const cr = __fmaf_rn(fay, fbx, -(fax * fby));
+              float const eb = 2.0f * __fmaf_rn(tx, fabsf(fay) + fabsf(fby),
+                                                ty * (fabsf(fax) + fabsf(fbx)));
+              und            = !(fabsf(cr) > eb);
+              tog            = !und && (cr < 0.0f) != y1;
+            }
+          }
+        }
+        if (__any_sync(kAll, und)) {
+          // the edge in the reference's arithmetic
+          T bx, by, qpx, qpy;
+          if constexpr (Filtered) {
+            uint32_t const ek = __shfl_sync(kAll, e, k);
+            uint32_t const pk = __shfl_sync(kAll, pl, k);
+            uint32_t const sk = __shfl_sync(kAll, s, k);
+            uint32_t const u  = v == sk ? ek - 1u : v - 1u;
+            if (und) {
+              bx  = vx[u];
+              by  = vy[u];
+              qpx = x[base + pk];
+              qpy = y[base + pk];
+            }
+          } else {
+            bx  = fbx;
+            by  = fby;
+            qpx = __shfl_sync(kAll, rpx, k);
+            qpy = __shfl_sync(kAll, rpy, k);
+          }
+          if (und) {
+            bool const ex = same_bits(ax, bx), ey = same_bits(ay, by);
+            if (!(isfinite(ax) && isfinite(ay)) ||
+                ((ex || (tiny_bits(ax) && tiny_bits(bx))) &&
+                 (ey || (tiny_bits(ay) && tiny_bits(by))) && !(ex && ey))) {
+              lit = true;  // the reference's skip rule needs the sequential walk
+            } else if (!(ex && ey)) {  // a repeated vertex is skipped, b kept
+              if (Filtered) ++nref;
+              int const ee = exact_edge<T>(qpx, qpy, ax, ay, bx, by);
+              hit          = ee == 2;
+              tog          = ee == 1;
+            }
+          }
+        }
+        unsigned const bt = __ballot_sync(kAll, tog);
+        unsigned const bh = __ballot_sync(kAll, hit);
+        unsigned const bl = __ballot_sync(kAll, lit);
+        if ((bt | bh | bl) != 0u) {
+          // the lanes of ring j in this chunk
+          uint32_t const lo   = s > c ? (s - c < 32u ? s - c : 32u) : 0u;
+          uint32_t const hi   = e > c ? (e - c < 32u ? e - c : 32u) : 0u;
+          unsigned const upto = hi ? kAll >> (32u - hi) : 0u;
+          unsigned const from = lo < 32u ? kAll << lo : 0u;
+          unsigned const mine = lane < nr ? upto & from : 0u;
+          rpar                = rpar != static_cast<bool>(__popc(bt & mine) & 1u);
+          ron |= (bh & mine) != 0u;
+          rlit |= (bl & mine) != 0u;
+        }
+      }
+      // rings [r0, r1) of pair p within this batch
+      uint32_t const lo   = r0 > rr ? (r0 - rr < 32u ? r0 - rr : 32u) : 0u;
+      uint32_t const hi   = r1 > rr ? (r1 - rr < 32u ? r1 - rr : 32u) : 0u;
+      unsigned const upto = hi ? kAll >> (32u - hi) : 0u;
+      unsigned const from = lo < 32u ? kAll << lo : 0u;
+      unsigned const mine = upto & from;
+      unsigned const bp   = __ballot_sync(kAll, rpar);
+      unsigned const bo   = __ballot_sync(kAll, ron);
+      unsigned const bq   = __ballot_sync(kAll, rlit);
+      within              = within != static_cast<bool>(__popc(bp & mine) & 1u);
+      on |= (bo & mine) != 0u;
+      literal |= (bq & mine) != 0u;
     }
-    if (g == 0) {
+    if (have_p) {
       bool hit = !on && within;
       if (literal) {
         PolygonIndexView<T> v{};
@@ -344,9 +461,20 @@ __global__ void __launch_bounds__(kPointsBlock)
     }
   }
   if (Filtered && refined) {
-    for (int o = 16; o > 0; o >>= 1) nref += __shfl_xor_sync(0xFFFFFFFFu, nref, o);
+    for (int o = 16; o > 0; o >>= 1) nref += __shfl_xor_sync(kAll, nref, o);
     if (lane == 0 && nref) atomicAdd(refined, static_cast<unsigned long long>(nref));
   }
+}
+
+// One lane per pair walks its polygon with the reference's loop.
+template <typename T>
+__global__ void __launch_bounds__(kPointsBlock)
+  pairwise_lane_kernel(T const* __restrict__ x, T const* __restrict__ y, size_t n,
+                       PolygonIndexView<T> v, uint8_t* __restrict__ out)
+{
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x)
+    out[i] = ring_walk<T>(x[i], y[i], v, static_cast<uint32_t>(i)) ? 1 : 0;
 }
 
 unsigned points_grid(size_t n)
@@ -388,24 +516,6 @@ void bitmask(T const* x, T const* y, size_t n, uint32_t const* po, size_t npo, u
   *out_refined = filtered ? read_back(reinterpret_cast<uint64_t*>(refined.data()), s) : 0;
 }
 
-template <typename T, int G>
-void launch_pairwise(T const* x, T const* y, size_t n, uint32_t const* po, uint32_t const* ro,
-                     T const* vx, T const* vy, bool filtered, uint8_t* out,
-                     unsigned long long* refined, cudaStream_t s)
-{
-  size_t const threads = n * G;
-  unsigned const grd   = grid_for(threads, kPointsBlock, static_cast<unsigned>(num_sms()) * 8u);
-  if (filtered) {
-    if constexpr (std::is_same<T, double>::value)
-      pairwise_pip_kernel<double, G, true>
-        <<<grd, kPointsBlock, 0, s>>>(x, y, n, po, ro, vx, vy, out, refined);
-  } else {
-    pairwise_pip_kernel<T, G, false>
-      <<<grd, kPointsBlock, 0, s>>>(x, y, n, po, ro, vx, vy, out, nullptr);
-  }
-  CSPT_CHECK_LAUNCH();
-}
-
 template <typename T>
 void pairwise(T const* x, T const* y, size_t n, uint32_t const* po, uint32_t const* ro,
               T const* vx, T const* vy, size_t nv, bool filtered, Allocator const& alloc,
@@ -414,18 +524,34 @@ void pairwise(T const* x, T const* y, size_t n, uint32_t const* po, uint32_t con
   cudaStream_t const s = alloc.stream();
   Buffer<unsigned long long> refined(alloc, 1);
   CSPT_CUDA_TRY(cudaMemsetAsync(refined.data(), 0, sizeof(unsigned long long), s));
-  // lanes per polygon from the mean vertex count
-  double const mean = static_cast<double>(nv) / static_cast<double>(n);
+  // Pairs per warp: 32 where that leaves 48 warps for every SM, fewer for
+  // short columns, so that their polygons still spread over the GPU.
+  size_t const fill       = n / (static_cast<size_t>(num_sms()) * 48u);
+  uint32_t const per_warp = static_cast<uint32_t>(fill < 1 ? 1 : (fill > 32 ? 32 : fill));
+  unsigned const grd      = grid_for((n + per_warp - 1) / per_warp * 32, kPointsBlock, sm_grid(64u));
+  // Float32 polygons of a few vertices: a lane walks one in fewer
+  // instructions than a run of 32 costs (1M pairs of 4..8 vertices: 43 us a
+  // call against 64).  Around 12 vertices the two meet; above, lanes wait for
+  // the largest polygon of their warp and read it uncoalesced.
+  bool const lanes = std::is_same<T, float>::value && nv < 12 * n;
   {
     KernelTimer timer("pairwise_pip", s);
-    if (mean < 12.0)
-      launch_pairwise<T, 1>(x, y, n, po, ro, vx, vy, filtered, out, refined.data(), s);
-    else if (mean < 48.0)
-      launch_pairwise<T, 4>(x, y, n, po, ro, vx, vy, filtered, out, refined.data(), s);
-    else if (mean < 160.0)
-      launch_pairwise<T, 8>(x, y, n, po, ro, vx, vy, filtered, out, refined.data(), s);
-    else
-      launch_pairwise<T, 32>(x, y, n, po, ro, vx, vy, filtered, out, refined.data(), s);
+    if (lanes) {
+      PolygonIndexView<T> v{};
+      v.poly_offsets = po;
+      v.ring_offsets = ro;
+      v.vx           = vx;
+      v.vy           = vy;
+      pairwise_lane_kernel<T><<<points_grid(n), kPointsBlock, 0, s>>>(x, y, n, v, out);
+    } else if (filtered) {
+      if constexpr (std::is_same<T, double>::value)
+        pairwise_pip_kernel<double, true>
+          <<<grd, kPointsBlock, 0, s>>>(x, y, n, po, ro, vx, vy, per_warp, out, refined.data());
+    } else {
+      pairwise_pip_kernel<T, false>
+        <<<grd, kPointsBlock, 0, s>>>(x, y, n, po, ro, vx, vy, per_warp, out, nullptr);
+    }
+    CSPT_CHECK_LAUNCH();
   }
   *out_refined = filtered ? read_back(reinterpret_cast<uint64_t*>(refined.data()), s) : 0;
 }
