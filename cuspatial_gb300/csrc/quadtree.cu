@@ -5,16 +5,13 @@
 // sort, bottom-up levels) and phase_2.cuh:56-345 (pruning, offsets).
 //
 // The reference builds every level bottom-up with reduce_by_key and then
-// prunes.  Here the tree is read directly off the sorted keys: position i of
-// the sorted key array starts a node at level l exactly when the keys at i-1
-// and i differ in their level-l prefix, i.e. when l >= lvl[i] with
-// lvl[i] = max(0, d-1 - floor(msb(key[i] ^ key[i-1]) / 2)).  One scan per
-// level ranks those starts; node sizes are differences of starts, child
-// counts are differences of next-level ranks, and a node at level l >= 1 is
-// kept iff its parent holds more than max_size points — the reference's
-// remove_unqualified_quads rule (phase_2.cuh:206-236).  Leaves keep the first
-// sorted position they cover, which is what the reference's flattened-key
-// scan (phase_2.cuh:98-141) produces.
+// prunes.  Here the tree is read directly off the sorted keys, all levels in
+// one pass (node_levels below): position i starts a node at level l exactly
+// when the keys at i-1 and i differ in their level-l prefix, and a node at
+// level l >= 1 is kept iff its parent holds more than max_size points, the
+// reference's remove_unqualified_quads rule (phase_2.cuh:206-236).  Leaves
+// keep the first sorted position they cover, which is what the reference's
+// flattened-key scan (phase_2.cuh:98-141) produces.
 #include <functional>
 #include <limits>
 #include <vector>
@@ -77,7 +74,7 @@ __global__ void start_level_kernel(uint32_t const* __restrict__ skeys, size_t n,
 }
 
 // sizes of the nodes of one level: count[k] = start[k+1] - start[k]
-__global__ void node_count_kernel(uint32_t const* __restrict__ starts, size_t nl, size_t n,
+__global__ void bottom_count_kernel(uint32_t const* __restrict__ starts, size_t nl, size_t n,
                                   uint32_t* __restrict__ count)
 {
   for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < nl;
@@ -87,161 +84,212 @@ __global__ void node_count_kernel(uint32_t const* __restrict__ starts, size_t nl
   }
 }
 
-// finest level (d-1): every position whose key differs from its predecessor
-// Histogram of the start levels: hist[v] = positions whose coarsest start
-// level is v (kNoStart is not counted; v < d <= 16).  Level l has
-// sum_{v <= l} hist[v] nodes, so one read gives every level's size.
-__global__ void __launch_bounds__(256)
-  level_histogram_kernel(uint8_t const* __restrict__ lvl, size_t n, uint32_t* __restrict__ hist)
+// ---------------------------------------------------------------------------
+// Nodes of all levels in one pass over the sorted keys.
+//
+// A sorted position i that starts a node at level l0 (its start level) also
+// starts one at every finer level, and a level-l node is kept iff its parent
+// holds more than max_size points; counts shrink with the level, so the kept
+// nodes starting at i are the levels l0..K of one interval.  Both ends follow
+// from a few keys around i:
+//   * the level-l node starting at i (l >= l0) holds more than m points iff
+//     key[i + m] shares its level-l prefix, i.e. iff l <= c with c read off
+//     the highest differing bit of key[i] ^ key[i + m];
+//   * the parent of (i, l0), l0 > 0, starts before i; it holds more than m
+//     points if key[i + m] shares its prefix (c >= l0 - 1) or key[i - m] does,
+//     holds at most m if neither of two keys m + 1 apart around i does, and
+//     otherwise its start is searched in the m positions before i.
+// So K = min(d - 1, c + 1) where the deeper levels are kept, else l0, and a
+// node (i, l) is internal iff l < K.  Nodes are output level by level in key
+// order: counting them per (level, tile of positions) and scanning the counts
+// level-major gives every node its output row, and the first child of an
+// internal node (i, l) is node (i, l + 1), which is also the reference's
+// child offset (level_1_size plus the scan of child counts).
+//
+// Bound: the key stream (4 bytes a position, the window reads hit L1) and, on
+// small inputs, launches; this replaces a scan, a count, a scan and a
+// compaction per level (61 launches at depth 5, 171 at depth 15).
+// ---------------------------------------------------------------------------
+constexpr int kNodeBlock     = 256;
+constexpr int kNodeRounds    = 8;  // rounds of 32 positions per warp
+constexpr int kNodeTile      = kNodeBlock * kNodeRounds;
+constexpr int kNodeLevels    = 16;
+constexpr uint8_t kNoNodes   = 0xFF;  // no kept node starts here (l0 and K are below 15)
+
+// the deepest level at which two keys share their node, -1 if none
+__device__ inline int shared_level(uint32_t a, uint32_t b, int d)
 {
-  uint32_t c[16];
-#pragma unroll
-  for (int b = 0; b < 16; ++b) c[b] = 0;
-  size_t const stride = static_cast<size_t>(gridDim.x) * blockDim.x;
-  size_t const tid    = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
-  size_t const n4     = n / 4;
-  uint32_t const* l4  = reinterpret_cast<uint32_t const*>(lvl);
-  for (size_t i = tid; i < n4; i += stride) {
-    uint32_t const w = l4[i];
-#pragma unroll
-    for (int b = 0; b < 16; ++b) c[b] += __popc(__vcmpeq4(w, 0x01010101u * b)) >> 3;
+  uint32_t const diff = a ^ b;
+  if (diff == 0) return d - 1;
+  int const c = d - 2 - (31 - __clz(diff)) / 2;
+  return c < 0 ? -1 : c;
+}
+
+// l0 | K << 4 of position i, kNoNodes when no kept node starts there
+__device__ inline uint8_t node_levels(uint32_t const* __restrict__ skeys, size_t n, size_t i, int d,
+                                      size_t m)
+{
+  uint32_t const key = skeys[i];
+  int l0             = 0;
+  if (i > 0) {
+    uint32_t const diff = key ^ skeys[i - 1];
+    if (diff == 0) return kNoNodes;
+    l0 = d - 1 - (31 - __clz(diff)) / 2;
+    l0 = l0 < 0 ? 0 : l0;
   }
-  for (size_t i = n4 * 4 + tid; i < n; i += stride) {
-    uint32_t const v = lvl[i];
-#pragma unroll
-    for (int b = 0; b < 16; ++b) c[b] += v == static_cast<uint32_t>(b) ? 1u : 0u;
+  int const c = i + m < n ? shared_level(key, skeys[i + m], d) : -1;
+  int K       = l0;
+  if (c >= l0 - 1 && c >= 0) {
+    K = c + 1 < d - 1 ? c + 1 : d - 1;
+  } else if (l0 > 0) {
+    int const sh     = 2 * (d - l0);  // >= 2: the parent's prefix
+    uint32_t const P = key >> sh;
+    if (!(i >= m && (skeys[i - m] >> sh) == P)) {
+      // at most ha - 1 points of the parent before i and hb from i on
+      size_t const ha = (m + 1) / 2, hb = m + 1 - ha;
+      bool const before = i >= ha && (skeys[i - ha] >> sh) == P;
+      bool const after  = i + hb < n && (skeys[i + hb] >> sh) == P;
+      if (!before && !after) return kNoNodes;
+      // the parent's first position, in (i - m, i - 1] (i - 1 belongs to it)
+      size_t lo = i >= m ? i - m + 1 : 0, hi = i - 1;
+      while (lo < hi) {
+        size_t const mid = (lo + hi) >> 1;
+        if ((skeys[mid] >> sh) == P)
+          hi = mid;
+        else
+          lo = mid + 1;
+      }
+      if (!(lo + m < n && (skeys[lo + m] >> sh) == P)) return kNoNodes;
+    }
   }
-  __shared__ uint32_t sh[16];
-  if (threadIdx.x < 16) sh[threadIdx.x] = 0;
+  return static_cast<uint8_t>(l0 | (K << 4));
+}
+
+// Per position the levels of its kept nodes, per tile the nodes of each level
+// (counts[level * tiles + tile]).
+__global__ void __launch_bounds__(kNodeBlock)
+  node_count_kernel(uint32_t const* __restrict__ skeys, size_t n, int d, size_t max_size,
+                    uint8_t* __restrict__ codes, uint32_t* __restrict__ counts)
+{
+  __shared__ uint32_t cnt[kNodeLevels];
+  if (threadIdx.x < kNodeLevels) cnt[threadIdx.x] = 0;
   __syncthreads();
-#pragma unroll
-  for (int b = 0; b < 16; ++b) {
-    uint32_t const w = __reduce_add_sync(0xFFFFFFFFu, c[b]);
-    if ((threadIdx.x & 31) == 0 && w) atomicAdd(&sh[b], w);
+  size_t const base = static_cast<size_t>(blockIdx.x) * kNodeTile;
+#pragma unroll 2
+  for (int r = 0; r < kNodeRounds; ++r) {
+    size_t const i = base + static_cast<size_t>(r) * kNodeBlock + threadIdx.x;
+    if (i >= n) break;
+    uint8_t const code = node_levels(skeys, n, i, d, max_size);
+    codes[i]           = code;
+    if (code != kNoNodes)
+      for (int l = code & 15; l <= (code >> 4); ++l) atomicAdd(&cnt[l], 1u);
   }
   __syncthreads();
-  if (threadIdx.x < 16 && sh[threadIdx.x]) atomicAdd(&hist[threadIdx.x], sh[threadIdx.x]);
+  if (threadIdx.x < d) counts[static_cast<size_t>(threadIdx.x) * gridDim.x + blockIdx.x] =
+    cnt[threadIdx.x];
 }
 
-struct FinestStart {
-  uint8_t const* lvl;
-  __device__ uint32_t operator()(size_t i) const { return lvl[i] != kNoStart ? 1u : 0u; }
-};
-struct FinestStore {
-  uint8_t const* lvl;
-  uint32_t* S;
-  uint8_t* LV;
-  __device__ void operator()(size_t i, uint32_t e, uint32_t f) const
-  {
-    if (f) {
-      S[e]  = static_cast<uint32_t>(i);
-      LV[e] = lvl[i];
+// Writes the kept nodes of a tile at the rows that the scanned counts give.
+// Warp w owns 256 consecutive positions; lane l keeps the running row of
+// level l.  The child counts of internal nodes follow in child_count_kernel.
+__global__ void __launch_bounds__(kNodeBlock)
+  node_write_kernel(uint32_t const* __restrict__ skeys, size_t n, int d, size_t max_size,
+                    uint8_t const* __restrict__ codes, uint32_t const* __restrict__ rows,
+                    uint32_t* __restrict__ okey, uint8_t* __restrict__ olevel,
+                    uint8_t* __restrict__ ointernal, uint32_t* __restrict__ olength,
+                    uint32_t* __restrict__ ooffset)
+{
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  __shared__ uint32_t wcnt[kNodeBlock / 32][kNodeLevels];
+  int const lane    = threadIdx.x & 31;
+  int const warp    = threadIdx.x >> 5;
+  unsigned const lt = (1u << lane) - 1u;
+  size_t const base =
+    static_cast<size_t>(blockIdx.x) * kNodeTile + static_cast<size_t>(warp) * (32 * kNodeRounds);
+  uint8_t code[kNodeRounds];
+#pragma unroll
+  for (int r = 0; r < kNodeRounds; ++r) {
+    size_t const i = base + r * 32 + lane;
+    code[r]        = i < n ? codes[i] : kNoNodes;
+  }
+  uint32_t run = 0;  // lane l: nodes of level l in this warp's positions
+#pragma unroll
+  for (int r = 0; r < kNodeRounds; ++r) {
+    if (!__any_sync(kAll, code[r] != kNoNodes)) continue;
+    int const l0 = code[r] & 15, K = code[r] >> 4;
+    for (int l = 0; l < d; ++l) {
+      unsigned const b = __ballot_sync(kAll, code[r] != kNoNodes && l0 <= l && l <= K);
+      if (lane == l) run += __popc(b);
     }
   }
-};
-// level l from level l+1: the starts whose lvl is <= l
-struct CoarserStart {
-  uint8_t const* LV;
-  int l;
-  __device__ uint32_t operator()(size_t k) const
-  {
-    return static_cast<int>(LV[k]) <= l ? 1u : 0u;
+  if (lane < kNodeLevels) wcnt[warp][lane] = run;
+  __syncthreads();
+  run = 0;
+  if (lane < d) {
+    run = rows[static_cast<size_t>(lane) * gridDim.x + blockIdx.x];
+    for (int w = 0; w < warp; ++w) run += wcnt[w][lane];
   }
-};
-struct CoarserStore {
-  uint32_t const* FS;
-  uint8_t const* FLV;
-  uint32_t* S;
-  uint32_t* X;
-  uint8_t* LV;
-  uint32_t* FP;
-  __device__ void operator()(size_t k, uint32_t e, uint32_t f) const
-  {
-    if (f) {
-      S[e]  = FS[k];
-      X[e]  = static_cast<uint32_t>(k);
-      LV[e] = FLV[k];
+#pragma unroll
+  for (int r = 0; r < kNodeRounds; ++r) {
+    if (!__any_sync(kAll, code[r] != kNoNodes)) continue;
+    size_t const i     = base + r * 32 + lane;
+    bool const any     = code[r] != kNoNodes;
+    int const l0       = code[r] & 15, K = code[r] >> 4;
+    uint32_t const key = any ? skeys[i] : 0u;
+    uint32_t parent    = 0;  // row of (i, l - 1)
+    for (int l = 0; l < d; ++l) {
+      bool const mine  = any && l0 <= l && l <= K;
+      unsigned const b = __ballot_sync(kAll, mine);
+      if (b == 0u) continue;
+      uint32_t const o = __shfl_sync(kAll, run, l) + __popc(b & lt);
+      if (lane == l) run += __popc(b);
+      if (!mine) continue;
+      okey[o]      = key >> (2 * (d - 1 - l));
+      olevel[o]    = static_cast<uint8_t>(l);
+      ointernal[o] = l < K ? 1 : 0;
+      if (l > l0) ooffset[parent] = o;
+      parent = o;
     }
-    FP[k] = e + f - 1u;  // the level-l node holding level-(l+1) start k
-  }
-};
-
-// Point counts, child counts and the keep rule of one level's nodes.  A
-// level-l node (l >= 1) survives iff its parent holds more than max_size
-// points (phase_2.cuh:206-236).
-__global__ void level_nodes_kernel(uint32_t const* __restrict__ S, uint32_t const* __restrict__ X,
-                                   size_t nl, size_t n, size_t n_finer,
-                                   uint32_t const* __restrict__ P,
-                                   uint32_t const* __restrict__ parent_count, uint32_t max_size,
-                                   uint32_t* __restrict__ count, uint32_t* __restrict__ child,
-                                   uint8_t* __restrict__ keep)
-{
-  for (size_t j = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; j < nl;
-       j += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    size_t const e = j + 1 < nl ? S[j + 1] : n;
-    count[j]       = static_cast<uint32_t>(e - S[j]);
-    if (child) {
-      size_t const ce = j + 1 < nl ? X[j + 1] : n_finer;
-      child[j]        = static_cast<uint32_t>(ce - X[j]);
+    if (any) {
+      // the leaf (i, K): its points end at the first key beyond its prefix
+      int const sh     = 2 * (d - 1 - K);
+      uint32_t const P = key >> sh;
+      size_t lo = i + 1, hi = n;  // the end lies in [lo, hi]
+      for (size_t step = max_size; i + step < n; step *= 2) {
+        if ((skeys[i + step] >> sh) != P) {
+          hi = i + step;
+          break;
+        }
+        lo = i + step + 1;
+      }
+      while (lo < hi) {
+        size_t const mid = (lo + hi) >> 1;
+        if ((skeys[mid] >> sh) == P)
+          lo = mid + 1;
+        else
+          hi = mid;
+      }
+      ooffset[parent] = static_cast<uint32_t>(i);
+      olength[parent] = static_cast<uint32_t>(lo - i);
     }
-    keep[j] = P ? (parent_count[P[j]] > max_size ? 1 : 0) : 1;
   }
 }
 
-__global__ void compact_nodes_kernel(size_t nl, uint8_t const* __restrict__ keep,
-                                     uint32_t const* __restrict__ pos,
-                                     uint32_t const* __restrict__ S,
-                                     uint32_t const* __restrict__ count,
-                                     uint32_t const* __restrict__ child,
-                                     uint32_t const* __restrict__ skeys, int shift,
-                                     uint32_t* __restrict__ okey, uint32_t* __restrict__ ocount,
-                                     uint32_t* __restrict__ ochild, uint32_t* __restrict__ ostart)
-{
-  for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < nl;
-       k += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    if (!keep[k]) continue;
-    uint32_t const o = pos[k];
-    okey[o]          = skeys[S[k]] >> shift;
-    ocount[o]        = count[k];
-    ochild[o]        = child ? child[k] : 0u;
-    ostart[o]        = S[k];
-  }
-}
-
-struct LevelNodes {
-  Buffer<uint32_t> key, count, child, start;
-  size_t size = 0;
-};
-
-__global__ void assemble_kernel(uint32_t const* __restrict__ key, uint32_t const* __restrict__ cnt,
-                                uint32_t const* __restrict__ child,
-                                uint32_t const* __restrict__ start, size_t nk, uint8_t level,
-                                bool may_be_internal, uint32_t max_size, size_t out_base,
-                                uint32_t* __restrict__ okey, uint8_t* __restrict__ olevel,
-                                uint8_t* __restrict__ ointernal, uint32_t* __restrict__ olength,
-                                uint32_t* __restrict__ ooffset,
-                                uint32_t* __restrict__ internal_children)
-{
-  for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < nk;
-       k += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    size_t const o      = out_base + k;
-    bool const internal = may_be_internal && cnt[k] > max_size;
-    okey[o]             = key[k];
-    olevel[o]           = level;
-    ointernal[o]        = internal ? 1 : 0;
-    olength[o]          = internal ? child[k] : cnt[k];
-    ooffset[o]          = start[k];
-    internal_children[o] = internal ? child[k] : 0u;
-  }
-}
-
-__global__ void internal_offset_kernel(uint8_t const* __restrict__ internal,
-                                       uint32_t const* __restrict__ child_pos, size_t q,
-                                       uint32_t level_1_size, uint32_t* __restrict__ offset)
+// Children of an internal node: the rows from its first child on whose key
+// extends the node's (at most four, all of the next level).
+__global__ void child_count_kernel(uint32_t const* __restrict__ key,
+                                   uint8_t const* __restrict__ level,
+                                   uint8_t const* __restrict__ internal,
+                                   uint32_t const* __restrict__ offset, size_t q,
+                                   uint32_t* __restrict__ length)
 {
   for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < q;
        k += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    if (internal[k]) offset[k] = child_pos[k] + level_1_size;
+    if (!internal[k]) continue;
+    size_t const c0 = offset[k];
+    uint32_t c      = 1;
+    while (c < 4 && c0 + c < q && level[c0 + c] == level[c0] && (key[c0 + c] >> 2) == key[k]) ++c;
+    length[k] = c;
   }
 }
 
@@ -412,15 +460,14 @@ void build(T const* x, T const* y, size_t n, double x1d, double x2d, double y1d,
   }
 
   KernelTimer levels_timer("quadtree_levels", s);
-  Buffer<uint8_t> lvl(alloc, n);
-  start_level_kernel<<<grd, blk, 0, s>>>(skeys.data(), n, d, lvl.data());
-  CSPT_CHECK_LAUNCH();
-
   Buffer<uint32_t> total(alloc, 1);
-  uint8_t const* lv = lvl.data();
 
   if (d <= 1) {
     // detail/point_quadtree.cuh:155-188: a tree of the bottom quadrants only
+    Buffer<uint8_t> lvl(alloc, n);
+    start_level_kernel<<<grd, blk, 0, s>>>(skeys.data(), n, d, lvl.data());
+    CSPT_CHECK_LAUNCH();
+    uint8_t const* lv = lvl.data();
     Buffer<uint32_t> starts(alloc, n);
     uint32_t* st = starts.data();
     scan_apply<uint32_t>(
@@ -432,7 +479,7 @@ void build(T const* x, T const* y, size_t n, double x1d, double x2d, double y1d,
     size_t const q = read_back(total.data(), s);
     Buffer<uint32_t> okey(alloc, q), olen(alloc, q), ooff(alloc, q);
     Buffer<uint8_t> olev(alloc, q), oint(alloc, q);
-    node_count_kernel<<<grid_for(q, blk, sm_grid(16u)), blk, 0, s>>>(st, q, n, olen.data());
+    bottom_count_kernel<<<grid_for(q, blk, sm_grid(16u)), blk, 0, s>>>(st, q, n, olen.data());
     CSPT_CHECK_LAUNCH();
     uint32_t const* sk = skeys.data();
     uint32_t* ok       = okey.data();
@@ -451,132 +498,25 @@ void build(T const* x, T const* y, size_t n, double x1d, double x2d, double y1d,
     return;
   }
 
-  // Levels, bottom-up.  A position starts a level-l node iff lvl <= l, so
-  // the level-l starts are the level-(l+1) starts whose lvl is <= l: each
-  // level is ranked by a scan over the next finer level only (about 1.3 N
-  // elements in all instead of d N).  For a level-l node j: S = first sorted
-  // position, X = its index among the level-(l+1) starts; for a level-(l+1)
-  // start k: P = the level-l node holding it (its parent).  Every level's
-  // size comes from one histogram of lvl, and the kept nodes of all levels
-  // are counted on the device and read once: the host waits twice in all.
-  std::vector<size_t> level_size(d);
-  {
-    Buffer<uint32_t> hist(alloc, 16);
-    CSPT_CUDA_TRY(cudaMemsetAsync(hist.data(), 0, 16 * sizeof(uint32_t), s));
-    level_histogram_kernel<<<grid_for((n + 3) / 4, blk, sm_grid(8u)), blk, 0, s>>>(lv, n,
-                                                                                  hist.data());
-    CSPT_CHECK_LAUNCH();
-    uint32_t h[16];
-    CSPT_CUDA_TRY(cudaMemcpyAsync(h, hist.data(), sizeof(h), cudaMemcpyDeviceToHost, s));
-    CSPT_CUDA_TRY(cudaStreamSynchronize(s));
-    size_t run = 0;
-    for (int l = 0; l < d; ++l) level_size[l] = run += h[l];
-  }
-  struct Raw {
-    Buffer<uint32_t> S, X, P, count;
-    Buffer<uint8_t> LV;
-    size_t n = 0;
-  };
-  std::vector<Raw> raw(d);
-  {
-    Raw& R = raw[d - 1];
-    R.S    = Buffer<uint32_t>(alloc, level_size[d - 1]);
-    R.LV   = Buffer<uint8_t>(alloc, level_size[d - 1]);
-    scan_apply<uint32_t>(FinestStart{lv}, FinestStore{lv, R.S.data(), R.LV.data()}, n,
-                         static_cast<uint32_t*>(nullptr), alloc);
-    R.n = level_size[d - 1];
-  }
-  for (int l = d - 2; l >= 0; --l) {
-    Raw& F = raw[l + 1];
-    Raw& R = raw[l];
-    R.n    = level_size[l];
-    R.S    = Buffer<uint32_t>(alloc, R.n);
-    R.X    = Buffer<uint32_t>(alloc, R.n);
-    R.LV   = Buffer<uint8_t>(alloc, R.n);
-    F.P    = Buffer<uint32_t>(alloc, F.n);
-    scan_apply<uint32_t>(CoarserStart{F.LV.data(), l},
-                         CoarserStore{F.S.data(), F.LV.data(), R.S.data(), R.X.data(),
-                                      R.LV.data(), F.P.data()},
-                         F.n, static_cast<uint32_t*>(nullptr), alloc);
-    F.LV.reset();
-  }
-  raw[0].LV.reset();
-  size_t const level_1_size = raw[0].n;
-  std::vector<LevelNodes> levels(d);
-  Buffer<uint32_t> kept(alloc, d);  // kept nodes per level
-  for (int l = 0; l < d; ++l) {
-    Raw& R        = raw[l];
-    size_t const nl = R.n;
-    R.count       = Buffer<uint32_t>(alloc, nl);
-    Buffer<uint32_t> child(alloc, l + 1 < d ? nl : 0);
-    Buffer<uint8_t> keep(alloc, nl);
-    if (nl) {
-      level_nodes_kernel<<<grid_for(nl, blk, sm_grid(16u)), blk, 0, s>>>(
-        R.S.data(), R.X.data(), nl, n, l + 1 < d ? raw[l + 1].n : 0, l > 0 ? R.P.data() : nullptr,
-        l > 0 ? raw[l - 1].count.data() : nullptr, max_size, R.count.data(),
-        l + 1 < d ? child.data() : nullptr, keep.data());
-      CSPT_CHECK_LAUNCH();
-    }
-    // compact the kept nodes of the level (at most nl of them)
-    LevelNodes& L = levels[l];
-    Buffer<uint32_t> pos(alloc, nl);
-    uint8_t const* kp = keep.data();
-    uint32_t* ps      = pos.data();
-    scan_apply<uint32_t>([kp] __device__(size_t k) { return static_cast<uint32_t>(kp[k]); },
-                         [ps] __device__(size_t k, uint32_t e, uint32_t) { ps[k] = e; }, nl,
-                         kept.data() + l, alloc);
-    L.key   = Buffer<uint32_t>(alloc, nl);
-    L.count = Buffer<uint32_t>(alloc, nl);
-    L.child = Buffer<uint32_t>(alloc, nl);
-    L.start = Buffer<uint32_t>(alloc, nl);
-    if (nl) {
-      compact_nodes_kernel<<<grid_for(nl, blk, sm_grid(16u)), blk, 0, s>>>(
-        nl, kp, ps, R.S.data(), R.count.data(), l + 1 < d ? child.data() : nullptr,
-        skeys.data(), 2 * (d - 1 - l), L.key.data(), L.count.data(), L.child.data(),
-        L.start.data());
-      CSPT_CHECK_LAUNCH();
-    }
-    // the parent level's counts are no longer needed
-    if (l > 0) {
-      raw[l - 1].count.reset();
-      raw[l - 1].S.reset();
-      raw[l - 1].X.reset();
-      raw[l - 1].P.reset();
-    }
-    R.P.reset();
-  }
-  raw.clear();
-  lvl.reset();
-  {
-    std::vector<uint32_t> hk(d);
-    CSPT_CUDA_TRY(
-      cudaMemcpyAsync(hk.data(), kept.data(), d * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    CSPT_CUDA_TRY(cudaStreamSynchronize(s));
-    for (int l = 0; l < d; ++l) levels[l].size = hk[l];
-  }
-
-  size_t q = 0;
-  for (auto& L : levels) q += L.size;
-  Buffer<uint32_t> okey(alloc, q), olen(alloc, q), ooff(alloc, q), ichild(alloc, q);
+  // every level's nodes from one pass (node_levels); the host waits once, for
+  // the number of nodes
+  unsigned const tiles = static_cast<unsigned>((n + kNodeTile - 1) / kNodeTile);
+  size_t const cells   = static_cast<size_t>(tiles) * d;
+  Buffer<uint8_t> codes(alloc, n);
+  Buffer<uint32_t> rows(alloc, cells);
+  node_count_kernel<<<tiles, kNodeBlock, 0, s>>>(skeys.data(), n, d, max_size, codes.data(),
+                                                 rows.data());
+  CSPT_CHECK_LAUNCH();
+  exclusive_scan<uint32_t>(rows.data(), rows.data(), cells, total.data(), alloc);
+  size_t const q = read_back(total.data(), s);
+  Buffer<uint32_t> okey(alloc, q), olen(alloc, q), ooff(alloc, q);
   Buffer<uint8_t> olev(alloc, q), oint(alloc, q);
-  size_t base = 0;
-  for (int l = 0; l < d; ++l) {
-    LevelNodes& L = levels[l];
-    if (L.size) {
-      assemble_kernel<<<grid_for(L.size, blk, sm_grid(16u)), blk, 0, s>>>(
-        L.key.data(), L.count.data(), L.child.data(), L.start.data(), L.size,
-        static_cast<uint8_t>(l), l <= d - 2, max_size, base, okey.data(), olev.data(),
-        oint.data(), olen.data(), ooff.data(), ichild.data());
-      CSPT_CHECK_LAUNCH();
-    }
-    base += L.size;
-    L = LevelNodes{};
-  }
-  // detail/point_quadtree.cuh:82-109: internal offsets = level_1_size + scan
-  exclusive_scan<uint32_t>(ichild.data(), ichild.data(), q, static_cast<uint32_t*>(nullptr),
-                           alloc);
-  internal_offset_kernel<<<grid_for(q, blk, sm_grid(16u)), blk, 0, s>>>(
-    oint.data(), ichild.data(), q, static_cast<uint32_t>(level_1_size), ooff.data());
+  node_write_kernel<<<tiles, kNodeBlock, 0, s>>>(skeys.data(), n, d, max_size, codes.data(),
+                                                 rows.data(), okey.data(), olev.data(),
+                                                 oint.data(), olen.data(), ooff.data());
+  CSPT_CHECK_LAUNCH();
+  child_count_kernel<<<grid_for(q, blk, sm_grid(16u)), blk, 0, s>>>(
+    okey.data(), olev.data(), oint.data(), ooff.data(), q, olen.data());
   CSPT_CHECK_LAUNCH();
   *out_point_indices = sidx.release();
   *out = cspt_quadtree{okey.release(), olev.release(), oint.release(), olen.release(),
