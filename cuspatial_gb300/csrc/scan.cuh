@@ -1,5 +1,9 @@
-// Device-wide exclusive scan and stream compaction (reduce / scan-partials /
-// downsweep, tiles of 2048 items per 256-thread block).
+// Device-wide exclusive scan and stream compaction over tiles of 2048 items
+// per 256-thread block, in as few launches as the size allows:
+//   one tile: the downsweep alone;
+//   up to kScanDirect tiles: reduce, then a downsweep whose blocks add up the
+//     partials before their tile themselves (at most 32 loads a thread, in L2);
+//   more: reduce, a scan of the partials by one block, downsweep.
 #pragma once
 
 #include "common.cuh"
@@ -95,9 +99,15 @@ __global__ void __launch_bounds__(1024) scan_partials_kernel(T* partials, size_t
 // the tile by thread t: coalesced), and scanned in blocked order (thread t
 // owns items [8 t, 8 t + 8)) through a shared-memory transpose padded by one
 // word per 32 (no bank conflicts for 4-byte items).
-template <typename T, typename InF, typename OutF>
+// ScanBase tells where the sum of the tiles before this one comes from: there
+// is only one tile, partials[tile] holds it, or the blocks add it up from the
+// tiles' own sums.  In the first and the last case the last block also writes
+// the total.
+enum class ScanBase { kNone, kScanned, kSums };
+
+template <typename T, ScanBase Base, typename InF, typename OutF>
 __global__ void __launch_bounds__(kScanBlock)
-  scan_down_kernel(InF in, OutF out, size_t n, T const* partials)
+  scan_down_kernel(InF in, OutF out, size_t n, T const* partials, T* total_out)
 {
   __shared__ T s_items[kScanTile + kScanTile / 32];
   size_t const base = static_cast<size_t>(blockIdx.x) * kScanTile;
@@ -119,7 +129,24 @@ __global__ void __launch_bounds__(kScanBlock)
     s += vals[j];
   }
   __shared__ T total;
-  T run = block_exclusive_scan<T, kScanBlock>(s, &total) + partials[blockIdx.x];
+  T run = block_exclusive_scan<T, kScanBlock>(s, &total);
+  if constexpr (Base == ScanBase::kScanned) {
+    run += partials[blockIdx.x];
+  } else {
+    T before = 0;
+    if constexpr (Base == ScanBase::kSums) {
+      T const own = total;
+      T v         = 0;
+      for (unsigned b = threadIdx.x; b < blockIdx.x; b += kScanBlock) v += partials[b];
+      (void)block_exclusive_scan<T, kScanBlock>(v, &total);
+      before = total;
+      run += before;
+      before += own;
+    } else {
+      before = total;
+    }
+    if (total_out && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) *total_out = before;
+  }
   // block_exclusive_scan ends with a barrier: every thread has read its
   // items before the prefixes overwrite them
 #pragma unroll
@@ -137,6 +164,38 @@ __global__ void __launch_bounds__(kScanBlock)
   }
 }
 
+// The launches of a scan over n > 0 items; partials holds ceil(n / kScanTile)
+// elements (unused for one tile).  kScanDirect: at 4096 tiles (8.4 M items) the
+// downsweep's own sums cost about what the one-block scan does, below it the
+// saved launch wins.
+constexpr size_t kScanDirect = 4096;
+
+template <typename T, typename InF, typename OutF>
+void scan_launch(InF in, OutF out, size_t n, T* total, T* partials, cudaStream_t s)
+{
+  size_t const nparts = (n + kScanTile - 1) / kScanTile;
+  unsigned const grd  = static_cast<unsigned>(nparts);
+  if (nparts == 1) {
+    scan_down_kernel<T, ScanBase::kNone, InF, OutF>
+      <<<1, kScanBlock, 0, s>>>(in, out, n, nullptr, total);
+    CSPT_CHECK_LAUNCH();
+    return;
+  }
+  scan_reduce_kernel<T, InF><<<grd, kScanBlock, 0, s>>>(in, n, partials);
+  CSPT_CHECK_LAUNCH();
+  if (nparts <= kScanDirect) {
+    scan_down_kernel<T, ScanBase::kSums, InF, OutF>
+      <<<grd, kScanBlock, 0, s>>>(in, out, n, partials, total);
+    CSPT_CHECK_LAUNCH();
+    return;
+  }
+  scan_partials_kernel<T><<<1, 1024, 0, s>>>(partials, nparts, total);
+  CSPT_CHECK_LAUNCH();
+  scan_down_kernel<T, ScanBase::kScanned, InF, OutF>
+    <<<grd, kScanBlock, 0, s>>>(in, out, n, partials, nullptr);
+  CSPT_CHECK_LAUNCH();
+}
+
 // Generic driver.  `total` (device pointer, may be null) receives the sum.
 template <typename T, typename InF, typename OutF>
 void scan_apply(InF in, OutF out, size_t n, T* total, Allocator const& alloc)
@@ -147,15 +206,8 @@ void scan_apply(InF in, OutF out, size_t n, T* total, Allocator const& alloc)
     return;
   }
   size_t const nparts = (n + kScanTile - 1) / kScanTile;
-  Buffer<T> partials(alloc, nparts);
-  scan_reduce_kernel<T, InF><<<static_cast<unsigned>(nparts), kScanBlock, 0, s>>>(
-    in, n, partials.data());
-  CSPT_CHECK_LAUNCH();
-  scan_partials_kernel<T><<<1, 1024, 0, s>>>(partials.data(), nparts, total);
-  CSPT_CHECK_LAUNCH();
-  scan_down_kernel<T, InF, OutF><<<static_cast<unsigned>(nparts), kScanBlock, 0, s>>>(
-    in, out, n, partials.data());
-  CSPT_CHECK_LAUNCH();
+  Buffer<T> partials(alloc, nparts > 1 ? nparts : 0);
+  scan_launch<T>(in, out, n, total, partials.data(), s);
 }
 
 template <typename T>
@@ -181,7 +233,7 @@ void exclusive_scan(T const* in, T* out, size_t n, T* total, Allocator const& al
 namespace cspt {
 
 // scan_apply over caller-provided partials (at least ceil(n / kScanTile)
-// elements): launches the same three kernels and allocates nothing.
+// elements): the same launches, no allocation.
 template <typename T, typename InF, typename OutF>
 void scan_apply_prealloc(InF in, OutF out, size_t n, T* total, T* partials, cudaStream_t s)
 {
@@ -189,14 +241,7 @@ void scan_apply_prealloc(InF in, OutF out, size_t n, T* total, T* partials, cuda
     if (total) CSPT_CUDA_TRY(cudaMemsetAsync(total, 0, sizeof(T), s));
     return;
   }
-  size_t const nparts = (n + kScanTile - 1) / kScanTile;
-  scan_reduce_kernel<T, InF><<<static_cast<unsigned>(nparts), kScanBlock, 0, s>>>(in, n, partials);
-  CSPT_CHECK_LAUNCH();
-  scan_partials_kernel<T><<<1, 1024, 0, s>>>(partials, nparts, total);
-  CSPT_CHECK_LAUNCH();
-  scan_down_kernel<T, InF, OutF>
-    <<<static_cast<unsigned>(nparts), kScanBlock, 0, s>>>(in, out, n, partials);
-  CSPT_CHECK_LAUNCH();
+  scan_launch<T>(in, out, n, total, partials, s);
 }
 
 }  // namespace cspt
