@@ -264,8 +264,7 @@ class TorchAllocator:
             # the block belongs to the stream the library will use it on:
             # torch's caching allocator reuses a freed block only for later
             # work on that same stream
-            cur = torch.cuda.current_stream(self.device)
-            if stream and int(stream) != cur.cuda_stream:
+            if stream and int(stream) != torch.cuda.current_stream(self.device).cuda_stream:
                 ext = self._streams.get(int(stream))
                 if ext is None:
                     ext = torch.cuda.ExternalStream(int(stream), device=self.device)
@@ -292,9 +291,9 @@ class TorchAllocator:
         if not ptr or count == 0:
             return torch.empty(0, dtype=dtype, device=self.device)
         t = self.blocks.pop(ptr)
-        nbytes = count * torch.empty(0, dtype=dtype).element_size()
+        nbytes = count * dtype.itemsize
         self.in_use -= t.numel()
-        return t[:nbytes].view(dtype)
+        return (t if t.numel() == nbytes else t[:nbytes]).view(dtype)
 
 
 def stream_ptr(stream=None):

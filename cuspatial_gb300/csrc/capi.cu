@@ -379,9 +379,10 @@ cspt_status cspt_quadtree_on_points(const void* x, const void* y, size_t num_poi
     check_dtype(dtype);
     if (num_points == 0) return;  // point_quadtree.cu:167-177
     CSPT_EXPECTS(x && y, "x and y columns must have the same length");
-    Allocator alloc(mr, as_stream(stream));
-    quadtree_on_points(x, y, num_points, dtype, x_min, x_max, y_min, y_max, scale, max_depth,
-                       max_size, alloc, out_point_indices, out_tree);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_on_points(x, y, num_points, dtype, x_min, x_max, y_min, y_max, scale, max_depth,
+                         max_size, alloc, out_point_indices, out_tree);
+    });
   });
 }
 
@@ -400,10 +401,11 @@ cspt_status cspt_quadtree_on_points_host(const void* host_x, const void* host_y,
     if (num_points == 0) return;  // point_quadtree.cu:167-177
     CSPT_EXPECTS(host_x && host_y && device_x && device_y,
                  "x and y columns must have the same length");
-    Allocator alloc(mr, as_stream(stream));
-    quadtree_on_points_from_host(host_x, host_y, device_x, device_y, num_points, dtype, x_min,
-                                 x_max, y_min, y_max, scale, max_depth, max_size, alloc,
-                                 out_point_indices, out_tree);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_on_points_from_host(host_x, host_y, device_x, device_y, num_points, dtype, x_min,
+                                   x_max, y_min, y_max, scale, max_depth, max_size, alloc,
+                                   out_point_indices, out_tree);
+    });
   });
 }
 
@@ -426,9 +428,10 @@ cspt_status cspt_quadtree_on_points_ordered(const void* x, const void* y, size_t
     CSPT_EXPECTS(out_ordered_xy && reinterpret_cast<uintptr_t>(out_ordered_xy) % vec == 0,
                  "the ordered points must start on a " + std::to_string(vec) +
                    "-byte boundary");
-    Allocator alloc(mr, as_stream(stream));
-    quadtree_on_points(x, y, num_points, dtype, x_min, x_max, y_min, y_max, scale, max_depth,
-                       max_size, alloc, out_point_indices, out_tree, out_ordered_xy);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_on_points(x, y, num_points, dtype, x_min, x_max, y_min, y_max, scale, max_depth,
+                         max_size, alloc, out_point_indices, out_tree, out_ordered_xy);
+    });
   });
 }
 
@@ -450,10 +453,11 @@ cspt_status cspt_quadtree_on_points_host_ordered(
     CSPT_EXPECTS(out_ordered_xy && reinterpret_cast<uintptr_t>(out_ordered_xy) % vec == 0,
                  "the ordered points must start on a " + std::to_string(vec) +
                    "-byte boundary");
-    Allocator alloc(mr, as_stream(stream));
-    quadtree_on_points_from_host(host_x, host_y, device_x, device_y, num_points, dtype, x_min,
-                                 x_max, y_min, y_max, scale, max_depth, max_size, alloc,
-                                 out_point_indices, out_tree, out_ordered_xy);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_on_points_from_host(host_x, host_y, device_x, device_y, num_points, dtype, x_min,
+                                   x_max, y_min, y_max, scale, max_depth, max_size, alloc,
+                                   out_point_indices, out_tree, out_ordered_xy);
+    });
   });
 }
 
@@ -544,10 +548,11 @@ cspt_status cspt_join_quadtree_and_bounding_boxes(
     CSPT_EXPECTS(max_depth > 0 && max_depth < 16,
                  "maximum depth must be positive and less than 16");
     if (tree->num_nodes == 0 || num_bboxes == 0) return;  // :108-114
-    Allocator alloc(mr, as_stream(stream));
-    join_quadtree_and_bounding_boxes(tree, bbox_min_x, bbox_min_y, bbox_max_x, bbox_max_y,
-                                     num_bboxes, dtype, x_min, y_min, scale, max_depth, alloc,
-                                     out_bbox_offset, out_quad_offset, out_num_pairs);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      join_quadtree_and_bounding_boxes(tree, bbox_min_x, bbox_min_y, bbox_max_x, bbox_max_y,
+                                       num_bboxes, dtype, x_min, y_min, scale, max_depth, alloc,
+                                       out_bbox_offset, out_quad_offset, out_num_pairs);
+    });
   });
 }
 
@@ -580,13 +585,14 @@ cspt_status cspt_quadtree_point_in_polygon(
       return;
     CSPT_EXPECTS(num_ring_offsets > 0,
                  "Polygon ring offsets must contain at least one (1) value");
-    Allocator alloc(mr, as_stream(stream));
     uint64_t refined = 0;
-    quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, point_indices,
-                              num_point_indices, x, y, poly_offsets, num_poly_offsets,
-                              ring_offsets, num_ring_offsets, poly_x, poly_y, num_poly_vertices,
-                              dtype, method, alloc, out_polygon_index, out_point_index,
-                              out_num_pairs, &refined);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, point_indices,
+                                num_point_indices, x, y, poly_offsets, num_poly_offsets,
+                                ring_offsets, num_ring_offsets, poly_x, poly_y, num_poly_vertices,
+                                dtype, method, alloc, out_polygon_index, out_point_index,
+                                out_num_pairs, &refined);
+    });
     t_last_refined = refined;
   });
 }
@@ -619,14 +625,15 @@ cspt_status cspt_quadtree_point_in_polygon_host(
       return;
     CSPT_EXPECTS(num_ring_offsets > 0,
                  "Polygon ring offsets must contain at least one (1) value");
-    Allocator alloc(mr, as_stream(stream));
     uint64_t refined = 0;
     HostRows const host{host_polygon_index, host_point_index, host_capacity};
-    quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, point_indices,
-                              num_point_indices, x, y, poly_offsets, num_poly_offsets,
-                              ring_offsets, num_ring_offsets, poly_x, poly_y, num_poly_vertices,
-                              dtype, method, alloc, nullptr, nullptr, out_num_pairs, &refined,
-                              &host);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, point_indices,
+                                num_point_indices, x, y, poly_offsets, num_poly_offsets,
+                                ring_offsets, num_ring_offsets, poly_x, poly_y, num_poly_vertices,
+                                dtype, method, alloc, nullptr, nullptr, out_num_pairs, &refined,
+                                &host);
+    });
     t_last_refined = refined;
   });
 }
@@ -702,12 +709,13 @@ cspt_status cspt_quadtree_point_to_nearest_linestring(
       return;
     CSPT_EXPECTS(out_point_index && out_linestring_index && out_distance,
                  "output pointers must not be null");
-    Allocator alloc(mr, as_stream(stream));
-    quadtree_point_to_nearest_linestring(pair_linestring, pair_quad, num_pairs, tree,
-                                         point_indices, num_point_indices, x, y,
-                                         linestring_offsets, num_linestring_offsets, ls_x, ls_y,
-                                         dtype, method, alloc, out_point_index,
-                                         out_linestring_index, out_distance);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_point_to_nearest_linestring(pair_linestring, pair_quad, num_pairs, tree,
+                                           point_indices, num_point_indices, x, y,
+                                           linestring_offsets, num_linestring_offsets, ls_x, ls_y,
+                                           dtype, method, alloc, out_point_index,
+                                           out_linestring_index, out_distance);
+    });
     *out_num_rows = num_point_indices;
   });
 }
@@ -746,13 +754,14 @@ cspt_status cspt_quadtree_point_in_polygon_ordered(
     check_ordered(ordered_xy, dtype);
     CSPT_EXPECTS(num_ring_offsets > 0,
                  "Polygon ring offsets must contain at least one (1) value");
-    Allocator alloc(mr, as_stream(stream));
     uint64_t refined = 0;
-    quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, nullptr, num_points,
-                              nullptr, nullptr, poly_offsets, num_poly_offsets, ring_offsets,
-                              num_ring_offsets, poly_x, poly_y, num_poly_vertices, dtype, method,
-                              alloc, out_polygon_index, out_point_index, out_num_pairs, &refined,
-                              nullptr, ordered_xy);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, nullptr, num_points,
+                                nullptr, nullptr, poly_offsets, num_poly_offsets, ring_offsets,
+                                num_ring_offsets, poly_x, poly_y, num_poly_vertices, dtype, method,
+                                alloc, out_polygon_index, out_point_index, out_num_pairs, &refined,
+                                nullptr, ordered_xy);
+    });
     t_last_refined = refined;
   });
 }
@@ -781,14 +790,15 @@ cspt_status cspt_quadtree_point_in_polygon_host_ordered(
     check_ordered(ordered_xy, dtype);
     CSPT_EXPECTS(num_ring_offsets > 0,
                  "Polygon ring offsets must contain at least one (1) value");
-    Allocator alloc(mr, as_stream(stream));
     uint64_t refined = 0;
     HostRows const host{host_polygon_index, host_point_index, host_capacity};
-    quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, nullptr, num_points,
-                              nullptr, nullptr, poly_offsets, num_poly_offsets, ring_offsets,
-                              num_ring_offsets, poly_x, poly_y, num_poly_vertices, dtype, method,
-                              alloc, nullptr, nullptr, out_num_pairs, &refined, &host,
-                              ordered_xy);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_point_in_polygon(pair_polygon, pair_quad, num_pairs, tree, nullptr, num_points,
+                                nullptr, nullptr, poly_offsets, num_poly_offsets, ring_offsets,
+                                num_ring_offsets, poly_x, poly_y, num_poly_vertices, dtype, method,
+                                alloc, nullptr, nullptr, out_num_pairs, &refined, &host,
+                                ordered_xy);
+    });
     t_last_refined = refined;
   });
 }
@@ -815,12 +825,13 @@ cspt_status cspt_quadtree_point_to_nearest_linestring_ordered(
     check_ordered(ordered_xy, dtype);
     CSPT_EXPECTS(out_point_index && out_linestring_index && out_distance,
                  "output pointers must not be null");
-    Allocator alloc(mr, as_stream(stream));
-    quadtree_point_to_nearest_linestring(pair_linestring, pair_quad, num_pairs, tree, nullptr,
-                                         num_points, nullptr, nullptr, linestring_offsets,
-                                         num_linestring_offsets, ls_x, ls_y, dtype, method,
-                                         alloc, out_point_index, out_linestring_index,
-                                         out_distance, ordered_xy);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      quadtree_point_to_nearest_linestring(pair_linestring, pair_quad, num_pairs, tree, nullptr,
+                                           num_points, nullptr, nullptr, linestring_offsets,
+                                           num_linestring_offsets, ls_x, ls_y, dtype, method,
+                                           alloc, out_point_index, out_linestring_index,
+                                           out_distance, ordered_xy);
+    });
     *out_num_rows = num_points;
   });
 }
@@ -844,7 +855,6 @@ cspt_status cspt_point_in_polygon(const void* x, const void* y, size_t num_point
     // detail/point_in_polygon.cuh:93-94
     CSPT_EXPECTS(npoly <= 31, "Number of polygons cannot exceed 31");
     CSPT_EXPECTS(out, "output pointers must not be null");
-    Allocator alloc(mr, as_stream(stream));
     if (npoly == 0) {
       CSPT_CUDA_TRY(cudaMemsetAsync(out, 0, num_points * sizeof(int32_t), as_stream(stream)));
       return;
@@ -852,9 +862,11 @@ cspt_status cspt_point_in_polygon(const void* x, const void* y, size_t num_point
     CSPT_EXPECTS(num_ring_offsets > 0,
                  "Polygon ring offsets must contain at least one (1) value");
     uint64_t refined = 0;
-    point_in_polygon(x, y, num_points, poly_offsets, num_poly_offsets, ring_offsets,
-                     num_ring_offsets, poly_x, poly_y, num_poly_vertices, dtype, method, alloc,
-                     out, &refined);
+    with_scratch(mr, as_stream(stream), [&](Allocator const& alloc) {
+      point_in_polygon(x, y, num_points, poly_offsets, num_poly_offsets, ring_offsets,
+                       num_ring_offsets, poly_x, poly_y, num_poly_vertices, dtype, method, alloc,
+                       out, &refined);
+    });
     t_last_refined = refined;
   });
 }

@@ -11,6 +11,7 @@
 #include <string>
 #include <type_traits>
 #include <utility>
+#include <vector>
 
 #include "../../include/cuspatial_gb300.h"
 
@@ -112,10 +113,12 @@ cudaStream_t library_stream();
 class Allocator {
  public:
   Allocator(cspt_allocator const* mr, cudaStream_t stream) : mr_(mr), stream_(stream) {}
-  void* allocate(size_t bytes) const
+  // scratch: the memory does not outlive the call (see ScratchArena)
+  void* allocate(size_t bytes, bool scratch = false) const
   {
     if (bytes == 0) return nullptr;
-    void* p = nullptr;
+    void* p = scratch && arena_ ? arena_take(bytes) : nullptr;
+    if (p) return p;
     if (mr_ && mr_->allocate) {
       p = mr_->allocate(mr_->ctx, bytes, stream_);
       if (!p) throw Error{CSPT_OUT_OF_MEMORY, "allocation of " + std::to_string(bytes) +
@@ -133,7 +136,7 @@ class Allocator {
   }
   void deallocate(void* p, size_t bytes) const
   {
-    if (!p) return;
+    if (!p || (arena_ && arena_give(p, bytes))) return;
     if (mr_ && mr_->deallocate) {
       mr_->deallocate(mr_->ctx, p, bytes, stream_);
     } else {
@@ -144,9 +147,122 @@ class Allocator {
   cspt_allocator const* resource() const { return mr_; }
 
  private:
+  friend class ScratchArena;
+  void* arena_take(size_t bytes) const;
+  bool arena_give(void* p, size_t bytes) const;
+
   cspt_allocator const* mr_;
   cudaStream_t stream_;
+  class ScratchArena* arena_ = nullptr;
 };
+
+// The scratch memory of one call.  A small join takes 60 to 150 buffers, most
+// of them a few kilobytes, and a caller's allocator is a callback (6 to 10 us
+// each from Python, a third of such a call); blocks of up to kMaxBlock bytes
+// are cut from slabs of the caller's memory instead, which go back when the
+// call ends.  Blocks are powers of two and are reused within the call in stream
+// order, as the allocator's own are.  Where the caller has no memory for a slab
+// the buffer is allocated as before.
+class ScratchArena {
+ public:
+  explicit ScratchArena(Allocator& a) : a_(a) { a_.arena_ = this; }
+  ~ScratchArena()
+  {
+    a_.arena_ = nullptr;
+    for (int i = 0; i < nslabs_; ++i) a_.deallocate(slabs_[i].p, slabs_[i].bytes);
+  }
+  ScratchArena(ScratchArena const&)            = delete;
+  ScratchArena& operator=(ScratchArena const&) = delete;
+
+  void* take(size_t bytes)
+  {
+    if (bytes > kMaxBlock) return nullptr;
+    int const c  = size_class(bytes);
+    size_t const size = kMinBlock << c;
+    if (!free_[c].empty()) {
+      void* const p = free_[c].back();
+      free_[c].pop_back();
+      return p;
+    }
+    if (end_ - at_ < static_cast<ptrdiff_t>(size) && !grow()) return nullptr;
+    if (end_ - at_ < static_cast<ptrdiff_t>(size)) return nullptr;
+    void* const p = at_;
+    at_ += size;
+    return p;
+  }
+  bool give(void* p, size_t bytes)
+  {
+    if (!owns(p)) return false;
+    free_[size_class(bytes)].push_back(p);
+    return true;
+  }
+  bool owns(void const* p) const
+  {
+    for (int i = 0; i < nslabs_; ++i) {
+      char const* const b = static_cast<char const*>(slabs_[i].p);
+      if (p >= b && p < b + slabs_[i].bytes) return true;
+    }
+    return false;
+  }
+
+ private:
+  static constexpr size_t kMinBlock = 256, kMaxBlock = size_t{1} << 20;
+  static constexpr int kClasses = 13, kMaxSlabs = 8;
+  static constexpr size_t kFirstSlab = size_t{2} << 20, kLastSlab = size_t{16} << 20;
+  static int size_class(size_t bytes)
+  {
+    int c = 0;
+    while ((kMinBlock << c) < bytes) ++c;
+    return c;
+  }
+  bool grow()
+  {
+    if (nslabs_ == kMaxSlabs) return false;
+    size_t const want = nslabs_ == 0 ? kFirstSlab : slabs_[nslabs_ - 1].bytes * 2;
+    size_t const size = want < kLastSlab ? want : kLastSlab;
+    void* p           = nullptr;
+    try {
+      p = a_.allocate(size);
+    } catch (Error const&) {
+      return false;
+    }
+    slabs_[nslabs_++] = Slab{p, size};
+    at_               = static_cast<char*>(p);
+    end_              = at_ + size;
+    return true;
+  }
+  struct Slab {
+    void* p;
+    size_t bytes;
+  };
+  Allocator& a_;
+  Slab slabs_[kMaxSlabs];
+  int nslabs_ = 0;
+  char *at_ = nullptr, *end_ = nullptr;
+  std::vector<void*> free_[kClasses];
+};
+
+inline void* Allocator::arena_take(size_t bytes) const { return arena_->take(bytes); }
+inline bool Allocator::arena_give(void* p, size_t bytes) const { return arena_->give(p, bytes); }
+
+// Runs body(alloc) with a scratch arena.  A call that runs out of memory so is
+// repeated without one: what fitted a caller's memory before still does.
+template <typename F>
+void with_scratch(cspt_allocator const* mr, cudaStream_t stream, F&& body)
+{
+  try {
+    Allocator alloc(mr, stream);
+    ScratchArena arena(alloc);
+    body(static_cast<Allocator const&>(alloc));
+  } catch (Error const& e) {
+    if (e.status != CSPT_OUT_OF_MEMORY) throw;
+    Allocator const alloc(mr, stream);
+    body(alloc);
+  }
+}
+
+// A buffer that is handed to the caller (release()): never from the arena.
+struct OutputBuffer {};
 
 // Owning typed device buffer (freed on scope exit unless released).
 template <typename T>
@@ -154,6 +270,10 @@ class Buffer {
  public:
   Buffer() = default;
   Buffer(Allocator const& a, size_t n) : a_(&a), n_(n)
+  {
+    p_ = static_cast<T*>(a.allocate(n * sizeof(T), true));
+  }
+  Buffer(Allocator const& a, size_t n, OutputBuffer) : a_(&a), n_(n)
   {
     p_ = static_cast<T*>(a.allocate(n * sizeof(T)));
   }

@@ -92,7 +92,7 @@ void run(cspt_quadtree const* tree, T const* bminx, T const* bminy, T const* bma
   if (k == 0) return;
   int key_bits = 1;
   while (key_bits < 32 && (host[1] >> key_bits) != 0) ++key_bits;
-  Buffer<uint32_t> ob(alloc, k), on(alloc, k);
+  Buffer<uint32_t> ob(alloc, k, OutputBuffer{}), on(alloc, k, OutputBuffer{});
   if (appended == k && k <= cap) {
     // Every pair was appended (in no particular order): sort them by
     // (leaf offset, box), one composite key, which is the order the write

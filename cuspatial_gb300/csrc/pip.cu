@@ -787,7 +787,7 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
     finish_counts();
     *out_n = m;
     if (m == 0) return;
-    Buffer<uint32_t> op(alloc, m), oq(alloc, m);
+    Buffer<uint32_t> op(alloc, m, OutputBuffer{}), oq(alloc, m, OutputBuffer{});
     expand(0, npairs, out_off, op.data(), oq.data(), m);
     *out_poly  = op.release();
     *out_point = oq.release();
@@ -1070,15 +1070,13 @@ template <typename T>
 void join_host(T const* hx, T const* hy, size_t n, double x_min, double x_max, double y_min,
                double y_max, double scale, int max_depth, int32_t max_size, uint32_t const* hpo,
                size_t npo, uint32_t const* hro, size_t nro, T const* hvx, T const* hvy,
-               size_t nv, cspt_method method, cspt_allocator const* mr, cudaStream_t s,
+               size_t nv, cspt_method method, Allocator const& alloc, Allocator const& palloc,
                HostRows const& out, size_t* out_n, uint64_t* out_refined)
 {
+  cudaStream_t const s = alloc.stream(), ps = palloc.stream();
   cspt_dtype const dtype = std::is_same<T, double>::value ? CSPT_FLOAT64 : CSPT_FLOAT32;
   bool const filtered    = method == CSPT_METHOD_FILTERED && std::is_same<T, double>::value;
   size_t const np        = npo - 1;
-  Allocator const alloc(mr, s);
-  cudaStream_t const ps = side_stream(1);
-  Allocator const palloc(mr, ps);
   // polygon columns, boxes and index: allocated and used on ps, read on s
   // once s has waited for ps
   Buffer<uint32_t> dpo(palloc, npo), dro(palloc, nro);
@@ -1142,16 +1140,20 @@ void point_in_polygon_join_host(void const* hx, void const* hy, size_t n, cspt_d
                                 cspt_method method, cspt_allocator const* mr, cudaStream_t s,
                                 HostRows const& out, size_t* out_n, uint64_t* out_refined)
 {
-  if (dtype == CSPT_FLOAT64)
-    join_host<double>(static_cast<double const*>(hx), static_cast<double const*>(hy), n, x_min,
-                      x_max, y_min, y_max, scale, max_depth, max_size, hpo, npo, hro, nro,
-                      static_cast<double const*>(hvx), static_cast<double const*>(hvy), nv,
-                      method, mr, s, out, out_n, out_refined);
-  else
-    join_host<float>(static_cast<float const*>(hx), static_cast<float const*>(hy), n, x_min,
-                     x_max, y_min, y_max, scale, max_depth, max_size, hpo, npo, hro, nro,
-                     static_cast<float const*>(hvx), static_cast<float const*>(hvy), nv, method,
-                     mr, s, out, out_n, out_refined);
+  with_scratch(mr, s, [&](Allocator const& alloc) {
+    with_scratch(mr, side_stream(1), [&](Allocator const& palloc) {
+      if (dtype == CSPT_FLOAT64)
+        join_host<double>(static_cast<double const*>(hx), static_cast<double const*>(hy), n, x_min,
+                          x_max, y_min, y_max, scale, max_depth, max_size, hpo, npo, hro, nro,
+                          static_cast<double const*>(hvx), static_cast<double const*>(hvy), nv,
+                          method, alloc, palloc, out, out_n, out_refined);
+      else
+        join_host<float>(static_cast<float const*>(hx), static_cast<float const*>(hy), n, x_min,
+                         x_max, y_min, y_max, scale, max_depth, max_size, hpo, npo, hro, nro,
+                         static_cast<float const*>(hvx), static_cast<float const*>(hvy), nv, method,
+                         alloc, palloc, out, out_n, out_refined);
+    });
+  });
 }
 
 }  // namespace cspt

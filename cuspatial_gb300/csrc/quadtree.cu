@@ -371,7 +371,8 @@ void build(T const* x, T const* y, size_t n, double x1d, double x2d, double y1d,
   KernelTimer timer("quadtree_build", s);
 
   Buffer<uint32_t> keys(alloc, n), keys_alt(alloc, n);
-  Buffer<uint32_t> idx(alloc, n), idx_alt(alloc, n);
+  // (either may become the output, depending on the number of passes)
+  Buffer<uint32_t> idx(alloc, n, OutputBuffer{}), idx_alt(alloc, n, OutputBuffer{});
   // ordered copy requested: the key pass also writes the points interleaved
   // (input order), so the gather after the sort reads one vector per point
   Buffer<T> xy_in(alloc, ordered ? 2 * n : 0);
@@ -477,8 +478,9 @@ void build(T const* x, T const* y, size_t n, double x1d, double x2d, double y1d,
       },
       n, total.data(), alloc);
     size_t const q = read_back(total.data(), s);
-    Buffer<uint32_t> okey(alloc, q), olen(alloc, q), ooff(alloc, q);
-    Buffer<uint8_t> olev(alloc, q), oint(alloc, q);
+    OutputBuffer const out_tag;
+    Buffer<uint32_t> okey(alloc, q, out_tag), olen(alloc, q, out_tag), ooff(alloc, q, out_tag);
+    Buffer<uint8_t> olev(alloc, q, out_tag), oint(alloc, q, out_tag);
     bottom_count_kernel<<<grid_for(q, blk, sm_grid(16u)), blk, 0, s>>>(st, q, n, olen.data());
     CSPT_CHECK_LAUNCH();
     uint32_t const* sk = skeys.data();
@@ -509,8 +511,9 @@ void build(T const* x, T const* y, size_t n, double x1d, double x2d, double y1d,
   CSPT_CHECK_LAUNCH();
   exclusive_scan<uint32_t>(rows.data(), rows.data(), cells, total.data(), alloc);
   size_t const q = read_back(total.data(), s);
-  Buffer<uint32_t> okey(alloc, q), olen(alloc, q), ooff(alloc, q);
-  Buffer<uint8_t> olev(alloc, q), oint(alloc, q);
+  OutputBuffer const out_tag;
+  Buffer<uint32_t> okey(alloc, q, out_tag), olen(alloc, q, out_tag), ooff(alloc, q, out_tag);
+  Buffer<uint8_t> olev(alloc, q, out_tag), oint(alloc, q, out_tag);
   node_write_kernel<<<tiles, kNodeBlock, 0, s>>>(skeys.data(), n, d, max_size, codes.data(),
                                                  rows.data(), okey.data(), olev.data(),
                                                  oint.data(), olen.data(), ooff.data());
