@@ -16,10 +16,15 @@
 // The distance is the reference's expression with its dot products contracted
 // the way nvcc contracts a.x*b.x + a.y*b.y (one FMA on the x term).
 //
+// Exact method: linestrings and chunks of segments whose bounding box is
+// certainly farther than the running winner are passed over (box_lower); the
+// distances that decide are the reference's expression in the input type.
+//
 // Filtered method (float64 inputs): each segment is first bounded in float32
 // with a forward error bound; only segments whose lower bound can still beat
 // the best upper bound of the point are evaluated with the float64
 // expression, so the winner and its distance are the exact ones.
+#include <algorithm>
 #include <memory>
 
 #include "common.cuh"
@@ -69,17 +74,6 @@ __device__ inline T segment_dist2(T px, T py, T ax, T ay, T bx, T by)
   return r >= d2 ? fmin(d0, d1) : d0 - r;
 }
 
-// point_linestring_distance.cuh:32-51
-template <typename T>
-__device__ inline T linestring_distance(T px, T py, T const* lx, T const* ly, uint32_t v0,
-                                        uint32_t v1)
-{
-  T ds = std::numeric_limits<T>::max();
-  for (uint32_t s = v0; s + 1 < v1; ++s)
-    ds = fmin(ds, segment_dist2<T>(px, py, lx[s], ly[s], lx[s + 1], ly[s + 1]));
-  return sqrt(ds);
-}
-
 // quadtree_point_to_nearest_linestring.cuh:279-294 — lhs is the running
 // value, rhs the next candidate.
 template <typename T>
@@ -105,46 +99,209 @@ __global__ void init_rows_kernel(size_t n, uint32_t* __restrict__ opt, uint32_t*
   }
 }
 
-template <typename T, bool Filtered>
+constexpr int kSegChunk = 8;  // segments per pruning box
+
+// Bounding boxes (minx, miny, maxx, maxy) of the linestrings and of their
+// chunks of kSegChunk segments, in float32 rounded outward; a box with a
+// non-finite coordinate is the whole plane.  Chunk c of linestring l is at
+// v0 / kSegChunk + l + c (v0 its first vertex): the ranges of successive
+// linestrings do not overlap, and no scan is needed to place them.
+struct LsBounds {
+  float4 const* ls;
+  float4 const* chunk;
+  uint32_t slots;  // chunk boxes; offsets that leave them are not pruned by chunk
+};
+__host__ __device__ inline size_t chunk_slots(size_t nv, size_t nls)
+{
+  return nv / kSegChunk + nls + 1;
+}
+
+__device__ inline float float_down(double v) { return __double2float_rd(v); }
+__device__ inline float float_up(double v) { return __double2float_ru(v); }
+__device__ inline float float_down(float v) { return v; }
+__device__ inline float float_up(float v) { return v; }
+
+struct BoundBox {
+  float4 b;  // empty: (inf, inf, -inf, -inf)
+  __device__ BoundBox() : b(make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY)) {}
+  template <typename T>
+  __device__ void add(T x, T y)
+  {
+    if (isfinite(x) && isfinite(y)) {
+      b.x = fminf(b.x, float_down(x));
+      b.y = fminf(b.y, float_down(y));
+      b.z = fmaxf(b.z, float_up(x));
+      b.w = fmaxf(b.w, float_up(y));
+    } else {
+      b = make_float4(-INFINITY, -INFINITY, INFINITY, INFINITY);
+    }
+  }
+  __device__ void add(float4 o)
+  {
+    b = make_float4(fminf(b.x, o.x), fminf(b.y, o.y), fmaxf(b.z, o.z), fmaxf(b.w, o.w));
+  }
+};
+
+// One warp per linestring, a lane per chunk.
+template <typename T>
 __global__ void __launch_bounds__(256)
-  nearest_kernel(uint32_t const* __restrict__ group_start, size_t ngroups, size_t npairs,
-                 uint32_t const* __restrict__ pair_ls, uint32_t const* __restrict__ pair_quad,
-                 uint32_t const* __restrict__ qlen, uint32_t const* __restrict__ qoff,
-                 PointSource<T> const src, size_t npi, uint32_t const* __restrict__ lso, size_t nls,
-                 T const* __restrict__ lx, T const* __restrict__ ly, uint32_t* __restrict__ opt,
+  ls_bounds_kernel(uint32_t const* __restrict__ lso, size_t nls, T const* __restrict__ lx,
+                   T const* __restrict__ ly, size_t slots, float4* __restrict__ ls_box,
+                   float4* __restrict__ chunk_box)
+{
+  int const lane      = threadIdx.x & 31;
+  size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
+  for (size_t l = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5; l < nls;
+       l += nwarps) {
+    uint32_t const v0   = lso[l], v1 = lso[l + 1];
+    uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
+    size_t const base   = v0 / kSegChunk + l;
+    BoundBox all;
+    for (uint32_t c = lane; c * kSegChunk < nseg; c += 32) {
+      BoundBox box;
+      uint32_t const s0 = v0 + c * kSegChunk, s1 = min(s0 + kSegChunk, v0 + nseg);
+      for (uint32_t v = s0; v <= s1; ++v) box.add(lx[v], ly[v]);
+      if (base + c < slots) chunk_box[base + c] = box.b;
+      all.add(box.b);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      all.add(make_float4(__shfl_xor_sync(0xFFFFFFFFu, all.b.x, o),
+                          __shfl_xor_sync(0xFFFFFFFFu, all.b.y, o),
+                          __shfl_xor_sync(0xFFFFFFFFu, all.b.z, o),
+                          __shfl_xor_sync(0xFFFFFFFFu, all.b.w, o)));
+    if (lane == 0) ls_box[l] = all.b;
+  }
+}
+
+// A lower bound of the squared segment distance that the reference's
+// expression gives in type T, for every segment with both ends in box b and a
+// finite point in [xl, xu] x [yl, yu].  The distance to the box is rounded
+// down throughout.  With u the type's unit roundoff (2^-53, 2^-24), D^2 the
+// largest squared distance to the box and v, e the expression's vectors, its
+// value is within 21 u D^2 of the exact one: 4 u |v|^2 for d0, 5 u |v| |e| for
+// d3 and 4 u |e|^2 for d2, hence 16 u |v|^2 for r = d3^2 / d2, and u for the
+// difference; underflow adds less than 2^-120.  The bound takes 32 u D^2.
+struct PointBounds {
+  float xl, xu, yl, yu;
+  bool finite;
+};
+template <typename T>
+__device__ inline PointBounds point_bounds(T x, T y)
+{
+  return PointBounds{float_down(x), float_up(x), float_down(y), float_up(y),
+                     isfinite(x) && isfinite(y)};
+}
+template <typename T>
+__device__ inline float box_lower(PointBounds const& p, float4 b)
+{
+  constexpr float k32u = sizeof(T) == 8 ? 3.5527136788005009e-15f : 1.9073486328125e-06f;
+  float const dx = fmaxf(fmaxf(__fsub_rd(b.x, p.xu), __fsub_rd(p.xl, b.z)), 0.0f);
+  float const dy = fmaxf(fmaxf(__fsub_rd(b.y, p.yu), __fsub_rd(p.yl, b.w)), 0.0f);
+  float const fx = fmaxf(__fsub_ru(p.xu, b.x), __fsub_ru(b.z, p.xl));
+  float const fy = fmaxf(__fsub_ru(p.yu, b.y), __fsub_ru(b.w, p.yl));
+  float const lb = __fadd_rd(__fmul_rd(dx, dx), __fmul_rd(dy, dy));
+  float const D2 = __fadd_ru(__fmul_ru(fx, fx), __fmul_ru(fy, fy));
+  return __fsub_rd(lb, __fmaf_ru(D2, k32u, 7.52316384526264e-37f));
+}
+
+// The running winner of the reference's fold, and the squared distance (in
+// float32, rounded up) beyond which a candidate's root is larger than the
+// winner's: such a candidate is not zero and never taken.  Nothing is passed
+// over while there is no winner, its distance is zero (it yields to the next
+// candidate whatever that is) or not a number.
+template <typename T>
+struct Fold {
+  bool have    = false;
+  uint32_t bid = 0;
+  T bd         = 0;
+  float far    = INFINITY;
+
+  __device__ void take(T d, uint32_t lid)
+  {
+    if (!have || take_rhs<T>(bd, bid, d, lid)) {
+      bid = lid;
+      bd  = d;
+      // (1 + 2^-20) covers the roundings of the root and of the square
+      far = bd > T{0} ? __fmul_ru(__fmul_ru(float_up(bd), float_up(bd)), 1.0000009536743164f)
+                      : INFINITY;
+    }
+    have = true;
+  }
+};
+
+// point_linestring_distance.cuh:32-51 without the chunks that cannot change
+// the fold: those beyond `far`, and those beyond the smallest distance so far.
+template <typename T>
+__device__ inline T linestring_distance(T px, T py, PointBounds const& pb, T const* lx,
+                                        T const* ly, uint32_t v0, uint32_t v1,
+                                        LsBounds const& bounds, uint32_t slot, float far)
+{
+  T ds                = std::numeric_limits<T>::max();
+  uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
+  for (uint32_t c = 0; c * kSegChunk < nseg; ++c) {
+    if (pb.finite && slot + c < bounds.slots && box_lower<T>(pb, bounds.chunk[slot + c]) > far)
+      continue;
+    uint32_t const s0 = v0 + c * kSegChunk, s1 = min(s0 + kSegChunk, v0 + nseg);
+    T ax = lx[s0], ay = ly[s0];
+    for (uint32_t s = s0; s < s1; ++s) {
+      T const bx = lx[s + 1], by = ly[s + 1];
+      ds = fmin(ds, segment_dist2<T>(px, py, ax, ay, bx, by));
+      ax = bx;
+      ay = by;
+    }
+    far = fminf(far, float_up(ds));
+  }
+  return sqrt(ds);
+}
+
+// A lane per point; the candidates of its group in pair order.  `split` warps
+// share a group.  Bound by the float64 pipe (two lanes a cycle and SM) and, on
+// few points, by one warp's chain of candidates, hence the split.  20k points,
+// 301 linestrings of 2 to 64 segments: the call took 7652 us with every
+// candidate evaluated, 881 us with the boxes.
+template <typename T>
+__global__ void __launch_bounds__(256)
+  nearest_kernel(uint32_t const* __restrict__ group_start, uint32_t const* __restrict__ ngroups_p,
+                 size_t npairs, uint32_t split, uint32_t const* __restrict__ pair_ls,
+                 uint32_t const* __restrict__ pair_quad, uint32_t const* __restrict__ qlen,
+                 uint32_t const* __restrict__ qoff, PointSource<T> const src, size_t npi,
+                 uint32_t const* __restrict__ lso, size_t nls, T const* __restrict__ lx,
+                 T const* __restrict__ ly, LsBounds const bounds, uint32_t* __restrict__ opt,
                  uint32_t* __restrict__ ols, T* __restrict__ od)
 {
-  int const lane     = threadIdx.x & 31;
-  size_t const warps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
-  for (size_t g = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5; g < ngroups;
-       g += warps) {
+  int const lane       = threadIdx.x & 31;
+  size_t const warps   = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
+  size_t const ngroups = *ngroups_p;
+  for (size_t t = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
+       t < ngroups * split; t += warps) {
+    size_t const g      = t / split;
+    uint32_t const part = static_cast<uint32_t>(t - g * split);
     uint32_t const k0   = group_start[g];
     uint32_t const k1   = (g + 1 < ngroups) ? group_start[g + 1] : static_cast<uint32_t>(npairs);
     uint32_t const quad = pair_quad[k0];
     uint32_t const len  = qlen[quad];
     uint64_t const off  = qoff[quad];
-    for (uint32_t c = lane; c < len; c += 32) {
+    for (uint32_t c = part * 32 + lane; c < len; c += 32 * split) {
       uint64_t const pos = off + c;
       if (pos >= npi) continue;
       T px, py;
       src.load(pos, px, py);
-      bool have    = false;
-      uint32_t bid = 0;
-      T bd         = 0;
+      PointBounds const pb = point_bounds<T>(px, py);
+      Fold<T> f;
       for (uint32_t k = k0; k < k1; ++k) {
         uint32_t const lid = pair_ls[k];
         if (lid >= nls) continue;
-        T const d = linestring_distance<T>(px, py, lx, ly, lso[lid], lso[lid + 1]);
-        if (!have || take_rhs<T>(bd, bid, d, lid)) {
-          bid = lid;
-          bd  = d;
-        }
-        have = true;
+        if (pb.finite && box_lower<T>(pb, bounds.ls[lid]) > f.far) continue;
+        uint32_t const v0 = lso[lid];
+        f.take(linestring_distance<T>(px, py, pb, lx, ly, v0, lso[lid + 1],
+                                      bounds, v0 / kSegChunk + lid, f.far),
+               lid);
       }
-      if (have) {
+      if (f.have) {
         opt[pos] = static_cast<uint32_t>(pos);
-        ols[pos] = bid;
-        od[pos]  = bd;
+        ols[pos] = f.bid;
+        od[pos]  = f.bd;
       }
     }
   }
@@ -153,15 +310,13 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 // float32 filter (float64 inputs)
 // ---------------------------------------------------------------------------
-constexpr int kSegChunk = 8;  // segments per pruning box
-
 // Per linestring, what the segment listing needs in one 64-byte record.
 struct __align__(16) LsRec {
   long long aix, aiy;  // anchor in grid steps
   float4 box;          // box of its float32 segments, anchor frame
   float maxoff;        // largest |float32 offset|
   uint32_t v0, nseg;   // first vertex, segments
-  uint32_t cb;         // first chunk
+  uint32_t cb;         // first chunk's slot
   uint32_t exact;      // non-finite coordinates: exact path only
   uint32_t pad[3];
 };
@@ -171,7 +326,6 @@ struct LinestringIndexView {
   long long const* aix;  // anchors in grid steps
   long long const* aiy;
   float const* maxoff;   // largest |float32 offset| of the linestring
-  uint32_t const* chunk_base;
   float4 const* chunk_box;  // (minx, miny, maxx, maxy) of 8 segments, anchor frame
   float4 const* seg32;      // per segment start vertex: (ax, ay, bx, by), anchor frame
   uint8_t const* exact;     // non-finite coordinates: exact path only
@@ -181,8 +335,7 @@ struct LinestringIndexView {
 // per linestring: box, anchor, float32 segments, chunk boxes (one warp each)
 __global__ void __launch_bounds__(256)
   ls_box_kernel(uint32_t const* __restrict__ lso, size_t nls, double const* __restrict__ lx,
-                double const* __restrict__ ly, double4_16a* __restrict__ box, uint8_t* exact,
-                uint32_t* nchunks)
+                double const* __restrict__ ly, double4_16a* __restrict__ box, uint8_t* exact)
 {
   int const lane      = threadIdx.x & 31;
   size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -209,8 +362,6 @@ __global__ void __launch_bounds__(256)
     if (lane == 0) {
       box[l]         = make_double4_16a(mnx, mny, mxx, mxy);
       exact[l]       = bad ? 1 : 0;
-      uint32_t const ns = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
-      nchunks[l]     = (ns + kSegChunk - 1) / kSegChunk;
     }
   }
 }
@@ -243,9 +394,10 @@ __global__ void __launch_bounds__(1024) ls_grid_kernel(double4_16a const* __rest
 __global__ void __launch_bounds__(256)
   ls_fill_kernel(uint32_t const* __restrict__ lso, size_t nls, double const* __restrict__ lx,
                  double const* __restrict__ ly, double4_16a const* __restrict__ box,
-                 double const* __restrict__ gridp, uint32_t const* __restrict__ chunk_base,
-                 uint8_t const* __restrict__ exact, long long* aix, long long* aiy,
-                 float* maxoff, float4* chunk_box, float4* seg32, LsRec* rec)
+                 double const* __restrict__ gridp, uint8_t const* __restrict__ exact,
+                 long long* aix, long long* aiy, float* maxoff, float4* chunk_box, float4* seg32,
+                 LsRec* rec, size_t slots, float4* __restrict__ abs_ls,
+                 float4* __restrict__ abs_chunk)
 {
   int const lane      = threadIdx.x & 31;
   size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -261,15 +413,19 @@ __global__ void __launch_bounds__(256)
     double const cx = rx * g, cy = ry * g;
     uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
     uint32_t const nch  = (nseg + kSegChunk - 1) / kSegChunk;
-    uint32_t const cb   = chunk_base[l];
+    uint32_t const cb   = v0 / kSegChunk + static_cast<uint32_t>(l);
     float m             = 0.0f;
     float4 lbx          = make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
+    BoundBox all;  // the boxes of LsBounds, for points folded over every candidate
     // lane per chunk
     for (uint32_t c = lane; c < nch; c += 32) {
       float4 cbx = make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
       uint32_t const s0 = v0 + c * kSegChunk;
       uint32_t const s1 = min(s0 + kSegChunk, v0 + nseg);
+      BoundBox abs_box;
+      abs_box.add(lx[s0], ly[s0]);
       for (uint32_t sg = s0; sg < s1; ++sg) {
+        abs_box.add(lx[sg + 1], ly[sg + 1]);
         float4 e;
         e.x       = static_cast<float>(lx[sg] - cx);
         e.y       = static_cast<float>(ly[sg] - cy);
@@ -282,7 +438,11 @@ __global__ void __launch_bounds__(256)
         cbx.w     = fmaxf(cbx.w, fmaxf(e.y, e.w));
         m = fmaxf(m, fmaxf(fmaxf(fabsf(e.x), fabsf(e.y)), fmaxf(fabsf(e.z), fabsf(e.w))));
       }
-      chunk_box[cb + c] = cbx;
+      all.add(abs_box.b);
+      if (cb + c < slots) {
+        chunk_box[cb + c] = cbx;
+        abs_chunk[cb + c] = abs_box.b;
+      }
       lbx = make_float4(fminf(lbx.x, cbx.x), fminf(lbx.y, cbx.y), fmaxf(lbx.z, cbx.z),
                         fmaxf(lbx.w, cbx.w));
     }
@@ -291,7 +451,10 @@ __global__ void __launch_bounds__(256)
     lbx.y = warp_min(lbx.y);
     lbx.z = warp_max(lbx.z);
     lbx.w = warp_max(lbx.w);
+    all.b = make_float4(warp_min(all.b.x), warp_min(all.b.y), warp_max(all.b.z),
+                        warp_max(all.b.w));
     if (lane == 0) {
+      abs_ls[l] = all.b;
       aix[l]    = static_cast<long long>(rx);
       aiy[l]    = static_cast<long long>(ry);
       maxoff[l] = m;
@@ -375,6 +538,7 @@ struct NearestArgs {
   float2 const* u;
   LeafFrame const* frames;
   LinestringIndexView li;
+  LsBounds bounds;
   float gf;
   uint32_t* opt;
   uint32_t* ols;
@@ -383,21 +547,61 @@ struct NearestArgs {
   unsigned long long* next_group;
 };
 
-// The reference's fold over every candidate of the group, in float64 (the
-// literal per-point loop of the reference).
-__device__ inline void fold_all(NearestArgs const& a, uint32_t k0, uint32_t k1, double px,
-                                double py, bool& have, uint32_t& bid, double& bd)
+// The reference's fold over every candidate of the group for one point, by the
+// whole warp: a lane per linestring tests its box, and those that may matter
+// are taken in pair order, a lane per segment.  (By one lane over every
+// segment, one point at distance zero among 5M cost 50 to 110 ms.)
+__device__ void fold_warp(NearestArgs const& a, uint32_t k0, uint32_t k1, double px, double py,
+                          Fold<double>& f)
 {
-  have = false;
-  for (uint32_t k = k0; k < k1; ++k) {
-    uint32_t const lid = a.pair_ls[k];
-    if (lid >= a.nls) continue;
-    double const d = linestring_distance<double>(px, py, a.lx, a.ly, a.lso[lid], a.lso[lid + 1]);
-    if (!have || take_rhs<double>(bd, bid, d, lid)) {
-      bid = lid;
-      bd  = d;
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  int const lane          = threadIdx.x & 31;
+  PointBounds const pb    = point_bounds<double>(px, py);
+  f                       = Fold<double>{};
+  for (uint32_t kb = k0; kb < k1; kb += 32) {
+    uint32_t const k = kb + static_cast<uint32_t>(lane);
+    uint32_t lid     = k < k1 ? a.pair_ls[k] : 0xFFFFFFFFu;
+    bool const valid = k < k1 && lid < a.nls;
+    float const lb   = valid && pb.finite ? box_lower<double>(pb, a.bounds.ls[lid]) : -INFINITY;
+    unsigned left    = __ballot_sync(kAll, valid);
+    for (;;) {
+      left &= __ballot_sync(kAll, !(lb > f.far));
+      if (!left) break;
+      int const src = __ffs(left) - 1;
+      left &= left - 1u;
+      uint32_t const l    = __shfl_sync(kAll, lid, src);
+      uint32_t const v0   = a.lso[l], v1 = a.lso[l + 1];
+      uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
+      uint32_t const slot = v0 / kSegChunk + l;
+      double ds           = std::numeric_limits<double>::max();
+      for (uint32_t s = lane; s < nseg; s += 32) {
+        uint32_t const c = slot + s / kSegChunk;
+        if (pb.finite && c < a.bounds.slots && box_lower<double>(pb, a.bounds.chunk[c]) > f.far)
+          continue;
+        uint32_t const v = v0 + s;
+        ds = fmin(ds, segment_dist2<double>(px, py, a.lx[v], a.ly[v], a.lx[v + 1], a.ly[v + 1]));
+      }
+      for (int o = 16; o > 0; o >>= 1) ds = fmin(ds, __shfl_xor_sync(kAll, ds, o));
+      f.take(sqrt(ds), l);
     }
-    have = true;
+  }
+}
+
+// Folds the points of the lanes that ask for it, one after the other.
+__device__ inline void fold_lanes(NearestArgs const& a, uint32_t k0, uint32_t k1, bool ask,
+                                  double px, double py, bool& have, uint32_t& bid, double& bd,
+                                  uint32_t& nfb)
+{
+  for (unsigned m = __ballot_sync(0xFFFFFFFFu, ask); m; m &= m - 1u) {
+    int const src = __ffs(m) - 1;
+    Fold<double> f;
+    fold_warp(a, k0, k1, __shfl_sync(0xFFFFFFFFu, px, src), __shfl_sync(0xFFFFFFFFu, py, src), f);
+    if (static_cast<int>(threadIdx.x & 31) == src) {
+      ++nfb;
+      have = f.have;
+      bid  = f.bid;
+      bd   = f.bd;
+    }
   }
 }
 
@@ -405,10 +609,12 @@ __device__ inline void fold_all(NearestArgs const& a, uint32_t k0, uint32_t k1, 
 // pass 1 bounds the running minimum U with float32 estimates and chunk
 // pruning, pass 2 evaluates in float64 only the segments whose estimate can
 // reach U, then the fold; a point whose candidates reach only zero distances
-// (or none) takes fold_all.  Used for groups the listing below cannot take.
-__device__ inline void nearest_point_scan(NearestArgs const& a, uint32_t k0, uint32_t k1,
+// (or none) is folded over every candidate (returns true).  Used for groups the
+// listing below cannot take.
+__device__ inline bool nearest_point_scan(NearestArgs const& a, uint32_t k0, uint32_t k1,
                                           LeafFrame const& lf, uint64_t pos, bool gok,
-                                          uint32_t& nfb)
+                                          double& px, double& py, bool& have, uint32_t& bid,
+                                          double& bd)
 {
   LinestringIndexView const& li = a.li;
   float const gf  = a.gf;
@@ -431,7 +637,7 @@ __device__ inline void nearest_point_scan(NearestArgs const& a, uint32_t k0, uin
     float const tol = 4.76837158203125e-07f * m;
     uint32_t const v0 = a.lso[lid], v1 = a.lso[lid + 1];
     uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
-    uint32_t const cb   = li.chunk_base[lid];
+    uint32_t const cb   = v0 / kSegChunk + lid;
     for (uint32_t ch = 0; ch * kSegChunk < nseg; ++ch) {
       if (box_lb(qx, qy, li.chunk_box[cb + ch], tol) > U) continue;
       uint32_t const s0 = v0 + ch * kSegChunk, s1 = min(s0 + kSegChunk, v0 + nseg);
@@ -442,11 +648,8 @@ __device__ inline void nearest_point_scan(NearestArgs const& a, uint32_t k0, uin
       }
     }
   }
-  double px = 0.0, py = 0.0;
   a.src.load(pos, px, py);
-  bool have = false, skipped = false, nonzero = false;
-  uint32_t bid = 0;
-  double bd    = 0.0;
+  bool skipped = false, nonzero = false;
   if (!full) {
     // pass 2: float64 on every segment that can reach U (widened so that
     // distances left out are larger even after the square root)
@@ -462,7 +665,7 @@ __device__ inline void nearest_point_scan(NearestArgs const& a, uint32_t k0, uin
       float const tol = 4.76837158203125e-07f * m;
       uint32_t const v0 = a.lso[lid], v1 = a.lso[lid + 1];
       uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
-      uint32_t const cb   = li.chunk_base[lid];
+      uint32_t const cb   = v0 / kSegChunk + lid;
       double dmin         = std::numeric_limits<double>::max();
       bool evaluated      = false;
       for (uint32_t ch = 0; ch * kSegChunk < nseg; ++ch) {
@@ -493,15 +696,7 @@ __device__ inline void nearest_point_scan(NearestArgs const& a, uint32_t k0, uin
     // the winner is the nearest non-zero one, find it exactly
     if (!have || (!nonzero && skipped)) full = true;
   }
-  if (full) {
-    ++nfb;
-    fold_all(a, k0, k1, px, py, have, bid, bd);
-  }
-  if (have) {
-    a.opt[pos] = static_cast<uint32_t>(pos);
-    a.ols[pos] = bid;
-    a.od[pos]  = bd;
-  }
+  return full;
 }
 
 // The group's segment list (per warp, in shared memory): the candidate
@@ -806,9 +1001,19 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
     if (!listed) {
       __syncwarp();
       ++nscan;
-      for (uint32_t c = lane; c < len; c += 32) {
-        uint64_t const pos = off + c;
-        if (pos < a.npi) nearest_point_scan(a, k0, k1, lf, pos, gok, nfb);
+      for (uint32_t c0 = 0; c0 < len; c0 += 32) {
+        uint64_t const pos = off + c0 + static_cast<uint32_t>(lane);
+        bool const act     = c0 + static_cast<uint32_t>(lane) < len && pos < a.npi;
+        double px = 0.0, py = 0.0, bd = 0.0;
+        bool have = false;
+        uint32_t bid    = 0;
+        bool const fold = act && nearest_point_scan(a, k0, k1, lf, pos, gok, px, py, have, bid, bd);
+        fold_lanes(a, k0, k1, fold, px, py, have, bid, bd, nfb);
+        if (act && have) {
+          a.opt[pos] = static_cast<uint32_t>(pos);
+          a.ols[pos] = bid;
+          a.od[pos]  = bd;
+        }
       }
       __syncwarp();
       continue;
@@ -886,16 +1091,11 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
         }
       }
       __syncwarp();  // the candidate slots are reused by the next chunk
-      if (act) {
-        if (!have || zero) {
-          ++nfb;
-          fold_all(a, k0, k1, px, py, have, bid, bd);
-        }
-        if (have) {
-          a.opt[pos] = static_cast<uint32_t>(pos);
-          a.ols[pos] = bid;
-          a.od[pos]  = bd;
-        }
+      fold_lanes(a, k0, k1, act && (!have || zero), px, py, have, bid, bd, nfb);
+      if (act && have) {
+        a.opt[pos] = static_cast<uint32_t>(pos);
+        a.ols[pos] = bid;
+        a.od[pos]  = bd;
       }
     }
     __syncwarp();  // the next group rewrites this warp's list
@@ -941,22 +1141,23 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       std::unique_ptr<KernelTimer> index_timer(new KernelTimer("nearest_index", s));
       Buffer<double4_16a> box(alloc, nls);
       Buffer<uint8_t> lexact(alloc, nls);
-      Buffer<uint32_t> nch(alloc, nls + 1), cbase(alloc, nls + 1);
       Buffer<double> grid(alloc, 1);
       unsigned const lgrd = grid_for(nls * 32, 256, sm_grid(32u));
-      ls_box_kernel<<<lgrd, 256, 0, s>>>(lso, nls, lx, ly, box.data(), lexact.data(), nch.data());
+      ls_box_kernel<<<lgrd, 256, 0, s>>>(lso, nls, lx, ly, box.data(), lexact.data());
       CSPT_CHECK_LAUNCH();
       ls_grid_kernel<<<1, 1024, 0, s>>>(box.data(), nls, grid.data());
       CSPT_CHECK_LAUNCH();
-      exclusive_scan<uint32_t>(nch.data(), cbase.data(), nls, cbase.data() + nls, alloc);
       size_t const nv = nls ? read_back(lso + nls, s) : 0;
       Buffer<long long> aix(alloc, nls), aiy(alloc, nls);
       Buffer<float> maxoff(alloc, nls);
-      Buffer<float4> cbox(alloc, nv / kSegChunk + nls + 1), seg32(alloc, nv);
+      size_t const slots = chunk_slots(nv, nls);
+      Buffer<float4> cbox(alloc, slots), seg32(alloc, nv), abs_ls(alloc, nls),
+        abs_chunk(alloc, slots);
       Buffer<LsRec> lrec(alloc, nls);
       ls_fill_kernel<<<lgrd, 256, 0, s>>>(lso, nls, lx, ly, box.data(), grid.data(),
-                                          cbase.data(), lexact.data(), aix.data(), aiy.data(),
-                                          maxoff.data(), cbox.data(), seg32.data(), lrec.data());
+                                          lexact.data(), aix.data(), aiy.data(),
+                                          maxoff.data(), cbox.data(), seg32.data(), lrec.data(),
+                                          slots, abs_ls.data(), abs_chunk.data());
       CSPT_CHECK_LAUNCH();
       double const g = read_back(grid.data(), s);
       index_timer.reset();
@@ -969,15 +1170,16 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
         frames.data());
       CSPT_CHECK_LAUNCH();
       frames_timer.reset();
-      LinestringIndexView liv{aix.data(),  aiy.data(),   maxoff.data(), cbase.data(),
-                              cbox.data(), seg32.data(), lexact.data(), lrec.data()};
+      LinestringIndexView liv{aix.data(),   aiy.data(),    maxoff.data(), cbox.data(),
+                              seg32.data(), lexact.data(), lrec.data()};
+      LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(slots)};
       // points folded whole, groups scanned, next group, float64 segment distances
       Buffer<unsigned long long> fb(alloc, 4);
       CSPT_CUDA_TRY(cudaMemsetAsync(fb.data(), 0, 4 * sizeof(unsigned long long), s));
       NearestArgs const na{gs,          gs + npairs,  npairs,     pair_ls,   pair_quad,
                            tree->length, qoff,        src,        npi,       lso,
                            nls,          lx,          ly,         u.data(),  frames.data(),
-                           liv,          static_cast<float>(g), opt, ols,    od,
+                           liv,          bounds,      static_cast<float>(g), opt, ols,    od,
                            fb.data(),    fb.data() + 2};
       KernelTimer timer("nearest", s);
       int per_sm = 0;
@@ -1000,12 +1202,28 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       return;
     }
   }
-  size_t const ng = read_back(gs + npairs, s);
+  // the sizes of the launch and of the boxes, in one wait
+  uint32_t h[2] = {0, 0};  // groups, vertices
+  CSPT_CUDA_TRY(cudaMemcpyAsync(h, gs + npairs, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  if (nls)
+    CSPT_CUDA_TRY(cudaMemcpyAsync(h + 1, lso + nls, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  CSPT_CUDA_TRY(cudaStreamSynchronize(s));
+  size_t const ng = h[0], slots = chunk_slots(h[1], nls);
+  Buffer<float4> ls_box(alloc, nls), chunk_box(alloc, slots);
+  ls_bounds_kernel<T><<<grid_for(nls * 32, 256, sm_grid(32u)), 256, 0, s>>>(
+    lso, nls, lx, ly, slots, ls_box.data(), chunk_box.data());
+  CSPT_CHECK_LAUNCH();
   {
     KernelTimer timer("nearest", s);
-    nearest_kernel<T, false><<<grid_for(ng * 32, 256, sm_grid(32u)), 256, 0, s>>>(
-      gs, ng, npairs, pair_ls, pair_quad, tree->length, qoff, src, npi, lso, nls, lx, ly, opt,
-      ols, od);
+    // warps per group: enough for 16 warps on every SM, at most 8 (a leaf of
+    // 256 points has no more rounds of 32)
+    size_t const fill    = static_cast<size_t>(num_sms()) * 16;
+    uint32_t const split = static_cast<uint32_t>(
+      ng == 0 ? 1 : std::min<size_t>(8, std::max<size_t>(1, fill / ng)));
+    nearest_kernel<T><<<grid_for(ng * split * 32, 256, sm_grid(32u)), 256, 0, s>>>(
+      gs, gs + npairs, npairs, split, pair_ls, pair_quad, tree->length, qoff, src, npi, lso, nls,
+      lx, ly, LsBounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots)}, opt, ols,
+      od);
     CSPT_CHECK_LAUNCH();
   }
 }
