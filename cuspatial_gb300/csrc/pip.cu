@@ -63,6 +63,19 @@ __device__ inline uint32_t slab_lookup(float qy, float y0, float invh, uint32_t 
   if (fs > 0.0f) sj = fs >= static_cast<float>(ns) ? ns - 1 : static_cast<uint32_t>(fs);
   return sj >= ns ? ns - 1 : sj;
 }
+// Exact joins on float64 points from this many points on compare bounds first
+// (pip_bounds_kernel): at 1M points x 256 polygons the call takes 858 us with
+// the bounds, 940 without; at 1k points x 17 the bounds' launches cost what they
+// save (667 to 697 us with, 655 to 680 without).
+#ifndef CSPT_BOUNDS_POINTS
+#define CSPT_BOUNDS_POINTS 65536
+#endif
+constexpr size_t kBoundsPoints = CSPT_BOUNDS_POINTS;
+template <typename T>
+bool use_bounds(bool filtered, size_t points)
+{
+  return !filtered && std::is_same<T, double>::value && points >= kBoundsPoints;
+}
 // Blocks of 256 threads per SM for the leaf frames (the index fill that runs
 // beside them takes what the frames leave; 2-8 measured within 1%).
 #ifndef CSPT_LEAF_BLOCKS_PER_SM
@@ -560,6 +573,234 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
   }
 }
 
+// ---------------------------------------------------------------------------
+// Exact method on float64 points: comparisons of float32 bounds in front of
+// the reference's float64 expression.
+//
+// The float64 pipe (two lanes a cycle and SM) bounds pip_pair_kernel<false>:
+// about ten float64 instructions per edge of the point's slab and six for the
+// slab.  Most of those edges lie wholly left, right, above or below the point.
+// Points, edges and polygons therefore carry float32 bounds rounded outward
+// (truncated_f32 widened by outward_width), and only comparisons are made of
+// them; each bound leaves at least 2^-24 of the coordinates' magnitude, and so
+// of an edge's run and rise, to spare, where the reference's products are
+// within 9 roundings of float64 (2^-50):
+//   left, above or below the point: no toggle, not on the edge;
+//   right, and the point's y certainly between the ends': a toggle;
+//   anything else: exact_edge, in float64.
+// Exactly vertical edges report "on edge" at their x whatever the y: the
+// points' x is looked up among them in float64 as before.
+// A quadrant whose points' box meets no edge's box and no vertical edge has
+// one result (the argument is at the edge-free quadrants above, here with
+// comparisons only): the first point's, evaluated with its slab.
+// 2M points x 10k polygons of 8 to 256 vertices: 621 us, pip_pair_kernel<false>
+// 3690 us; the call 4728 -> 1449 us.
+// ---------------------------------------------------------------------------
+struct QuadBounds {
+  float xl, yl, xu, yu;  // the points' bounds
+  uint32_t nonfinite;    // some point is beyond float32 or not finite
+};
+
+// Per group of pairs sharing a quadrant: the points cut to float32 in
+// quadtree order, and their box.  One warp per group.
+__global__ void __launch_bounds__(256)
+  quad_bounds_kernel(uint32_t const* __restrict__ group_start,
+                     uint32_t const* __restrict__ ngroups_p,
+                     uint32_t const* __restrict__ pair_quad, uint32_t const* __restrict__ qlen,
+                     uint32_t const* __restrict__ qoff, PointSource<double> const src, size_t npi,
+                     float2* __restrict__ t, QuadBounds* __restrict__ out)
+{
+  int const lane      = threadIdx.x & 31;
+  size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
+  uint32_t const ng   = *ngroups_p;
+  for (size_t g = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5; g < ng;
+       g += nwarps) {
+    uint32_t const quad = pair_quad[group_start[g]];
+    uint32_t const len  = qlen[quad];
+    uint64_t const off  = qoff[quad];
+    float xl = INFINITY, yl = INFINITY, xu = -INFINITY, yu = -INFINITY;
+    bool bad = false;
+#pragma unroll 4
+    for (uint32_t c = lane; c < len; c += 32) {
+      if (off + c >= npi) break;
+      double px, py;
+      src.load(off + c, px, py);
+      float2 const v = make_float2(truncated_f32(px), truncated_f32(py));
+      t[off + c]     = v;
+      bad |= !(isfinite(v.x) && isfinite(v.y));
+      float const wx = outward_width(v.x), wy = outward_width(v.y);
+      xl = fminf(xl, __fsub_rd(v.x, wx));
+      yl = fminf(yl, __fsub_rd(v.y, wy));
+      xu = fmaxf(xu, __fadd_ru(v.x, wx));
+      yu = fmaxf(yu, __fadd_ru(v.y, wy));
+    }
+    xl  = warp_min(xl);
+    yl  = warp_min(yl);
+    xu  = warp_max(xu);
+    yu  = warp_max(yu);
+    bad = __any_sync(0xFFFFFFFFu, bad);
+    if (lane == 0) out[g] = QuadBounds{xl, yl, xu, yu, bad ? 1u : 0u};
+  }
+}
+
+// One edge against one point by bounds: 0 neither toggles nor holds the point,
+// 1 toggles, 2 undecided.  `inner` covers the widening of the edge's y bounds.
+__device__ inline int edge_by_bounds(float4 const& e, float xl, float yl, float xu, float yu,
+                                     float inner)
+{
+  if (xl > e.z || yl > e.w || yu < e.y) return 0;
+  return xu < e.x && yl > e.y + inner && yu < e.w - inner ? 1 : 2;
+}
+
+__global__ void __launch_bounds__(kPipBlock)
+  pip_bounds_kernel(uint32_t const* __restrict__ pair_poly, uint32_t const* __restrict__ pair_quad,
+                    uint32_t const* __restrict__ pair_group, size_t npairs,
+                    uint32_t const* __restrict__ qlen, uint32_t const* __restrict__ qoff,
+                    PointSource<double> const src, size_t npi, float2 const* __restrict__ t,
+                    QuadBounds const* __restrict__ quads, PolygonIndexView<double> ix,
+                    uint64_t const* __restrict__ word_off, uint32_t* __restrict__ bits,
+                    uint32_t* __restrict__ counts, unsigned long long* __restrict__ next_pair)
+{
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  int const lane          = threadIdx.x & 31;
+  for (;;) {
+    unsigned long long kk = 0;
+    if (lane == 0) kk = atomicAdd(next_pair, 1ull);
+    size_t const k = static_cast<size_t>(__shfl_sync(kAll, kk, 0));
+    if (k >= npairs) break;
+    uint32_t const poly = pair_poly[k];
+    uint32_t const quad = pair_quad[k];
+    uint32_t const len  = qlen[quad];
+    uint64_t const off  = qoff[quad];
+    uint64_t const wb   = word_off[k];
+    uint32_t const nw   = (len + 31) >> 5;
+    bool const known    = poly < ix.num_polygons;
+    QuadBounds const q  = quads[pair_group[k]];
+    float4 const box    = known ? ix.box32[poly] : make_float4(0.f, 0.f, 0.f, 0.f);
+    bool const walk     = known && ix.exact_only[poly];
+    if (!known || (!walk && !q.nonfinite &&
+                   (q.xl > box.z || q.xu < box.x || q.yl > box.w || q.yu < box.y))) {
+      for (uint32_t w = lane; w < nw; w += 32) bits[wb + w] = 0u;
+      if (lane == 0) counts[k] = 0;
+      continue;
+    }
+    float const invh     = ix.inv_slab_h32[poly];
+    uint32_t const ns    = ix.num_slabs[poly];
+    uint32_t const slab0 = ix.slab_base[poly];
+    uint32_t const vb = ix.vert_begin[poly], ve = ix.vert_end[poly];
+    float const y0    = truncated_f32(ix.pminy[poly]);
+    // the polygon's largest |y|; the float32 slab lookup is off by less than
+    // 1/64 slab while largest |y| x slabs per unit stays below 2^14
+    float const my    = fmaxf(fabsf(box.y), fabsf(box.w));
+    float const inner = __fmaf_ru(my, 9.5367431640625e-07f, 1.0e-36f);  // 2^-20
+    bool const lookup = fmaxf(my, fmaxf(fabsf(q.yl), fabsf(q.yu))) * invh <= 16384.0f;
+    bool verts        = vb < ve;  // some point may have a vertical edge's x
+    if (!walk && lookup && !q.nonfinite && len > 0 && off < npi) {
+      if (verts) {
+        uint32_t lo = vb, hi = ve;
+        while (lo < hi) {
+          uint32_t const mid = (lo + hi) >> 1;
+          if (ix.vert_x[mid] < static_cast<double>(q.xl))
+            lo = mid + 1;
+          else
+            hi = mid;
+        }
+        verts = lo < ve && ix.vert_x[lo] <= static_cast<double>(q.xu);
+      }
+      uint32_t const j0 = slab_lookup(q.yl, y0, invh, ns), j1 = slab_lookup(q.yu, y0, invh, ns);
+      uint32_t const E0 = ix.slab_start[slab0 + j0], E1 = ix.slab_start[slab0 + j1 + 1];
+      bool meets        = verts || E1 - E0 > kFreeScan;
+      for (uint32_t e0 = E0; e0 < E1 && !meets; e0 += 32) {
+        bool m = false;
+        if (e0 + lane < E1) {
+          float4 const e = ix.slab_e32[e0 + lane];
+          m              = !(q.xl > e.z || q.xu < e.x || q.yl > e.w || q.yu < e.y);
+        }
+        meets = __any_sync(kAll, m);
+      }
+      if (!meets) {
+        double px, py;
+        src.load(off, px, py);
+        float2 const v    = t[off];
+        float const wx    = outward_width(v.x), wy = outward_width(v.y);
+        uint32_t const jr = slab_lookup(v.y, y0, invh, ns);
+        uint32_t const R0 = ix.slab_start[slab0 + jr], R1 = ix.slab_start[slab0 + jr + 1];
+        unsigned par      = 0u;
+        bool on           = false;
+        for (uint32_t e0 = R0; e0 < R1; e0 += 32) {
+          int c = 0;
+          if (e0 + lane < R1) {
+            c = edge_by_bounds(ix.slab_e32[e0 + lane], v.x - wx, v.y - wy, v.x + wx, v.y + wy,
+                               inner);
+            if (c == 2) {
+              uint32_t const a = ix.slab_edges[e0 + lane] & kEntryVertex, b = ix.prev_vertex[a];
+              c = exact_edge<double>(px, py, ix.vx[a], ix.vy[a], ix.vx[b], ix.vy[b]);
+            }
+          }
+          par ^= __ballot_sync(kAll, c == 1);
+          on = __any_sync(kAll, c == 2) || on;
+        }
+        if (!on) {  // (on an edge: contradicts the premise, tested point by point)
+          bool const all      = (__popc(par) & 1u) != 0u;
+          uint64_t const vmax = npi - off < len ? npi - off : len;
+          for (uint32_t w = lane; w < nw; w += 32) {
+            uint64_t const b0 = static_cast<uint64_t>(w) * 32u;
+            uint32_t word     = 0u;
+            if (all && vmax > b0) word = vmax - b0 >= 32 ? kAll : (1u << (vmax - b0)) - 1u;
+            bits[wb + w] = word;
+          }
+          if (lane == 0) counts[k] = all ? static_cast<uint32_t>(vmax) : 0u;
+          continue;
+        }
+      }
+    }
+    uint32_t cnt = 0;
+    for (uint32_t c = 0; c < len; c += 32) {
+      uint64_t const pos = off + c + lane;
+      bool hit           = false;
+      if (c + lane < len && pos < npi) {
+        float2 const v = t[pos];
+        float const wx = outward_width(v.x), wy = outward_width(v.y);
+        float const xl = __fsub_rd(v.x, wx), xu = __fadd_ru(v.x, wx);
+        float const yl = __fsub_rd(v.y, wy), yu = __fadd_ru(v.y, wy);
+        if (walk || !lookup) {
+          double px, py;
+          src.load(pos, px, py);
+          hit = pip_exact<double>(px, py, ix, poly);
+        } else if (!(xl > box.z || xu < box.x || yl > box.w || yu < box.y)) {
+          double px = 0.0, py = 0.0;
+          bool have64 = false, on = false;
+          if (verts) {
+            src.load(pos, px, py);
+            have64 = true;
+            on     = sorted_has<double>(ix.vert_x, vb, ve, px);
+          }
+          uint32_t const s  = slab0 + slab_lookup(v.y, y0, invh, ns);
+          uint32_t const e1 = ix.slab_start[s + 1];
+          for (uint32_t e = ix.slab_start[s]; e < e1 && !on; ++e) {
+            int d = edge_by_bounds(ix.slab_e32[e], xl, yl, xu, yu, inner);
+            if (d == 2) {
+              if (!have64) {
+                src.load(pos, px, py);
+                have64 = true;
+              }
+              uint32_t const a = ix.slab_edges[e] & kEntryVertex, b = ix.prev_vertex[a];
+              d  = exact_edge<double>(px, py, ix.vx[a], ix.vy[a], ix.vx[b], ix.vy[b]);
+              on = d == 2;
+            }
+            if (d == 1) hit = !hit;
+          }
+          hit = hit && !on;
+        }
+      }
+      unsigned const w = __ballot_sync(kAll, hit);
+      if (lane == 0) bits[wb + (c >> 5)] = w;
+      cnt += __popc(w);
+    }
+    if (lane == 0) counts[k] = cnt;
+  }
+}
+
 // float inputs: the reference's test in float, one warp per pair.
 __global__ void __launch_bounds__(256)
   pip_pair_kernel_f32(uint32_t const* __restrict__ pair_poly,
@@ -683,7 +924,9 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
   Buffer<uint32_t> gstart, pgroup;
   Buffer<float2> u;
   Buffer<LeafFrame> frames;
-  if (filtered) {
+  Buffer<QuadBounds> quads;
+  bool const bounded = prebuilt ? prebuilt->edge_bounds() : use_bounds<T>(filtered, npi);
+  if (filtered || bounded) {
     gstart       = Buffer<uint32_t>(alloc, npairs + 1);
     pgroup       = Buffer<uint32_t>(alloc, npairs);
     uint32_t* gs = gstart.data();
@@ -698,7 +941,8 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
       },
       npairs, gs + npairs, alloc);
     u      = Buffer<float2>(alloc, npi);
-    frames = Buffer<LeafFrame>(alloc, npairs);
+    frames = Buffer<LeafFrame>(alloc, filtered ? npairs : 0);
+    quads  = Buffer<QuadBounds>(alloc, bounded ? npairs : 0);
   }
   // The leaf frames (bound by HBM) run on a second stream while the index
   // writes its slab entries: they start once everything enqueued above,
@@ -709,7 +953,7 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
   // (a prebuilt index, filled, may come with the call)
   std::unique_ptr<PolygonIndex<T>> own;
   if (!prebuilt)
-    own.reset(new PolygonIndex<T>(po, npo, ro, nro, vx, vy, nv, filtered, alloc, false, filtered));
+    own.reset(new PolygonIndex<T>(po, npo, ro, nro, vx, vy, nv, filtered, alloc, false, filtered, bounded));
   PolygonIndex<T>& index  = prebuilt ? *prebuilt : *own;
   cudaStream_t const side = filtered ? side_stream() : nullptr;
   StreamJoin join(s, side);
@@ -720,6 +964,14 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
       leaf_frame_kernel<<<leaf_frame_grid(npairs), blk, 0, side>>>(
         gstart.data(), gstart.data() + npairs, pair_quad, qlen, qoff, src, npi, index.grid(),
         u.data(), frames.data());
+      CSPT_CHECK_LAUNCH();
+    }
+  }
+  if constexpr (std::is_same<T, double>::value) {
+    if (bounded) {
+      quad_bounds_kernel<<<leaf_frame_grid(npairs), blk, 0, s>>>(
+        gstart.data(), gstart.data() + npairs, pair_quad, qlen, qoff, src, npi, u.data(),
+        quads.data());
       CSPT_CHECK_LAUNCH();
     }
   }
@@ -740,6 +992,11 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
           pair_poly + k0, pair_quad + k0, pgroup.data() + k0, n, qlen, qoff, src, npi, u.data(),
           frames.data(), index.view(), word_off.data() + k0, bits.data(), counts.data() + k0,
           refined.data(), refined.data() + 1, refined.data() + 2);
+      else if (bounded)
+        pip_bounds_kernel<<<pair_grid(pip_bounds_kernel, kPipBlock, n), kPipBlock, 0, s>>>(
+          pair_poly + k0, pair_quad + k0, pgroup.data() + k0, n, qlen, qoff, src, npi, u.data(),
+          quads.data(), index.view(), word_off.data() + k0, bits.data(), counts.data() + k0,
+          refined.data() + 1);
       else
         pip_pair_kernel<false>
           <<<pair_grid(pip_pair_kernel<false>, kPipBlock, n), kPipBlock, 0, s>>>(
@@ -1098,7 +1355,7 @@ void join_host(T const* hx, T const* hy, size_t n, double x_min, double x_max, d
     polygon_bounding_boxes(dpo.data(), npo, dro.data(), nro, dvx.data(), dvy.data(), nv, dtype,
                            0.0, bminx.data(), bminy.data(), bmaxx.data(), bmaxy.data(), palloc);
     index.reset(new PolygonIndex<T>(dpo.data(), npo, dro.data(), nro, dvx.data(), dvy.data(), nv,
-                                    filtered, palloc, false, false));
+                                    filtered, palloc, false, false, use_bounds<T>(filtered, n)));
   };
   uint32_t* pi_raw = nullptr;
   cspt_quadtree tree{nullptr, nullptr, nullptr, nullptr, nullptr, 0};

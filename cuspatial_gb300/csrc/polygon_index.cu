@@ -28,13 +28,19 @@ constexpr int kMaxSlabs = 4096;
 // set (build + evaluation): density 2 for the one-shot float32 index, whose
 // pair kernel classifies a quadrant's slab entries once (1: 12.90 ms,
 // 2: 12.51, 3: 12.71, 4: 13.29); 4 for the ordered index, whose per-point
-// windows gain from shorter slabs; 8 for the float64-only evaluation.
+// windows gain from shorter slabs; 8 for the float64-only evaluation; 1 for the
+// edge bounds, whose entries cost a comparison (2M points x 10k polygons, whole
+// call: 1: 1.449 ms, 2: 1.534, 4: 1.588).
 #ifndef CSPT_SLAB_DENSITY32
 #define CSPT_SLAB_DENSITY32 2.0
 #endif
 constexpr double kSlabDensityFloat32 = CSPT_SLAB_DENSITY32;
 constexpr double kSlabDensityOrdered = 4.0;
 constexpr double kSlabDensityFloat64 = 8.0;
+#ifndef CSPT_SLAB_DENSITY_BOUNDS
+#define CSPT_SLAB_DENSITY_BOUNDS 1.0
+#endif
+constexpr double kSlabDensityBounds = CSPT_SLAB_DENSITY_BOUNDS;
 __device__ inline uint32_t choose_slabs(uint32_t nv, double height, double sum_rise,
                                         double density)
 {
@@ -184,20 +190,6 @@ __device__ inline uint32_t edge_span(T ax, T ay, T bx, T by, float fa, float fb,
   uint32_t const j0 = !(l > 0.0f) ? 0u : (l >= top ? ns - 1 : min(static_cast<uint32_t>(l), ns - 1));
   uint32_t const j1 = !(h > 0.0f) ? 0u : (h >= top ? ns - 1 : min(static_cast<uint32_t>(h), ns - 1));
   return j0 | (j1 << 12) | (ex ? kSpanVertical : 0u);
-}
-
-// A double cut to float32 on the integer pipe (mantissa truncated; below
-// float32's normal range -> 0, beyond it or non-finite -> infinity), for the
-// slab-count heuristic only: any slab count gives a valid index.
-__device__ inline float truncated_f32(double v)
-{
-  unsigned long long const b = static_cast<unsigned long long>(__double_as_longlong(v));
-  uint32_t const sign        = static_cast<uint32_t>(b >> 32) & 0x80000000u;
-  int const e                = static_cast<int>((b >> 52) & 0x7FFull) - 1023 + 127;
-  if (e <= 0) return __uint_as_float(sign);
-  if (e >= 255) return __uint_as_float(sign | 0x7F800000u);
-  return __uint_as_float(sign | (static_cast<uint32_t>(e) << 23) |
-                         static_cast<uint32_t>((b >> 29) & 0x7FFFFFull));
 }
 
 // Order-preserving integer image of a non-NaN double (min/max on the
@@ -426,7 +418,7 @@ __global__ void __launch_bounds__(kIdxBlock)
                     T const* __restrict__ invh, uint32_t const* __restrict__ nslab,
                     uint32_t const* __restrict__ slab_base, uint32_t const* __restrict__ entry_base,
                     uint32_t const* __restrict__ vert_base, T const* __restrict__ grid,
-                    bool float32, T* anchor_x, T* anchor_y, long long* aix, long long* aiy,
+                    bool float32, bool bounds, T* anchor_x, T* anchor_y, long long* aix, long long* aiy,
                     float4* box32, float* invh32, float* maxoff, uint32_t const* __restrict__ prev,
                     uint32_t const* __restrict__ spans, float4* edge32, uint32_t* slab_start,
                     uint32_t* slab_edges, float4* slab_e32, T* vert_x, float* vert_x32,
@@ -463,6 +455,8 @@ __global__ void __launch_bounds__(kIdxBlock)
       box32[p]    = make_float4(static_cast<float>(pminx[p] - cx), static_cast<float>(ymin - cy),
                                 static_cast<float>(pmaxx[p] - cx), static_cast<float>(pmaxy[p] - cy));
       invh32[p]   = static_cast<float>(invh[p]);
+      if constexpr (std::is_same<T, double>::value)
+        if (bounds) box32[p] = outward_box(pminx[p], ymin, pmaxx[p], pmaxy[p]);
       vcur        = 0;
     }
     for (uint32_t j = threadIdx.x; j < ns; j += kIdxBlock) cur[j] = 0;
@@ -499,6 +493,8 @@ __global__ void __launch_bounds__(kIdxBlock)
                                            fmaxf(fabsf(ef.z), fabsf(ef.w))));
       }
       if (sp & kSpanSkip) continue;
+      if constexpr (std::is_same<T, double>::value)
+        if (bounds) ef = outward_box(vx[v], vy[v], vx[pv], vy[pv]);
       float const fa = yslab[v], fb = yslab[pv];
       float const flo = fminf(fa, fb), fhi = fmaxf(fa, fb);
       for (uint32_t j = span_j0(sp); j <= span_j1(sp); ++j) {
@@ -508,7 +504,7 @@ __global__ void __launch_bounds__(kIdxBlock)
         bool const crossing = flo < static_cast<float>(j) - 0.0625f &&
                               fhi > static_cast<float>(j) + 1.0625f;
         slab_edges[k]       = v | (crossing ? kEntryCrossing : 0u);
-        if (float32) slab_e32[k] = ef;
+        if (float32 || bounds) slab_e32[k] = ef;
       }
       if (sp & kSpanVertical) {
         uint32_t const k  = atomicAdd(&vcur, 1u);
@@ -732,7 +728,7 @@ struct PolygonIndex<T>::Sizing {
   uint32_t const *po, *ro;
   T const *vx, *vy;
   size_t np, nslabs_total, nentries, nvertical;
-  bool build_float32, order_slabs;
+  bool build_float32, order_slabs, edge_bounds;
   unsigned grd;
   Buffer<uint32_t> ebase, nvert, spans;
   Buffer<float> yslab;
@@ -742,9 +738,13 @@ struct PolygonIndex<T>::Sizing {
 template <typename T>
 PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro, size_t nro,
                               T const* vx, T const* vy, size_t nv, bool build_float32,
-                              Allocator const& alloc, bool order_slabs, bool defer_fill)
+                              Allocator const& alloc, bool order_slabs, bool defer_fill,
+                              bool edge_bounds)
 {
   (void)nro;
+  CSPT_EXPECTS(!edge_bounds || (std::is_same<T, double>::value && !build_float32),
+               "edge bounds belong to the float64 index");
+  edge_bounds_         = edge_bounds;
   cudaStream_t const s = alloc.stream();
   KernelTimer timer("polygon_index", s);
   size_t const np = npo > 0 ? npo - 1 : 0;
@@ -774,6 +774,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
   Buffer<float> yslab(alloc, nv);
 
   double const density = build_float32 ? (order_slabs ? kSlabDensityOrdered : kSlabDensityFloat32)
+                         : edge_bounds ? kSlabDensityBounds
                                        : kSlabDensityFloat64;
   unsigned const grd = static_cast<unsigned>(np < sm_grid(64u) ? (np ? np : 1) : sm_grid(64u));
   if (np > 0) {
@@ -829,7 +830,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
     nvertical    = tot[2];
   }
   sizing_.reset(new Sizing{po, ro, vx, vy, np, nslabs_total, nentries, nvertical, build_float32,
-                           order_slabs, grd, std::move(ebase), std::move(nvert), std::move(spans),
+                           order_slabs, edge_bounds, grd, std::move(ebase), std::move(nvert), std::move(spans),
                            std::move(yslab), &alloc});
   if (!defer_fill) fill();
 }
@@ -854,7 +855,7 @@ void PolygonIndex<T>::fill()
   unsigned const grd       = z->grd;
   slab_start_ = Buffer<uint32_t>(alloc, nslabs_total + 1);
   slab_edges_ = Buffer<uint32_t>(alloc, nentries);
-  if (build_float32) slab_e32_ = Buffer<float4>(alloc, nentries);
+  if (build_float32 || z->edge_bounds) slab_e32_ = Buffer<float4>(alloc, nentries);
   vert_x_ = Buffer<T>(alloc, nvertical);
   if (build_float32) vert_x32_ = Buffer<float>(alloc, nvertical);
   if (np == 0) CSPT_CUDA_TRY(cudaMemsetAsync(slab_start_.data(), 0, sizeof(uint32_t), s));
@@ -863,7 +864,7 @@ void PolygonIndex<T>::fill()
     index_fill_kernel<T><<<grd, kIdxBlock, 0, s>>>(
       po, ro, vx, vy, np, pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
       invh_.data(), nslab_.data(), slab_base_.data(), z->ebase.data(), vbeg_.data(), grid_.data(),
-      build_float32, ax_.data(), ay_.data(), aix_.data(), aiy_.data(), box32_.data(),
+      build_float32, z->edge_bounds, ax_.data(), ay_.data(), aix_.data(), aiy_.data(), box32_.data(),
       invh32_.data(), maxoff_.data(), prev_.data(), z->spans.data(), edge32_.data(),
       slab_start_.data(),
       slab_edges_.data(), slab_e32_.data(), vert_x_.data(), vert_x32_.data(), vxy32.data(),

@@ -51,6 +51,42 @@ constexpr int kSlabBins = 8;
 constexpr uint32_t kEntryCrossing = 1u << 31;
 constexpr uint32_t kEntryVertex   = kEntryCrossing - 1u;
 
+// A double cut to float32 on the integer pipe: mantissa truncated; below
+// float32's normal range -> 0, beyond it or non-finite -> infinity.  Within
+// 2^-23 |v| (1.2e-38 below the normal range) of v, toward zero.
+__device__ inline float truncated_f32(double v)
+{
+  unsigned long long const b = static_cast<unsigned long long>(__double_as_longlong(v));
+  uint32_t const sign        = static_cast<uint32_t>(b >> 32) & 0x80000000u;
+  int const e                = static_cast<int>((b >> 52) & 0x7FFull) - 1023 + 127;
+  if (e <= 0) return __uint_as_float(sign);
+  if (e >= 255) return __uint_as_float(sign | 0x7F800000u);
+  return __uint_as_float(sign | (static_cast<uint32_t>(e) << 23) |
+                         static_cast<uint32_t>((b >> 29) & 0x7FFFFFull));
+}
+// The width that a truncated value t is widened by on both sides: twice its
+// truncation error, so that the value itself lies inside by at least
+// 2^-23 |t| (not a number for an infinite t: its comparisons decide nothing).
+__device__ inline float outward_width(float t)
+{
+  return __fmaf_ru(fabsf(t), 2.384185791015625e-07f, 1.0e-37f);
+}
+// The box (xmin, ymin, xmax, ymax) of two points in float32, wider than them
+// by 2^-23 of the larger magnitude on each side, which is more than 2^-24 of
+// the difference of their coordinates; the whole plane when a coordinate is
+// beyond float32 or not finite.
+__device__ inline float4 outward_box(double ax, double ay, double bx, double by)
+{
+  float const x0 = truncated_f32(ax), x1 = truncated_f32(bx);
+  float const y0 = truncated_f32(ay), y1 = truncated_f32(by);
+  float const mx = fmaxf(fabsf(x0), fabsf(x1)), my = fmaxf(fabsf(y0), fabsf(y1));
+  float const wx = outward_width(mx), wy = outward_width(my);
+  if (!(wx < INFINITY && wy < INFINITY))
+    return make_float4(-INFINITY, -INFINITY, INFINITY, INFINITY);
+  return make_float4(__fsub_rd(fminf(x0, x1), wx), __fsub_rd(fminf(y0, y1), wy),
+                     __fadd_ru(fmaxf(x0, x1), wx), __fadd_ru(fmaxf(y0, y1), wy));
+}
+
 template <typename T>
 struct PolygonIndexView {
   // polygon topology (caller's arrays)
@@ -73,6 +109,7 @@ struct PolygonIndexView {
   T const* inv_slab_h;         // slabs per unit of y
   float const* max_offset;     // largest |float32 offset| over the polygon's vertices
   float4 const* box32;         // vertex box as float32 offsets from the anchor
+                               // (edge bounds: the vertex box itself, outward)
   uint32_t const* num_slabs;
   uint32_t const* slab_base;   // first slab of the polygon in slab_start
   uint8_t const* exact_only;   // 1: walk the reference loop, no index
@@ -84,6 +121,7 @@ struct PolygonIndexView {
   uint32_t const* slab_start;
   uint32_t const* slab_edges;  // vertex index of the edge's end point | kEntryCrossing
   float4 const* slab_e32;      // the entry's edge (ax, ay, bx, by) as float32 offsets
+                               // (edge bounds: its box, outward_box)
   // per vertex
   uint32_t const* prev_vertex;
   float4 const* edge32;        // (ax, ay, bx, by) offsets from the anchor
@@ -102,6 +140,8 @@ class PolygonIndex {
   // build the per-(slab, x-bin) windows.  It costs a pass over all slab
   // entries and pays off where the index is evaluated many times (batched
   // plans, resident polygon sets).
+  // edge_bounds (float64 index without float32 edges): slab entries carry
+  // their edge's box in float32, rounded outward (outward_box).
   // defer_fill: return once the per-polygon boxes, slab counts and the anchor
   // grid are enqueued (array sizes come from bounds on the host, so the call
   // does not wait for the device); fill() then writes the slab entries.  Work
@@ -110,7 +150,7 @@ class PolygonIndex {
   PolygonIndex(uint32_t const* poly_offsets, size_t num_poly_offsets,
                uint32_t const* ring_offsets, size_t num_ring_offsets, T const* vx, T const* vy,
                size_t num_vertices, bool build_float32, Allocator const& alloc,
-               bool order_slabs = false, bool defer_fill = false);
+               bool order_slabs = false, bool defer_fill = false, bool edge_bounds = false);
   ~PolygonIndex();
   PolygonIndex(PolygonIndex const&)            = delete;
   PolygonIndex& operator=(PolygonIndex const&) = delete;
@@ -118,10 +158,12 @@ class PolygonIndex {
   // device scalar: the anchor grid step (valid before fill())
   T const* grid() const { return grid_.data(); }
   PolygonIndexView<T> view() const { return v_; }
+  bool edge_bounds() const { return edge_bounds_; }
 
  private:
   struct Sizing;  // state carried from the sizing pass to fill()
   std::unique_ptr<Sizing> sizing_;
+  bool edge_bounds_ = false;
   Buffer<T> pminx_, pminy_, pmaxx_, pmaxy_, ax_, ay_, invh_, vert_x_, grid_;
   Buffer<float> maxoff_, vert_x32_, invh32_;
   Buffer<long long> aix_, aiy_;
