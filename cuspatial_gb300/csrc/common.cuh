@@ -489,26 +489,45 @@ __device__ inline bool outside_closed(double v, double lo, double hi)
 __device__ inline bool outside_closed(float v, float lo, float hi) { return v < lo || v > hi; }
 
 // static_cast<uint16_t>(t / s) for t >= 0 (the reference's cell index,
-// phase_1.cuh:73-85) without a float64 division in the common case.  With
+// phase_1.cuh:73-85) without a float64 division in the common cases.  With
 // r = fl(1/s) (host-rounded) and q0 = fl(t * r):
 //   |q0 - t/s| <= (t/s)(2^-52 + 2^-106)   and   |fl(t/s) - t/s| <= 2^-53 t/s,
 // so for t/s < 2^16 the two differ by less than 2^-35.  When q0 lies more
 // than 2^-30 away from every integer, q0 and fl(t/s) have the same integer
-// part; the fraction test reads q0's bits.  Every other case (near an
-// integer, below 2^-30, 2^16 and above, non-finite) divides.
+// part; the fraction test reads q0's bits.  Below 2^-30 the cell is 0.  Near an
+// integer k (points on cell boundaries and clamped to the box are: with a few
+// percent of them nearly every warp took the division, 50M keys in 1478 us),
+// fl(t/s) >= k exactly when t/s >= k - h, h half the spacing below k (the tie
+// goes to k, whose last bit is zero), i.e. when t - k s >= -s h: one fma, whose
+// rounding keeps the order against the representable -s h unless they come out
+// equal.  That, 2^16 and above and non-finite values divide.
 __device__ inline uint16_t cell_of_quotient(double t, double s, double r)
 {
-  double const q0          = t * r;
+  double const q0            = t * r;
   unsigned long long const b = static_cast<unsigned long long>(__double_as_longlong(q0));
-  int const e              = static_cast<int>((b >> 52) & 0x7FFull) - 1023;
-  if (e >= 0 && e < 16 && !(b >> 63)) {
+  if (b < 0x3FEFFFFFFF800000ull) {  // 0 <= q0 < 1 - 2^-30 (positive doubles order as integers)
+    return 0;
+  }
+  if (b < 0x40F0000000000000ull) {  // below 2^16
+    int const e                   = static_cast<int>(b >> 52) - 1023;  // >= -1
     unsigned long long const m    = (b & ((1ull << 52) - 1ull)) | (1ull << 52);
     int const sh                  = 52 - e;  // fraction bits, >= 37
     unsigned long long const frac = m & ((1ull << sh) - 1ull);
     unsigned long long const mg   = 1ull << (sh - 30);
     if (frac > mg && frac < (1ull << sh) - mg) return static_cast<uint16_t>(m >> sh);
-  } else if (b > 0x3E10000000000000ull && b < 0x3FEFFFFFFF800000ull) {
-    return 0;  // 2^-30 < q0 < 1 - 2^-30 (positive doubles order as integers)
+    uint32_t const k = static_cast<uint32_t>((m + (1ull << (sh - 1))) >> sh);
+    // k >= 1; s at or above 2^-900, so that nothing below underflows
+    if (k < 65536u &&
+        static_cast<unsigned long long>(__double_as_longlong(s)) >= 0x07B0000000000000ull) {
+      double const kd = __uint2double_rn(k);
+      // 2^(E-53), or 2^(E-54) below a power of two, with E k's exponent
+      int const E    = 31 - __clz(k);
+      int const hexp = (k & (k - 1u)) ? E - 53 : E - 54;
+      double const h = __longlong_as_double(static_cast<long long>(hexp + 1023) << 52);
+      double const d = __fma_rn(-kd, s, t), limit = -(s * h);
+      if (d > limit) return static_cast<uint16_t>(k);
+      if (d < limit) return static_cast<uint16_t>(k - 1u);
+    }
   }
   return static_cast<uint16_t>(t / s);
 }

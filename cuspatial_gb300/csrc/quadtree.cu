@@ -137,32 +137,30 @@ __device__ inline uint8_t node_levels(uint32_t const* __restrict__ skeys, size_t
     l0 = d - 1 - (31 - __clz(diff)) / 2;
     l0 = l0 < 0 ? 0 : l0;
   }
-  int const c = i + m < n ? shared_level(key, skeys[i + m], d) : -1;
-  int K       = l0;
-  if (c >= l0 - 1 && c >= 0) {
-    K = c + 1 < d - 1 ? c + 1 : d - 1;
-  } else if (l0 > 0) {
-    int const sh     = 2 * (d - l0);  // >= 2: the parent's prefix
-    uint32_t const P = key >> sh;
-    if (!(i >= m && (skeys[i - m] >> sh) == P)) {
-      // at most ha - 1 points of the parent before i and hb from i on
-      size_t const ha = (m + 1) / 2, hb = m + 1 - ha;
-      bool const before = i >= ha && (skeys[i - ha] >> sh) == P;
-      bool const after  = i + hb < n && (skeys[i + hb] >> sh) == P;
-      if (!before && !after) return kNoNodes;
-      // the parent's first position, in (i - m, i - 1] (i - 1 belongs to it)
-      size_t lo = i >= m ? i - m + 1 : 0, hi = i - 1;
-      while (lo < hi) {
-        size_t const mid = (lo + hi) >> 1;
-        if ((skeys[mid] >> sh) == P)
-          hi = mid;
-        else
-          lo = mid + 1;
-      }
-      if (!(lo + m < n && (skeys[lo + m] >> sh) == P)) return kNoNodes;
-    }
+  int const sh     = 2 * (d - l0);  // the parent's prefix (l0 > 0: 2 <= sh < 32)
+  uint32_t const P = l0 > 0 ? key >> sh : 0u;
+  if (l0 > 0) {
+    // first the common case, a small parent: at most ha - 1 of its points lie
+    // before i and hb from i on
+    size_t const ha = (m + 1) / 2, hb = m + 1 - ha;
+    if (!(i >= ha && (skeys[i - ha] >> sh) == P) && !(i + hb < n && (skeys[i + hb] >> sh) == P))
+      return kNoNodes;
   }
-  return static_cast<uint8_t>(l0 | (K << 4));
+  int const c = i + m < n ? shared_level(key, skeys[i + m], d) : -1;
+  if (c >= 0 && c >= l0 - 1) return static_cast<uint8_t>(l0 | (min(c + 1, d - 1) << 4));
+  if (l0 > 0 && !(i >= m && (skeys[i - m] >> sh) == P)) {
+    // the parent's first position, in (i - m, i - 1] (i - 1 belongs to it)
+    size_t lo = i >= m ? i - m + 1 : 0, hi = i - 1;
+    while (lo < hi) {
+      size_t const mid = (lo + hi) >> 1;
+      if ((skeys[mid] >> sh) == P)
+        hi = mid;
+      else
+        lo = mid + 1;
+    }
+    if (!(lo + m < n && (skeys[lo + m] >> sh) == P)) return kNoNodes;
+  }
+  return static_cast<uint8_t>(l0 | (l0 << 4));
 }
 
 // Per position the levels of its kept nodes, per tile the nodes of each level
@@ -201,6 +199,7 @@ __global__ void __launch_bounds__(kNodeBlock)
 {
   constexpr unsigned kAll = 0xFFFFFFFFu;
   __shared__ uint32_t wcnt[kNodeBlock / 32][kNodeLevels];
+  __shared__ uint32_t wfirst[kNodeBlock / 32];  // first position with nodes, in the tile
   int const lane    = threadIdx.x & 31;
   int const warp    = threadIdx.x >> 5;
   unsigned const lt = (1u << lane) - 1u;
@@ -212,10 +211,17 @@ __global__ void __launch_bounds__(kNodeBlock)
     size_t const i = base + r * 32 + lane;
     code[r]        = i < n ? codes[i] : kNoNodes;
   }
-  uint32_t run = 0;  // lane l: nodes of level l in this warp's positions
+  uint32_t run   = 0;  // lane l: nodes of level l in this warp's positions
+  uint32_t first = kNodeTile;
+  unsigned starts[kNodeRounds];
+#pragma unroll
+  for (int r = kNodeRounds - 1; r >= 0; --r) {
+    starts[r] = __ballot_sync(kAll, code[r] != kNoNodes);
+    if (starts[r]) first = warp * (32 * kNodeRounds) + r * 32 + __ffs(starts[r]) - 1;
+  }
 #pragma unroll
   for (int r = 0; r < kNodeRounds; ++r) {
-    if (!__any_sync(kAll, code[r] != kNoNodes)) continue;
+    if (!starts[r]) continue;
     int const l0 = code[r] & 15, K = code[r] >> 4;
     for (int l = 0; l < d; ++l) {
       unsigned const b = __ballot_sync(kAll, code[r] != kNoNodes && l0 <= l && l <= K);
@@ -223,7 +229,12 @@ __global__ void __launch_bounds__(kNodeBlock)
     }
   }
   if (lane < kNodeLevels) wcnt[warp][lane] = run;
+  if (lane == 0) wfirst[warp] = first;
   __syncthreads();
+  // the next position with nodes after this warp's, if it lies in the tile
+  uint32_t after = kNodeTile;
+  for (int w = kNodeBlock / 32 - 1; w > warp; --w)
+    if (wfirst[w] < kNodeTile) after = wfirst[w];
   run = 0;
   if (lane < d) {
     run = rows[static_cast<size_t>(lane) * gridDim.x + blockIdx.x];
@@ -231,7 +242,7 @@ __global__ void __launch_bounds__(kNodeBlock)
   }
 #pragma unroll
   for (int r = 0; r < kNodeRounds; ++r) {
-    if (!__any_sync(kAll, code[r] != kNoNodes)) continue;
+    if (!starts[r]) continue;
     size_t const i     = base + r * 32 + lane;
     bool const any     = code[r] != kNoNodes;
     int const l0       = code[r] & 15, K = code[r] >> 4;
@@ -251,23 +262,36 @@ __global__ void __launch_bounds__(kNodeBlock)
       parent = o;
     }
     if (any) {
-      // the leaf (i, K): its points end at the first key beyond its prefix
-      int const sh     = 2 * (d - 1 - K);
-      uint32_t const P = key >> sh;
-      size_t lo = i + 1, hi = n;  // the end lies in [lo, hi]
-      for (size_t step = max_size; i + step < n; step *= 2) {
-        if ((skeys[i + step] >> sh) != P) {
-          hi = i + step;
-          break;
-        }
-        lo = i + step + 1;
+      // The leaf (i, K) ends where the next kept node starts: no kept node
+      // starts inside a leaf, and the node after it is a sibling of it or of
+      // one of its ancestors, which their parent's size keeps.  The tile's
+      // last leaf looks for the first key beyond its prefix.
+      uint32_t next = after;
+#pragma unroll
+      for (int t = kNodeRounds - 1; t >= r; --t) {
+        unsigned const later = t == r ? starts[t] & ~lt & ~(1u << lane) : starts[t];
+        if (later) next = warp * (32 * kNodeRounds) + t * 32 + __ffs(later) - 1;
       }
-      while (lo < hi) {
-        size_t const mid = (lo + hi) >> 1;
-        if ((skeys[mid] >> sh) == P)
-          lo = mid + 1;
-        else
-          hi = mid;
+      size_t lo = static_cast<size_t>(blockIdx.x) * kNodeTile + next;  // the end
+      if (next == kNodeTile) {
+        int const sh     = 2 * (d - 1 - K);
+        uint32_t const P = key >> sh;
+        size_t hi        = n;
+        lo               = i + 1;  // the end lies in [lo, hi]
+        for (size_t step = max_size; i + step < n; step *= 2) {
+          if ((skeys[i + step] >> sh) != P) {
+            hi = i + step;
+            break;
+          }
+          lo = i + step + 1;
+        }
+        while (lo < hi) {
+          size_t const mid = (lo + hi) >> 1;
+          if ((skeys[mid] >> sh) == P)
+            lo = mid + 1;
+          else
+            hi = mid;
+        }
       }
       ooffset[parent] = static_cast<uint32_t>(i);
       olength[parent] = static_cast<uint32_t>(lo - i);
