@@ -55,14 +55,6 @@ constexpr uint32_t kFastSlabs = 31;
 // the edge-free quadrant test streams at most this many slab entries
 constexpr uint32_t kFreeScan = 1024;
 
-// The float32 slab of offset y (the lookup of filtered_test).
-__device__ inline uint32_t slab_lookup(float qy, float y0, float invh, uint32_t ns)
-{
-  float const fs = (qy - y0) * invh;
-  uint32_t sj    = 0;
-  if (fs > 0.0f) sj = fs >= static_cast<float>(ns) ? ns - 1 : static_cast<uint32_t>(fs);
-  return sj >= ns ? ns - 1 : sj;
-}
 // Exact joins on float64 points from this many points on compare bounds first
 // (pip_bounds_kernel): at 1M points x 256 polygons the call takes 858 us with
 // the bounds, 940 without; at 1k points x 17 the bounds' launches cost what they
@@ -643,15 +635,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// One edge against one point by bounds: 0 neither toggles nor holds the point,
-// 1 toggles, 2 undecided.  `inner` covers the widening of the edge's y bounds.
-__device__ inline int edge_by_bounds(float4 const& e, float xl, float yl, float xu, float yu,
-                                     float inner)
-{
-  if (xl > e.z || yl > e.w || yu < e.y) return 0;
-  return xu < e.x && yl > e.y + inner && yu < e.w - inner ? 1 : 2;
-}
-
 __global__ void __launch_bounds__(kPipBlock)
   pip_bounds_kernel(uint32_t const* __restrict__ pair_poly, uint32_t const* __restrict__ pair_quad,
                     uint32_t const* __restrict__ pair_group, size_t npairs,
@@ -663,6 +646,7 @@ __global__ void __launch_bounds__(kPipBlock)
 {
   constexpr unsigned kAll = 0xFFFFFFFFu;
   int const lane          = threadIdx.x & 31;
+  uint32_t nref           = 0;  // (not reported: the exact method refines nothing)
   for (;;) {
     unsigned long long kk = 0;
     if (lane == 0) kk = atomicAdd(next_pair, 1ull);
@@ -768,29 +752,9 @@ __global__ void __launch_bounds__(kPipBlock)
           src.load(pos, px, py);
           hit = pip_exact<double>(px, py, ix, poly);
         } else if (!(xl > box.z || xu < box.x || yl > box.w || yu < box.y)) {
-          double px = 0.0, py = 0.0;
-          bool have64 = false, on = false;
-          if (verts) {
-            src.load(pos, px, py);
-            have64 = true;
-            on     = sorted_has<double>(ix.vert_x, vb, ve, px);
-          }
-          uint32_t const s  = slab0 + slab_lookup(v.y, y0, invh, ns);
-          uint32_t const e1 = ix.slab_start[s + 1];
-          for (uint32_t e = ix.slab_start[s]; e < e1 && !on; ++e) {
-            int d = edge_by_bounds(ix.slab_e32[e], xl, yl, xu, yu, inner);
-            if (d == 2) {
-              if (!have64) {
-                src.load(pos, px, py);
-                have64 = true;
-              }
-              uint32_t const a = ix.slab_edges[e] & kEntryVertex, b = ix.prev_vertex[a];
-              d  = exact_edge<double>(px, py, ix.vx[a], ix.vy[a], ix.vx[b], ix.vy[b]);
-              on = d == 2;
-            }
-            if (d == 1) hit = !hit;
-          }
-          hit = hit && !on;
+          hit = bounds_test(ix, xl, yl, xu, yu, inner, slab0 + slab_lookup(v.y, y0, invh, ns),
+                            verts ? vb : ve, ve,
+                            [&](double& px, double& py) { src.load(pos, px, py); }, nref);
         }
       }
       unsigned const w = __ballot_sync(kAll, hit);

@@ -273,5 +273,56 @@ __device__ __forceinline__ bool filtered_test(PolygonIndexView<double> const& ix
   return r == 1;
 }
 
+// The float32 slab of offset y (the lookup of filtered_test).
+__device__ inline uint32_t slab_lookup(float qy, float y0, float invh, uint32_t ns)
+{
+  float const fs = (qy - y0) * invh;
+  uint32_t sj    = 0;
+  if (fs > 0.0f) sj = fs >= static_cast<float>(ns) ? ns - 1 : static_cast<uint32_t>(fs);
+  return sj >= ns ? ns - 1 : sj;
+}
+// One edge against one point by bounds: 0 neither toggles nor holds the point,
+// 1 toggles, 2 undecided.  `inner` covers the widening of the edge's y bounds.
+__device__ inline int edge_by_bounds(float4 const& e, float xl, float yl, float xu, float yu,
+                                     float inner)
+{
+  if (xl > e.z || yl > e.w || yu < e.y) return 0;
+  return xu < e.x && yl > e.y + inner && yu < e.w - inner ? 1 : 2;
+}
+
+// A point known by its bounds against the edges of slab s (their outward boxes,
+// edge_by_bounds; what those leave undecided takes the reference's float64
+// expression, counted in nref) and the exactly vertical edges [vb, ve).
+template <class Load>
+__device__ __forceinline__ bool bounds_test(PolygonIndexView<double> const& ix, float xl, float yl,
+                                            float xu, float yu, float inner, uint32_t s,
+                                            uint32_t vb, uint32_t ve, Load const& load,
+                                            uint32_t& nref)
+{
+  double px = 0.0, py = 0.0;
+  bool have64 = false, hit = false;
+  if (vb < ve) {
+    load(px, py);
+    have64 = true;
+    if (sorted_has<double>(ix.vert_x, vb, ve, px)) return false;
+  }
+  uint32_t const e1 = ix.slab_start[s + 1];
+  for (uint32_t e = ix.slab_start[s]; e < e1; ++e) {
+    int d = edge_by_bounds(ix.slab_e32[e], xl, yl, xu, yu, inner);
+    if (d == 2) {
+      ++nref;
+      if (!have64) {
+        load(px, py);
+        have64 = true;
+      }
+      uint32_t const a = ix.slab_edges[e] & kEntryVertex, b = ix.prev_vertex[a];
+      d = exact_edge<double>(px, py, ix.vx[a], ix.vy[a], ix.vx[b], ix.vy[b]);
+      if (d == 2) return false;
+    }
+    if (d == 1) hit = !hit;
+  }
+  return hit;
+}
+
 }  // namespace
 }  // namespace cspt

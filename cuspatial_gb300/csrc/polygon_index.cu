@@ -156,7 +156,10 @@ __device__ inline uint32_t span_j1(uint32_t s) { return (s >> 12) & 0xFFFu; }
 // coordinates the reference's float_equal(b - a, 0) holds exactly when
 // a == b, except where both coordinates lie below 2^-1019, where distinct
 // neighbours can be within 4 ULP of each other; such edges are flagged
-// (kSpanTiny) and their polygon is walked with the reference loop.
+// (kSpanTiny) and their polygon is walked with the reference loop.  So are,
+// in float64, polygons with an edge between different y both below 2^-800: the
+// products of a smaller rise can underflow, where deciding an edge by its
+// bounds and the reference's comparison could part.
 template <typename T>
 __device__ inline bool same_value(T a, T b)
 {
@@ -175,6 +178,15 @@ __device__ inline bool below_tiny(double a)
   return ((static_cast<unsigned long long>(__double_as_longlong(a)) >> 52) & 0x7FFull) <= 3ull;
 }
 
+__device__ inline bool vanishing_rise(float, float) { return false; }
+__device__ inline bool vanishing_rise(double ay, double by)
+{
+  auto const e = [](double a) {
+    return static_cast<int>((static_cast<unsigned long long>(__double_as_longlong(a)) >> 52) & 0x7FFull);
+  };
+  return e(ay) < 223 && e(by) < 223;
+}
+
 template <typename T>
 __device__ inline uint32_t edge_span(T ax, T ay, T bx, T by, float fa, float fb, uint32_t ns)
 {
@@ -189,7 +201,8 @@ __device__ inline uint32_t edge_span(T ax, T ay, T bx, T by, float fa, float fb,
   float const top = static_cast<float>(ns);
   uint32_t const j0 = !(l > 0.0f) ? 0u : (l >= top ? ns - 1 : min(static_cast<uint32_t>(l), ns - 1));
   uint32_t const j1 = !(h > 0.0f) ? 0u : (h >= top ? ns - 1 : min(static_cast<uint32_t>(h), ns - 1));
-  return j0 | (j1 << 12) | (ex ? kSpanVertical : 0u);
+  uint32_t const tiny = !ey && vanishing_rise(ay, by) ? kSpanTiny : 0u;
+  return j0 | (j1 << 12) | (ex ? kSpanVertical : 0u) | tiny;
 }
 
 // Order-preserving integer image of a non-NaN double (min/max on the
