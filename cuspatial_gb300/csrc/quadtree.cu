@@ -19,6 +19,7 @@
 #include "common.cuh"
 #include "radix_sort.cuh"
 #include "scan.cuh"
+#include "tree_nodes.cuh"
 
 namespace cspt {
 namespace {
@@ -81,239 +82,6 @@ __global__ void bottom_count_kernel(uint32_t const* __restrict__ starts, size_t 
        k += static_cast<size_t>(gridDim.x) * blockDim.x) {
     size_t const e = (k + 1 < nl) ? starts[k + 1] : n;
     count[k]       = static_cast<uint32_t>(e - starts[k]);
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Nodes of all levels in one pass over the sorted keys.
-//
-// A sorted position i that starts a node at level l0 (its start level) also
-// starts one at every finer level, and a level-l node is kept iff its parent
-// holds more than max_size points; counts shrink with the level, so the kept
-// nodes starting at i are the levels l0..K of one interval.  Both ends follow
-// from a few keys around i:
-//   * the level-l node starting at i (l >= l0) holds more than m points iff
-//     key[i + m] shares its level-l prefix, i.e. iff l <= c with c read off
-//     the highest differing bit of key[i] ^ key[i + m];
-//   * the parent of (i, l0), l0 > 0, starts before i; it holds more than m
-//     points if key[i + m] shares its prefix (c >= l0 - 1) or key[i - m] does,
-//     holds at most m if neither of two keys m + 1 apart around i does, and
-//     otherwise its start is searched in the m positions before i.
-// So K = min(d - 1, c + 1) where the deeper levels are kept, else l0, and a
-// node (i, l) is internal iff l < K.  Nodes are output level by level in key
-// order: counting them per (level, tile of positions) and scanning the counts
-// level-major gives every node its output row, and the first child of an
-// internal node (i, l) is node (i, l + 1), which is also the reference's
-// child offset (level_1_size plus the scan of child counts).
-//
-// Bound: the key stream (4 bytes a position, the window reads hit L1) and, on
-// small inputs, launches; this replaces a scan, a count, a scan and a
-// compaction per level (61 launches at depth 5, 171 at depth 15).
-// ---------------------------------------------------------------------------
-constexpr int kNodeBlock     = 256;
-constexpr int kNodeRounds    = 8;  // rounds of 32 positions per warp
-constexpr int kNodeTile      = kNodeBlock * kNodeRounds;
-constexpr int kNodeLevels    = 16;
-constexpr uint8_t kNoNodes   = 0xFF;  // no kept node starts here (l0 and K are below 15)
-
-// the deepest level at which two keys share their node, -1 if none
-__device__ inline int shared_level(uint32_t a, uint32_t b, int d)
-{
-  uint32_t const diff = a ^ b;
-  if (diff == 0) return d - 1;
-  int const c = d - 2 - (31 - __clz(diff)) / 2;
-  return c < 0 ? -1 : c;
-}
-
-// l0 | K << 4 of position i, kNoNodes when no kept node starts there
-__device__ inline uint8_t node_levels(uint32_t const* __restrict__ skeys, size_t n, size_t i, int d,
-                                      size_t m)
-{
-  uint32_t const key = skeys[i];
-  int l0             = 0;
-  if (i > 0) {
-    uint32_t const diff = key ^ skeys[i - 1];
-    if (diff == 0) return kNoNodes;
-    l0 = d - 1 - (31 - __clz(diff)) / 2;
-    l0 = l0 < 0 ? 0 : l0;
-  }
-  int const sh     = 2 * (d - l0);  // the parent's prefix (l0 > 0: 2 <= sh < 32)
-  uint32_t const P = l0 > 0 ? key >> sh : 0u;
-  if (l0 > 0) {
-    // first the common case, a small parent: at most ha - 1 of its points lie
-    // before i and hb from i on
-    size_t const ha = (m + 1) / 2, hb = m + 1 - ha;
-    if (!(i >= ha && (skeys[i - ha] >> sh) == P) && !(i + hb < n && (skeys[i + hb] >> sh) == P))
-      return kNoNodes;
-  }
-  int const c = i + m < n ? shared_level(key, skeys[i + m], d) : -1;
-  if (c >= 0 && c >= l0 - 1) return static_cast<uint8_t>(l0 | (min(c + 1, d - 1) << 4));
-  if (l0 > 0 && !(i >= m && (skeys[i - m] >> sh) == P)) {
-    // the parent's first position, in (i - m, i - 1] (i - 1 belongs to it)
-    size_t lo = i >= m ? i - m + 1 : 0, hi = i - 1;
-    while (lo < hi) {
-      size_t const mid = (lo + hi) >> 1;
-      if ((skeys[mid] >> sh) == P)
-        hi = mid;
-      else
-        lo = mid + 1;
-    }
-    if (!(lo + m < n && (skeys[lo + m] >> sh) == P)) return kNoNodes;
-  }
-  return static_cast<uint8_t>(l0 | (l0 << 4));
-}
-
-// Per position the levels of its kept nodes, per tile the nodes of each level
-// (counts[level * tiles + tile]).
-__global__ void __launch_bounds__(kNodeBlock)
-  node_count_kernel(uint32_t const* __restrict__ skeys, size_t n, int d, size_t max_size,
-                    uint8_t* __restrict__ codes, uint32_t* __restrict__ counts)
-{
-  __shared__ uint32_t cnt[kNodeLevels];
-  if (threadIdx.x < kNodeLevels) cnt[threadIdx.x] = 0;
-  __syncthreads();
-  size_t const base = static_cast<size_t>(blockIdx.x) * kNodeTile;
-#pragma unroll 2
-  for (int r = 0; r < kNodeRounds; ++r) {
-    size_t const i = base + static_cast<size_t>(r) * kNodeBlock + threadIdx.x;
-    if (i >= n) break;
-    uint8_t const code = node_levels(skeys, n, i, d, max_size);
-    codes[i]           = code;
-    if (code != kNoNodes)
-      for (int l = code & 15; l <= (code >> 4); ++l) atomicAdd(&cnt[l], 1u);
-  }
-  __syncthreads();
-  if (threadIdx.x < d) counts[static_cast<size_t>(threadIdx.x) * gridDim.x + blockIdx.x] =
-    cnt[threadIdx.x];
-}
-
-// Writes the kept nodes of a tile at the rows that the scanned counts give.
-// Warp w owns 256 consecutive positions; lane l keeps the running row of
-// level l.  The child counts of internal nodes follow in child_count_kernel.
-__global__ void __launch_bounds__(kNodeBlock)
-  node_write_kernel(uint32_t const* __restrict__ skeys, size_t n, int d, size_t max_size,
-                    uint8_t const* __restrict__ codes, uint32_t const* __restrict__ rows,
-                    uint32_t* __restrict__ okey, uint8_t* __restrict__ olevel,
-                    uint8_t* __restrict__ ointernal, uint32_t* __restrict__ olength,
-                    uint32_t* __restrict__ ooffset)
-{
-  constexpr unsigned kAll = 0xFFFFFFFFu;
-  __shared__ uint32_t wcnt[kNodeBlock / 32][kNodeLevels];
-  __shared__ uint32_t wfirst[kNodeBlock / 32];  // first position with nodes, in the tile
-  int const lane    = threadIdx.x & 31;
-  int const warp    = threadIdx.x >> 5;
-  unsigned const lt = (1u << lane) - 1u;
-  size_t const base =
-    static_cast<size_t>(blockIdx.x) * kNodeTile + static_cast<size_t>(warp) * (32 * kNodeRounds);
-  uint8_t code[kNodeRounds];
-#pragma unroll
-  for (int r = 0; r < kNodeRounds; ++r) {
-    size_t const i = base + r * 32 + lane;
-    code[r]        = i < n ? codes[i] : kNoNodes;
-  }
-  uint32_t run   = 0;  // lane l: nodes of level l in this warp's positions
-  uint32_t first = kNodeTile;
-  unsigned starts[kNodeRounds];
-#pragma unroll
-  for (int r = kNodeRounds - 1; r >= 0; --r) {
-    starts[r] = __ballot_sync(kAll, code[r] != kNoNodes);
-    if (starts[r]) first = warp * (32 * kNodeRounds) + r * 32 + __ffs(starts[r]) - 1;
-  }
-#pragma unroll
-  for (int r = 0; r < kNodeRounds; ++r) {
-    if (!starts[r]) continue;
-    int const l0 = code[r] & 15, K = code[r] >> 4;
-    for (int l = 0; l < d; ++l) {
-      unsigned const b = __ballot_sync(kAll, code[r] != kNoNodes && l0 <= l && l <= K);
-      if (lane == l) run += __popc(b);
-    }
-  }
-  if (lane < kNodeLevels) wcnt[warp][lane] = run;
-  if (lane == 0) wfirst[warp] = first;
-  __syncthreads();
-  // the next position with nodes after this warp's, if it lies in the tile
-  uint32_t after = kNodeTile;
-  for (int w = kNodeBlock / 32 - 1; w > warp; --w)
-    if (wfirst[w] < kNodeTile) after = wfirst[w];
-  run = 0;
-  if (lane < d) {
-    run = rows[static_cast<size_t>(lane) * gridDim.x + blockIdx.x];
-    for (int w = 0; w < warp; ++w) run += wcnt[w][lane];
-  }
-#pragma unroll
-  for (int r = 0; r < kNodeRounds; ++r) {
-    if (!starts[r]) continue;
-    size_t const i     = base + r * 32 + lane;
-    bool const any     = code[r] != kNoNodes;
-    int const l0       = code[r] & 15, K = code[r] >> 4;
-    uint32_t const key = any ? skeys[i] : 0u;
-    uint32_t parent    = 0;  // row of (i, l - 1)
-    for (int l = 0; l < d; ++l) {
-      bool const mine  = any && l0 <= l && l <= K;
-      unsigned const b = __ballot_sync(kAll, mine);
-      if (b == 0u) continue;
-      uint32_t const o = __shfl_sync(kAll, run, l) + __popc(b & lt);
-      if (lane == l) run += __popc(b);
-      if (!mine) continue;
-      okey[o]      = key >> (2 * (d - 1 - l));
-      olevel[o]    = static_cast<uint8_t>(l);
-      ointernal[o] = l < K ? 1 : 0;
-      if (l > l0) ooffset[parent] = o;
-      parent = o;
-    }
-    if (any) {
-      // The leaf (i, K) ends where the next kept node starts: no kept node
-      // starts inside a leaf, and the node after it is a sibling of it or of
-      // one of its ancestors, which their parent's size keeps.  The tile's
-      // last leaf looks for the first key beyond its prefix.
-      uint32_t next = after;
-#pragma unroll
-      for (int t = kNodeRounds - 1; t >= r; --t) {
-        unsigned const later = t == r ? starts[t] & ~lt & ~(1u << lane) : starts[t];
-        if (later) next = warp * (32 * kNodeRounds) + t * 32 + __ffs(later) - 1;
-      }
-      size_t lo = static_cast<size_t>(blockIdx.x) * kNodeTile + next;  // the end
-      if (next == kNodeTile) {
-        int const sh     = 2 * (d - 1 - K);
-        uint32_t const P = key >> sh;
-        size_t hi        = n;
-        lo               = i + 1;  // the end lies in [lo, hi]
-        for (size_t step = max_size; i + step < n; step *= 2) {
-          if ((skeys[i + step] >> sh) != P) {
-            hi = i + step;
-            break;
-          }
-          lo = i + step + 1;
-        }
-        while (lo < hi) {
-          size_t const mid = (lo + hi) >> 1;
-          if ((skeys[mid] >> sh) == P)
-            lo = mid + 1;
-          else
-            hi = mid;
-        }
-      }
-      ooffset[parent] = static_cast<uint32_t>(i);
-      olength[parent] = static_cast<uint32_t>(lo - i);
-    }
-  }
-}
-
-// Children of an internal node: the rows from its first child on whose key
-// extends the node's (at most four, all of the next level).
-__global__ void child_count_kernel(uint32_t const* __restrict__ key,
-                                   uint8_t const* __restrict__ level,
-                                   uint8_t const* __restrict__ internal,
-                                   uint32_t const* __restrict__ offset, size_t q,
-                                   uint32_t* __restrict__ length)
-{
-  for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < q;
-       k += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    if (!internal[k]) continue;
-    size_t const c0 = offset[k];
-    uint32_t c      = 1;
-    while (c < 4 && c0 + c < q && level[c0 + c] == level[c0] && (key[c0 + c] >> 2) == key[k]) ++c;
-    length[k] = c;
   }
 }
 
@@ -526,25 +294,24 @@ void build(T const* x, T const* y, size_t n, double x1d, double x2d, double y1d,
 
   // every level's nodes from one pass (node_levels); the host waits once, for
   // the number of nodes
-  unsigned const tiles = static_cast<unsigned>((n + kNodeTile - 1) / kNodeTile);
-  size_t const cells   = static_cast<size_t>(tiles) * d;
+  OneTreeTiles const tiles{n, static_cast<unsigned>((n + kNodeTile - 1) / kNodeTile), d, max_size};
+  size_t const cells = static_cast<size_t>(tiles.ntiles) * d;
   Buffer<uint8_t> codes(alloc, n);
   Buffer<uint32_t> rows(alloc, cells);
-  node_count_kernel<<<tiles, kNodeBlock, 0, s>>>(skeys.data(), n, d, max_size, codes.data(),
-                                                 rows.data());
+  Buffer<unsigned long long> wide = wide_node_total(n * d, alloc);
+  node_count_kernel<uint32_t, OneTreeTiles><<<tiles.ntiles, kNodeBlock, 0, s>>>(
+    skeys.data(), tiles, d, codes.data(), rows.data(), nullptr, nullptr, wide.data());
   CSPT_CHECK_LAUNCH();
+  check_node_total(wide, s);
   exclusive_scan<uint32_t>(rows.data(), rows.data(), cells, total.data(), alloc);
   size_t const q = read_back(total.data(), s);
   OutputBuffer const out_tag;
   Buffer<uint32_t> okey(alloc, q, out_tag), olen(alloc, q, out_tag), ooff(alloc, q, out_tag);
   Buffer<uint8_t> olev(alloc, q, out_tag), oint(alloc, q, out_tag);
-  node_write_kernel<<<tiles, kNodeBlock, 0, s>>>(skeys.data(), n, d, max_size, codes.data(),
-                                                 rows.data(), okey.data(), olev.data(),
-                                                 oint.data(), olen.data(), ooff.data());
-  CSPT_CHECK_LAUNCH();
-  child_count_kernel<<<grid_for(q, blk, sm_grid(16u)), blk, 0, s>>>(
-    okey.data(), olev.data(), oint.data(), ooff.data(), q, olen.data());
-  CSPT_CHECK_LAUNCH();
+  write_nodes<uint32_t>(skeys.data(), tiles, tiles.ntiles, codes.data(), rows.data(),
+                        NodeColumns{okey.data(), olev.data(), oint.data(), olen.data(),
+                                    ooff.data(), nullptr},
+                        q, s);
   *out_point_indices = sidx.release();
   *out = cspt_quadtree{okey.release(), olev.release(), oint.release(), olen.release(),
                        ooff.release(), q};
