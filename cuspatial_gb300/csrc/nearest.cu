@@ -480,8 +480,10 @@ __global__ void __launch_bounds__(256)
 //   d2: 4 d t + 4 u32 t^2, d3: 2 d (s + t) + 4 u32 s t,
 //   d0 - d3^2/d2 adds r (dd3/d3 * 2 + dd2/d2), i.e. up to 4 d s^2 / t;
 // the branch choice near a projection end changes the value by the square
-// of those errors only (the two branches meet there).  The bound below takes
-// four times their sum plus 2^-40 of the magnitudes for the float64
+// of those errors only (the two branches meet there).  1/t comes from the
+// approximate reciprocal square root (2^-22.9) and s from the approximate square
+// root: r = d3^2 (1/t)^2 is off by 6 u32 s^2 more.  The bound below takes more
+// than twice the sum of all that plus 2^-40 of the magnitudes for the float64
 // rounding; t -> 0 makes it infinite, which sends the segment to float64.
 __device__ inline void seg_estimate(float qx, float qy, float4 e, float dm, float& est,
                                     float& err)
@@ -493,11 +495,15 @@ __device__ inline void seg_estimate(float qx, float qy, float4 e, float dm, floa
   float const d1 = __fmaf_rn(v2x, v2x, v2y * v2y);
   float const d2 = __fmaf_rn(ex, ex, ey * ey);
   float const d3 = __fmaf_rn(v1x, ex, v1y * ey);
-  float const r  = d3 * d3 / d2;
+  float it, sv;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(it) : "f"(d2));
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(sv) : "f"(d0));
+  float const q  = d3 * it;
+  float const r  = q * q;
   est            = (d3 <= 0.0f || r >= d2) ? fminf(d0, d1) : d0 - r;
-  float const sv = sqrtf(d0), tv = sqrtf(d2);
+  float const tv = d2 * it;
   float const u32 = 5.960464477539063e-08f;
-  err = 4.0f * (dm * (8.0f * sv + 4.0f * tv + 4.0f * d0 / tv) +
+  err = 4.0f * (dm * (8.0f * sv + 4.0f * tv + 4.0f * d0 * it) +
                 u32 * (12.0f * d0 + 8.0f * sv * tv + 4.0f * d2)) +
         9.094947017729282e-13f * (d0 + d2) + 7.52316384526264e-37f;
   if (!(err < INFINITY)) err = INFINITY;
@@ -933,7 +939,8 @@ __device__ inline bool seg_can_reach(NearList const& L, uint32_t t, float qx, fl
 //   3. list the segments within r2 of the leaf box: a segment left out has
 //      a float64 distance above r2 >= U for every point, so it can neither
 //      win nor tie;
-//   4. per point: U over the list, then float64 (the reference's expression)
+//   4. per point: U over the list from step 2's on (one pass over the list: most
+//      segments' boxes lie beyond it), then float64 (the reference's expression)
 //      on every listed segment whose estimate can reach U; the winner is the
 //      smallest (distance, linestring id) among them, which is the
 //      reference's fold (:279-294) whenever no distance is exactly 0.  A
@@ -988,7 +995,10 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
         uint64_t const pos = off + c;
         if (pos >= a.npi) continue;
         float2 const uv = a.u[pos];
-        r2              = fmaxf(r2, list_upper(L, n, uv.x, uv.y, dm, tol));
+        float const U   = list_upper(L, n, uv.x, uv.y, dm, tol);
+        r2              = fmaxf(r2, U);
+        // kept for step 4 (the same lane reads it) where the distance will be
+        *reinterpret_cast<float*>(a.od + pos) = U;
       }
       r2 = warp_max(r2);
       __syncwarp();  // every lane is done with the first list
@@ -1009,10 +1019,12 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
         uint32_t bid    = 0;
         bool const fold = act && nearest_point_scan(a, k0, k1, lf, pos, gok, px, py, have, bid, bd);
         fold_lanes(a, k0, k1, fold, px, py, have, bid, bd, nfb);
-        if (act && have) {
-          a.opt[pos] = static_cast<uint32_t>(pos);
-          a.ols[pos] = bid;
-          a.od[pos]  = bd;
+        if (act) {
+          if (have) {
+            a.opt[pos] = static_cast<uint32_t>(pos);
+            a.ols[pos] = bid;
+          }
+          a.od[pos] = have ? bd : 0.0;  // (step 2 may have left its bound here)
         }
       }
       __syncwarp();
@@ -1025,18 +1037,35 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
       uint64_t const pos = off + c0 + static_cast<uint32_t>(lane);
       bool const act     = c0 + static_cast<uint32_t>(lane) < len && pos < a.npi;
       // this point's candidates: the listed segments whose estimate can
-      // reach U (the smallest upper bound over the list), the first
-      // kNearCand of them kept in list order
+      // reach U, which starts at the bound of step 2 and shrinks on the way;
+      // the first kNearCand of them are kept in list order
       float2 const uv = act ? a.u[pos] : make_float2(0.0f, 0.0f);
       float Uw        = 0.0f;
       uint32_t nc     = 0;
       if (act) {
-        float const U = list_upper(L, n, uv.x, uv.y, dm, tol);
-        Uw            = U * 1.0000000009313226f + 7.52316384526264e-37f;
+        float U = *reinterpret_cast<float const*>(a.od + pos);
+        Uw      = U * 1.0000000009313226f + 7.52316384526264e-37f;
         for (uint32_t t = 0; t < n; ++t) {
-          if (!seg_can_reach(L, t, uv.x, uv.y, dm, tol, Uw)) continue;
+          float4 const e  = L.e[t];
+          float4 const sb = make_float4(fminf(e.x, e.z), fminf(e.y, e.w), fmaxf(e.x, e.z),
+                                        fmaxf(e.y, e.w));
+          if (box_lb(uv.x, uv.y, sb, tol) > Uw) continue;
+          float est, err;
+          seg_estimate(uv.x, uv.y, e, dm, est, err);
+          if (est - err > Uw) continue;
+          U  = fminf(U, est + err);
+          Uw = U * 1.0000000009313226f + 7.52316384526264e-37f;
           if (nc < kNearCand) cand[nc][lane] = static_cast<uint16_t>(t);
           ++nc;
+        }
+        if (nc > kNearCand) {
+          // some may no longer reach the final bound: list them again
+          nc = 0;
+          for (uint32_t t = 0; t < n; ++t) {
+            if (!seg_can_reach(L, t, uv.x, uv.y, dm, tol, Uw)) continue;
+            if (nc < kNearCand) cand[nc][lane] = static_cast<uint16_t>(t);
+            ++nc;
+          }
         }
       }
       double px = 0.0, py = 0.0;
@@ -1092,10 +1121,12 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
       }
       __syncwarp();  // the candidate slots are reused by the next chunk
       fold_lanes(a, k0, k1, act && (!have || zero), px, py, have, bid, bd, nfb);
-      if (act && have) {
-        a.opt[pos] = static_cast<uint32_t>(pos);
-        a.ols[pos] = bid;
-        a.od[pos]  = bd;
+      if (act) {
+        if (have) {
+          a.opt[pos] = static_cast<uint32_t>(pos);
+          a.ols[pos] = bid;
+        }
+        a.od[pos] = have ? bd : 0.0;
       }
     }
     __syncwarp();  // the next group rewrites this warp's list
