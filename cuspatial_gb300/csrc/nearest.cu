@@ -310,6 +310,11 @@ __global__ void __launch_bounds__(256)
 // ---------------------------------------------------------------------------
 // float32 filter (float64 inputs)
 // ---------------------------------------------------------------------------
+constexpr int kSegSuper = 64;  // segments per coarse pruning box (8 chunks)
+// (the coarse boxes' slots, as chunk_slots: box c of linestring l is at
+// v0 / kSegSuper + l + c)
+inline size_t super_slots(size_t nv, size_t nls) { return nv / kSegSuper + nls + 1; }
+
 // Per linestring, what the segment listing needs in one 64-byte record.
 struct __align__(16) LsRec {
   long long aix, aiy;  // anchor in grid steps
@@ -317,8 +322,9 @@ struct __align__(16) LsRec {
   float maxoff;        // largest |float32 offset|
   uint32_t v0, nseg;   // first vertex, segments
   uint32_t cb;         // first chunk's slot
+  uint32_t sb;         // first coarse box's slot
   uint32_t exact;      // non-finite coordinates: exact path only
-  uint32_t pad[3];
+  uint32_t pad[2];
 };
 static_assert(sizeof(LsRec) == 64, "one 64-byte record per linestring");
 
@@ -327,6 +333,7 @@ struct LinestringIndexView {
   long long const* aiy;
   float const* maxoff;   // largest |float32 offset| of the linestring
   float4 const* chunk_box;  // (minx, miny, maxx, maxy) of 8 segments, anchor frame
+  float4 const* super_box;  // the same of 64 segments
   float4 const* seg32;      // per segment start vertex: (ax, ay, bx, by), anchor frame
   uint8_t const* exact;     // non-finite coordinates: exact path only
   LsRec const* rec;
@@ -397,7 +404,7 @@ __global__ void __launch_bounds__(256)
                  double const* __restrict__ gridp, uint8_t const* __restrict__ exact,
                  long long* aix, long long* aiy, float* maxoff, float4* chunk_box, float4* seg32,
                  LsRec* rec, size_t slots, float4* __restrict__ abs_ls,
-                 float4* __restrict__ abs_chunk)
+                 float4* __restrict__ abs_chunk, size_t sslots, float4* __restrict__ super_box)
 {
   int const lane      = threadIdx.x & 31;
   size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -417,32 +424,44 @@ __global__ void __launch_bounds__(256)
     float m             = 0.0f;
     float4 lbx          = make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
     BoundBox all;  // the boxes of LsBounds, for points folded over every candidate
-    // lane per chunk
-    for (uint32_t c = lane; c < nch; c += 32) {
+    // lane per chunk, eight lanes per coarse box
+    uint32_t const sb = v0 / kSegSuper + static_cast<uint32_t>(l);
+    for (uint32_t c0 = 0; c0 < nch; c0 += 32) {
+      uint32_t const c = c0 + static_cast<uint32_t>(lane);
       float4 cbx = make_float4(INFINITY, INFINITY, -INFINITY, -INFINITY);
-      uint32_t const s0 = v0 + c * kSegChunk;
-      uint32_t const s1 = min(s0 + kSegChunk, v0 + nseg);
-      BoundBox abs_box;
-      abs_box.add(lx[s0], ly[s0]);
-      for (uint32_t sg = s0; sg < s1; ++sg) {
-        abs_box.add(lx[sg + 1], ly[sg + 1]);
-        float4 e;
-        e.x       = static_cast<float>(lx[sg] - cx);
-        e.y       = static_cast<float>(ly[sg] - cy);
-        e.z       = static_cast<float>(lx[sg + 1] - cx);
-        e.w       = static_cast<float>(ly[sg + 1] - cy);
-        seg32[sg] = e;
-        cbx.x     = fminf(cbx.x, fminf(e.x, e.z));
-        cbx.y     = fminf(cbx.y, fminf(e.y, e.w));
-        cbx.z     = fmaxf(cbx.z, fmaxf(e.x, e.z));
-        cbx.w     = fmaxf(cbx.w, fmaxf(e.y, e.w));
-        m = fmaxf(m, fmaxf(fmaxf(fabsf(e.x), fabsf(e.y)), fmaxf(fabsf(e.z), fabsf(e.w))));
+      if (c < nch) {
+        uint32_t const s0 = v0 + c * kSegChunk;
+        uint32_t const s1 = min(s0 + kSegChunk, v0 + nseg);
+        BoundBox abs_box;
+        abs_box.add(lx[s0], ly[s0]);
+        for (uint32_t sg = s0; sg < s1; ++sg) {
+          abs_box.add(lx[sg + 1], ly[sg + 1]);
+          float4 e;
+          e.x       = static_cast<float>(lx[sg] - cx);
+          e.y       = static_cast<float>(ly[sg] - cy);
+          e.z       = static_cast<float>(lx[sg + 1] - cx);
+          e.w       = static_cast<float>(ly[sg + 1] - cy);
+          seg32[sg] = e;
+          cbx.x     = fminf(cbx.x, fminf(e.x, e.z));
+          cbx.y     = fminf(cbx.y, fminf(e.y, e.w));
+          cbx.z     = fmaxf(cbx.z, fmaxf(e.x, e.z));
+          cbx.w     = fmaxf(cbx.w, fmaxf(e.y, e.w));
+          m = fmaxf(m, fmaxf(fmaxf(fabsf(e.x), fabsf(e.y)), fmaxf(fabsf(e.z), fabsf(e.w))));
+        }
+        all.add(abs_box.b);
+        if (cb + c < slots) {
+          chunk_box[cb + c] = cbx;
+          abs_chunk[cb + c] = abs_box.b;
+        }
       }
-      all.add(abs_box.b);
-      if (cb + c < slots) {
-        chunk_box[cb + c] = cbx;
-        abs_chunk[cb + c] = abs_box.b;
-      }
+      float4 sbx = cbx;
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1)
+        sbx = make_float4(fminf(sbx.x, __shfl_xor_sync(0xFFFFFFFFu, sbx.x, o)),
+                          fminf(sbx.y, __shfl_xor_sync(0xFFFFFFFFu, sbx.y, o)),
+                          fmaxf(sbx.z, __shfl_xor_sync(0xFFFFFFFFu, sbx.z, o)),
+                          fmaxf(sbx.w, __shfl_xor_sync(0xFFFFFFFFu, sbx.w, o)));
+      if (c < nch && (lane & 7) == 0 && sb + (c >> 3) < sslots) super_box[sb + (c >> 3)] = sbx;
       lbx = make_float4(fminf(lbx.x, cbx.x), fminf(lbx.y, cbx.y), fmaxf(lbx.z, cbx.z),
                         fmaxf(lbx.w, cbx.w));
     }
@@ -466,6 +485,7 @@ __global__ void __launch_bounds__(256)
       r.v0     = v0;
       r.nseg   = nseg;
       r.cb     = cb;
+      r.sb     = sb;
       r.exact  = exact[l];
       rec[l]   = r;
     }
@@ -727,13 +747,13 @@ constexpr uint32_t kListFrame    = 0xFFFFFFFFu;  // a linestring outside the flo
 // distance r2 of the leaf's point box (box-to-box lower bound with the
 // filter's margin tol, computed in each linestring's frame; the leaf box
 // maps into that frame monotonically, so it holds every point's mapped
-// offset and the bound is below each point's own box_lb).  Three filters,
+// offset and the bound is below each point's own box_lb).  Four filters,
 // each on every lane: 32 candidate linestrings at a time, each lane loading
-// one linestring's 64-byte record and testing its whole box; the chunks of
-// the linestrings that pass, flattened over the lanes (a lane finds its
-// chunk's linestring by a binary search over the lanes' running chunk
-// counts); four near chunks at a time, eight lanes per chunk, one segment
-// each.  Listed segments are stored in the leaf frame, rounded once from the
+// one linestring's 64-byte record and testing its whole box; the coarse boxes
+// (64 segments) of the linestrings that pass, flattened over the lanes (a lane
+// finds its box's linestring by a binary search over the lanes' running
+// counts); four near coarse boxes at a time, eight lanes per box, one chunk
+// each; four near chunks at a time, eight lanes per chunk, one segment each.  Listed segments are stored in the leaf frame, rounded once from the
 // float64 vertices; mg receives the largest magnitude of the leaf frame (its
 // points' and the listed segments' offsets), which bounds their errors.
 // Returns the count, kListOverflow or kListFrame.
@@ -761,7 +781,7 @@ __device__ uint32_t list_segments(NearestArgs const& a, NearList& L, uint32_t k0
     bool bad = false;
     float4 lb{};
     float tol    = 0.0f;
-    uint32_t nch = 0;
+    uint32_t nsb = 0;
     if (valid) {
       long long const dix = r.aix - lf.ix, diy = r.aiy - lf.iy;
       bad = r.exact || dix <= -16777216LL || dix >= 16777216LL || diy <= -16777216LL ||
@@ -773,12 +793,12 @@ __device__ uint32_t list_segments(NearestArgs const& a, NearList& L, uint32_t k0
         float const mk = fmaxf(fmaxf(r.maxoff, lf.m), fmaxf(fmaxf(fabsf(lb.x), fabsf(lb.y)),
                                                             fmaxf(fabsf(lb.z), fabsf(lb.w))));
         tol            = 4.76837158203125e-07f * mk;
-        if (boxbox_lb(lb, r.box, tol) <= r2) nch = (r.nseg + kSegChunk - 1) / kSegChunk;
+        if (boxbox_lb(lb, r.box, tol) <= r2) nsb = (r.nseg + kSegSuper - 1) / kSegSuper;
       }
     }
     if (__any_sync(kAll, bad)) return kListFrame;
-    // running chunk counts over the lanes
-    uint32_t incl = nch;
+    // running coarse box counts over the lanes
+    uint32_t incl = nsb;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       uint32_t const t = __shfl_up_sync(kAll, incl, o);
@@ -787,7 +807,7 @@ __device__ uint32_t list_segments(NearestArgs const& a, NearList& L, uint32_t k0
     uint32_t const total = __shfl_sync(kAll, incl, 31);
     for (uint32_t c0 = 0; c0 < total; c0 += 32) {
       uint32_t const c = c0 + static_cast<uint32_t>(lane);
-      // the chunk's linestring: the first lane whose running count exceeds c
+      // the coarse box's linestring: the first lane whose running count exceeds c
       int ow = 0;
 #pragma unroll
       for (int step = 16; step > 0; step >>= 1) {
@@ -795,58 +815,76 @@ __device__ uint32_t list_segments(NearestArgs const& a, NearList& L, uint32_t k0
         if (v <= c) ow += step;
       }
       ow = ow < 31 ? ow : 31;
-      float4 const olb     = make_float4(__shfl_sync(kAll, lb.x, ow), __shfl_sync(kAll, lb.y, ow),
-                                         __shfl_sync(kAll, lb.z, ow), __shfl_sync(kAll, lb.w, ow));
-      float const otol     = __shfl_sync(kAll, tol, ow);
-      uint32_t const olid  = __shfl_sync(kAll, lid, ow);
-      uint32_t const ov0   = __shfl_sync(kAll, r.v0, ow);
-      uint32_t const onseg = __shfl_sync(kAll, r.nseg, ow);
-      uint32_t const ocb   = __shfl_sync(kAll, r.cb, ow);
-      uint32_t const oinc  = __shfl_sync(kAll, incl, ow);
-      uint32_t const onch  = __shfl_sync(kAll, nch, ow);
-      uint32_t const ch    = c - (oinc - onch);  // the chunk within its linestring
-      bool const near      = c < total && boxbox_lb(olb, li.chunk_box[ocb + ch], otol) <= r2;
-      unsigned cm          = __ballot_sync(kAll, near);
-      while (cm) {
-        // lane l expands the (l / 8)-th remaining near chunk, segment l % 8;
-        // that chunk's linestring fields are held by lane src
-        unsigned mm = cm;
-        for (int t = 0; t < (lane >> 3); ++t) mm &= mm - 1u;
-        int const src       = mm ? __ffs(mm) - 1 : 0;
-        float4 const slb    = make_float4(__shfl_sync(kAll, olb.x, src), __shfl_sync(kAll, olb.y, src),
-                                          __shfl_sync(kAll, olb.z, src), __shfl_sync(kAll, olb.w, src));
-        float const stol    = __shfl_sync(kAll, otol, src);
-        uint32_t const slid = __shfl_sync(kAll, olid, src);
-        uint32_t const sv0  = __shfl_sync(kAll, ov0, src);
-        uint32_t const snsg = __shfl_sync(kAll, onseg, src);
-        uint32_t const sch  = __shfl_sync(kAll, ch, src);
-        uint32_t const sg   = sv0 + sch * kSegChunk + static_cast<uint32_t>(lane & 7);
-        bool keep           = false;
-        if (mm && sg < sv0 + snsg) {
-          float4 const e   = li.seg32[sg];
-          float4 const sbx = make_float4(fminf(e.x, e.z), fminf(e.y, e.w), fmaxf(e.x, e.z),
-                                         fmaxf(e.y, e.w));
-          keep             = boxbox_lb(slb, sbx, stol) <= r2;
+      float4 const wlb    = make_float4(__shfl_sync(kAll, lb.x, ow), __shfl_sync(kAll, lb.y, ow),
+                                        __shfl_sync(kAll, lb.z, ow), __shfl_sync(kAll, lb.w, ow));
+      float const wtol    = __shfl_sync(kAll, tol, ow);
+      uint32_t const wsb  = __shfl_sync(kAll, r.sb, ow);
+      uint32_t const winc = __shfl_sync(kAll, incl, ow);
+      uint32_t const wnsb = __shfl_sync(kAll, nsb, ow);
+      uint32_t const sc   = c - (winc - wnsb);  // the box within its linestring
+      bool const wnear    = c < total && boxbox_lb(wlb, li.super_box[wsb + sc], wtol) <= r2;
+      unsigned wm         = __ballot_sync(kAll, wnear);
+      while (wm) {
+        // lane l expands the (l / 8)-th remaining near box, chunk l % 8; its
+        // linestring is held by lane ow of that box's lane
+        unsigned wl = wm;
+        for (int t = 0; t < (lane >> 3); ++t) wl &= wl - 1u;
+        int const wsrc       = wl ? __ffs(wl) - 1 : 0;
+        int const own        = __shfl_sync(kAll, ow, wsrc);
+        uint32_t const ch    = __shfl_sync(kAll, sc, wsrc) * (kSegSuper / kSegChunk) +
+                               static_cast<uint32_t>(lane & 7);
+        float4 const olb     = make_float4(__shfl_sync(kAll, lb.x, own), __shfl_sync(kAll, lb.y, own),
+                                           __shfl_sync(kAll, lb.z, own), __shfl_sync(kAll, lb.w, own));
+        float const otol     = __shfl_sync(kAll, tol, own);
+        uint32_t const olid  = __shfl_sync(kAll, lid, own);
+        uint32_t const ov0   = __shfl_sync(kAll, r.v0, own);
+        uint32_t const onseg = __shfl_sync(kAll, r.nseg, own);
+        uint32_t const ocb   = __shfl_sync(kAll, r.cb, own);
+        for (int t = 0; t < 4 && wm; ++t) wm &= wm - 1u;
+        bool const near = wl && ch * kSegChunk < onseg &&
+                          boxbox_lb(olb, li.chunk_box[ocb + ch], otol) <= r2;
+        unsigned cm     = __ballot_sync(kAll, near);
+        while (cm) {
+          // lane l expands the (l / 8)-th remaining near chunk, segment l % 8;
+          // that chunk's linestring fields are held by lane src
+          unsigned mm = cm;
+          for (int t = 0; t < (lane >> 3); ++t) mm &= mm - 1u;
+          int const src       = mm ? __ffs(mm) - 1 : 0;
+          float4 const slb    = make_float4(__shfl_sync(kAll, olb.x, src), __shfl_sync(kAll, olb.y, src),
+                                            __shfl_sync(kAll, olb.z, src), __shfl_sync(kAll, olb.w, src));
+          float const stol    = __shfl_sync(kAll, otol, src);
+          uint32_t const slid = __shfl_sync(kAll, olid, src);
+          uint32_t const sv0  = __shfl_sync(kAll, ov0, src);
+          uint32_t const snsg = __shfl_sync(kAll, onseg, src);
+          uint32_t const sch  = __shfl_sync(kAll, ch, src);
+          uint32_t const sg   = sv0 + sch * kSegChunk + static_cast<uint32_t>(lane & 7);
+          bool keep           = false;
+          if (mm && sg < sv0 + snsg) {
+            float4 const e   = li.seg32[sg];
+            float4 const sbx = make_float4(fminf(e.x, e.z), fminf(e.y, e.w), fmaxf(e.x, e.z),
+                                           fmaxf(e.y, e.w));
+            keep             = boxbox_lb(slb, sbx, stol) <= r2;
+          }
+          unsigned const km = __ballot_sync(kAll, keep);
+          if (n + __popc(km) > kNearCap) return kListOverflow;
+          if (keep) {
+            // the segment in the leaf frame, rounded once from the float64
+            // vertices: its error is a float32 rounding of a leaf-local value,
+            // not of the linestring-frame offset (which grows with the
+            // linestring's extent), so the estimates' bound stays tight
+            uint32_t const slot = n + __popc(km & lt);
+            float4 const el     = make_float4(static_cast<float>(a.lx[sg] - lf.ax),
+                                              static_cast<float>(a.ly[sg] - lf.ay),
+                                              static_cast<float>(a.lx[sg + 1] - lf.ax),
+                                              static_cast<float>(a.ly[sg + 1] - lf.ay));
+            L.e[slot]   = el;
+            L.seg[slot] = sg;
+            L.lid[slot] = slid;
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(el.x), fabsf(el.y)), fmaxf(fabsf(el.z), fabsf(el.w))));
+          }
+          n += __popc(km);
+          for (int t = 0; t < 4 && cm; ++t) cm &= cm - 1u;
         }
-        unsigned const km = __ballot_sync(kAll, keep);
-        if (n + __popc(km) > kNearCap) return kListOverflow;
-        if (keep) {
-          // the segment in the leaf frame, rounded once from the float64
-          // vertices: its error is a float32 rounding of a leaf-local value,
-          // not of the linestring-frame offset (which grows with the
-          // linestring's extent), so the estimates' bound stays tight
-          uint32_t const slot = n + __popc(km & lt);
-          float4 const el     = make_float4(static_cast<float>(a.lx[sg] - lf.ax),
-                                            static_cast<float>(a.ly[sg] - lf.ay),
-                                            static_cast<float>(a.lx[sg + 1] - lf.ax),
-                                            static_cast<float>(a.ly[sg + 1] - lf.ay));
-          L.e[slot]   = el;
-          L.seg[slot] = sg;
-          L.lid[slot] = slid;
-          m = fmaxf(m, fmaxf(fmaxf(fabsf(el.x), fabsf(el.y)), fmaxf(fabsf(el.z), fabsf(el.w))));
-        }
-        n += __popc(km);
-        for (int t = 0; t < 4 && cm; ++t) cm &= cm - 1u;
       }
     }
   }
@@ -932,13 +970,15 @@ __device__ inline bool seg_can_reach(NearList const& L, uint32_t t, float qx, fl
 
 // One warp per group of pairs sharing a quadrant (handed out from a device
 // counter), one lane per point.
-//   1. list the segments whose box meets the leaf's point box (radius 0);
+//   1. list the segments whose box is within a radius of the leaf's point box,
+//      taken from the warp's last groups (a guess: it only decides whether 3 is
+//      needed; the listings are most of the kernel's instructions);
 //   2. each point's float32 upper bound U over that list; r2 = the largest U
 //      of the group's points: every point's nearest segment lies within r2
 //      of the leaf box;
-//   3. list the segments within r2 of the leaf box: a segment left out has
-//      a float64 distance above r2 >= U for every point, so it can neither
-//      win nor tie;
+//   3. unless 1 went that far, list the segments within r2 of the leaf box: a
+//      segment left out has a float64 distance above r2 >= U for every point,
+//      so it can neither win nor tie;
 //   4. per point: U over the list from step 2's on (one pass over the list: most
 //      segments' boxes lie beyond it), then float64 (the reference's expression)
 //      on every listed segment whose estimate can reach U; the winner is the
@@ -960,6 +1000,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
   uint32_t const ng = *a.ngroups_p;
   bool const gok    = a.gf >= 1.17549435e-38f && a.gf < 1.0e30f;
   uint32_t nfb = 0, nscan = 0, nf64 = 0;
+  float guess  = 0.0f;  // squared radius expected to hold the next group's list
   for (;;) {
     unsigned long long gg = 0;
     if (lane == 0) gg = atomicAdd(a.next_group, 1ull);
@@ -973,16 +1014,22 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
     LeafFrame const lf  = a.frames[gi];
     bool listed         = !lf.nonfinite && gok;
     float mg            = 0.0f;
+    float rad           = guess;  // squared radius of the list
     uint32_t n          = 0;
     if (listed) {
-      n = list_segments(a, L, k0, k1, lf, 0.0f, mg);
+      n = list_segments(a, L, k0, k1, lf, rad, mg);
+      if (n == kListOverflow && rad > 0.0f) {
+        __syncwarp();
+        rad = 0.0f;
+        n   = list_segments(a, L, k0, k1, lf, rad, mg);
+      }
       listed = n != kListOverflow && n != kListFrame;
       if (listed && n == 0) {
-        // no segment meets the leaf box: a radius from the chunks' vertices
-        float const r2 = group_upper(a, k0, k1, lf);
-        listed         = r2 < INFINITY;
+        // no segment within the radius: one from the chunks' vertices
+        rad    = group_upper(a, k0, k1, lf);
+        listed = rad < INFINITY;
         if (listed) {
-          n      = list_segments(a, L, k0, k1, lf, r2, mg);
+          n      = list_segments(a, L, k0, k1, lf, rad, mg);
           listed = n != kListOverflow && n != kListFrame && n > 0;
         }
       }
@@ -1004,8 +1051,12 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
       __syncwarp();  // every lane is done with the first list
       listed = r2 < INFINITY;
       if (listed) {
-        n      = list_segments(a, L, k0, k1, lf, r2 * 1.0000009536743164f, mg);
-        listed = n != kListOverflow && n != kListFrame && n > 0;
+        float const need = r2 * 1.0000009536743164f;
+        if (need > rad) {
+          n      = list_segments(a, L, k0, k1, lf, need, mg);
+          listed = n != kListOverflow && n != kListFrame && n > 0;
+        }
+        guess = fmaxf(0.7f * guess, 1.3f * need);
       }
     }
     if (!listed) {
@@ -1182,13 +1233,14 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       Buffer<long long> aix(alloc, nls), aiy(alloc, nls);
       Buffer<float> maxoff(alloc, nls);
       size_t const slots = chunk_slots(nv, nls);
+      size_t const sslots = super_slots(nv, nls);
       Buffer<float4> cbox(alloc, slots), seg32(alloc, nv), abs_ls(alloc, nls),
-        abs_chunk(alloc, slots);
+        abs_chunk(alloc, slots), sbox(alloc, sslots);
       Buffer<LsRec> lrec(alloc, nls);
       ls_fill_kernel<<<lgrd, 256, 0, s>>>(lso, nls, lx, ly, box.data(), grid.data(),
                                           lexact.data(), aix.data(), aiy.data(),
                                           maxoff.data(), cbox.data(), seg32.data(), lrec.data(),
-                                          slots, abs_ls.data(), abs_chunk.data());
+                                          slots, abs_ls.data(), abs_chunk.data(), sslots, sbox.data());
       CSPT_CHECK_LAUNCH();
       double const g = read_back(grid.data(), s);
       index_timer.reset();
@@ -1201,8 +1253,8 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
         frames.data());
       CSPT_CHECK_LAUNCH();
       frames_timer.reset();
-      LinestringIndexView liv{aix.data(),   aiy.data(),    maxoff.data(), cbox.data(),
-                              seg32.data(), lexact.data(), lrec.data()};
+      LinestringIndexView liv{aix.data(),  aiy.data(),   maxoff.data(), cbox.data(),
+                              sbox.data(), seg32.data(), lexact.data(), lrec.data()};
       LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(slots)};
       // points folded whole, groups scanned, next group, float64 segment distances
       Buffer<unsigned long long> fb(alloc, 4);
