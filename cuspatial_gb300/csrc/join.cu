@@ -40,6 +40,26 @@ __global__ void composite_key_kernel(uint32_t const* __restrict__ node,
     key[i] = (static_cast<uint64_t>(offset[node[i]]) << box_bits) | box[i];
 }
 
+// What the count pass leaves for the host, read back in one copy.
+struct JoinTotals {
+  uint32_t max_offset;  // largest leaf first-point offset found
+  int error;
+  unsigned long long appended;
+  uint32_t pairs;
+  uint32_t level0;  // the tree's level-0 nodes
+};
+
+__global__ void count_level0_kernel(uint8_t const* __restrict__ level, size_t nq,
+                                    uint32_t* __restrict__ out)
+{
+  uint32_t c = 0;
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < nq;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x)
+    c += level[i] == 0 ? 1u : 0u;
+  c = __reduce_add_sync(0xFFFFFFFFu, c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
+}
+
 template <typename T>
 void run(cspt_quadtree const* tree, T const* bminx, T const* bminy, T const* bmaxx,
          T const* bmaxy, size_t nb, T vminx, T vminy, T scale, int max_depth,
@@ -48,58 +68,47 @@ void run(cspt_quadtree const* tree, T const* bminx, T const* bminy, T const* bma
   cudaStream_t const s = alloc.stream();
   TreeView tv{tree->key, tree->level, tree->is_internal_node, tree->length, tree->offset,
               tree->num_nodes};
+  Buffer<JoinTotals> totals(alloc, 1);
+  JoinTotals* const tot = totals.data();
+  CSPT_CUDA_TRY(cudaMemsetAsync(tot, 0, sizeof(JoinTotals), s));
   // seeds: the number of level-0 nodes (quadtree_bbox_filtering.cuh:53-56)
-  Buffer<uint32_t> L0(alloc, 1);
-  uint8_t const* lev = tree->level;
-  scan_apply<uint32_t>([lev] __device__(size_t i) { return lev[i] == 0 ? 1u : 0u; },
-                       [] __device__(size_t, uint32_t, uint32_t) {}, tree->num_nodes, L0.data(),
-                       alloc);
+  count_level0_kernel<<<grid_for(tree->num_nodes, 256, sm_grid(4u)), 256, 0, s>>>(
+    tree->level, tree->num_nodes, &tot->level0);
+  CSPT_CHECK_LAUNCH();
   CSPT_EXPECTS(tree->num_nodes < (size_t{1} << 28), "quadtree has too many nodes");
-  OneTree<T> const trees{L0.data(), static_cast<uint32_t>(tree->num_nodes), vminx, vminy, scale,
+  OneTree<T> const trees{&tot->level0, static_cast<uint32_t>(tree->num_nodes), vminx, vminy, scale,
                          max_depth};
-  Buffer<uint32_t> counts(alloc, nb + 1);
-  Buffer<uint32_t> status(alloc, 2);  // [0] max leaf offset, [1] error flag
-  CSPT_CUDA_TRY(cudaMemsetAsync(status.data(), 0, 2 * sizeof(uint32_t), s));
-  int* err           = reinterpret_cast<int*>(status.data() + 1);
+  Buffer<uint32_t> counts(alloc, nb);
+  int* const err     = &tot->error;
   unsigned const blk = kJoinWarps * 32;
   unsigned const grd = grid_for(nb * 32, blk, sm_grid(16u));
   // the count pass also appends each (node, box) it finds while they fit
   size_t const cap = join_append_capacity(nb);
   Buffer<uint32_t> app_node(alloc, cap), app_box(alloc, cap);
-  Buffer<unsigned long long> app_n(alloc, 1);
-  CSPT_CUDA_TRY(cudaMemsetAsync(app_n.data(), 0, sizeof(unsigned long long), s));
   {
     KernelTimer timer("join_count", s);
     join_warp_kernel<T, false><<<grd, blk, 0, s>>>(
-      tv, trees, bminx, bminy, bmaxx, bmaxy, nb, counts.data(), status.data(), nullptr, nullptr,
-      nullptr, nullptr, err, JoinAppend{app_node.data(), app_box.data(), app_n.data(), cap});
+      tv, trees, bminx, bminy, bmaxx, bmaxy, nb, counts.data(), &tot->max_offset, nullptr,
+      nullptr, nullptr, nullptr, err,
+      JoinAppend{app_node.data(), app_box.data(), &tot->appended, cap});
     CSPT_CHECK_LAUNCH();
   }
-  exclusive_scan<uint32_t>(counts.data(), counts.data(), nb, counts.data() + nb, alloc);
-  uint32_t host[3];
-  unsigned long long appended = 0;
-  CSPT_CUDA_TRY(cudaMemcpyAsync(host, counts.data() + nb, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                                s));
-  CSPT_CUDA_TRY(
-    cudaMemcpyAsync(host + 1, status.data(), 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  CSPT_CUDA_TRY(cudaMemcpyAsync(&appended, app_n.data(), sizeof(appended),
-                                cudaMemcpyDeviceToHost, s));
-  CSPT_CUDA_TRY(cudaStreamSynchronize(s));
-  size_t const k = host[0];
-  CSPT_EXPECTS(host[2] == 0,
+  exclusive_scan<uint32_t>(counts.data(), counts.data(), nb, &tot->pairs, alloc);
+  JoinTotals const h = read_back(tot, s);
+  size_t const k     = h.pairs;
+  CSPT_EXPECTS(h.error == 0,
                "quadtree is malformed: a node index or child count is out of range");
   *out_n = k;
   if (k == 0) return;
   int key_bits = 1;
-  while (key_bits < 32 && (host[1] >> key_bits) != 0) ++key_bits;
+  while (key_bits < 32 && (h.max_offset >> key_bits) != 0) ++key_bits;
   Buffer<uint32_t> ob(alloc, k, OutputBuffer{}), on(alloc, k, OutputBuffer{});
-  if (appended == k && k <= cap) {
+  if (h.appended == k && k <= cap) {
     // Every pair was appended (in no particular order): sort them by
     // (leaf offset, box), one composite key, which is the order the write
     // pass and a stable sort by leaf offset give.
     int box_bits = 1;
     while (box_bits < 32 && ((nb - 1) >> box_bits) != 0) ++box_bits;
-    app_n.reset();
     Buffer<uint64_t> key(alloc, k), key_alt(alloc, k);
     Buffer<uint32_t> perm(alloc, k), perm_alt(alloc, k);
     {

@@ -878,9 +878,9 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
     [wo] __device__(size_t k, uint64_t e, uint64_t) { wo[k] = e; }, npairs, wo + npairs, alloc);
   Buffer<uint32_t> counts(alloc, npairs);
   // [0] refined candidates, [1] next pair, [2] pairs decided by the
-  // edge-free test
-  Buffer<unsigned long long> refined(alloc, 3);
-  CSPT_CUDA_TRY(cudaMemsetAsync(refined.data(), 0, 3 * sizeof(unsigned long long), s));
+  // edge-free test, [3] rows of the last evaluated pairs
+  Buffer<unsigned long long> refined(alloc, 4);
+  CSPT_CUDA_TRY(cudaMemsetAsync(refined.data(), 0, 4 * sizeof(unsigned long long), s));
   unsigned const blk = 256;
   // filtered: groups of consecutive pairs sharing a quadrant, each pair's
   // group, and the leaf frames (float32 point offsets from the quadrant's
@@ -950,7 +950,8 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
   auto evaluate = [&](size_t k0, size_t n) {
     KernelTimer timer("pip_bits", s);
     if constexpr (std::is_same<T, double>::value) {
-      CSPT_CUDA_TRY(cudaMemsetAsync(refined.data() + 1, 0, sizeof(unsigned long long), s));
+      if (k0 > 0)
+        CSPT_CUDA_TRY(cudaMemsetAsync(refined.data() + 1, 0, sizeof(unsigned long long), s));
       if (filtered)
         pip_pair_kernel<true><<<pair_grid(pip_pair_kernel<true>, kPipBlock, n), kPipBlock, 0, s>>>(
           pair_poly + k0, pair_quad + k0, pgroup.data() + k0, n, qlen, qoff, src, npi, u.data(),
@@ -974,15 +975,21 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
     }
     CSPT_CHECK_LAUNCH();
   };
-  // row offsets of pairs [k0, k0 + n) from their counts; returns the rows
+  // row offsets of pairs [k0, k0 + n) from their counts; returns the rows (and
+  // the kernel's counters so far, in the same copy)
   auto row_offsets = [&](size_t k0, size_t n, Buffer<uint64_t>& out_off) {
-    out_off             = Buffer<uint64_t>(alloc, n + 1);
+    out_off             = Buffer<uint64_t>(alloc, n);
     uint64_t* oo        = out_off.data();
     uint32_t const* cnt = counts.data() + k0;
     scan_apply<uint64_t>([cnt] __device__(size_t k) { return static_cast<uint64_t>(cnt[k]); },
                          [oo] __device__(size_t k, uint64_t e, uint64_t) { oo[k] = e; }, n,
-                         oo + n, alloc);
-    return static_cast<size_t>(read_back(oo + n, s));
+                         reinterpret_cast<uint64_t*>(refined.data() + 3), alloc);
+    unsigned long long h[4];
+    CSPT_CUDA_TRY(cudaMemcpyAsync(h, refined.data(), sizeof(h), cudaMemcpyDeviceToHost, s));
+    CSPT_CUDA_TRY(cudaStreamSynchronize(s));
+    if (out_refined) *out_refined = filtered ? h[0] : 0;
+    last_edge_free_pairs() = filtered ? h[2] : 0;
+    return static_cast<size_t>(h[3]);
   };
   auto expand = [&](size_t k0, size_t n, Buffer<uint64_t> const& out_off, uint32_t* op,
                     uint32_t* oq, size_t m) {
@@ -993,19 +1000,10 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
     CSPT_CHECK_LAUNCH();
   };
 
-  // the kernel's counters (read once the stream is idle)
-  auto finish_counts = [&] {
-    unsigned long long h[3] = {0, 0, 0};
-    CSPT_CUDA_TRY(cudaMemcpyAsync(h, refined.data(), sizeof(h), cudaMemcpyDeviceToHost, s));
-    CSPT_CUDA_TRY(cudaStreamSynchronize(s));
-    if (out_refined) *out_refined = filtered ? h[0] : 0;
-    last_edge_free_pairs() = filtered ? h[2] : 0;
-  };
   if (!host) {
     evaluate(0, npairs);
     Buffer<uint64_t> out_off;
     size_t const m = row_offsets(0, npairs, out_off);
-    finish_counts();
     *out_n = m;
     if (m == 0) return;
     Buffer<uint32_t> op(alloc, m, OutputBuffer{}), oq(alloc, m, OutputBuffer{});
@@ -1052,7 +1050,7 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
     rows += m;
   }
   copies.join();
-  finish_counts();
+  CSPT_CUDA_TRY(cudaStreamSynchronize(s));  // the rows are in the caller's arrays
   *out_n = rows;
   CSPT_EXPECTS(rows <= host->capacity,
                "the host buffers hold " + std::to_string(host->capacity) +

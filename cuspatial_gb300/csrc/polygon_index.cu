@@ -381,9 +381,9 @@ __global__ void __launch_bounds__(kIdxBlock)
 // non-finite skipped), which order as the magnitudes: integer work only, so
 // the FP64 pipe of the one SM this runs on stays out of the loop.
 template <typename T>
-__global__ void __launch_bounds__(1024)
-  grid_kernel(T const* __restrict__ pminx, T const* __restrict__ pminy,
-              T const* __restrict__ pmaxx, T const* __restrict__ pmaxy, size_t np, T* grid)
+__device__ inline void anchor_grid(T const* __restrict__ pminx, T const* __restrict__ pminy,
+                                   T const* __restrict__ pmaxx, T const* __restrict__ pmaxy,
+                                   size_t np, T* grid)
 {
   using U             = typename uint_of<T>::type;
   constexpr U kMag    = ~(U{1} << (8 * sizeof(U) - 1));
@@ -418,6 +418,50 @@ __global__ void __launch_bounds__(1024)
       frexp(mv > T{0} ? mv : T{1}, &e);  // mv < 2^e
       *grid = ldexp(T{1}, e - 22);
     }
+  }
+}
+template <typename T>
+__global__ void __launch_bounds__(1024)
+  grid_kernel(T const* __restrict__ pminx, T const* __restrict__ pminy,
+              T const* __restrict__ pmaxx, T const* __restrict__ pmaxy, size_t np, T* grid)
+{
+  anchor_grid<T>(pminx, pminy, pmaxx, pmaxy, np, grid);
+}
+
+// Few polygons: the anchor grid (as grid_kernel) and the three scans (slabs,
+// entries and vertical edges per polygon; each total follows its array) by one
+// block, instead of one launch and three scans.  Up to kFewPolygons the block's
+// rounds of 1024 cost less than the launches.
+constexpr size_t kFewPolygons = 4096;
+
+template <typename T>
+__global__ void __launch_bounds__(1024)
+  few_polygons_kernel(T const* __restrict__ pminx, T const* __restrict__ pminy,
+                      T const* __restrict__ pmaxx, T const* __restrict__ pmaxy, uint32_t np,
+                      T* grid, uint32_t const* __restrict__ nslab,
+                      uint32_t const* __restrict__ nent, uint32_t const* __restrict__ nvert,
+                      uint32_t* __restrict__ slab_base, uint32_t* __restrict__ ebase,
+                      uint32_t* __restrict__ vbeg, uint32_t* __restrict__ vend)
+{
+  anchor_grid<T>(pminx, pminy, pmaxx, pmaxy, np, grid);
+  __shared__ uint32_t total;
+  uint32_t const* const in[3] = {nslab, nent, nvert};
+  uint32_t* const out[3]      = {slab_base, ebase, vbeg};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    uint32_t carry = 0;
+    for (uint32_t b = 0; b < np; b += 1024) {
+      uint32_t const p = b + threadIdx.x;
+      uint32_t const v = p < np ? in[a][p] : 0u;
+      uint32_t const e = carry + block_exclusive_scan<uint32_t, 1024>(v, &total);
+      if (p < np) {
+        out[a][p] = e;
+        if (a == 2) vend[p] = e + v;
+      }
+      carry += total;
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) out[a][np] = carry;
   }
 }
 
@@ -743,7 +787,7 @@ struct PolygonIndex<T>::Sizing {
   size_t np, nslabs_total, nentries, nvertical;
   bool build_float32, order_slabs, edge_bounds;
   unsigned grd;
-  Buffer<uint32_t> ebase, nvert, spans;
+  Buffer<uint32_t> ebase, spans;
   Buffer<float> yslab;
   Allocator const* alloc;  // the caller's: the index's buffers keep pointing to it
 };
@@ -797,12 +841,23 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
       spans.data(), yslab.data(), density);
     CSPT_CHECK_LAUNCH();
   }
-  grid_kernel<T><<<1, 1024, 0, s>>>(pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
-                                    np, grid_.data());
-  CSPT_CHECK_LAUNCH();
-  exclusive_scan<uint32_t>(nslab_.data(), slab_base_.data(), np, slab_base_.data() + np, alloc);
-  exclusive_scan<uint32_t>(nent.data(), ebase.data(), np, ebase.data() + np, alloc);
-  exclusive_scan<uint32_t>(nvert.data(), vbeg_.data(), np, vbeg_.data() + np, alloc);
+  if (np <= kFewPolygons) {
+    few_polygons_kernel<T><<<1, 1024, 0, s>>>(
+      pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(), static_cast<uint32_t>(np),
+      grid_.data(), nslab_.data(), nent.data(), nvert.data(), slab_base_.data(), ebase.data(),
+      vbeg_.data(), vend_.data());
+    CSPT_CHECK_LAUNCH();
+  } else {
+    grid_kernel<T><<<1, 1024, 0, s>>>(pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
+                                      np, grid_.data());
+    CSPT_CHECK_LAUNCH();
+    exclusive_scan<uint32_t>(nslab_.data(), slab_base_.data(), np, slab_base_.data() + np, alloc);
+    exclusive_scan<uint32_t>(nent.data(), ebase.data(), np, ebase.data() + np, alloc);
+    exclusive_scan<uint32_t>(nvert.data(), vbeg_.data(), np, vbeg_.data() + np, alloc);
+    vert_end_kernel<<<grid_for(np, 256, sm_grid(16u)), 256, 0, s>>>(vbeg_.data(), nvert.data(), np,
+                                                                    vend_.data());
+    CSPT_CHECK_LAUNCH();
+  }
   // Sizes of the slab arrays.  A polygon of V vertices gets
   // ns <= max(1, density V / 2) slabs, and its edges' slab spans add up to
   // at most (density + 1.07) V entries: with ns = s <= density V H / sum|rise|
@@ -843,7 +898,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
     nvertical    = tot[2];
   }
   sizing_.reset(new Sizing{po, ro, vx, vy, np, nslabs_total, nentries, nvertical, build_float32,
-                           order_slabs, edge_bounds, grd, std::move(ebase), std::move(nvert), std::move(spans),
+                           order_slabs, edge_bounds, grd, std::move(ebase), std::move(spans),
                            std::move(yslab), &alloc});
   if (!defer_fill) fill();
 }
@@ -882,9 +937,6 @@ void PolygonIndex<T>::fill()
       slab_start_.data(),
       slab_edges_.data(), slab_e32_.data(), vert_x_.data(), vert_x32_.data(), vxy32.data(),
       z->yslab.data());
-    CSPT_CHECK_LAUNCH();
-    vert_end_kernel<<<grid_for(np, 256, sm_grid(16u)), 256, 0, s>>>(vbeg_.data(), z->nvert.data(),
-                                                                  np, vend_.data());
     CSPT_CHECK_LAUNCH();
   }
   vxy32.reset();
