@@ -579,14 +579,16 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
 // within 9 roundings of float64 (2^-50):
 //   left, above or below the point: no toggle, not on the edge;
 //   right, and the point's y certainly between the ends': a toggle;
+//   across the point, its y certainly between the ends': the side of the edge's
+//   line it lies on, where that is certain (edge_by_side);
 //   anything else: exact_edge, in float64.
 // Exactly vertical edges report "on edge" at their x whatever the y: the
 // points' x is looked up among them in float64 as before.
 // A quadrant whose points' box meets no edge's box and no vertical edge has
 // one result (the argument is at the edge-free quadrants above, here with
 // comparisons only): the first point's, evaluated with its slab.
-// 2M points x 10k polygons of 8 to 256 vertices: 621 us, pip_pair_kernel<false>
-// 3690 us; the call 4728 -> 1449 us.
+// 2M points x 10k polygons of 8 to 256 vertices: 423 us, pip_pair_kernel<false>
+// 3690 us; the call 4728 -> 1212 us (621 and 1535 us without the sides).
 // ---------------------------------------------------------------------------
 struct QuadBounds {
   float xl, yl, xu, yu;  // the points' bounds
@@ -677,6 +679,7 @@ __global__ void __launch_bounds__(kPipBlock)
     // 1/64 slab while largest |y| x slabs per unit stays below 2^14
     float const my    = fmaxf(fabsf(box.y), fabsf(box.w));
     float const inner = __fmaf_ru(my, 9.5367431640625e-07f, 1.0e-36f);  // 2^-20
+    float const m     = 1.001f * fmaxf(my, fmaxf(fabsf(box.x), fabsf(box.z)));
     bool const lookup = fmaxf(my, fmaxf(fabsf(q.yl), fabsf(q.yu))) * invh <= 16384.0f;
     bool verts        = vb < ve;  // some point may have a vertical edge's x
     if (!walk && lookup && !q.nonfinite && len > 0 && off < npi) {
@@ -752,8 +755,8 @@ __global__ void __launch_bounds__(kPipBlock)
           src.load(pos, px, py);
           hit = pip_exact<double>(px, py, ix, poly);
         } else if (!(xl > box.z || xu < box.x || yl > box.w || yu < box.y)) {
-          hit = bounds_test(ix, xl, yl, xu, yu, inner, slab0 + slab_lookup(v.y, y0, invh, ns),
-                            verts ? vb : ve, ve,
+          hit = bounds_test(ix, v.x, v.y, xl, yl, xu, yu, inner, m,
+                            slab0 + slab_lookup(v.y, y0, invh, ns), verts ? vb : ve, ve,
                             [&](double& px, double& py) { src.load(pos, px, py); }, nref);
         }
       }

@@ -432,8 +432,9 @@ __global__ void __launch_bounds__(kPointsBlock)
           ++nref;
           hit = pip_exact<double>(px, py, ix, p);
         } else {
-          hit = bounds_test(ix, __fsub_rd(tx, wx), __fsub_rd(ty, wy), __fadd_ru(tx, wx),
+          hit = bounds_test(ix, tx, ty, __fsub_rd(tx, wx), __fsub_rd(ty, wy), __fadd_ru(tx, wx),
                             __fadd_ru(ty, wy), f.inner,
+                            1.001f * fmaxf(f.my, fmaxf(fabsf(f.box.x), fabsf(f.box.z))),
                             f.slab0 + slab_lookup(ty, f.y0, f.invh, f.ns), f.vb, f.ve,
                             [&](double& a, double& b) {
                               a = px;
