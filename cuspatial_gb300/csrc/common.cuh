@@ -517,14 +517,18 @@ __device__ inline uint16_t cell_of_quotient(double t, double s, double r)
     if (frac > mg && frac < (1ull << sh) - mg) return static_cast<uint16_t>(m >> sh);
     uint32_t const k = static_cast<uint32_t>((m + (1ull << (sh - 1))) >> sh);
     // k >= 1; s at or above 2^-900, so that nothing below underflows
-    if (k < 65536u &&
-        static_cast<unsigned long long>(__double_as_longlong(s)) >= 0x07B0000000000000ull) {
-      double const kd = __uint2double_rn(k);
-      // 2^(E-53), or 2^(E-54) below a power of two, with E k's exponent
+    unsigned long long const sb = static_cast<unsigned long long>(__double_as_longlong(s));
+    if (k < 65536u && sb >= 0x07B0000000000000ull && sb < 0x7FF0000000000000ull) {
+      // everything but the fma on the integer pipe (the float64 pipe bounds the
+      // keys): -k by its bits; h = 2^(E-53), or 2^(E-54) below a power of two,
+      // with E k's exponent, so -s h is s with its exponent lowered, negative
       int const E    = 31 - __clz(k);
-      int const hexp = (k & (k - 1u)) ? E - 53 : E - 54;
-      double const h = __longlong_as_double(static_cast<long long>(hexp + 1023) << 52);
-      double const d = __fma_rn(-kd, s, t), limit = -(s * h);
+      int const hexp = (k & (k - 1u)) ? 53 - E : 54 - E;
+      double const nk = __longlong_as_double(static_cast<long long>(
+        (static_cast<unsigned long long>(E + 1023 + 2048) << 52) |
+        ((static_cast<unsigned long long>(k) << (52 - E)) & ((1ull << 52) - 1ull))));
+      long long const d     = ordered_bits(__fma_rn(nk, s, t));
+      long long const limit = -static_cast<long long>(sb - (static_cast<unsigned long long>(hexp) << 52));
       if (d > limit) return static_cast<uint16_t>(k);
       if (d < limit) return static_cast<uint16_t>(k - 1u);
     }

@@ -8,6 +8,7 @@
 // contiguous segments in place (tiles never cross a segment boundary).
 #pragma once
 
+#include <algorithm>
 #include <vector>
 
 #include "common.cuh"
@@ -23,6 +24,7 @@ constexpr int kSortWarps = kSortBlock / 32;
 constexpr int kSortRound = 8;
 constexpr int kSortTile  = kSortBlock * kSortRound;
 constexpr unsigned kNoDigit = 0xFFFFu;
+constexpr uint32_t kNoItem  = 0xFFFFFFFFu;
 
 // Where a tile's items lie and where its digit counts go.
 // PlainTiles: fixed tiles over [0, n); counts digit-major over all tiles, so
@@ -63,32 +65,49 @@ struct SegmentTiles {
   }
 };
 
+// Digit counts of the tiles.  A block takes tile after tile, the next tile's keys
+// loading while this one's are counted: one tile a block left the kernel waiting
+// for its loads (50M keys: 116 us a pass, 59 this way).
 template <typename K, typename Tiles>
 __global__ void __launch_bounds__(kSortBlock)
-  radix_histogram_kernel(K const* keys, Tiles tiles, int shift, unsigned mask, uint32_t* counts)
+  radix_histogram_kernel(K const* keys, Tiles tiles, unsigned ntiles, int shift, unsigned mask,
+                         uint32_t* counts)
 {
   __shared__ uint32_t hist[kSortWarps][256];
-  for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortBlock) (&hist[0][0])[i] = 0;
-  __syncthreads();
   int const warp = threadIdx.x >> 5;
   int const lane = threadIdx.x & 31;
-  size_t tb, te;
-  tiles.range(blockIdx.x, tb, te);
-  size_t const base = tb + warp * (32 * kSortRound);
+  K key[kSortRound];
+  unsigned valid = 0;  // rounds with a key
+  auto const load = [&](unsigned t) {
+    size_t tb, te;
+    tiles.range(t, tb, te);
+    size_t const base = tb + warp * (32 * kSortRound) + lane;
+    valid             = 0;
 #pragma unroll
-  for (int r = 0; r < kSortRound; ++r) {
-    size_t const i = base + r * 32 + lane;
-    if (i < te) {
-      unsigned const d = static_cast<unsigned>((keys[i] >> shift) & mask);
-      atomicAdd(&hist[warp][d], 1u);
+    for (int r = 0; r < kSortRound; ++r) {
+      bool const ok = base + r * 32 < te;
+      key[r]        = ok ? keys[base + r * 32] : K{0};
+      valid |= ok ? 1u << r : 0u;
     }
-  }
-  __syncthreads();
-  for (int d = threadIdx.x; d < 256; d += kSortBlock) {
+  };
+  if (blockIdx.x < ntiles) load(blockIdx.x);
+  for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortBlock) (&hist[0][0])[i] = 0;
+    unsigned d[kSortRound];
+    unsigned const own = valid;
+#pragma unroll
+    for (int r = 0; r < kSortRound; ++r) d[r] = static_cast<unsigned>((key[r] >> shift) & mask);
+    if (t + gridDim.x < ntiles) load(t + gridDim.x);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kSortRound; ++r)
+      if ((own >> r) & 1u) atomicAdd(&hist[warp][d[r]], 1u);
+    __syncthreads();
     uint32_t s = 0;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) s += hist[w][d];
-    counts[tiles.slot(blockIdx.x, d)] = s;
+    for (int w = 0; w < kSortWarps; ++w) s += hist[w][threadIdx.x];
+    counts[tiles.slot(t, threadIdx.x)] = s;
+    __syncthreads();
   }
 }
 
@@ -97,18 +116,23 @@ static_assert(kSortBlock == 256, "the scatter assigns one thread per digit");
 // Stable scatter of one tile: items are ranked per warp with
 // __match_any_sync (rounds in input order), placed in shared memory in the
 // tile's digit order, then written out in that order, so the global writes
-// of each digit's run are contiguous.
+// of each digit's run are contiguous.  Bound by the shared-memory pipe and the
+// waits of few blocks: 50M pairs, four passes: 1657 us with keys and values
+// apart and 61 registers (four blocks an SM), 1423 us as here with six.
 template <typename K, typename Tiles>
-__global__ void __launch_bounds__(kSortBlock)
+__global__ void __launch_bounds__(kSortBlock, 6)
   radix_scatter_kernel(K const* keys_in, uint32_t const* vals_in, K* keys_out, uint32_t* vals_out,
                        Tiles tiles, int shift, unsigned mask, uint32_t const* offsets,
                        uint32_t iota_base)
 {
   __shared__ uint32_t wcount[kSortWarps][256];
-  __shared__ uint32_t tile_start[256];
-  __shared__ uint32_t global_base[256];
-  __shared__ K skey[kSortTile];
-  __shared__ uint32_t sval[kSortTile];
+  __shared__ uint32_t global_base[256];  // the digit's output start minus its tile start
+  // (32-bit keys beside their values: one 64-bit access for both; the shared
+  // memory pipe bounds the kernel)
+  constexpr bool kPacked = sizeof(K) == 4;
+  __shared__ K skey[kPacked ? 1 : kSortTile];
+  __shared__ uint32_t sval[kPacked ? 1 : kSortTile];
+  __shared__ uint2 spair[kPacked ? kSortTile : 1];
   __shared__ uint32_t total_s;
   for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortBlock) (&wcount[0][0])[i] = 0;
   __syncthreads();
@@ -120,23 +144,22 @@ __global__ void __launch_bounds__(kSortBlock)
   size_t const base    = tb + warp * (32 * kSortRound);
   K key[kSortRound];
   uint32_t val[kSortRound];
-  uint32_t pos[kSortRound];
-  unsigned dig[kSortRound];
+  uint32_t meta[kSortRound];  // digit | rank in the warp's digit << 8, kNoItem
 #pragma unroll
   for (int r = 0; r < kSortRound; ++r) {
     size_t const i = base + r * 32 + lane;
     bool const ok  = i < te;
     key[r]         = ok ? keys_in[i] : K{0};
     val[r]         = ok ? (vals_in ? vals_in[i] : static_cast<uint32_t>(i) + iota_base) : 0u;
-    dig[r]         = ok ? static_cast<unsigned>((key[r] >> shift) & mask) : kNoDigit;
-    unsigned const peers = __match_any_sync(0xFFFFFFFFu, dig[r]);
+    unsigned const dig   = ok ? static_cast<unsigned>((key[r] >> shift) & mask) : kNoDigit;
+    unsigned const peers = __match_any_sync(0xFFFFFFFFu, dig);
     unsigned const below = __popc(peers & lt);
     uint32_t prior       = 0;
-    if (ok) prior = wcount[warp][dig[r]];
-    pos[r] = prior + below;
+    if (ok) prior = wcount[warp][dig];
+    meta[r] = ok ? dig | ((prior + below) << 8) : kNoItem;
     __syncwarp();
     // the lowest lane of each digit group advances the warp's counter
-    if (ok && below == 0) wcount[warp][dig[r]] = prior + __popc(peers);
+    if (ok && below == 0) wcount[warp][dig] = prior + __popc(peers);
     __syncwarp();
   }
   __syncthreads();
@@ -146,32 +169,45 @@ __global__ void __launch_bounds__(kSortBlock)
     int const d    = threadIdx.x;  // kSortBlock == 256 digits
     uint32_t run   = 0;
 #pragma unroll
-    for (int w = 0; w < kSortWarps; ++w) {
+    for (int w = 0; w < kSortWarps; ++w) run += wcount[w][d];
+    uint32_t at = block_exclusive_scan<uint32_t, kSortBlock>(run, &total_s);
+    global_base[d] = offsets[tiles.slot(blockIdx.x, d)] - at;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {  // where the warp's items of the digit go
       uint32_t const c = wcount[w][d];
-      wcount[w][d]     = run;
-      run += c;
+      wcount[w][d]     = at;
+      at += c;
     }
-    uint32_t const start = block_exclusive_scan<uint32_t, kSortBlock>(run, &total_s);
-    tile_start[d]        = start;
-    global_base[d]       = offsets[tiles.slot(blockIdx.x, d)];
   }
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < kSortRound; ++r) {
-    if (dig[r] != kNoDigit) {
-      uint32_t const t = tile_start[dig[r]] + wcount[warp][dig[r]] + pos[r];
-      skey[t]          = key[r];
-      sval[t]          = val[r];
+    if (meta[r] != kNoItem) {
+      uint32_t const t = wcount[warp][meta[r] & 255u] + (meta[r] >> 8);
+      if constexpr (kPacked) {
+        spair[t] = make_uint2(static_cast<uint32_t>(key[r]), val[r]);
+      } else {
+        skey[t] = key[r];
+        sval[t] = val[r];
+      }
     }
   }
   __syncthreads();
   uint32_t const m = total_s;
   for (uint32_t t = threadIdx.x; t < m; t += kSortBlock) {
-    K const k        = skey[t];
-    unsigned const d = static_cast<unsigned>((k >> shift) & mask);
-    uint32_t const g = global_base[d] + (t - tile_start[d]);
+    K k;
+    uint32_t v;
+    if constexpr (kPacked) {
+      uint2 const p = spair[t];
+      k             = p.x;
+      v             = p.y;
+    } else {
+      k = skey[t];
+      v = sval[t];
+    }
+    uint32_t const g = global_base[static_cast<unsigned>((k >> shift) & mask)] + t;
     keys_out[g]      = k;
-    vals_out[g]      = sval[t];
+    vals_out[g]      = v;
   }
 }
 
@@ -207,7 +243,8 @@ bool radix_sort_tiles(K* keys, uint32_t* vals, K* keys_alt, uint32_t* vals_alt, 
     int const width     = end_bit - shift < 8 ? end_bit - shift : 8;
     unsigned const mask = (1u << width) - 1u;
     radix_histogram_kernel<K, Tiles>
-      <<<ntiles, kSortBlock, 0, s>>>(kin, tiles, shift, mask, counts.data());
+      <<<std::min(ntiles, sm_grid(8u)), kSortBlock, 0, s>>>(kin, tiles, ntiles, shift, mask,
+                                                            counts.data());
     CSPT_CHECK_LAUNCH();
     exclusive_scan<uint32_t>(counts.data(), counts.data(), static_cast<size_t>(ntiles) * 256,
                              static_cast<uint32_t*>(nullptr), alloc);
