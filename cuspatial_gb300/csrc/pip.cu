@@ -102,6 +102,23 @@ unsigned pair_grid(K kernel, unsigned block, size_t npairs)
   size_t const cap  = static_cast<size_t>(num_sms()) * static_cast<size_t>(per_sm);
   return static_cast<unsigned>(want < 1 ? 1 : (want < cap ? want : cap));
 }
+// Which side of edge e = (ax, ay, bx, by) a quadrant's point box lies on (centre
+// (cx, cy), half sides (hw, hh), widened by tol): 1 every point is left of the
+// edge's line (it toggles where its y-range holds the point's y), 2 right of it
+// (it never does), 0 the line may meet the box.  The filter's cross product is
+// beyond its error eb, on the same side, at every point of a box that the line
+// misses by more than eb, so the float64 expression agrees and no point is on the
+// edge.
+__device__ inline int box_side(float4 const& e, float cx, float cy, float hw, float hh, float tol,
+                               float eb)
+{
+  float const ex = e.z - e.x, ey = e.w - e.y;
+  float const cr = __fmaf_rn(cx - e.x, ey, -(ex * (cy - e.y)));
+  float const reach = __fmaf_rn(hw + tol, fabsf(ey), (hh + tol) * fabsf(ex));
+  if (!(fabsf(cr) > __fmaf_rn(reach, 1.001f, eb))) return 0;
+  return (cr < 0.0f) == (ey > 0.0f) ? 1 : 2;
+}
+
 // One warp per (polygon, quadrant) pair, lanes over the quadrant's points.
 // Filtered: float32 test in the leaf frame (bounds above), undecided points
 // re-evaluated with pip_exact.  Exact: pip_exact on float64 coordinates.
@@ -200,7 +217,9 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
       //     than tol and the edge rises by more than 2 tol, so the
       //     reference's float64 comparison is decided) -> a common parity;
       //   x entirely right, y partly: the toggle is the y-flags test alone;
-      //   x overlapping the box: the full per-point test.
+      //   x overlapping the box, but the edge's line misses it: as entirely
+      //     right or left, by the side the box lies on (box_side);
+      //   otherwise: the full per-point test.
       // Exactly vertical edges keep their x-only check (the vertical list).
       // (the ordered index, used by plans evaluated many times, keeps its
       // per-bin windows: its launches use small blocks that these per-warp
@@ -209,11 +228,16 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
       uint32_t base = 0, j0 = 0, jspan = 0, npart_all = 0;
       if constexpr (!Ordered) {
         if (!exact && mall * invh <= 16384.0f) {
+          float const eb  = __fmaf_rn(7.62939453125e-06f * mall, mall, 7.52316384526264e-37f);
+          float const qcx = 0.5f * (qxmin + qxmax), qhw = 0.5f * (qxmax - qxmin);
+          float const qcy = 0.5f * (qymin + qymax), qhh = 0.5f * (qymax - qymin);
           j0                  = slab_lookup(qymin, bx.y, invh, ns);
           uint32_t const j1   = slab_lookup(qymax, bx.y, invh, ns);
           jspan               = j1 - j0;
-          // Edge-free quadrant.  When no edge's box, widened by tol, meets
-          // the quadrant's point box [qxmin, qxmax] x [qymin, qymax] and no
+          // Edge-free quadrant.  When no edge meets the quadrant's point box
+          // [qxmin, qxmax] x [qymin, qymax] widened by tol (its own box beyond
+          // it, or its line missing it: a region that no edge of the closed
+          // rings enters has one parity) and no
           // exactly vertical edge lies within tol of its x-range, every
           // point of the quadrant gets the reference's result of any one of
           // them: no point can be on an edge (each edge is more than tol
@@ -238,7 +262,8 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
               if (kk < E1) {
                 float4 const e = ix.slab_e32[kk];
                 m = !(fmaxf(e.x, e.z) < qxmin - tol || fminf(e.x, e.z) > qxmax + tol ||
-                      fmaxf(e.y, e.w) < qymin - tol || fminf(e.y, e.w) > qymax + tol);
+                      fmaxf(e.y, e.w) < qymin - tol || fminf(e.y, e.w) > qymax + tol) &&
+                    box_side(e, qcx, qcy, qhw, qhh, tol, eb) == 0;
               }
               meets = __any_sync(0xFFFFFFFFu, m);
             }
@@ -257,7 +282,6 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
             if (!meets) {
               float2 const uv   = u[off];
               float const qx    = uv.x - dx, qy = uv.y - dy;
-              float const eb    = __fmaf_rn(7.62939453125e-06f * mall, mall, 7.52316384526264e-37f);
               uint32_t const jr = slab_lookup(qy, bx.y, invh, ns);
               uint32_t const R0 = ix.slab_start[slab0 + jr];
               uint32_t const R1 = ix.slab_start[slab0 + jr + 1];
@@ -346,9 +370,11 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
               float const eymin = fminf(e.y, e.w), eymax = fmaxf(e.y, e.w);
               int cls = 0;  // 0 none, 1 every point, 2 y-test, 3 full test
               if (has && !(exmax < qxmin - tol) && !(eymin > yhi + tol || eymax < ylo - tol)) {
-                if (exmin > qxmax + tol)
+                int const side =
+                  exmin > qxmax + tol ? 1 : box_side(e, qcx, qcy, qhw, qhh, tol, eb);
+                if (side == 1)
                   cls = (eymin < ylo - tol && eymax > yhi + tol) ? 1 : 2;
-                else
+                else if (side == 0)
                   cls = 3;
               }
               if (cls == 1) atomicXor(&s_base[wid], 1u << jj);
