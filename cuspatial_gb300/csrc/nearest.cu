@@ -110,6 +110,8 @@ struct LsBounds {
   float4 const* ls;
   float4 const* chunk;
   uint32_t slots;  // chunk boxes; offsets that leave them are not pruned by chunk
+  float2 const* vertex;  // the vertices to nearest float32 (exact method)
+  uint32_t nv;           // how many; offsets beyond are not pruned by segment
 };
 __host__ __device__ inline size_t chunk_slots(size_t nv, size_t nls)
 {
@@ -147,7 +149,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
   ls_bounds_kernel(uint32_t const* __restrict__ lso, size_t nls, T const* __restrict__ lx,
                    T const* __restrict__ ly, size_t slots, float4* __restrict__ ls_box,
-                   float4* __restrict__ chunk_box)
+                   float4* __restrict__ chunk_box, uint32_t nv, float2* __restrict__ vertex)
 {
   int const lane      = threadIdx.x & 31;
   size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -160,7 +162,12 @@ __global__ void __launch_bounds__(256)
     for (uint32_t c = lane; c * kSegChunk < nseg; c += 32) {
       BoundBox box;
       uint32_t const s0 = v0 + c * kSegChunk, s1 = min(s0 + kSegChunk, v0 + nseg);
-      for (uint32_t v = s0; v <= s1; ++v) box.add(lx[v], ly[v]);
+      for (uint32_t v = s0; v <= s1; ++v) {
+        T const x = lx[v], y = ly[v];
+        box.add(x, y);
+        if ((v < s1 || v + 1 == v1) && v < nv)
+          vertex[v] = make_float2(static_cast<float>(x), static_cast<float>(y));
+      }
       if (base + c < slots) chunk_box[base + c] = box.b;
       all.add(box.b);
     }
@@ -205,6 +212,33 @@ __device__ inline float box_lower(PointBounds const& p, float4 b)
   return __fsub_rd(lb, __fmaf_ru(D2, k32u, 7.52316384526264e-37f));
 }
 
+// An upper bound of the squared distance that the reference's expression gives
+// for a segment that starts at a vertex known to nearest float32: at most |p - v|^2
+// (its d0), the coordinates off by 2^-24 of their magnitude and the roundings of d0
+// and of this by less than 2^-20.  Infinite where a coordinate is not finite.
+__device__ inline float vertex_upper(PointBounds const& p, float2 v)
+{
+  float const dx = fmaxf(__fsub_ru(p.xu, v.x), __fsub_ru(v.x, p.xl));
+  float const dy = fmaxf(__fsub_ru(p.yu, v.y), __fsub_ru(v.y, p.yl));
+  float const ex = __fmaf_ru(fabsf(v.x), 1.1920928955078125e-07f, dx);  // 2^-23
+  float const ey = __fmaf_ru(fabsf(v.y), 1.1920928955078125e-07f, dy);
+  float const u  = __fmul_ru(__fadd_ru(__fmul_ru(ex, ex), __fmul_ru(ey, ey)), 1.000002f);
+  return u < INFINITY ? __fadd_ru(u, 1.0e-37f) : INFINITY;
+}
+
+// box_lower of a segment between two such vertices (not finite: a bound below
+// everything).
+template <typename T>
+__device__ inline float segment_lower(PointBounds const& p, float2 a, float2 b)
+{
+  float const ex = 1.1920928955078125e-07f * fmaxf(fabsf(a.x), fabsf(b.x));
+  float const ey = 1.1920928955078125e-07f * fmaxf(fabsf(a.y), fabsf(b.y));
+  if (!(ex < INFINITY && ey < INFINITY)) return -INFINITY;
+  return box_lower<T>(p, make_float4(__fsub_rd(fminf(a.x, b.x), ex), __fsub_rd(fminf(a.y, b.y), ey),
+                                     __fadd_ru(fmaxf(a.x, b.x), ex),
+                                     __fadd_ru(fmaxf(a.y, b.y), ey)));
+}
+
 // The running winner of the reference's fold, and the squared distance (in
 // float32, rounded up) beyond which a candidate's root is larger than the
 // winner's: such a candidate is not zero and never taken.  Nothing is passed
@@ -230,8 +264,9 @@ struct Fold {
   }
 };
 
-// point_linestring_distance.cuh:32-51 without the chunks that cannot change
-// the fold: those beyond `far`, and those beyond the smallest distance so far.
+// point_linestring_distance.cuh:32-51 without the chunks and segments that
+// cannot change the fold: those beyond `far`, and those beyond the smallest
+// distance so far.
 template <typename T>
 __device__ inline T linestring_distance(T px, T py, PointBounds const& pb, T const* lx,
                                         T const* ly, uint32_t v0, uint32_t v1,
@@ -243,14 +278,18 @@ __device__ inline T linestring_distance(T px, T py, PointBounds const& pb, T con
     if (pb.finite && slot + c < bounds.slots && box_lower<T>(pb, bounds.chunk[slot + c]) > far)
       continue;
     uint32_t const s0 = v0 + c * kSegChunk, s1 = min(s0 + kSegChunk, v0 + nseg);
-    T ax = lx[s0], ay = ly[s0];
+    bool const cull = pb.finite && s1 < bounds.nv;
+    float2 fa       = cull ? bounds.vertex[s0] : make_float2(0.0f, 0.0f);
     for (uint32_t s = s0; s < s1; ++s) {
-      T const bx = lx[s + 1], by = ly[s + 1];
-      ds = fmin(ds, segment_dist2<T>(px, py, ax, ay, bx, by));
-      ax = bx;
-      ay = by;
+      if (cull) {
+        float2 const fb = bounds.vertex[s + 1];
+        bool const out  = segment_lower<T>(pb, fa, fb) > far;
+        fa              = fb;
+        if (out) continue;
+      }
+      ds  = fmin(ds, segment_dist2<T>(px, py, lx[s], ly[s], lx[s + 1], ly[s + 1]));
+      far = fminf(far, float_up(ds));
     }
-    far = fminf(far, float_up(ds));
   }
   return sqrt(ds);
 }
@@ -258,8 +297,10 @@ __device__ inline T linestring_distance(T px, T py, PointBounds const& pb, T con
 // A lane per point; the candidates of its group in pair order.  `split` warps
 // share a group.  Bound by the float64 pipe (two lanes a cycle and SM) and, on
 // few points, by one warp's chain of candidates, hence the split.  20k points,
-// 301 linestrings of 2 to 64 segments: the call took 7652 us with every
-// candidate evaluated, 881 us with the boxes.
+// 301 linestrings of 2 to 64 segments: the kernel took 6960 us with every
+// candidate evaluated, 595 us with the boxes of linestrings and chunks, 280 us
+// with those of segments and the bound from the chunks' first vertices (the call
+// 7652, 881 and 572 us).
 template <typename T>
 __global__ void __launch_bounds__(256)
   nearest_kernel(uint32_t const* __restrict__ group_start, uint32_t const* __restrict__ ngroups_p,
@@ -288,15 +329,36 @@ __global__ void __launch_bounds__(256)
       T px, py;
       src.load(pos, px, py);
       PointBounds const pb = point_bounds<T>(px, py);
-      Fold<T> f;
-      for (uint32_t k = k0; k < k1; ++k) {
+      // No candidate beyond the distance to some chunk's first vertex can win,
+      // unless that vertex's linestring turns out at distance zero (or not a
+      // number), which the fold passes over: then the point is folded again
+      // without the bound.
+      float bound = INFINITY;
+      for (uint32_t k = k0; k < k1 && pb.finite; ++k) {
         uint32_t const lid = pair_ls[k];
-        if (lid >= nls) continue;
-        if (pb.finite && box_lower<T>(pb, bounds.ls[lid]) > f.far) continue;
-        uint32_t const v0 = lso[lid];
-        f.take(linestring_distance<T>(px, py, pb, lx, ly, v0, lso[lid + 1],
-                                      bounds, v0 / kSegChunk + lid, f.far),
-               lid);
+        if (lid >= nls || box_lower<T>(pb, bounds.ls[lid]) > bound) continue;
+        uint32_t const v0 = lso[lid], v1 = lso[lid + 1];
+        for (uint32_t v = v0; v + 1 < v1 && v < bounds.nv; v += kSegChunk)
+          bound = fminf(bound, vertex_upper(pb, bounds.vertex[v]));
+      }
+      Fold<T> f;
+      for (;;) {
+        f         = Fold<T>{};
+        f.far     = bound;
+        bool zero = false;
+        for (uint32_t k = k0; k < k1; ++k) {
+          uint32_t const lid = pair_ls[k];
+          if (lid >= nls) continue;
+          if (pb.finite && box_lower<T>(pb, bounds.ls[lid]) > f.far) continue;
+          uint32_t const v0 = lso[lid];
+          T const d = linestring_distance<T>(px, py, pb, lx, ly, v0, lso[lid + 1], bounds,
+                                             v0 / kSegChunk + lid, f.far);
+          f.take(d, lid);
+          f.far = fminf(f.far, bound);
+          zero |= !(d > T{0});
+        }
+        if (!zero || bound == INFINITY) break;
+        bound = INFINITY;
       }
       if (f.have) {
         opt[pos] = static_cast<uint32_t>(pos);
@@ -1255,7 +1317,7 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       frames_timer.reset();
       LinestringIndexView liv{aix.data(),  aiy.data(),   maxoff.data(), cbox.data(),
                               sbox.data(), seg32.data(), lexact.data(), lrec.data()};
-      LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(slots)};
+      LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(slots), nullptr, 0u};
       // points folded whole, groups scanned, next group, float64 segment distances
       Buffer<unsigned long long> fb(alloc, 4);
       CSPT_CUDA_TRY(cudaMemsetAsync(fb.data(), 0, 4 * sizeof(unsigned long long), s));
@@ -1293,8 +1355,9 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
   CSPT_CUDA_TRY(cudaStreamSynchronize(s));
   size_t const ng = h[0], slots = chunk_slots(h[1], nls);
   Buffer<float4> ls_box(alloc, nls), chunk_box(alloc, slots);
+  Buffer<float2> vertex(alloc, h[1]);
   ls_bounds_kernel<T><<<grid_for(nls * 32, 256, sm_grid(32u)), 256, 0, s>>>(
-    lso, nls, lx, ly, slots, ls_box.data(), chunk_box.data());
+    lso, nls, lx, ly, slots, ls_box.data(), chunk_box.data(), h[1], vertex.data());
   CSPT_CHECK_LAUNCH();
   {
     KernelTimer timer("nearest", s);
@@ -1305,8 +1368,8 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       ng == 0 ? 1 : std::min<size_t>(8, std::max<size_t>(1, fill / ng)));
     nearest_kernel<T><<<grid_for(ng * split * 32, 256, sm_grid(32u)), 256, 0, s>>>(
       gs, gs + npairs, npairs, split, pair_ls, pair_quad, tree->length, qoff, src, npi, lso, nls,
-      lx, ly, LsBounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots)}, opt, ols,
-      od);
+      lx, ly, LsBounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots), vertex.data(), h[1]},
+      opt, ols, od);
     CSPT_CHECK_LAUNCH();
   }
 }
