@@ -180,7 +180,14 @@ __device__ inline bool walk(TreeView const& t, BoxTree<T> const& bt, T bminx, T 
 }
 
 constexpr int kJoinWarps = 4;       // warps per block
-constexpr int kWarpStack = 2048;    // stack entries per warp (shared memory)
+// Stack entries per warp (shared memory).  A round takes as many nodes as leave
+// room for four children each and for a walk node by node from there (three more
+// entries a level), so that a small stack does not overflow on a quadtree: with
+// 32 nodes every round 2048 entries were needed, and their 8 KB a warp held the
+// kernel to seven blocks an SM.
+constexpr int kWarpStack   = 512;
+constexpr int kStackSpare  = 64;
+constexpr uint32_t kFoundRoom = 96;  // pairs held per warp before they are appended
 
 // Where the count pass appends each (node, box) it finds, in any order, while
 // fewer than `cap` have been found (`n` counts them all, also past cap).
@@ -194,11 +201,12 @@ struct JoinAppend {
 // One warp per box.  Each round pops up to 32 entries (node << 4 | depth)
 // from the warp's shared stack, one per lane, classifies them, counts or
 // writes the leaves with a ballot, and pushes the children of internal nodes
-// (warp scan of the child counts).  If the stack would overflow the warp
+// (warp scan of the child counts).  If the stack would overflow (nodes of more
+// than four children) the warp
 // restarts the box on lane 0 with the private-stack walk above.  Seeds (the
 // level-0 nodes) are fed 32 at a time whenever the stack runs empty.
 template <typename T, bool Write, typename Trees>
-__global__ void __launch_bounds__(kJoinWarps * 32)
+__global__ void __launch_bounds__(kJoinWarps * 32, 10)
   join_warp_kernel(TreeView t, Trees trees, T const* __restrict__ bminx,
                    T const* __restrict__ bminy, T const* __restrict__ bmaxx,
                    T const* __restrict__ bmaxy, size_t nb, uint32_t* __restrict__ counts,
@@ -208,7 +216,26 @@ __global__ void __launch_bounds__(kJoinWarps * 32)
                    int* __restrict__ error, JoinAppend app = JoinAppend{nullptr, nullptr, nullptr, 0})
 {
   __shared__ uint32_t stack_s[kJoinWarps][kWarpStack];
+  // pairs found and not appended yet (one atomic a flush: one a round took about
+  // a third of the count pass of 100k boxes)
+  __shared__ uint2 found_s[Write ? 1 : kJoinWarps][Write ? 1 : kFoundRoom];
   uint32_t* stack      = stack_s[threadIdx.x >> 5];
+  uint2* const pending = found_s[Write ? 0 : threadIdx.x >> 5];
+  uint32_t held        = 0;
+  auto const flush     = [&] {
+    __syncwarp();
+    unsigned long long at = 0;
+    if ((threadIdx.x & 31) == 0) at = atomicAdd(app.n, static_cast<unsigned long long>(held));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    for (uint32_t i = threadIdx.x & 31; i < held; i += 32) {
+      if (at + i < app.cap) {
+        app.node[at + i] = pending[i].x;
+        app.box[at + i]  = pending[i].y;
+      }
+    }
+    held = 0;
+    __syncwarp();
+  };
   int const lane       = threadIdx.x & 31;
   unsigned const lt    = (1u << lane) - 1u;
   size_t const nwarps  = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -229,7 +256,9 @@ __global__ void __launch_bounds__(kJoinWarps * 32)
     while (sp > 0 || seed < L0) {
       uint32_t e     = 0;
       bool have      = false;
-      int const take = sp > 0 ? (sp < 32 ? sp : 32) : 0;
+      int const room = (kWarpStack - kStackSpare - sp) / 3;
+      int const want = room < 1 ? 1 : (room < 32 ? room : 32);
+      int const take = sp < want ? sp : want;
       if (take > 0) {
         if (lane < take) {
           e    = stack[sp - 1 - lane];
@@ -259,16 +288,10 @@ __global__ void __launch_bounds__(kJoinWarps * 32)
       }
       unsigned const leaves = __ballot_sync(0xFFFFFFFFu, c == 0);
       if (!Write && app.n && leaves) {
-        unsigned long long at = 0;
-        if (lane == 0) at = atomicAdd(app.n, static_cast<unsigned long long>(__popc(leaves)));
-        at = __shfl_sync(0xFFFFFFFFu, at, 0);
-        if (c == 0) {
-          unsigned long long const d = at + __popc(leaves & lt);
-          if (d < app.cap) {
-            app.node[d] = g;
-            app.box[d]  = static_cast<uint32_t>(b);
-          }
-        }
+        if (c == 0)
+          pending[held + __popc(leaves & lt)] = make_uint2(g, static_cast<uint32_t>(b));
+        held += __popc(leaves);
+        if (held > kFoundRoom - 32) flush();
       }
       if (c == 0) {
         uint32_t const key = bt.pt_base + t.offset[g];
@@ -331,6 +354,7 @@ __global__ void __launch_bounds__(kJoinWarps * 32)
     if (!Write && lane == 0) counts[b] = found;
   }
   if (!Write) {
+    if (held) flush();
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) {
       uint32_t const o = __shfl_xor_sync(0xFFFFFFFFu, local_max, off);
