@@ -184,8 +184,7 @@ class ScratchArena {
       free_[c].pop_back();
       return p;
     }
-    if (end_ - at_ < static_cast<ptrdiff_t>(size) && !grow()) return nullptr;
-    if (end_ - at_ < static_cast<ptrdiff_t>(size)) return nullptr;
+    if (end_ - at_ < static_cast<ptrdiff_t>(size) && !grow(size)) return nullptr;
     void* const p = at_;
     at_ += size;
     return p;
@@ -206,19 +205,21 @@ class ScratchArena {
   }
 
  private:
-  static constexpr size_t kMinBlock = 256, kMaxBlock = size_t{1} << 20;
-  static constexpr int kClasses = 13, kMaxSlabs = 8;
-  static constexpr size_t kFirstSlab = size_t{2} << 20, kLastSlab = size_t{16} << 20;
+  static constexpr size_t kMinBlock = 256, kMaxBlock = size_t{4} << 20;
+  static constexpr int kClasses = 15, kMaxSlabs = 8;
+  static constexpr size_t kFirstSlab = size_t{2} << 20, kLastSlab = size_t{32} << 20;
+  static_assert(kMinBlock << (kClasses - 1) == kMaxBlock && kLastSlab >= kMaxBlock, "sizes");
   static int size_class(size_t bytes)
   {
     int c = 0;
     while ((kMinBlock << c) < bytes) ++c;
     return c;
   }
-  bool grow()
+  bool grow(size_t least)
   {
     if (nslabs_ == kMaxSlabs) return false;
-    size_t const want = nslabs_ == 0 ? kFirstSlab : slabs_[nslabs_ - 1].bytes * 2;
+    size_t const next = nslabs_ == 0 ? kFirstSlab : slabs_[nslabs_ - 1].bytes * 2;
+    size_t const want = next < least ? least : next;
     size_t const size = want < kLastSlab ? want : kLastSlab;
     void* p           = nullptr;
     try {
