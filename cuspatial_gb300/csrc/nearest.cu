@@ -295,7 +295,8 @@ __device__ inline T linestring_distance(T px, T py, PointBounds const& pb, T con
 }
 
 // A lane per point; the candidates of its group in pair order.  `split` warps
-// share a group.  Bound by the float64 pipe (two lanes a cycle and SM) and, on
+// share a group.  `groups`: those that the filtered kernel left (which may have
+// left its bound in place of the distance), or all where it is null.  Bound by the float64 pipe (two lanes a cycle and SM) and, on
 // few points, by one warp's chain of candidates, hence the split.  20k points,
 // 301 linestrings of 2 to 64 segments: the kernel took 6960 us with every
 // candidate evaluated, 595 us with the boxes of linestrings and chunks, 280 us
@@ -303,7 +304,8 @@ __device__ inline T linestring_distance(T px, T py, PointBounds const& pb, T con
 // 7652, 881 and 572 us).
 template <typename T>
 __global__ void __launch_bounds__(256)
-  nearest_kernel(uint32_t const* __restrict__ group_start, uint32_t const* __restrict__ ngroups_p,
+  nearest_kernel(uint32_t const* __restrict__ groups, uint32_t const* __restrict__ count,
+                 uint32_t const* __restrict__ group_start, uint32_t const* __restrict__ ngroups_p,
                  size_t npairs, uint32_t split, uint32_t const* __restrict__ pair_ls,
                  uint32_t const* __restrict__ pair_quad, uint32_t const* __restrict__ qlen,
                  uint32_t const* __restrict__ qoff, PointSource<T> const src, size_t npi,
@@ -313,17 +315,19 @@ __global__ void __launch_bounds__(256)
 {
   int const lane       = threadIdx.x & 31;
   size_t const warps   = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
-  size_t const ngroups = *ngroups_p;
+  size_t const ngroups = *ngroups_p, n = *count;
   for (size_t t = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
-       t < ngroups * split; t += warps) {
-    size_t const g      = t / split;
-    uint32_t const part = static_cast<uint32_t>(t - g * split);
+       t < n * split; t += warps) {
+    // (all groups' first parts, then their second parts: leaves with few points
+    // have no later ones, and every warp must get its share of the first)
+    size_t const part = t / n, i = t - part * n;
+    size_t const g      = groups ? groups[i] : i;
     uint32_t const k0   = group_start[g];
     uint32_t const k1   = (g + 1 < ngroups) ? group_start[g + 1] : static_cast<uint32_t>(npairs);
     uint32_t const quad = pair_quad[k0];
     uint32_t const len  = qlen[quad];
     uint64_t const off  = qoff[quad];
-    for (uint32_t c = part * 32 + lane; c < len; c += 32 * split) {
+    for (uint32_t c = static_cast<uint32_t>(part) * 32 + lane; c < len; c += 32 * split) {
       uint64_t const pos = off + c;
       if (pos >= npi) continue;
       T px, py;
@@ -363,7 +367,130 @@ __global__ void __launch_bounds__(256)
       if (f.have) {
         opt[pos] = static_cast<uint32_t>(pos);
         ols[pos] = f.bid;
-        od[pos]  = f.bd;
+      }
+      if (f.have || groups) od[pos] = f.have ? f.bd : T{0};
+    }
+  }
+}
+
+// The reference's fold over every candidate of a group for one point, by the
+// whole warp: a lane per linestring tests its box, and those that may matter
+// are taken in pair order, a lane per segment.  (By one lane over every
+// segment, one point at distance zero among 5M cost 50 to 110 ms.)
+template <typename T>
+struct FoldArgs {
+  uint32_t const* pair_ls;
+  uint32_t const* lso;
+  size_t nls;
+  T const* lx;
+  T const* ly;
+  LsBounds bounds;
+};
+
+template <typename T>
+__device__ void fold_warp(FoldArgs<T> const& a, uint32_t k0, uint32_t k1, T px, T py,
+                          bool use_bound, Fold<T>& f)
+{
+  constexpr unsigned kAll = 0xFFFFFFFFu;
+  int const lane          = threadIdx.x & 31;
+  PointBounds const pb    = point_bounds<T>(px, py);
+  // the bound of nearest_kernel, from the chunks' first vertices
+  float bound = INFINITY;
+  for (uint32_t kb = k0; kb < k1 && use_bound && pb.finite; kb += 32) {
+    uint32_t const k   = kb + static_cast<uint32_t>(lane);
+    uint32_t const lid = k < k1 ? a.pair_ls[k] : 0xFFFFFFFFu;
+    if (k < k1 && lid < a.nls && !(box_lower<T>(pb, a.bounds.ls[lid]) > bound)) {
+      uint32_t const v1 = a.lso[lid + 1];
+      for (uint32_t v = a.lso[lid]; v + 1 < v1 && v < a.bounds.nv; v += kSegChunk)
+        bound = fminf(bound, vertex_upper(pb, a.bounds.vertex[v]));
+    }
+    // (not negative: ordered as integers)
+    bound = __uint_as_float(__reduce_min_sync(kAll, __float_as_uint(bound)));
+  }
+  for (;;) {
+    f         = Fold<T>{};
+    f.far     = bound;
+    bool zero = false;
+    for (uint32_t kb = k0; kb < k1; kb += 32) {
+      uint32_t const k   = kb + static_cast<uint32_t>(lane);
+      uint32_t const lid = k < k1 ? a.pair_ls[k] : 0xFFFFFFFFu;
+      bool const valid   = k < k1 && lid < a.nls;
+      float const lb     = valid && pb.finite ? box_lower<T>(pb, a.bounds.ls[lid]) : -INFINITY;
+      unsigned left      = __ballot_sync(kAll, valid);
+      for (;;) {
+        // the next in order that is not beyond the winner so far (which a zero
+        // distance or one that is not a number may give up again, so those
+        // beyond it are only passed over up to here)
+        unsigned const near = left & __ballot_sync(kAll, !(lb > f.far));
+        if (!near) break;
+        int const src = __ffs(near) - 1;
+        left &= ~((2u << src) - 1u);
+        uint32_t const l    = __shfl_sync(kAll, lid, src);
+        uint32_t const v0   = a.lso[l], v1 = a.lso[l + 1];
+        uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
+        uint32_t const slot = v0 / kSegChunk + l;
+        T ds                = std::numeric_limits<T>::max();
+        for (uint32_t s = lane; s < nseg; s += 32) {
+          uint32_t const c = slot + s / kSegChunk, v = v0 + s;
+          if (pb.finite && c < a.bounds.slots && box_lower<T>(pb, a.bounds.chunk[c]) > f.far)
+            continue;
+          if (pb.finite && v + 1 < a.bounds.nv &&
+              segment_lower<T>(pb, a.bounds.vertex[v], a.bounds.vertex[v + 1]) > f.far)
+            continue;
+          ds = fmin(ds, segment_dist2<T>(px, py, a.lx[v], a.ly[v], a.lx[v + 1], a.ly[v + 1]));
+        }
+        for (int o = 16; o > 0; o >>= 1) ds = fmin(ds, __shfl_xor_sync(kAll, ds, o));
+        T const d = sqrt(ds);
+        f.take(d, l);
+        f.far = fminf(f.far, bound);
+        zero |= !(d > T{0});
+      }
+    }
+    if (!zero || bound == INFINITY) break;
+    bound = INFINITY;
+  }
+}
+
+// nearest_kernel with a warp per point, for few points, whose lanes would leave
+// the GPU idle.
+template <typename T>
+__global__ void __launch_bounds__(256)
+  nearest_point_kernel(uint32_t const* __restrict__ groups, uint32_t const* __restrict__ count,
+                       uint32_t const* __restrict__ group_start,
+                       uint32_t const* __restrict__ ngroups_p, size_t npairs, uint32_t split,
+                       uint32_t const* __restrict__ pair_quad, uint32_t const* __restrict__ qlen,
+                       uint32_t const* __restrict__ qoff, PointSource<T> const src, size_t npi,
+                       FoldArgs<T> const a, uint32_t* __restrict__ opt,
+                       uint32_t* __restrict__ ols, T* __restrict__ od)
+{
+  int const lane       = threadIdx.x & 31;
+  size_t const warps   = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
+  size_t const ngroups = *ngroups_p, n = *count;
+  for (size_t t = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
+       t < n * split; t += warps) {
+    // (all groups' first parts, then their second parts: leaves with few points
+    // have no later ones, and every warp must get its share of the first)
+    size_t const part = t / n, i = t - part * n;
+    size_t const g      = groups ? groups[i] : i;
+    uint32_t const k0   = group_start[g];
+    uint32_t const k1   = g + 1 < ngroups ? group_start[g + 1] : static_cast<uint32_t>(npairs);
+    uint32_t const quad = pair_quad[k0];
+    uint32_t const len  = qlen[quad];
+    uint64_t const off  = qoff[quad];
+    for (uint32_t c = static_cast<uint32_t>(part); c < len; c += split) {
+      uint64_t const pos = off + c;
+      if (pos >= npi) break;
+      T px, py;
+      src.load(pos, px, py);
+      Fold<T> f;
+      fold_warp<T>(a, k0, k1, px, py, true, f);
+      if (lane == 0) {
+        if (f.have) {
+          opt[pos] = static_cast<uint32_t>(pos);
+          ols[pos] = f.bid;
+        }
+        // (the filtered kernel may have left its bound here)
+        od[pos] = f.have ? f.bd : T{0};
       }
     }
   }
@@ -466,7 +593,8 @@ __global__ void __launch_bounds__(256)
                  double const* __restrict__ gridp, uint8_t const* __restrict__ exact,
                  long long* aix, long long* aiy, float* maxoff, float4* chunk_box, float4* seg32,
                  LsRec* rec, size_t slots, float4* __restrict__ abs_ls,
-                 float4* __restrict__ abs_chunk, size_t sslots, float4* __restrict__ super_box)
+                 float4* __restrict__ abs_chunk, size_t sslots, float4* __restrict__ super_box,
+                 uint32_t nv, float2* __restrict__ vertex)
 {
   int const lane      = threadIdx.x & 31;
   size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
@@ -498,6 +626,11 @@ __global__ void __launch_bounds__(256)
         abs_box.add(lx[s0], ly[s0]);
         for (uint32_t sg = s0; sg < s1; ++sg) {
           abs_box.add(lx[sg + 1], ly[sg + 1]);
+          if (sg < nv)
+            vertex[sg] = make_float2(static_cast<float>(lx[sg]), static_cast<float>(ly[sg]));
+          if (sg + 2 == v1 && sg + 1 < nv)
+            vertex[sg + 1] =
+              make_float2(static_cast<float>(lx[sg + 1]), static_cast<float>(ly[sg + 1]));
           float4 e;
           e.x       = static_cast<float>(lx[sg] - cx);
           e.y       = static_cast<float>(ly[sg] - cy);
@@ -633,47 +766,9 @@ struct NearestArgs {
   double* od;
   unsigned long long* stats;  // [0] points folded over every candidate, [1] groups scanned whole
   unsigned long long* next_group;
+  uint32_t* left;   // groups that the listing cannot take
+  uint32_t* nleft;
 };
-
-// The reference's fold over every candidate of the group for one point, by the
-// whole warp: a lane per linestring tests its box, and those that may matter
-// are taken in pair order, a lane per segment.  (By one lane over every
-// segment, one point at distance zero among 5M cost 50 to 110 ms.)
-__device__ void fold_warp(NearestArgs const& a, uint32_t k0, uint32_t k1, double px, double py,
-                          Fold<double>& f)
-{
-  constexpr unsigned kAll = 0xFFFFFFFFu;
-  int const lane          = threadIdx.x & 31;
-  PointBounds const pb    = point_bounds<double>(px, py);
-  f                       = Fold<double>{};
-  for (uint32_t kb = k0; kb < k1; kb += 32) {
-    uint32_t const k = kb + static_cast<uint32_t>(lane);
-    uint32_t lid     = k < k1 ? a.pair_ls[k] : 0xFFFFFFFFu;
-    bool const valid = k < k1 && lid < a.nls;
-    float const lb   = valid && pb.finite ? box_lower<double>(pb, a.bounds.ls[lid]) : -INFINITY;
-    unsigned left    = __ballot_sync(kAll, valid);
-    for (;;) {
-      left &= __ballot_sync(kAll, !(lb > f.far));
-      if (!left) break;
-      int const src = __ffs(left) - 1;
-      left &= left - 1u;
-      uint32_t const l    = __shfl_sync(kAll, lid, src);
-      uint32_t const v0   = a.lso[l], v1 = a.lso[l + 1];
-      uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
-      uint32_t const slot = v0 / kSegChunk + l;
-      double ds           = std::numeric_limits<double>::max();
-      for (uint32_t s = lane; s < nseg; s += 32) {
-        uint32_t const c = slot + s / kSegChunk;
-        if (pb.finite && c < a.bounds.slots && box_lower<double>(pb, a.bounds.chunk[c]) > f.far)
-          continue;
-        uint32_t const v = v0 + s;
-        ds = fmin(ds, segment_dist2<double>(px, py, a.lx[v], a.ly[v], a.lx[v + 1], a.ly[v + 1]));
-      }
-      for (int o = 16; o > 0; o >>= 1) ds = fmin(ds, __shfl_xor_sync(kAll, ds, o));
-      f.take(sqrt(ds), l);
-    }
-  }
-}
 
 // Folds the points of the lanes that ask for it, one after the other.
 __device__ inline void fold_lanes(NearestArgs const& a, uint32_t k0, uint32_t k1, bool ask,
@@ -683,7 +778,10 @@ __device__ inline void fold_lanes(NearestArgs const& a, uint32_t k0, uint32_t k1
   for (unsigned m = __ballot_sync(0xFFFFFFFFu, ask); m; m &= m - 1u) {
     int const src = __ffs(m) - 1;
     Fold<double> f;
-    fold_warp(a, k0, k1, __shfl_sync(0xFFFFFFFFu, px, src), __shfl_sync(0xFFFFFFFFu, py, src), f);
+    // (mostly points at a zero distance, which would drop the bound again)
+    fold_warp<double>(FoldArgs<double>{a.pair_ls, a.lso, a.nls, a.lx, a.ly, a.bounds}, k0, k1,
+                      __shfl_sync(0xFFFFFFFFu, px, src), __shfl_sync(0xFFFFFFFFu, py, src), false,
+                      f);
     if (static_cast<int>(threadIdx.x & 31) == src) {
       ++nfb;
       have = f.have;
@@ -691,100 +789,6 @@ __device__ inline void fold_lanes(NearestArgs const& a, uint32_t k0, uint32_t k1
       bd   = f.bd;
     }
   }
-}
-
-// One point against every candidate linestring of its group, chunk by chunk:
-// pass 1 bounds the running minimum U with float32 estimates and chunk
-// pruning, pass 2 evaluates in float64 only the segments whose estimate can
-// reach U, then the fold; a point whose candidates reach only zero distances
-// (or none) is folded over every candidate (returns true).  Used for groups the
-// listing below cannot take.
-__device__ inline bool nearest_point_scan(NearestArgs const& a, uint32_t k0, uint32_t k1,
-                                          LeafFrame const& lf, uint64_t pos, bool gok,
-                                          double& px, double& py, bool& have, uint32_t& bid,
-                                          double& bd)
-{
-  LinestringIndexView const& li = a.li;
-  float const gf  = a.gf;
-  float2 const uv = a.u[pos];
-  bool full       = lf.nonfinite || !gok;
-  float U         = INFINITY;
-  for (uint32_t k = k0; k < k1 && !full; ++k) {
-    uint32_t const lid = a.pair_ls[k];
-    if (lid >= a.nls) continue;
-    long long const dix = li.aix[lid] - lf.ix, diy = li.aiy[lid] - lf.iy;
-    if (li.exact[lid] || dix <= -16777216LL || dix >= 16777216LL || diy <= -16777216LL ||
-        diy >= 16777216LL) {
-      full = true;
-      break;
-    }
-    float const qx  = uv.x - static_cast<float>(static_cast<int>(dix)) * gf;
-    float const qy  = uv.y - static_cast<float>(static_cast<int>(diy)) * gf;
-    float const m   = fmaxf(fmaxf(li.maxoff[lid], lf.m), fmaxf(fabsf(qx), fabsf(qy)));
-    float const dm  = 1.1920928955078125e-07f * m;  // 2 u32 M
-    float const tol = 4.76837158203125e-07f * m;
-    uint32_t const v0 = a.lso[lid], v1 = a.lso[lid + 1];
-    uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
-    uint32_t const cb   = v0 / kSegChunk + lid;
-    for (uint32_t ch = 0; ch * kSegChunk < nseg; ++ch) {
-      if (box_lb(qx, qy, li.chunk_box[cb + ch], tol) > U) continue;
-      uint32_t const s0 = v0 + ch * kSegChunk, s1 = min(s0 + kSegChunk, v0 + nseg);
-      for (uint32_t sg = s0; sg < s1; ++sg) {
-        float est, err;
-        seg_estimate(qx, qy, li.seg32[sg], dm, est, err);
-        U = fminf(U, est + err);
-      }
-    }
-  }
-  a.src.load(pos, px, py);
-  bool skipped = false, nonzero = false;
-  if (!full) {
-    // pass 2: float64 on every segment that can reach U (widened so that
-    // distances left out are larger even after the square root)
-    float const Uw = U * 1.0000000009313226f + 7.52316384526264e-37f;
-    for (uint32_t k = k0; k < k1; ++k) {
-      uint32_t const lid = a.pair_ls[k];
-      if (lid >= a.nls) continue;
-      long long const dix = li.aix[lid] - lf.ix, diy = li.aiy[lid] - lf.iy;
-      float const qx  = uv.x - static_cast<float>(static_cast<int>(dix)) * gf;
-      float const qy  = uv.y - static_cast<float>(static_cast<int>(diy)) * gf;
-      float const m   = fmaxf(fmaxf(li.maxoff[lid], lf.m), fmaxf(fabsf(qx), fabsf(qy)));
-      float const dm  = 1.1920928955078125e-07f * m;
-      float const tol = 4.76837158203125e-07f * m;
-      uint32_t const v0 = a.lso[lid], v1 = a.lso[lid + 1];
-      uint32_t const nseg = v1 > v0 + 1 ? v1 - v0 - 1 : 0;
-      uint32_t const cb   = v0 / kSegChunk + lid;
-      double dmin         = std::numeric_limits<double>::max();
-      bool evaluated      = false;
-      for (uint32_t ch = 0; ch * kSegChunk < nseg; ++ch) {
-        if (box_lb(qx, qy, li.chunk_box[cb + ch], tol) > Uw) continue;
-        uint32_t const s0 = v0 + ch * kSegChunk, s1 = min(s0 + kSegChunk, v0 + nseg);
-        for (uint32_t sg = s0; sg < s1; ++sg) {
-          float est, err;
-          seg_estimate(qx, qy, li.seg32[sg], dm, est, err);
-          if (est - err > Uw) continue;
-          dmin = fmin(dmin, segment_dist2<double>(px, py, a.lx[sg], a.ly[sg], a.lx[sg + 1],
-                                                  a.ly[sg + 1]));
-          evaluated = true;
-        }
-      }
-      if (!evaluated || !(dmin <= static_cast<double>(Uw))) {
-        skipped = true;  // farther than the best: cannot win
-        continue;
-      }
-      double const d = sqrt(dmin);
-      if (!have || take_rhs<double>(bd, bid, d, lid)) {
-        bid = lid;
-        bd  = d;
-      }
-      have = true;
-      nonzero |= d != 0.0;
-    }
-    // only zero distances among the candidates while others were left out:
-    // the winner is the nearest non-zero one, find it exactly
-    if (!have || (!nonzero && skipped)) full = true;
-  }
-  return full;
 }
 
 // The group's segment list (per warp, in shared memory): the candidate
@@ -1050,8 +1054,9 @@ __device__ inline bool seg_can_reach(NearList const& L, uint32_t t, float qx, fl
 //      that linestring, whose other segments may be unlisted) or none is
 //      folded over every candidate.
 // A group whose list overflows, or that meets a linestring outside the
-// float32 frames, a non-finite point or an unusable grid, is scanned whole
-// per point (nearest_point_scan).
+// float32 frames, a non-finite point or an unusable grid, is left to the exact
+// method's kernels, which spread it over several warps.  (Scanned by its own
+// warp, 1081 points of sparse leaves x 3190 linestrings took 11.5 ms.)
 __global__ void __launch_bounds__(kNearWarps * 32, 6)
   nearest_filtered_kernel(NearestArgs const a)
 {
@@ -1123,24 +1128,8 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
     }
     if (!listed) {
       __syncwarp();
+      if (lane == 0) a.left[atomicAdd(a.nleft, 1u)] = static_cast<uint32_t>(gi);
       ++nscan;
-      for (uint32_t c0 = 0; c0 < len; c0 += 32) {
-        uint64_t const pos = off + c0 + static_cast<uint32_t>(lane);
-        bool const act     = c0 + static_cast<uint32_t>(lane) < len && pos < a.npi;
-        double px = 0.0, py = 0.0, bd = 0.0;
-        bool have = false;
-        uint32_t bid    = 0;
-        bool const fold = act && nearest_point_scan(a, k0, k1, lf, pos, gok, px, py, have, bid, bd);
-        fold_lanes(a, k0, k1, fold, px, py, have, bid, bd, nfb);
-        if (act) {
-          if (have) {
-            a.opt[pos] = static_cast<uint32_t>(pos);
-            a.ols[pos] = bid;
-          }
-          a.od[pos] = have ? bd : 0.0;  // (step 2 may have left its bound here)
-        }
-      }
-      __syncwarp();
       continue;
     }
     float const dm  = 1.1920928955078125e-07f * mg;
@@ -1255,6 +1244,15 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
   }
 }
 
+// Up to this many points take a warp each (exact method, and the groups the
+// filtered kernel leaves).  Whole calls, a warp per point against a lane: 1081
+// points x 3190 linestrings 585 and 1234 us, 2000 x 20k 4.7 and 19.4 ms, 1620 x 72
+// 459 and 541 us; 5000 x 1000 1081 to 1422 and 998 to 1067 us, 20k x 301 2003 and
+// 715 us.
+constexpr size_t kWarpPoints = 4096;
+// warps that share a group: a warp per point, a lane per point
+constexpr uint32_t kPointSplit = 64, kLaneSplit = 8;
+
 template <typename T>
 void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
          cspt_quadtree const* tree, uint32_t const* point_indices, size_t npi, T const* x,
@@ -1298,11 +1296,13 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       size_t const sslots = super_slots(nv, nls);
       Buffer<float4> cbox(alloc, slots), seg32(alloc, nv), abs_ls(alloc, nls),
         abs_chunk(alloc, slots), sbox(alloc, sslots);
+      Buffer<float2> vertex(alloc, nv);
       Buffer<LsRec> lrec(alloc, nls);
       ls_fill_kernel<<<lgrd, 256, 0, s>>>(lso, nls, lx, ly, box.data(), grid.data(),
                                           lexact.data(), aix.data(), aiy.data(),
                                           maxoff.data(), cbox.data(), seg32.data(), lrec.data(),
-                                          slots, abs_ls.data(), abs_chunk.data(), sslots, sbox.data());
+                                          slots, abs_ls.data(), abs_chunk.data(), sslots, sbox.data(),
+                                          static_cast<uint32_t>(nv), vertex.data());
       CSPT_CHECK_LAUNCH();
       double const g = read_back(grid.data(), s);
       index_timer.reset();
@@ -1317,15 +1317,19 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       frames_timer.reset();
       LinestringIndexView liv{aix.data(),  aiy.data(),   maxoff.data(), cbox.data(),
                               sbox.data(), seg32.data(), lexact.data(), lrec.data()};
-      LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(slots), nullptr, 0u};
+      LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(slots),
+                            vertex.data(), static_cast<uint32_t>(nv)};
       // points folded whole, groups scanned, next group, float64 segment distances
-      Buffer<unsigned long long> fb(alloc, 4);
-      CSPT_CUDA_TRY(cudaMemsetAsync(fb.data(), 0, 4 * sizeof(unsigned long long), s));
+      // (and the groups left, as 32 bits)
+      Buffer<unsigned long long> fb(alloc, 5);
+      CSPT_CUDA_TRY(cudaMemsetAsync(fb.data(), 0, 5 * sizeof(unsigned long long), s));
+      Buffer<uint32_t> left(alloc, npairs);
+      uint32_t* const nleft = reinterpret_cast<uint32_t*>(fb.data() + 4);
       NearestArgs const na{gs,          gs + npairs,  npairs,     pair_ls,   pair_quad,
                            tree->length, qoff,        src,        npi,       lso,
                            nls,          lx,          ly,         u.data(),  frames.data(),
                            liv,          bounds,      static_cast<float>(g), opt, ols,    od,
-                           fb.data(),    fb.data() + 2};
+                           fb.data(),    fb.data() + 2, left.data(), nleft};
       KernelTimer timer("nearest", s);
       int per_sm = 0;
       if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nearest_filtered_kernel,
@@ -1337,6 +1341,15 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       nearest_filtered_kernel<<<grid_for(npairs * 32, kNearWarps * 32,
                                          sm_grid(static_cast<unsigned>(per_sm))),
                                 kNearWarps * 32, 0, s>>>(na);
+      CSPT_CHECK_LAUNCH();
+      if (npi <= kWarpPoints)
+        nearest_point_kernel<double><<<sm_grid(4u), 256, 0, s>>>(
+          left.data(), nleft, gs, gs + npairs, npairs, kPointSplit, pair_quad, tree->length, qoff,
+          src, npi, FoldArgs<double>{pair_ls, lso, nls, lx, ly, bounds}, opt, ols, od);
+      else
+        nearest_kernel<double><<<sm_grid(8u), 256, 0, s>>>(
+          left.data(), nleft, gs, gs + npairs, npairs, kLaneSplit, pair_ls, pair_quad,
+          tree->length, qoff, src, npi, lso, nls, lx, ly, bounds, opt, ols, od);
       CSPT_CHECK_LAUNCH();
       unsigned long long st[4];
       CSPT_CUDA_TRY(cudaMemcpyAsync(st, fb.data(), sizeof(st), cudaMemcpyDeviceToHost, s));
@@ -1359,15 +1372,25 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
   ls_bounds_kernel<T><<<grid_for(nls * 32, 256, sm_grid(32u)), 256, 0, s>>>(
     lso, nls, lx, ly, slots, ls_box.data(), chunk_box.data(), h[1], vertex.data());
   CSPT_CHECK_LAUNCH();
-  {
+  if (npi <= kWarpPoints) {
     KernelTimer timer("nearest", s);
-    // warps per group: enough for 16 warps on every SM, at most 8 (a leaf of
-    // 256 points has no more rounds of 32)
+    nearest_point_kernel<T><<<grid_for(npi * 32, 256, sm_grid(8u)), 256, 0, s>>>(
+      nullptr, gs + npairs, gs, gs + npairs, npairs, kPointSplit, pair_quad, tree->length, qoff,
+      src, npi,
+      FoldArgs<T>{pair_ls, lso, nls, lx, ly,
+                  LsBounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots),
+                           vertex.data(), h[1]}},
+      opt, ols, od);
+    CSPT_CHECK_LAUNCH();
+  } else {
+    KernelTimer timer("nearest", s);
+    // warps per group: enough for 16 warps on every SM, at most kLaneSplit (a
+    // leaf of 256 points has no more rounds of 32)
     size_t const fill    = static_cast<size_t>(num_sms()) * 16;
     uint32_t const split = static_cast<uint32_t>(
-      ng == 0 ? 1 : std::min<size_t>(8, std::max<size_t>(1, fill / ng)));
+      ng == 0 ? 1 : std::min<size_t>(kLaneSplit, std::max<size_t>(1, fill / ng)));
     nearest_kernel<T><<<grid_for(ng * split * 32, 256, sm_grid(32u)), 256, 0, s>>>(
-      gs, gs + npairs, npairs, split, pair_ls, pair_quad, tree->length, qoff, src, npi, lso, nls,
+      nullptr, gs + npairs, gs, gs + npairs, npairs, split, pair_ls, pair_quad, tree->length, qoff, src, npi, lso, nls,
       lx, ly, LsBounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots), vertex.data(), h[1]},
       opt, ols, od);
     CSPT_CHECK_LAUNCH();
