@@ -18,6 +18,7 @@
 // of instance i land at [row_offsets_i, row_offsets_{i+1}) with
 // instance-local polygon and point indices.
 #include <memory>
+#include <optional>
 #include <vector>
 
 #include "forest.cuh"
@@ -77,11 +78,15 @@ class BatchedPip {
              uint64_t const* h_poly_off, uint32_t const* po, size_t npo, uint32_t const* ro,
              size_t nro, double const* vx, double const* vy, size_t nv,
              cspt_instance_params const* params, cspt_method method, bool ordered, int block,
-             cspt_allocator const* mr, cudaStream_t stream)
+             cspt_allocator const* mr, cudaStream_t stream, bool arenas)
     : mr_copy_(mr ? *mr : cspt_allocator{}), alloc_(mr ? &mr_copy_ : nullptr, stream),
       palloc_(mr ? &mr_copy_ : nullptr, nullptr), ni_(ni), f_(alloc_)
   {
     try {
+      if (arenas) {
+        arena_.emplace(alloc_);
+        parena_.emplace(palloc_);
+      }
       plan(h_pt_off, x, y, h_poly_off, po, npo, ro, nro, vx, vy, nv, params, method, ordered,
            block);
     } catch (...) {
@@ -214,7 +219,7 @@ class BatchedPip {
     CSPT_EXPECTS(np_ + 1 <= npo, "polygon offsets do not cover the instances' polygons");
     f_.setup(ni_, h_pt_off, params, h_poly_off);
     uint32_t const ni = static_cast<uint32_t>(ni_);
-    row_off_          = Buffer<uint64_t>(a, ni_ + 1);
+    row_off_          = Buffer<uint64_t>(a, ni_ + 1, OutputBuffer{});
     bool const filtered = method == CSPT_METHOD_FILTERED;
     // the ordered index's windows serve small blocks; the one-shot index's
     // quadrant fast path keeps per-warp lists sized for blocks of 256
@@ -228,7 +233,7 @@ class BatchedPip {
     // aligned with the polygons (empty geometries shift rows).
     if (np_ > 0) {
       poly_stream_ = library_stream();
-      palloc_      = Allocator(alloc_.resource(), poly_stream_);
+      palloc_.set_stream(poly_stream_);
       stream_wait(poly_stream_, s);  // the polygon columns were written on s
       Allocator const& pa = palloc_;
       bminx_              = Buffer<double>(pa, np_);
@@ -267,8 +272,8 @@ class BatchedPip {
     // one evaluation sizes the outputs
     pip_->evaluate(s);
     m_  = read_back(pip_->total(), s);
-    op_ = Buffer<uint32_t>(a, m_);
-    oq_ = Buffer<uint32_t>(a, m_);
+    op_ = Buffer<uint32_t>(a, m_, OutputBuffer{});
+    oq_ = Buffer<uint32_t>(a, m_, OutputBuffer{});
     evaluated_ = true;
   }
 
@@ -325,6 +330,10 @@ class BatchedPip {
   cspt_allocator mr_copy_;
   Allocator alloc_;
   Allocator palloc_;  // the polygon side's memory, ordered on poly_stream_
+  // The plan's memory comes from slabs that live as long as it does, but for what
+  // info() hands out.  A block freed while planning is reused on the plan's stream
+  // only, and the plan waits for that before it ends.
+  std::optional<ScratchArena> arena_, parena_;
   cudaStream_t poly_stream_ = nullptr;  // library_stream(), not owned
   size_t ni_;
   Forest f_;
@@ -375,13 +384,23 @@ cspt_status cspt_batched_pip_plan(size_t num_instances, const uint64_t* point_of
                  "block_threads must be a multiple of 32 in [32, 256]");
     CSPT_EXPECTS(point_offsets[0] == 0 && polygon_offsets[0] == 0,
                  "instance offsets must start at 0");
-    *out_plan = reinterpret_cast<cspt_batched_pip*>(new BatchedPip(
-      num_instances, point_offsets, static_cast<double const*>(x),
-      static_cast<double const*>(y), polygon_offsets, poly_offsets, num_poly_offsets,
-      ring_offsets, num_ring_offsets, static_cast<double const*>(poly_x),
-      static_cast<double const*>(poly_y), num_poly_vertices, params, method, ordered_index != 0,
-      block_threads, mr,
-      static_cast<cudaStream_t>(stream)));
+    auto const make = [&](bool arenas) {
+      return new BatchedPip(num_instances, point_offsets, static_cast<double const*>(x),
+                            static_cast<double const*>(y), polygon_offsets, poly_offsets,
+                            num_poly_offsets, ring_offsets, num_ring_offsets,
+                            static_cast<double const*>(poly_x),
+                            static_cast<double const*>(poly_y), num_poly_vertices, params, method,
+                            ordered_index != 0, block_threads, mr,
+                            static_cast<cudaStream_t>(stream), arenas);
+    };
+    BatchedPip* plan = nullptr;
+    try {
+      plan = make(true);
+    } catch (Error const& e) {  // a plan that fits without slabs still does
+      if (e.status != CSPT_OUT_OF_MEMORY) throw;
+      plan = make(false);
+    }
+    *out_plan = reinterpret_cast<cspt_batched_pip*>(plan);
   });
 }
 

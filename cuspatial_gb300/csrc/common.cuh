@@ -145,6 +145,8 @@ class Allocator {
   }
   cudaStream_t stream() const { return stream_; }
   cspt_allocator const* resource() const { return mr_; }
+  // before the first allocation
+  void set_stream(cudaStream_t stream) { stream_ = stream; }
 
  private:
   friend class ScratchArena;

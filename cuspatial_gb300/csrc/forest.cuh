@@ -300,7 +300,7 @@ class Forest {
     Allocator const& a   = *alloc_;
     cudaStream_t const s = a.stream();
     size_t const n       = n_;
-    node_off_            = Buffer<uint64_t>(a, ni_ + 1);
+    node_off_            = Buffer<uint64_t>(a, ni_ + 1, OutputBuffer{});
     if (n == 0) {
       CSPT_CUDA_TRY(cudaMemsetAsync(node_off_.data(), 0, (ni_ + 1) * 8, s));
       return;
@@ -342,7 +342,7 @@ class Forest {
     unsigned const ntiles = static_cast<unsigned>(sort_tiles_.size());
     ForestTiles const tiles{sort_tiles_.data(), inst_.data(), kb};
     size_t const cells = static_cast<size_t>(ntiles) * kNodeLevels;
-    pidx_              = Buffer<uint32_t>(a, n);
+    pidx_              = Buffer<uint32_t>(a, n, OutputBuffer{});
     Buffer<uint8_t> codes(a, n);
     Buffer<uint32_t> rows(a, cells), total(a, 2);  // nodes, error flag
     CSPT_CUDA_TRY(cudaMemsetAsync(total.data(), 0, 2 * sizeof(uint32_t), s));
@@ -364,12 +364,13 @@ class Forest {
     CSPT_CUDA_TRY(cudaStreamSynchronize(s));
     CSPT_EXPECTS(h[1] == 0, kTooMany);
     size_t const q = q_ = h[0];
-    key_      = Buffer<uint32_t>(a, q);
-    length_   = Buffer<uint32_t>(a, q);
-    offset_   = Buffer<uint32_t>(a, q);
+    OutputBuffer const out_tag;
+    key_      = Buffer<uint32_t>(a, q, out_tag);
+    length_   = Buffer<uint32_t>(a, q, out_tag);
+    offset_   = Buffer<uint32_t>(a, q, out_tag);
     goff_     = Buffer<uint32_t>(a, q);
-    level_    = Buffer<uint8_t>(a, q);
-    internal_ = Buffer<uint8_t>(a, q);
+    level_    = Buffer<uint8_t>(a, q, out_tag);
+    internal_ = Buffer<uint8_t>(a, q, out_tag);
     write_nodes<K>(sk.data(), tiles, ntiles, codes.data(), rows.data(),
                    NodeColumns{key_.data(), level_.data(), internal_.data(), length_.data(),
                                offset_.data(), goff_.data()},
