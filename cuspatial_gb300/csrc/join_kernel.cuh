@@ -54,12 +54,10 @@ struct OneTree {
 // intersection.cuh:104-128; the node corners are v_min + k * level_scale,
 // which the reference's build contracts into one FMA.
 template <typename T>
-__device__ inline int classify(TreeView const& t, uint32_t node, T bminx, T bminy, T bmaxx,
+__device__ inline int classify(uint32_t key, int lev, bool internal, T bminx, T bminy, T bmaxx,
                                T bmaxy, T vminx, T vminy, T scale, int max_depth)
 {
-  uint32_t const key = t.key[node];
-  int const lev      = t.level[node];
-  int const sh       = max_depth - 1 - lev;
+  int const sh = max_depth - 1 - lev;
   if (sh < 0) return 2;
   T const kx  = static_cast<T>(gather16(key));
   T const ky  = static_cast<T>(gather16(key >> 1));
@@ -69,7 +67,7 @@ __device__ inline int classify(TreeView const& t, uint32_t node, T bminx, T bmin
   T const x1  = fma_rn(kx + T{1}, ls, vminx);
   T const y1  = fma_rn(ky + T{1}, ls, vminy);
   if (x0 > bmaxx || x1 < bminx || y0 > bmaxy || y1 < bminy) return 2;
-  return t.internal[node] ? 1 : 0;
+  return internal ? 1 : 0;
 }
 
 // float32 pre-classification of a node for float64 trees.  The reference's
@@ -132,20 +130,30 @@ __device__ inline int classify_float(uint32_t key, int sh, FloatBox const& f)
   return -1;
 }
 
+// A node's columns, loaded together: the walk is a chain of rounds, and reading
+// the type and the children only once the box test passed made each round three
+// loads long.
+struct NodeFields {
+  uint32_t key, level, internal, length, offset;
+};
+__device__ inline NodeFields load_node(TreeView const& t, uint32_t node)
+{
+  return NodeFields{t.key[node], t.level[node], t.internal[node], t.length[node], t.offset[node]};
+}
+
 template <typename T>
-__device__ inline int classify_filtered(TreeView const& t, uint32_t node, FloatBox const& f,
-                                        T bminx, T bminy, T bmaxx, T bmaxy, T vminx, T vminy,
-                                        T scale, int max_depth)
+__device__ inline int classify_filtered(NodeFields const& n, FloatBox const& f, T bminx, T bminy,
+                                        T bmaxx, T bmaxy, T vminx, T vminy, T scale, int max_depth)
 {
   if constexpr (std::is_same<T, double>::value) {
-    uint32_t const key = t.key[node];
-    int const sh       = max_depth - 1 - t.level[node];
+    int const sh = max_depth - 1 - static_cast<int>(n.level);
     if (sh < 0) return 2;
-    int const c = classify_float(key, sh, f);
+    int const c = classify_float(n.key, sh, f);
     if (c == 2) return 2;
-    if (c == 1) return t.internal[node] ? 1 : 0;
+    if (c == 1) return n.internal ? 1 : 0;
   }
-  return classify<T>(t, node, bminx, bminy, bmaxx, bmaxy, vminx, vminy, scale, max_depth);
+  return classify<T>(n.key, static_cast<int>(n.level), n.internal != 0, bminx, bminy, bmaxx, bmaxy,
+                     vminx, vminy, scale, max_depth);
 }
 
 // Walks the tree for box b; calls emit(node) for every intersecting leaf.
@@ -164,8 +172,8 @@ __device__ inline bool walk(TreeView const& t, BoxTree<T> const& bt, T bminx, T 
       int const depth     = top & 15;
       if (node >= bt.nq) return false;
       uint32_t const g = bt.base + node;
-      int const c      = classify<T>(t, g, bminx, bminy, bmaxx, bmaxy, bt.vminx, bt.vminy,
-                                bt.scale, bt.max_depth);
+      int const c      = classify<T>(t.key[g], t.level[g], t.internal[g] != 0, bminx, bminy, bmaxx,
+                                bmaxy, bt.vminx, bt.vminy, bt.scale, bt.max_depth);
       if (c == 0) {
         emit(g);
       } else if (c == 1 && depth + 1 < bt.max_depth) {
@@ -180,13 +188,13 @@ __device__ inline bool walk(TreeView const& t, BoxTree<T> const& bt, T bminx, T 
 }
 
 constexpr int kJoinWarps = 4;       // warps per block
-// Stack entries per warp (shared memory).  A round takes as many nodes as leave
-// room for four children each and for a walk node by node from there (three more
-// entries a level), so that a small stack does not overflow on a quadtree: with
-// 32 nodes every round 2048 entries were needed, and their 8 KB a warp held the
-// kernel to seven blocks an SM.
-constexpr int kWarpStack   = 512;
-constexpr int kStackSpare  = 64;
+// Stack entries per warp (shared memory).  A round takes as many of the top 32
+// nodes as leave room for three more entries each on every level below them, so
+// that a quadtree's walk never overflows, and a wide one keeps its width (22 nodes
+// at depth 15).  With 32 nodes every round 2048 entries were needed, and their
+// 32 KB a block held the kernel to seven blocks an SM.  (512 entries are 10% faster
+// on small boxes, but leave a box over the whole tree 11 nodes a round.)
+constexpr int kWarpStack      = 1024;
 constexpr uint32_t kFoundRoom = 96;  // pairs held per warp before they are appended
 
 // Where the count pass appends each (node, box) it finds, in any order, while
@@ -206,7 +214,7 @@ struct JoinAppend {
 // restarts the box on lane 0 with the private-stack walk above.  Seeds (the
 // level-0 nodes) are fed 32 at a time whenever the stack runs empty.
 template <typename T, bool Write, typename Trees>
-__global__ void __launch_bounds__(kJoinWarps * 32, 10)
+__global__ void __launch_bounds__(kJoinWarps * 32, 8)
   join_warp_kernel(TreeView t, Trees trees, T const* __restrict__ bminx,
                    T const* __restrict__ bminy, T const* __restrict__ bmaxx,
                    T const* __restrict__ bmaxy, size_t nb, uint32_t* __restrict__ counts,
@@ -256,14 +264,15 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 10)
     while (sp > 0 || seed < L0) {
       uint32_t e     = 0;
       bool have      = false;
-      int const room = (kWarpStack - kStackSpare - sp) / 3;
-      int const want = room < 1 ? 1 : (room < 32 ? room : 32);
-      int const take = sp < want ? sp : want;
-      if (take > 0) {
-        if (lane < take) {
-          e    = stack[sp - 1 - lane];
-          have = true;
-        }
+      int take = 0;
+      if (sp > 0) {
+        if (lane < sp) e = stack[sp - 1 - lane];
+        int const below = bt.max_depth - static_cast<int>(e & 15u);  // levels, at least 1
+        unsigned const fits =
+          __ballot_sync(0xFFFFFFFFu, lane < sp && (lane == 0 || sp + 3 * (lane + 1) * below <=
+                                                                  kWarpStack));
+        take = ~fits ? __ffs(~fits) - 1 : 32;
+        have = lane < take;
         sp -= take;
       } else {
         uint32_t const s = seed + lane;
@@ -278,11 +287,13 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 10)
       int const depth     = e & 15;
       int c               = 2;
       uint32_t const g    = bt.base + node;
+      NodeFields f{};
       if (have) {
         if (node >= bt.nq) {
           bad = true;
         } else {
-          c = classify_filtered<T>(t, g, fbox, x0, y0, x1, y1, bt.vminx, bt.vminy, bt.scale,
+          f = load_node(t, g);
+          c = classify_filtered<T>(f, fbox, x0, y0, x1, y1, bt.vminx, bt.vminy, bt.scale,
                                    bt.max_depth);
         }
       }
@@ -294,7 +305,7 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 10)
         if (held > kFoundRoom - 32) flush();
       }
       if (c == 0) {
-        uint32_t const key = bt.pt_base + t.offset[g];
+        uint32_t const key = bt.pt_base + f.offset;
         if (Write) {
           uint32_t const d = p + __popc(leaves & lt);
           okey[d]          = key;
@@ -308,8 +319,8 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 10)
       found += __popc(leaves);
       uint32_t nchild = 0, first = 0;
       if (c == 1 && depth + 1 < bt.max_depth) {
-        first  = t.offset[g];
-        nchild = t.length[g];
+        first  = f.offset;
+        nchild = f.length;
       }
       uint32_t const incl  = warp_inclusive_scan(nchild);
       uint32_t const total = __shfl_sync(0xFFFFFFFFu, incl, 31);
