@@ -15,18 +15,34 @@
 // same order.
 // A node at traversal depth t is expanded only while t + 1 < max_depth, the
 // reference's loop bound (quadtree_bbox_filtering.cuh:118).
+#include <algorithm>
+#include <cstddef>
+
 #include "join_kernel.cuh"
 #include "radix_sort.cuh"
 
 namespace cspt {
 namespace {
 
-// Pairs the count pass may append (node + box, 8 bytes each): 64 per box, at
-// most 64 Mi pairs; a join with more runs the write pass instead.
-inline size_t join_append_capacity(size_t nb)
+// Pairs the count pass may append (node + box, 8 bytes each): 64 per box, or, for
+// few boxes over a large tree, all there can be up to 4 Mi; at most 64 Mi.  A join
+// with more runs the write pass instead.
+inline size_t join_append_capacity(size_t nb, size_t nodes)
 {
-  size_t const c = nb * 64;
+  size_t const all = nodes < (size_t{4} << 20) / nb ? nodes * nb : size_t{4} << 20;
+  size_t const c   = std::max(nb * 64, all);
   return c < (size_t{64} << 20) ? c : (size_t{64} << 20);
+}
+
+// Warps per box: as many as give every SM 32 warps, with at least 256 nodes of the
+// tree for each; the nodes four levels times as many are handed out.
+inline JoinSplit join_split(size_t nb, size_t nodes, uint32_t* failed)
+{
+  JoinSplit p{1u, 0, failed};
+  while (p.warps < 256u && nb * p.warps * 2 <= sm_grid(32u) && nodes >= p.warps * 512u)
+    p.warps *= 2;
+  while ((1u << (2 * p.level)) < 4u * p.warps) ++p.level;
+  return p;
 }
 
 // (leaf first-point offset << box_bits) | box of each appended pair.
@@ -47,6 +63,8 @@ struct JoinTotals {
   unsigned long long appended;
   uint32_t pairs;
   uint32_t level0;  // the tree's level-0 nodes
+  uint32_t failed;  // a walk by several warps per box gave up
+  uint32_t pad;
 };
 
 __global__ void count_level0_kernel(uint8_t const* __restrict__ level, size_t nq,
@@ -83,18 +101,26 @@ void run(cspt_quadtree const* tree, T const* bminx, T const* bminy, T const* bma
   unsigned const blk = kJoinWarps * 32;
   unsigned const grd = grid_for(nb * 32, blk, sm_grid(16u));
   // the count pass also appends each (node, box) it finds while they fit
-  size_t const cap = join_append_capacity(nb);
+  size_t const cap = join_append_capacity(nb, tree->num_nodes);
   Buffer<uint32_t> app_node(alloc, cap), app_box(alloc, cap);
-  {
+  auto const count = [&](JoinSplit const& split) {
     KernelTimer timer("join_count", s);
-    join_warp_kernel<T, false><<<grd, blk, 0, s>>>(
+    if (split.warps > 1u)
+      CSPT_CUDA_TRY(cudaMemsetAsync(counts.data(), 0, nb * sizeof(uint32_t), s));
+    unsigned const g = grid_for(nb * split.warps * 32, blk, sm_grid(16u));
+    join_warp_kernel<T, false><<<g, blk, 0, s>>>(
       tv, trees, bminx, bminy, bmaxx, bmaxy, nb, counts.data(), &tot->max_offset, nullptr,
       nullptr, nullptr, nullptr, err,
-      JoinAppend{app_node.data(), app_box.data(), &tot->appended, cap});
+      JoinAppend{app_node.data(), app_box.data(), &tot->appended, cap}, split);
     CSPT_CHECK_LAUNCH();
+    exclusive_scan<uint32_t>(counts.data(), counts.data(), nb, &tot->pairs, alloc);
+    return read_back(tot, s);
+  };
+  JoinTotals h = count(join_split(nb, tree->num_nodes, &tot->failed));
+  if (h.failed && h.error == 0) {  // (only nodes of more than four children)
+    CSPT_CUDA_TRY(cudaMemsetAsync(&tot->max_offset, 0, offsetof(JoinTotals, level0), s));
+    h = count(JoinSplit{1u, 0, nullptr});
   }
-  exclusive_scan<uint32_t>(counts.data(), counts.data(), nb, &tot->pairs, alloc);
-  JoinTotals const h = read_back(tot, s);
   size_t const k     = h.pairs;
   CSPT_EXPECTS(h.error == 0,
                "quadtree is malformed: a node index or child count is out of range");

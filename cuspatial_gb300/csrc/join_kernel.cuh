@@ -206,7 +206,18 @@ struct JoinAppend {
   size_t cap;
 };
 
-// One warp per box.  Each round pops up to 32 entries (node << 4 | depth)
+// Several warps per box (a power of two; 1: the whole walk is one warp's), for
+// boxes too few to fill the GPU.  Each of them walks the levels above `level`;
+// a node at `level`, and a leaf above it, belongs to the warp that its index
+// selects.  Counts are then added to (zero before).  A stack that would overflow
+// sets *failed: the pass is run again with one warp per box.
+struct JoinSplit {
+  uint32_t warps;
+  int level;
+  uint32_t* failed;
+};
+
+// One warp per box (or several, JoinSplit).  Each round pops up to 32 entries (node << 4 | depth)
 // from the warp's shared stack, one per lane, classifies them, counts or
 // writes the leaves with a ballot, and pushes the children of internal nodes
 // (warp scan of the child counts).  If the stack would overflow (nodes of more
@@ -221,7 +232,8 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 8)
                    uint32_t* __restrict__ maxkey,
                    uint32_t const* __restrict__ pos, uint32_t* __restrict__ okey,
                    uint32_t* __restrict__ onode, uint32_t* __restrict__ obox,
-                   int* __restrict__ error, JoinAppend app = JoinAppend{nullptr, nullptr, nullptr, 0})
+                   int* __restrict__ error, JoinAppend app = JoinAppend{nullptr, nullptr, nullptr, 0},
+                   JoinSplit const split = JoinSplit{1u, 0, nullptr})
 {
   __shared__ uint32_t stack_s[kJoinWarps][kWarpStack];
   // pairs found and not appended yet (one atomic a flush: one a round took about
@@ -248,8 +260,10 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 8)
   unsigned const lt    = (1u << lane) - 1u;
   size_t const nwarps  = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
   uint32_t local_max   = 0;
-  for (size_t b = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5; b < nb;
-       b += nwarps) {
+  for (size_t w = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5;
+       w < nb * split.warps; w += nwarps) {
+    size_t const b       = split.warps == 1u ? w : w / split.warps;
+    uint32_t const share = static_cast<uint32_t>(w) & (split.warps - 1u);
     T const x0 = bminx[b], y0 = bminy[b], x1 = bmaxx[b], y1 = bmaxy[b];
     BoxTree<T> const bt = trees(b);
     FloatBox const fbox = float_box<T>(x0, y0, x1, y1, bt.vminx, bt.vminy, bt.scale,
@@ -292,9 +306,13 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 8)
         if (node >= bt.nq) {
           bad = true;
         } else {
-          f = load_node(t, g);
-          c = classify_filtered<T>(f, fbox, x0, y0, x1, y1, bt.vminx, bt.vminy, bt.scale,
-                                   bt.max_depth);
+          bool const mine = depth > split.level || (node & (split.warps - 1u)) == share;
+          if (mine || depth < split.level) {
+            f = load_node(t, g);
+            c = classify_filtered<T>(f, fbox, x0, y0, x1, y1, bt.vminx, bt.vminy, bt.scale,
+                                     bt.max_depth);
+            if (!mine && c == 0) c = 2;
+          }
         }
       }
       unsigned const leaves = __ballot_sync(0xFFFFFFFFu, c == 0);
@@ -337,6 +355,10 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 8)
       if (lane == 0) atomicExch(error, 1);
       continue;
     }
+    if (overflow && split.warps > 1u) {
+      if (lane == 0) atomicExch(split.failed, 1u);
+      continue;
+    }
     if (overflow) {
       // rare: restart the box serially on lane 0.  The box's pairs appended
       // so far would repeat, so the appended set is given up (its count is
@@ -362,7 +384,12 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 8)
       }
       found = __shfl_sync(0xFFFFFFFFu, found, 0);
     }
-    if (!Write && lane == 0) counts[b] = found;
+    if (!Write && lane == 0) {
+      if (split.warps == 1u)
+        counts[b] = found;
+      else if (found)
+        atomicAdd(counts + b, found);
+    }
   }
   if (!Write) {
     if (held) flush();
