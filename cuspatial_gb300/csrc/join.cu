@@ -10,9 +10,9 @@
 // shared memory (join_kernel.cuh).  The count pass sizes the output and
 // appends every (node, box) it finds; a radix sort of the composite key
 // (leaf first-point offset, box) gives the reference's order.  When the
-// appended pairs would not fit, a write pass emits (leaf offset, node, box)
-// in box-major order and a stable radix sort by the leaf offset gives the
-// same order.
+// appended pairs would not fit, a write pass emits (leaf offset, box) in
+// box-major order, a stable radix sort by the leaf offset gives the same order,
+// and the nodes are looked up by their offsets.
 // A node at traversal depth t is expanded only while t + 1 < max_depth, the
 // reference's loop bound (quadtree_bbox_filtering.cuh:118).
 #include <algorithm>
@@ -54,6 +54,29 @@ __global__ void composite_key_kernel(uint32_t const* __restrict__ node,
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < k;
        i += static_cast<size_t>(gridDim.x) * blockDim.x)
     key[i] = (static_cast<uint64_t>(offset[node[i]]) << box_bits) | box[i];
+}
+
+// at[first point of a leaf] = the leaf's node + 1, over zeros; *shared is set where
+// two leaves begin at the same point.
+__global__ void leaf_at_kernel(TreeView t, uint32_t max_offset, uint32_t* __restrict__ at,
+                               uint32_t* __restrict__ shared)
+{
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < t.nq;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x) {
+    uint32_t const o = t.offset[i];
+    if (t.internal[i] || o > max_offset) continue;
+    if (atomicExch(at + o, static_cast<uint32_t>(i) + 1u) != 0u) *shared = 1u;
+  }
+}
+
+// Bound by the read of the sorted first points and the write of the nodes: equal
+// first points stand together, so the table is read from the L1 cache.
+__global__ void node_lookup_kernel(uint32_t const* __restrict__ first, size_t k,
+                                   uint32_t const* __restrict__ at, uint32_t* __restrict__ node)
+{
+  for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < k;
+       i += static_cast<size_t>(gridDim.x) * blockDim.x)
+    node[i] = at[first[i]] - 1u;
 }
 
 // What the count pass leaves for the host, read back in one copy.
@@ -153,15 +176,47 @@ void run(cspt_quadtree const* tree, T const* bminx, T const* bminy, T const* bma
   } else {
     app_node.reset();
     app_box.reset();
-    Buffer<uint32_t> key(alloc, k), key_alt(alloc, k), node(alloc, k), box(alloc, k),
-      perm(alloc, k), perm_alt(alloc, k);
-    {
+    Buffer<uint32_t> key(alloc, k), key_alt(alloc, k);
+    auto const write = [&](uint32_t* node, uint32_t* box) {
       KernelTimer timer("join_write", s);
       join_warp_kernel<T, true><<<grd, blk, 0, s>>>(tv, trees, bminx, bminy, bmaxx, bmaxy, nb,
                                                     nullptr, nullptr, counts.data(), key.data(),
-                                                    node.data(), box.data(), err);
+                                                    node, box, err);
       CSPT_CHECK_LAUNCH();
+    };
+    // Where every leaf has its own first point (any tree of the quadtree build) the
+    // boxes are sorted along with the first points and the nodes are looked up from
+    // the sorted first points, next to one another, in place of a random gather of
+    // both columns (0.52 ms for 43M pairs; a nearest-linestring call over 5M points and
+    // 20k linestrings 10.95 -> 10.51 ms).  The table has an entry per point up to the
+    // last leaf found; it is made for at most four entries per pair, so that its
+    // clearing costs less than the gather.
+    size_t const entries = static_cast<size_t>(h.max_offset) + 1;
+    bool lookup          = entries <= 4 * k;
+    Buffer<uint32_t> at;
+    if (lookup) {
+      at = Buffer<uint32_t>(alloc, entries + 1);
+      CSPT_CUDA_TRY(cudaMemsetAsync(at.data(), 0, (entries + 1) * sizeof(uint32_t), s));
+      leaf_at_kernel<<<grid_for(tree->num_nodes, 256, sm_grid(8u)), 256, 0, s>>>(
+        tv, h.max_offset, at.data(), at.data() + entries);
+      CSPT_CHECK_LAUNCH();
+      lookup = read_back(at.data() + entries, s) == 0;
     }
+    if (lookup) {
+      Buffer<uint32_t> ob_alt(alloc, k, OutputBuffer{});
+      write(nullptr, ob.data());
+      bool const alt = radix_sort_pairs<uint32_t>(key.data(), ob.data(), key_alt.data(),
+                                                  ob_alt.data(), k, 0, key_bits, false, alloc);
+      node_lookup_kernel<<<grid_for(k, 256, sm_grid(16u)), 256, 0, s>>>(
+        alt ? key_alt.data() : key.data(), k, at.data(), on.data());
+      CSPT_CHECK_LAUNCH();
+      *out_box  = (alt ? ob_alt : ob).release();
+      *out_node = on.release();
+      return;
+    }
+    at.reset();
+    Buffer<uint32_t> node(alloc, k), box(alloc, k), perm(alloc, k), perm_alt(alloc, k);
+    write(node.data(), box.data());
     bool const alt = radix_sort_pairs<uint32_t>(key.data(), perm.data(), key_alt.data(),
                                                 perm_alt.data(), k, 0, key_bits, true, alloc);
     gather_pairs_kernel<<<grid_for(k, 256, sm_grid(16u)), 256, 0, s>>>(

@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 8)
         if (Write) {
           uint32_t const d = p + __popc(leaves & lt);
           okey[d]          = key;
-          onode[d]         = g;
+          if (onode) onode[d] = g;
           obox[d]          = static_cast<uint32_t>(b);
         } else {
           local_max = key > local_max ? key : local_max;
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(kJoinWarps * 32, 8)
             uint32_t const key = bt.pt_base + t.offset[node];
             if (Write) {
               okey[q]  = key;
-              onode[q] = node;
+              if (onode) onode[q] = node;
               obox[q]  = static_cast<uint32_t>(b);
             } else {
               local_max = key > local_max ? key : local_max;
