@@ -213,9 +213,12 @@ __device__ inline float box_lower(PointBounds const& p, float4 b)
 }
 
 // An upper bound of the squared distance that the reference's expression gives
-// for a segment that starts at a vertex known to nearest float32: at most |p - v|^2
-// (its d0), the coordinates off by 2^-24 of their magnitude and the roundings of d0
-// and of this by less than 2^-20.  Infinite where a coordinate is not finite.
+// for a segment that starts at a vertex known to nearest float32, where it gives a
+// number: at most |p - v|^2 (its d0), the coordinates off by 2^-24 of their
+// magnitude and the roundings of d0 and of this by less than 2^-20.  Infinite where
+// v or the point is not finite.  Where the segment's other end is not finite, or its
+// squares overflow or underflow, the expression is not a number and the segment
+// gives no distance at all: whoever uses the bound asks holds_bound afterwards.
 __device__ inline float vertex_upper(PointBounds const& p, float2 v)
 {
   float const dx = fmaxf(__fsub_ru(p.xu, v.x), __fsub_ru(v.x, p.xl));
@@ -263,6 +266,18 @@ struct Fold {
     have = true;
   }
 };
+
+// Whether a fold that passed over what lies beyond `bound` is the whole fold's:
+// every linestring it took is at a positive distance, and its winner lies within
+// the bound, so what was passed over is beyond the winner.  (A fold of no
+// candidates holds too.)  The bound is above the square of any distance that it
+// comes from by 2^-19, so its own linestring passes.
+template <typename T>
+__device__ inline bool holds_bound(Fold<T> const& f, bool zero, float bound)
+{
+  if (bound == INFINITY || !f.have) return true;
+  return !zero && __fmul_rd(float_down(f.bd), float_down(f.bd)) < bound;
+}
 
 // point_linestring_distance.cuh:32-51 without the chunks and segments that
 // cannot change the fold: those beyond `far`, and those beyond the smallest
@@ -335,8 +350,8 @@ __global__ void __launch_bounds__(256)
       PointBounds const pb = point_bounds<T>(px, py);
       // No candidate beyond the distance to some chunk's first vertex can win,
       // unless that vertex's linestring turns out at distance zero (or not a
-      // number), which the fold passes over: then the point is folded again
-      // without the bound.
+      // number), which the fold passes over, or the vertex's segment gives no
+      // distance: then the point is folded again without the bound.
       float bound = INFINITY;
       for (uint32_t k = k0; k < k1 && pb.finite; ++k) {
         uint32_t const lid = pair_ls[k];
@@ -361,7 +376,7 @@ __global__ void __launch_bounds__(256)
           f.far = fminf(f.far, bound);
           zero |= !(d > T{0});
         }
-        if (!zero || bound == INFINITY) break;
+        if (holds_bound(f, zero, bound)) break;
         bound = INFINITY;
       }
       if (f.have) {
@@ -446,7 +461,7 @@ __device__ void fold_warp(FoldArgs<T> const& a, uint32_t k0, uint32_t k1, T px, 
         zero |= !(d > T{0});
       }
     }
-    if (!zero || bound == INFINITY) break;
+    if (holds_bound(f, zero, bound)) break;
     bound = INFINITY;
   }
 }
