@@ -563,7 +563,9 @@ __device__ inline bool tiny_bits(float a) { return ((__float_as_uint(a) >> 23) &
 //     toggles exactly when px is left of the edge.
 //   * Flags differ otherwise: cr = a_y b_x - a_x b_y in float32 against
 //     eb = 2 (t_x (|a_y| + |b_y|) + t_y (|a_x| + |b_x|)), above the offsets'
-//     errors, float32's roundings (2^-23 of each product) and float64's.
+//     errors, float32's roundings (2^-23 of each product) and float64's.  Offsets
+//     from about 2^64 on have products beyond float32: an infinite cr decides
+//     nothing (eb, 2^-20 of them, may still be finite).
 // Anything else, and any vertex with a coordinate that does not split (zero,
 // below 2^-100, 2^100 and above, non-finite), takes the reference's float64
 // edge test, which also finds the polygons that need the sequential walk
@@ -716,7 +718,7 @@ __global__ void __launch_bounds__(kPointsBlock, 5)
               float const cr = __fmaf_rn(fay, fbx, -(fax * fby));
               float const eb = 2.0f * __fmaf_rn(tx, fabsf(fay) + fabsf(fby),
                                                 ty * (fabsf(fax) + fabsf(fbx)));
-              und            = !(fabsf(cr) > eb);
+              und            = !(fabsf(cr) > eb && fabsf(cr) < INFINITY);
               tog            = !und && (cr < 0.0f) != y1;
             }
           }
