@@ -328,7 +328,9 @@ __device__ inline int edge_by_bounds(float4 const& e, float xl, float yl, float 
 // float32 from truncated coordinates of magnitude at most m: they are off by
 // 2^-23 m, their differences by less than 2^-21 m and the cross product by less
 // than 2^-20 m times the differences' sum, a quarter of the margin; float64's
-// roundings and the reference's collinear band (4 ULP) are far below it.
+// roundings and the reference's collinear band (4 ULP) are far below it.  From
+// differences of about 2^64 on the products are beyond float32 while the margin is
+// not yet: an infinite cross product tells nothing.
 __device__ inline int edge_by_side(float px, float py, double ax64, double ay64, double bx64,
                                    double by64, float m)
 {
@@ -337,7 +339,7 @@ __device__ inline int edge_by_side(float px, float py, double ax64, double ay64,
   float const dx = px - ax, dy = py - ay;
   float const cr  = __fmaf_rn(dx, ey, -(dy * ex));
   float const err = 3.814697265625e-06f * m * (fabsf(ex) + fabsf(ey) + fabsf(dx) + fabsf(dy));
-  if (!(fabsf(cr) > err + 1.0e-36f)) return 2;
+  if (!(fabsf(cr) > err + 1.0e-36f && fabsf(cr) < INFINITY)) return 2;
   return (cr < 0.0f) == (ey > 0.0f) ? 1 : 0;
 }
 

@@ -310,7 +310,8 @@ __device__ inline int edge_by_line(PolygonIndexView<double> const& ix, uint32_t 
   float const cr    = __fmaf_rn(dx, ey, -(dy * ex));
   float const reach = __fmaf_rn(hw, fabsf(ey), hh * fabsf(ex));
   float const err   = 3.814697265625e-06f * m * (fabsf(ex) + fabsf(ey) + fabsf(dx) + fabsf(dy));
-  if (!(fabsf(cr) > 1.001f * reach + err + 1.0e-36f)) return 2;
+  // (an infinite cross product tells nothing, as in edge_by_side)
+  if (!(fabsf(cr) > 1.001f * reach + err + 1.0e-36f && fabsf(cr) < INFINITY)) return 2;
   if (cy > e.w || cy < e.y) return 0;
   if (!(cy > e.y + inner && cy < e.w - inner)) return 2;
   return (cr < 0.0f) == (ey > 0.0f) ? 1 : 0;
