@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
       bool fast = false, vcheck = false;
       uint32_t base = 0, j0 = 0, jspan = 0, npart_all = 0;
       if constexpr (!Ordered) {
-        if (!exact && mall * invh <= 16384.0f) {
+        if (!exact && mall < kFilterMax && mall * invh <= 16384.0f) {
           float const eb  = __fmaf_rn(7.62939453125e-06f * mall, mall, 7.52316384526264e-37f);
           float const qcx = 0.5f * (qxmin + qxmax), qhw = 0.5f * (qxmax - qxmin);
           float const qcy = 0.5f * (qymin + qymax), qhh = 0.5f * (qymax - qymin);

@@ -172,6 +172,9 @@ __device__ bool pip_exact(T px, T py, PolygonIndexView<T> const& ix, uint32_t po
 
 constexpr int kUndecided = 2;
 
+// The magnitudes that the float32 filter takes (its bounds below).
+constexpr float kFilterMax = 1.152921504606847e18f;  // 2^60
+
 // float32 filter, in a frame anchored on the polygon grid (a quadrant's
 // leaf frame, or a single point's own frame).
 //
@@ -191,7 +194,9 @@ constexpr int kUndecided = 2;
 //     2^-17 M^2 = 128 u32 M^2, plus 2^-120 for float32 underflow;
 //   * the float32 slab index is off by at most 8 u32 M invh + 2 u32 nslab
 //     slabs; edges are binned 1/64 slab wide of their range, so the filter
-//     requires M invh <= 2^14.
+//     requires M invh <= 2^14;
+//   * cross32 is finite while M < 2^60 (its products stay below 2^122), which the
+//     filter requires too: an infinite one would pass any bound with either sign.
 // Undecided points are re-evaluated with pip_exact.  The polygon box is kept
 // in the polygon's frame (f_p), so the box reject is a cross-frame comparison
 // with tol as well.
@@ -216,7 +221,7 @@ __device__ __forceinline__ bool filtered_test(PolygonIndexView<double> const& ix
   float const tol = 4.76837158203125e-07f * m;  // 2^-21 M
   if (qx < bx.x - tol || qx > bx.z + tol || qy < bx.y - tol || qy > bx.w + tol) {
     r = 0;
-  } else if (m * invh <= 16384.0f) {
+  } else if (m < kFilterMax && m * invh <= 16384.0f) {
     r = -1;  // in progress
     if (vb < ve) {
       // a vertical edge within tol: decide the px == x quirk exactly
