@@ -602,9 +602,9 @@ __global__ void __launch_bounds__(kPipBlock, Filtered ? kPipMinBlocksFiltered : 
 // The float64 pipe (two lanes a cycle and SM) bounds pip_pair_kernel<false>:
 // about ten float64 instructions per edge of the point's slab and six for the
 // slab.  Most of those edges lie wholly left, right, above or below the point.
-// Points, edges and polygons therefore carry float32 bounds rounded outward
-// (truncated_f32 widened by outward_width), and only comparisons are made of
-// them; each bound leaves at least 2^-24 of the coordinates' magnitude, and so
+// Points, edges and polygons therefore carry float32 bounds, relative to an
+// origin amid the layer and rounded outward (truncated_f32 widened by
+// outward_width), and only comparisons are made of them; each bound leaves at least 2^-24 of the coordinates' magnitude, and so
 // of an edge's run and rise, to spare, where the reference's products are
 // within 9 roundings of float64 (2^-50):
 //   left, above or below the point: no toggle, not on the edge;
@@ -625,16 +625,18 @@ struct QuadBounds {
   uint32_t nonfinite;    // some point is beyond float32 or not finite
 };
 
-// Per group of pairs sharing a quadrant: the points cut to float32 in
-// quadtree order, and their box.  One warp per group.
+// Per group of pairs sharing a quadrant: the points relative to the index's
+// origin, cut to float32, in quadtree order, and their box.  One warp per group.
 __global__ void __launch_bounds__(256)
   quad_bounds_kernel(uint32_t const* __restrict__ group_start,
                      uint32_t const* __restrict__ ngroups_p,
                      uint32_t const* __restrict__ pair_quad, uint32_t const* __restrict__ qlen,
                      uint32_t const* __restrict__ qoff, PointSource<double> const src, size_t npi,
-                     float2* __restrict__ t, QuadBounds* __restrict__ out)
+                     double const* __restrict__ origin, float2* __restrict__ t,
+                     QuadBounds* __restrict__ out)
 {
   int const lane      = threadIdx.x & 31;
+  double const ox     = origin[0], oy = origin[1];
   size_t const nwarps = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
   uint32_t const ng   = *ngroups_p;
   for (size_t g = (blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x) >> 5; g < ng;
@@ -649,7 +651,7 @@ __global__ void __launch_bounds__(256)
       if (off + c >= npi) break;
       double px, py;
       src.load(off + c, px, py);
-      float2 const v = make_float2(truncated_f32(px), truncated_f32(py));
+      float2 const v = make_float2(truncated_f32(px - ox), truncated_f32(py - oy));
       t[off + c]     = v;
       bad |= !(isfinite(v.x) && isfinite(v.y));
       float const wx = outward_width(v.x), wy = outward_width(v.y);
@@ -679,6 +681,7 @@ __global__ void __launch_bounds__(kPipBlock)
   constexpr unsigned kAll = 0xFFFFFFFFu;
   int const lane          = threadIdx.x & 31;
   uint32_t nref           = 0;  // (not reported: the exact method refines nothing)
+  double const ox = ix.origin[0], oy = ix.origin[1];
   for (;;) {
     unsigned long long kk = 0;
     if (lane == 0) kk = atomicAdd(next_pair, 1ull);
@@ -693,7 +696,8 @@ __global__ void __launch_bounds__(kPipBlock)
     bool const known    = poly < ix.num_polygons;
     QuadBounds const q  = quads[pair_group[k]];
     float4 const box    = known ? ix.box32[poly] : make_float4(0.f, 0.f, 0.f, 0.f);
-    bool const walk     = known && ix.exact_only[poly];
+    // (a polygon beyond float32 or without vertices has the whole plane as its box)
+    bool const walk     = known && (ix.exact_only[poly] || !(box.z < INFINITY));
     if (!known || (!walk && !q.nonfinite &&
                    (q.xl > box.z || q.xu < box.x || q.yl > box.w || q.yu < box.y))) {
       for (uint32_t w = lane; w < nw; w += 32) bits[wb + w] = 0u;
@@ -704,27 +708,35 @@ __global__ void __launch_bounds__(kPipBlock)
     uint32_t const ns    = ix.num_slabs[poly];
     uint32_t const slab0 = ix.slab_base[poly];
     uint32_t const vb = ix.vert_begin[poly], ve = ix.vert_end[poly];
-    float const y0    = truncated_f32(ix.pminy[poly]);
+    double const y064 = ix.pminy[poly] - oy;
+    float const y0    = truncated_f32(y064);
     // the polygon's largest |y|; the float32 slab lookup is off by less than
-    // 1/64 slab while largest |y| x slabs per unit stays below 2^14
+    // 1/64 slab while largest |y| x slabs per unit stays below 2^14 (the float64
+    // one of a bound below 2^30)
     float const my    = fmaxf(fabsf(box.y), fabsf(box.w));
     float const inner = __fmaf_ru(my, 9.5367431640625e-07f, 1.0e-36f);  // 2^-20
     float const m     = 1.001f * fmaxf(my, fmaxf(fabsf(box.x), fabsf(box.z)));
-    bool const lookup = fmaxf(my, fmaxf(fabsf(q.yl), fabsf(q.yu))) * invh <= 16384.0f;
+    float const slabs = fmaxf(my, fmaxf(fabsf(q.yl), fabsf(q.yu))) * invh;
+    bool const lookup = slabs <= 16384.0f;
     bool verts        = vb < ve;  // some point may have a vertical edge's x
-    if (!walk && lookup && !q.nonfinite && len > 0 && off < npi) {
+    auto const slab_of_bound = [&](float y) {
+      if (lookup) return slab_lookup(y, y0, invh, ns);
+      double const f = (static_cast<double>(y) - y064) * ix.inv_slab_h[poly];
+      return f > 0.0 ? (f >= static_cast<double>(ns) ? ns - 1 : static_cast<uint32_t>(f)) : 0u;
+    };
+    if (!walk && slabs <= 1073741824.0f && !q.nonfinite && len > 0 && off < npi) {
       if (verts) {
         uint32_t lo = vb, hi = ve;
         while (lo < hi) {
           uint32_t const mid = (lo + hi) >> 1;
-          if (ix.vert_x[mid] < static_cast<double>(q.xl))
+          if (ix.vert_x[mid] - ox < static_cast<double>(q.xl))
             lo = mid + 1;
           else
             hi = mid;
         }
-        verts = lo < ve && ix.vert_x[lo] <= static_cast<double>(q.xu);
+        verts = lo < ve && ix.vert_x[lo] - ox <= static_cast<double>(q.xu);
       }
-      uint32_t const j0 = slab_lookup(q.yl, y0, invh, ns), j1 = slab_lookup(q.yu, y0, invh, ns);
+      uint32_t const j0 = slab_of_bound(q.yl), j1 = slab_of_bound(q.yu);
       uint32_t const E0 = ix.slab_start[slab0 + j0], E1 = ix.slab_start[slab0 + j1 + 1];
       bool meets        = verts || E1 - E0 > kFreeScan;
       for (uint32_t e0 = E0; e0 < E1 && !meets; e0 += 32) {
@@ -740,7 +752,8 @@ __global__ void __launch_bounds__(kPipBlock)
         src.load(off, px, py);
         float2 const v    = t[off];
         float const wx    = outward_width(v.x), wy = outward_width(v.y);
-        uint32_t const jr = slab_lookup(v.y, y0, invh, ns);
+        uint32_t const jr =
+          lookup ? slab_lookup(v.y, y0, invh, ns) : point_slab<double>(py, ix, poly);
         uint32_t const R0 = ix.slab_start[slab0 + jr], R1 = ix.slab_start[slab0 + jr + 1];
         unsigned par      = 0u;
         bool on           = false;
@@ -780,14 +793,15 @@ __global__ void __launch_bounds__(kPipBlock)
         float const wx = outward_width(v.x), wy = outward_width(v.y);
         float const xl = __fsub_rd(v.x, wx), xu = __fadd_ru(v.x, wx);
         float const yl = __fsub_rd(v.y, wy), yu = __fadd_ru(v.y, wy);
-        if (walk || !lookup) {
+        auto const load = [&](double& px, double& py) { src.load(pos, px, py); };
+        if (walk) {
           double px, py;
-          src.load(pos, px, py);
+          load(px, py);
           hit = pip_exact<double>(px, py, ix, poly);
         } else if (!(xl > box.z || xu < box.x || yl > box.w || yu < box.y)) {
           hit = bounds_test(ix, v.x, v.y, xl, yl, xu, yu, inner, m,
-                            slab0 + slab_lookup(v.y, y0, invh, ns), verts ? vb : ve, ve,
-                            [&](double& px, double& py) { src.load(pos, px, py); }, nref);
+                            slab0 + bounds_slab(ix, poly, lookup, v.y, y0, invh, ns, load),
+                            verts ? vb : ve, ve, load, nref);
         }
       }
       unsigned const w = __ballot_sync(kAll, hit);
@@ -980,8 +994,8 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
   if constexpr (std::is_same<T, double>::value) {
     if (bounded) {
       quad_bounds_kernel<<<leaf_frame_grid(npairs), blk, 0, s>>>(
-        gstart.data(), gstart.data() + npairs, pair_quad, qlen, qoff, src, npi, u.data(),
-        quads.data());
+        gstart.data(), gstart.data() + npairs, pair_quad, qlen, qoff, src, npi, index.origin(),
+        u.data(), quads.data());
       CSPT_CHECK_LAUNCH();
     }
   }

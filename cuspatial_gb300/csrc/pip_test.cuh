@@ -329,23 +329,36 @@ __device__ inline int edge_by_bounds(float4 const& e, float xl, float yl, float 
 }
 
 // An edge that a point's y certainly lies between the ends of, by the side of
-// its line the point is on: 1 toggles, 0 does not, 2 too near to tell.  All in
-// float32 from truncated coordinates of magnitude at most m: they are off by
+// its line the point is on: 1 toggles, 0 does not, 2 too near to tell.  e: the ends
+// (ax, ay, bx, by).  All in float32 from truncated coordinates of magnitude at most
+// m, relative to the index's origin (a float64 difference is within 2^-53 of
+// itself, which is nothing beside the truncation): they are off by
 // 2^-23 m, their differences by less than 2^-21 m and the cross product by less
 // than 2^-20 m times the differences' sum, a quarter of the margin; float64's
 // roundings and the reference's collinear band (4 ULP) are far below it.  From
 // differences of about 2^64 on the products are beyond float32 while the margin is
 // not yet: an infinite cross product tells nothing.
-__device__ inline int edge_by_side(float px, float py, double ax64, double ay64, double bx64,
-                                   double by64, float m)
+__device__ inline int edge_by_side(float px, float py, float4 const& e, float m)
 {
-  float const ax = truncated_f32(ax64), ay = truncated_f32(ay64);
-  float const ex = truncated_f32(bx64) - ax, ey = truncated_f32(by64) - ay;
-  float const dx = px - ax, dy = py - ay;
+  float const ex = e.z - e.x, ey = e.w - e.y;
+  float const dx = px - e.x, dy = py - e.y;
   float const cr  = __fmaf_rn(dx, ey, -(dy * ex));
   float const err = 3.814697265625e-06f * m * (fabsf(ex) + fabsf(ey) + fabsf(dx) + fabsf(dy));
   if (!(fabsf(cr) > err + 1.0e-36f && fabsf(cr) < INFINITY)) return 2;
   return (cr < 0.0f) == (ey > 0.0f) ? 1 : 0;
+}
+
+// The slab of a point for its bounds: in float32 (ty: its truncated y) where the
+// polygon's `lookup` allows, else from its float64 y.
+template <class Load>
+__device__ __forceinline__ uint32_t bounds_slab(PolygonIndexView<double> const& ix, uint32_t poly,
+                                                bool lookup, float ty, float y0, float invh,
+                                                uint32_t ns, Load const& load)
+{
+  if (lookup) return slab_lookup(ty, y0, invh, ns);
+  double px, py;
+  load(px, py);
+  return point_slab<double>(py, ix, poly);
 }
 
 // A point (truncated (tx, ty) and bounds) against the edges of slab s: their
@@ -372,16 +385,16 @@ __device__ __forceinline__ bool bounds_test(PolygonIndexView<double> const& ix, 
     float4 const e = ix.slab_e32[k];
     int d          = edge_by_bounds(e, xl, yl, xu, yu, inner);
     if (d == 2) {
-      uint32_t const a = ix.slab_edges[k] & kEntryVertex, b = ix.prev_vertex[a];
-      double const ax = ix.vx[a], ay = ix.vy[a], bx = ix.vx[b], by = ix.vy[b];
-      if (yl > e.y + inner && yu < e.w - inner) d = edge_by_side(tx, ty, ax, ay, bx, by, m);
+      uint32_t const a = ix.slab_edges[k] & kEntryVertex;
+      if (yl > e.y + inner && yu < e.w - inner) d = edge_by_side(tx, ty, ix.edge32[a], m);
       if (d == 2) {
+        uint32_t const b = ix.prev_vertex[a];
         ++nref;
         if (!have64) {
           load(px, py);
           have64 = true;
         }
-        d = exact_edge<double>(px, py, ax, ay, bx, by);
+        d = exact_edge<double>(px, py, ix.vx[a], ix.vy[a], ix.vx[b], ix.vy[b]);
         if (d == 2) return false;
       }
     }

@@ -253,7 +253,7 @@ __device__ inline void load_cells(PolygonIndexView<double> const& ix, uint32_t g
       f.box   = walk || empty ? b : v;
       f.my    = fmaxf(fabsf(f.box.y), fabsf(f.box.w));
       f.inner = __fmaf_ru(f.my, 9.5367431640625e-07f, 1.0e-36f);  // 2^-20
-      f.y0    = truncated_f32(ix.pminy[p]);
+      f.y0    = truncated_f32(ix.pminy[p] - ix.origin[1]);
       f.invh  = ix.inv_slab_h32[p];
       f.ns    = ix.num_slabs[p];
       f.slab0 = ix.slab_base[p];
@@ -298,15 +298,14 @@ __device__ inline void cell_range(uint32_t c, float origin, float end, float per
 // An edge whose box meets the cell: 2 when the edge may meet the cell or the
 // centre's result is not certain, 1 when the centre sees it as a toggle, else 0.
 // (cx, cy) the centre, (hw, hh) half the cell, m the largest coordinate.
-// Truncated coordinates are off by 2^-23 m, their differences by less than
-// 2^-21 m, the cross product by less than 2^-20 m times the differences' sum.
+// Truncated coordinates (relative to the index's origin, as all here) are off by
+// 2^-23 m, their differences by less than 2^-21 m, the cross product by less than 2^-20 m times the differences' sum.
 __device__ inline int edge_by_line(PolygonIndexView<double> const& ix, uint32_t k, float4 const& e,
                                    float cx, float cy, float hw, float hh, float m, float inner)
 {
-  uint32_t const v = ix.slab_edges[k] & kEntryVertex, u = ix.prev_vertex[v];
-  float const ax = truncated_f32(ix.vx[v]), ay = truncated_f32(ix.vy[v]);
-  float const ex = truncated_f32(ix.vx[u]) - ax, ey = truncated_f32(ix.vy[u]) - ay;
-  float const dx = cx - ax, dy = cy - ay;
+  float4 const t = ix.edge32[ix.slab_edges[k] & kEntryVertex];
+  float const ex = t.z - t.x, ey = t.w - t.y;
+  float const dx = cx - t.x, dy = cy - t.y;
   float const cr    = __fmaf_rn(dx, ey, -(dy * ex));
   float const reach = __fmaf_rn(hw, fabsf(ey), hh * fabsf(ex));
   float const err   = 3.814697265625e-06f * m * (fabsf(ex) + fabsf(ey) + fabsf(dx) + fabsf(dy));
@@ -329,6 +328,7 @@ __global__ void __launch_bounds__(kPointsBlock)
   __shared__ CellPoly s_poly[32];
   __shared__ CellGrid grid;
   load_cells(ix, g, s_poly, grid);
+  double const ox       = ix.origin[0];
   uint32_t const npoly  = static_cast<uint32_t>(ix.num_polygons);
   uint32_t const lane   = threadIdx.x & 31u;
   uint32_t const warps  = gridDim.x * (kPointsBlock / 32);
@@ -355,12 +355,12 @@ __global__ void __launch_bounds__(kPointsBlock)
         uint32_t lo = f.vb, hi = f.ve;
         while (lo < hi) {
           uint32_t const mid = (lo + hi) >> 1;
-          if (ix.vert_x[mid] < static_cast<double>(xl))
+          if (ix.vert_x[mid] - ox < static_cast<double>(xl))
             lo = mid + 1;
           else
             hi = mid;
         }
-        meets = lo < f.ve && ix.vert_x[lo] <= static_cast<double>(xu);
+        meets = lo < f.ve && ix.vert_x[lo] - ox <= static_cast<double>(xu);
       }
       bool in = false;
       if (__any_sync(kAll, open && !meets)) {
@@ -409,6 +409,7 @@ __global__ void __launch_bounds__(kPointsBlock)
   __shared__ uint16_t s_queue[kWarps][64];  // point of the warp | polygon << 7
   static_assert(kPts == 128, "queue entries hold 7 bits of point");
   load_cells(ix, g, s_poly, grid);
+  double const ox = ix.origin[0], oy = ix.origin[1];
   int const lane       = threadIdx.x & 31;
   int const warp       = threadIdx.x >> 5;
   unsigned const lt    = (1u << lane) - 1u;
@@ -426,22 +427,23 @@ __global__ void __launch_bounds__(kPointsBlock)
         uint32_t const slot = q & (kPts - 1), p = q >> 7;
         CellPoly const& f   = s_poly[p];
         double const px = x[base + slot], py = y[base + slot];
-        float const tx = truncated_f32(px), ty = truncated_f32(py);
+        float const tx = truncated_f32(px - ox), ty = truncated_f32(py - oy);
         float const wx = outward_width(tx), wy = outward_width(ty);
         bool hit;
-        if (((grid.walked >> p) & 1u) || !((f.my + fabsf(ty)) * f.invh <= 16384.0f)) {
+        if (((grid.walked >> p) & 1u) || !(f.my < INFINITY)) {  // (or without vertices)
           ++nref;
           hit = pip_exact<double>(px, py, ix, p);
         } else {
+          auto const load = [&](double& a, double& b) {
+            a = px;
+            b = py;
+          };
+          bool const lookup = (f.my + fabsf(ty)) * f.invh <= 16384.0f;
           hit = bounds_test(ix, tx, ty, __fsub_rd(tx, wx), __fsub_rd(ty, wy), __fadd_ru(tx, wx),
                             __fadd_ru(ty, wy), f.inner,
                             1.001f * fmaxf(f.my, fmaxf(fabsf(f.box.x), fabsf(f.box.z))),
-                            f.slab0 + slab_lookup(ty, f.y0, f.invh, f.ns), f.vb, f.ve,
-                            [&](double& a, double& b) {
-                              a = px;
-                              b = py;
-                            },
-                            nref);
+                            f.slab0 + bounds_slab(ix, p, lookup, ty, f.y0, f.invh, f.ns, load),
+                            f.vb, f.ve, load, nref);
         }
         if (hit) atomicOr(&s_mask[warp][slot], 1u << p);
       }
@@ -455,7 +457,8 @@ __global__ void __launch_bounds__(kPointsBlock)
     for (int r = 0; r < kPointSets; ++r) {
       size_t const i = base + r * 32 + lane;
       bool const have = static_cast<uint32_t>(r) < sets && i < n;
-      t[r] = have ? make_float2(truncated_f32(x[i]), truncated_f32(y[i])) : make_float2(0.f, 0.f);
+      t[r] = have ? make_float2(truncated_f32(x[i] - ox), truncated_f32(y[i] - oy))
+                  : make_float2(0.f, 0.f);
     }
 #pragma unroll
     for (int r = 0; r < kPointSets; ++r) {

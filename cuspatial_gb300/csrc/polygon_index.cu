@@ -376,7 +376,34 @@ __global__ void __launch_bounds__(kIdxBlock)
   }
 }
 
-// The anchor grid: 2^(e-22) where 2^e bounds every finite polygon coordinate.
+// The origin that edge bounds are relative to (origin[0], origin[1]), by one
+// warp: on each axis the median of the lower sides of 32 polygons spread over the
+// layer.  Float32 then resolves the layer wherever it lies, and a few polygons
+// that lie apart from the others (or without vertices) do not move it.  Relative
+// to (0, 0) instead, 31 polygons of 100 sides and 10M points at (10000, 20000)
+// took 14.1 ms (326 us there now, 325 at the origin), as the bounds told nothing.
+template <typename T>
+__device__ inline void bounds_origin(T const* __restrict__ pminx, T const* __restrict__ pminy,
+                                     size_t np, T* origin)
+{
+  int const lane = static_cast<int>(threadIdx.x & 31u);
+  T const* const low[2] = {pminx, pminy};
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
+    T const v            = np ? low[a][np * static_cast<size_t>(lane) / 32] : T{0};
+    bool const finite    = isfinite(v);
+    int const of         = __popc(__ballot_sync(0xFFFFFFFFu, finite));
+    int rank             = 0;  // among the finite ones
+    for (int l = 0; l < 32; ++l) {
+      T const o = __shfl_sync(0xFFFFFFFFu, v, l);
+      rank += isfinite(o) && (o < v || (o == v && l < lane)) ? 1 : 0;
+    }
+    if (of == 0 ? lane == 0 : finite && rank == (of - 1) / 2) origin[a] = of == 0 ? T{0} : v;
+  }
+}
+
+// The anchor grid: 2^(e-22) where 2^e bounds every finite polygon coordinate
+// (grid[0]), and the origin of the edge bounds (grid[1], grid[2]).
 // The largest magnitude is taken on the bit patterns (sign cleared,
 // non-finite skipped), which order as the magnitudes: integer work only, so
 // the FP64 pipe of the one SM this runs on stays out of the loop.
@@ -418,6 +445,8 @@ __device__ inline void anchor_grid(T const* __restrict__ pminx, T const* __restr
       frexp(mv > T{0} ? mv : T{1}, &e);  // mv < 2^e
       *grid = ldexp(T{1}, e - 22);
     }
+  } else if (threadIdx.x < 64) {
+    bounds_origin<T>(pminx, pminy, np, grid + 1);
   }
 }
 template <typename T>
@@ -489,6 +518,7 @@ __global__ void __launch_bounds__(kIdxBlock)
   T const g    = *grid;
   T const ginv = T{1} / g;  // g is a power of two: v * ginv == v / g while 1/g is finite
   bool const gi = isfinite(ginv);
+  T const ox = grid[1], oy = grid[2];  // the bounds' origin
   for (size_t p = blockIdx.x; p < np; p += gridDim.x) {
     uint32_t const r0 = po[p], r1 = po[p + 1];
     uint32_t const vb = ro[r0], ve = ro[r1];
@@ -513,7 +543,9 @@ __global__ void __launch_bounds__(kIdxBlock)
                                 static_cast<float>(pmaxx[p] - cx), static_cast<float>(pmaxy[p] - cy));
       invh32[p]   = static_cast<float>(invh[p]);
       if constexpr (std::is_same<T, double>::value)
-        if (bounds) box32[p] = outward_box(pminx[p], ymin, pmaxx[p], pmaxy[p]);
+        if (bounds)
+          box32[p] = outward_box(truncated_f32(pminx[p] - ox), truncated_f32(ymin - oy),
+                                 truncated_f32(pmaxx[p] - ox), truncated_f32(pmaxy[p] - oy));
       vcur        = 0;
     }
     for (uint32_t j = threadIdx.x; j < ns; j += kIdxBlock) cur[j] = 0;
@@ -550,8 +582,14 @@ __global__ void __launch_bounds__(kIdxBlock)
                                            fmaxf(fabsf(ef.z), fabsf(ef.w))));
       }
       if (sp & kSpanSkip) continue;
-      if constexpr (std::is_same<T, double>::value)
-        if (bounds) ef = outward_box(vx[v], vy[v], vx[pv], vy[pv]);
+      if constexpr (std::is_same<T, double>::value) {
+        if (bounds) {
+          ef        = make_float4(truncated_f32(vx[v] - ox), truncated_f32(vy[v] - oy),
+                                  truncated_f32(vx[pv] - ox), truncated_f32(vy[pv] - oy));
+          edge32[v] = ef;
+          ef        = outward_box(ef.x, ef.y, ef.z, ef.w);
+        }
+      }
       float const fa = yslab[v], fb = yslab[pv];
       float const flo = fminf(fa, fb), fhi = fmaxf(fa, fb);
       for (uint32_t j = span_j0(sp); j <= span_j1(sp); ++j) {
@@ -813,7 +851,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
   ax_        = Buffer<T>(alloc, np);
   ay_        = Buffer<T>(alloc, np);
   invh_      = Buffer<T>(alloc, np);
-  grid_      = Buffer<T>(alloc, 1);
+  grid_      = Buffer<T>(alloc, 3);
   maxoff_    = Buffer<float>(alloc, np);
   invh32_    = Buffer<float>(alloc, np);
   box32_     = Buffer<float4>(alloc, np);
@@ -825,7 +863,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
   vend_      = Buffer<uint32_t>(alloc, np + 1);
   exact_     = Buffer<uint8_t>(alloc, np);
   prev_      = Buffer<uint32_t>(alloc, nv);
-  if (build_float32) edge32_ = Buffer<float4>(alloc, nv);
+  if (build_float32 || edge_bounds) edge32_ = Buffer<float4>(alloc, nv);
   Buffer<uint32_t> nent(alloc, np + 1), ebase(alloc, np + 1), nvert(alloc, np + 1);
   Buffer<uint32_t> spans(alloc, nv);
   Buffer<float> yslab(alloc, nv);
@@ -968,6 +1006,7 @@ void PolygonIndex<T>::fill()
                            ax_.data(),
                            ay_.data(),
                            grid_.data(),
+                           grid_.data() + 1,
                            aix_.data(),
                            aiy_.data(),
                            invh32_.data(),

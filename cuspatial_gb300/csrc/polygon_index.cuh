@@ -71,14 +71,12 @@ __device__ inline float outward_width(float t)
 {
   return __fmaf_ru(fabsf(t), 2.384185791015625e-07f, 1.0e-37f);
 }
-// The box (xmin, ymin, xmax, ymax) of two points in float32, wider than them
-// by 2^-23 of the larger magnitude on each side, which is more than 2^-24 of
+// The box (xmin, ymin, xmax, ymax) of two points given truncated, wider than
+// them by 2^-23 of the larger magnitude on each side, which is more than 2^-24 of
 // the difference of their coordinates; the whole plane when a coordinate is
 // beyond float32 or not finite.
-__device__ inline float4 outward_box(double ax, double ay, double bx, double by)
+__device__ inline float4 outward_box(float x0, float y0, float x1, float y1)
 {
-  float const x0 = truncated_f32(ax), x1 = truncated_f32(bx);
-  float const y0 = truncated_f32(ay), y1 = truncated_f32(by);
   float const mx = fmaxf(fabsf(x0), fabsf(x1)), my = fmaxf(fabsf(y0), fabsf(y1));
   float const wx = outward_width(mx), wy = outward_width(my);
   if (!(wx < INFINITY && wy < INFINITY))
@@ -103,13 +101,14 @@ struct PolygonIndexView {
   T const* anchor_x;           // box centre rounded to the grid
   T const* anchor_y;
   T const* grid;               // device scalar: the anchor grid step
+  T const* origin;             // (x, y) that edge bounds are relative to
   long long const* anchor_ix;  // anchors in grid steps
   long long const* anchor_iy;
   float const* inv_slab_h32;   // inv_slab_h rounded to float
   T const* inv_slab_h;         // slabs per unit of y
   float const* max_offset;     // largest |float32 offset| over the polygon's vertices
   float4 const* box32;         // vertex box as float32 offsets from the anchor
-                               // (edge bounds: the vertex box itself, outward)
+                               // (edge bounds: the vertex box from the origin, outward)
   uint32_t const* num_slabs;
   uint32_t const* slab_base;   // first slab of the polygon in slab_start
   uint8_t const* exact_only;   // 1: walk the reference loop, no index
@@ -121,10 +120,11 @@ struct PolygonIndexView {
   uint32_t const* slab_start;
   uint32_t const* slab_edges;  // vertex index of the edge's end point | kEntryCrossing
   float4 const* slab_e32;      // the entry's edge (ax, ay, bx, by) as float32 offsets
-                               // (edge bounds: its box, outward_box)
+                               // (edge bounds: its box from the origin, outward_box)
   // per vertex
   uint32_t const* prev_vertex;
   float4 const* edge32;        // (ax, ay, bx, by) offsets from the anchor
+                               // (edge bounds: from the origin, truncated)
   // float32 index: per slab, the entries crossing the whole slab come first
   // (sorted left to right); per (slab, x-bin) a window record
   // lo | hi << 15 | parity << 30 (see slab_order_kernel)
@@ -157,6 +157,8 @@ class PolygonIndex {
   void fill();
   // device scalar: the anchor grid step (valid before fill())
   T const* grid() const { return grid_.data(); }
+  // device: x and y of the edge bounds' origin (valid before fill())
+  T const* origin() const { return grid_.data() + 1; }
   PolygonIndexView<T> view() const { return v_; }
   bool edge_bounds() const { return edge_bounds_; }
 

@@ -1,0 +1,71 @@
+"""Float32 bounds of points and edges wherever the layer lies (projected and
+geographic coordinates, small polygons over a large extent, a few polygons apart
+from the others or without vertices): rows equal to the oracle's, and few
+candidates left to float64."""
+
+import numpy as np
+import pytest
+
+import cuspatial_gb300 as cs
+from cuspatial_gb300.api import last_refined_count
+from oracle import oracle as O
+
+from helpers import gpu_polygons, to_np
+from test_pip_large_offsets import join, join_oracle, layer, points
+
+pytestmark = pytest.mark.gpu
+
+PLACES = [(0.0, 1.0), (5.0e3, 1.0), (-4.5e6, 1.0), (48.2, 1e-5), (3.0e9, 1.0), (1e17, 1e5)]
+
+
+@pytest.mark.parametrize("n,method", [(70_000, "exact"), (140_000, "filtered")])
+@pytest.mark.parametrize("at,unit", PLACES)
+def test_bitmask(at, unit, n, method):
+    rng = np.random.default_rng(21)
+    P = layer(rng, 25, unit, at)
+    x, y = points(rng, P, n, unit, at)
+    got = cs.point_in_polygon_bitmask(cs.GeoSeries.from_points(x, y), gpu_polygons(P), method)
+    want = O.point_in_polygon(x, y, P.part_offset, P.ring_offset, P.x, P.y)
+    np.testing.assert_array_equal(to_np(got).view(np.uint32), want.view(np.uint32))
+    if method == "filtered" and at * 2.0 ** -44 < unit:
+        # an eighth of the points are on or level with vertices; a point meets two
+        # or three of the polygons' edges
+        assert last_refined_count() < n // 2
+
+
+@pytest.mark.parametrize("at,unit", PLACES)
+def test_exact_join(at, unit):
+    rng = np.random.default_rng(22)
+    P = layer(rng, 40, unit, at)
+    x, y = points(rng, P, 70_000, unit, at)
+    a = (at - 4 * unit, at + 24 * unit, 6, 100)
+    got, want = join(x, y, P, *a, "exact"), join_oracle(x, y, P, *a)
+    for k in ("polygon_index", "point_index"):
+        np.testing.assert_array_equal(to_np(got[k]), want[k].astype(np.int32))
+
+
+@pytest.mark.parametrize("outlier", [0.0, 1e12, 1e37, 1e60, -1e300])
+@pytest.mark.parametrize("extent", [1e3, 1e7])
+def test_small_polygons_over_a_large_extent(extent, outlier):
+    # slabs far thinner than float32 resolves the extent: looked up in float64
+    rng = np.random.default_rng(23)
+    count, n = 31, 70_000
+    P = layer(rng, count, 1.0)
+    ids = np.repeat(np.arange(count), np.diff(P.ring_offset))
+    move = rng.uniform(-extent, extent, (2, count))
+    move[:, -1] += outlier
+    P.x += move[0][ids]
+    P.y += move[1][ids]
+    j = rng.integers(0, count, n)
+    k = P.ring_offset[j] + rng.integers(0, 10 ** 6, n) % np.diff(P.ring_offset)[j]
+    spread = rng.choice([0.0, 1e-3, 3.0], n)
+    x = P.x[k] + spread * rng.standard_normal(n)
+    y = P.y[k] + spread * rng.standard_normal(n)
+    want = O.point_in_polygon(x, y, P.part_offset, P.ring_offset, P.x, P.y)
+    pts, polys = cs.GeoSeries.from_points(x, y), gpu_polygons(P)
+    got = cs.point_in_polygon_bitmask(pts, polys, "exact")
+    np.testing.assert_array_equal(to_np(got).view(np.uint32), want.view(np.uint32))
+    a = (-1.1 * extent, 1.1 * extent, 9, 50)
+    got, want = join(x, y, P, *a, "exact"), join_oracle(x, y, P, *a)
+    for c in ("polygon_index", "point_index"):
+        np.testing.assert_array_equal(to_np(got[c]), want[c].astype(np.int32))
