@@ -87,9 +87,11 @@ __device__ inline bool grid_split(double v, int k, long long& q, float& u)
 template <typename T, bool Filtered>
 __global__ void __launch_bounds__(kPointsBlock)
   points_pip_kernel(T const* __restrict__ x, T const* __restrict__ y, size_t n,
-                    PolygonIndexView<T> ix, uint32_t lp, int32_t* __restrict__ out,
-                    unsigned long long* __restrict__ refined)
+                    PolygonIndexView<T> ix, T bounds_share, uint32_t lp,
+                    int32_t* __restrict__ out, unsigned long long* __restrict__ refined)
 {
+  // (bounds_share > 0: the index may carry bounds instead, for the grid of cells)
+  if (bounds_share > T{0} && has_bounds(ix.origin[2], bounds_share)) return;
   int const lane       = threadIdx.x & 31;
   uint32_t const P     = 1u << lp;
   uint32_t const S     = 32u >> lp;
@@ -230,7 +232,6 @@ struct CellPoly {
 struct CellGrid {
   float x0, y0, x1, y1;  // common box (outward)
   float iw, ih;          // cells per unit
-  uint32_t g;            // cells along an axis
   uint32_t walked;       // polygons tested for every point
 };
 
@@ -271,7 +272,7 @@ __device__ inline void load_cells(PolygonIndexView<double> const& ix, uint32_t g
     unsigned const walked = __ballot_sync(0xFFFFFFFFu, walk);
     if (threadIdx.x == 0)
       s_grid = CellGrid{b.x, b.y, b.z, b.w, static_cast<float>(g) / (b.z - b.x),
-                        static_cast<float>(g) / (b.w - b.y), g, walked};
+                        static_cast<float>(g) / (b.w - b.y), walked};
   }
   __syncthreads();
 }
@@ -321,9 +322,10 @@ __device__ inline int edge_by_line(PolygonIndexView<double> const& ix, uint32_t 
 // fill the GPU (a warp's chain of polygons, each a few dependent loads, bounds
 // the kernel).  cells[row g + column] |= (inside, test), zero before.
 __global__ void __launch_bounds__(kPointsBlock)
-  points_cells_kernel(PolygonIndexView<double> ix, uint32_t g, uint32_t share,
-                      uint2* __restrict__ cells)
+  points_cells_kernel(PolygonIndexView<double> ix, double bounds_share, uint32_t g,
+                      uint32_t share, uint2* __restrict__ cells)
 {
+  if (!has_bounds(ix.origin[2], bounds_share)) return;
   constexpr unsigned kAll = 0xFFFFFFFFu;
   __shared__ CellPoly s_poly[32];
   __shared__ CellGrid grid;
@@ -350,7 +352,9 @@ __global__ void __launch_bounds__(kPointsBlock)
       if (yl > f.box.w || yu < f.box.y) continue;  // the row lies beyond the polygon
       bool const open = !(xl > f.box.z || xu < f.box.x);  // still to be decided
       if (!__any_sync(kAll, open)) continue;
-      bool meets = !((f.my + fmaxf(fabsf(yl), fabsf(yu))) * f.invh <= 16384.0f);
+      // (a row that holds the polygon's whole height decides nothing)
+      bool meets = !((f.my + fmaxf(fabsf(yl), fabsf(yu))) * f.invh <= 16384.0f) ||
+                   (yl <= f.box.y && yu >= f.box.w);
       if (f.vb < f.ve && !meets) {
         uint32_t lo = f.vb, hi = f.ve;
         while (lo < hi) {
@@ -397,10 +401,11 @@ __global__ void __launch_bounds__(kPointsBlock)
 
 __global__ void __launch_bounds__(kPointsBlock)
   points_grid_kernel(double const* __restrict__ x, double const* __restrict__ y, size_t n,
-                     PolygonIndexView<double> ix, uint32_t g, uint2 const* __restrict__ cells,
-                     uint32_t sets, int32_t* __restrict__ out,
+                     PolygonIndexView<double> ix, double bounds_share, uint32_t g,
+                     uint2 const* __restrict__ cells, uint32_t sets, int32_t* __restrict__ out,
                      unsigned long long* __restrict__ refined)
 {
+  if (!has_bounds(ix.origin[2], bounds_share)) return;
   constexpr unsigned kAll = 0xFFFFFFFFu;
   constexpr int kWarps = kPointsBlock / 32, kPts = 32 * kPointSets;
   __shared__ CellPoly s_poly[32];
@@ -835,11 +840,24 @@ uint32_t lanes_log2(size_t npoly)
 // Whether the bitmask call takes the grid of cells: where building it costs less
 // than it saves.  31 polygons of 400 sides, 130k points, whole call: filtered
 // 144 us with the grid, 155 without, exact 129 and 304; 65536 points of 1000
-// sides: filtered 175 and 150, exact 157 and 229.
-bool points_use_grid(size_t n, bool filtered)
+// sides: filtered 175 and 150, exact 157 and 229.  5 polygons of 20000 sides, 140k
+// points: filtered 1251 and 888, exact 1224 and 1487 (2M points: 998 and 1402), so
+// the filtered method asks for two points a vertex.
+bool points_use_grid(size_t n, size_t nv, bool filtered)
 {
-  return n >= (size_t{1} << (filtered ? 17 : 16));
+  return filtered ? n >= (size_t{1} << 17) && n / 2 >= nv : n >= (size_t{1} << 16);
 }
+// The filtered method takes the grid where the median polygon's box is this many
+// cells wide and high at least.  Cells that are large beside the polygons, or
+// farther from the origin than float32 resolves them, decide little, and the tests
+// they leave cost more than the filter's: 31 polygons of 100 sides in two places
+// 10000 radii apart, 10M points around them: 23.7 ms with the grid, 7.2 without; one
+// of 31 polygons of 1000 sides 100 radii off, 2M points around the others (5 cells a
+// polygon): 1069 us and 639, 10M points (10 cells): 2536 and 2610.  (Where few
+// polygons overlap fewer cells would do: 31 of 1000 sides spread over 20 radii, 140k
+// points, 6 cells: 458 us and 1021.)  The exact method gains in all of these but at
+// small sizes in the second (200k points, 1 cell: 790 us and 663).
+constexpr double kCellsPerPolygon = 8.0;
 
 // Cells along an axis: one cell for every kPointsPerCell points.
 uint32_t grid_side(size_t n)
@@ -857,24 +875,22 @@ uint32_t points_sets(size_t n)
   return static_cast<uint32_t>(k < 1 ? 1 : (k > kPointSets ? kPointSets : k));
 }
 
-void bitmask_grid(double const* x, double const* y, size_t n, uint32_t const* po, size_t npo,
-                  uint32_t const* ro, size_t nro, double const* vx, double const* vy, size_t nv,
-                  Allocator const& alloc, int32_t* out, unsigned long long* refined)
+void bitmask_grid(double const* x, double const* y, size_t n, PolygonIndex<double>& index,
+                  size_t npoly, double bounds_share, Allocator const& alloc, int32_t* out,
+                  unsigned long long* refined)
 {
   cudaStream_t const s = alloc.stream();
-  PolygonIndex<double> index(po, npo, ro, nro, vx, vy, nv, false, alloc, false, false, true);
   uint32_t const g = grid_side(n), sets = points_sets(n);
   Buffer<uint2> cells(alloc, static_cast<size_t>(g) * g);
-  KernelTimer timer("points_pip", s);
   CSPT_CUDA_TRY(cudaMemsetAsync(cells.data(), 0, static_cast<size_t>(g) * g * sizeof(uint2), s));
   uint32_t const segs  = g * (g / 32u);
-  uint32_t const share = std::max(1u, std::min(static_cast<uint32_t>(npo - 1), 32768u / segs));
+  uint32_t const share = std::max(1u, std::min(static_cast<uint32_t>(npoly), 32768u / segs));
   points_cells_kernel<<<grid_for(static_cast<size_t>(segs) * share * 32, kPointsBlock,
                                  sm_grid(8u)),
-                        kPointsBlock, 0, s>>>(index.view(), g, share, cells.data());
+                        kPointsBlock, 0, s>>>(index.view(), bounds_share, g, share, cells.data());
   CSPT_CHECK_LAUNCH();
   points_grid_kernel<<<points_grid((n + sets - 1) / sets), kPointsBlock, 0, s>>>(
-    x, y, n, index.view(), g, cells.data(), sets, out, refined);
+    x, y, n, index.view(), bounds_share, g, cells.data(), sets, out, refined);
   CSPT_CHECK_LAUNCH();
 }
 
@@ -886,24 +902,26 @@ void bitmask(T const* x, T const* y, size_t n, uint32_t const* po, size_t npo, u
   cudaStream_t const s = alloc.stream();
   Buffer<unsigned long long> refined(alloc, 1);
   CSPT_CUDA_TRY(cudaMemsetAsync(refined.data(), 0, sizeof(unsigned long long), s));
-  bool grid = false;
-  if constexpr (std::is_same<T, double>::value) {
-    grid = points_use_grid(n, filtered);
-    if (grid) bitmask_grid(x, y, n, po, npo, ro, nro, vx, vy, nv, alloc, out, refined.data());
-  }
-  if (!grid) {
-    PolygonIndex<T> index(po, npo, ro, nro, vx, vy, nv, filtered, alloc);
-    uint32_t const lp = lanes_log2(npo - 1);
-    KernelTimer timer("points_pip", s);
-    if (filtered) {
-      if constexpr (std::is_same<T, double>::value) {
-        points_pip_kernel<double, true><<<points_grid(n), kPointsBlock, 0, s>>>(
-          x, y, n, index.view(), lp, out, refined.data());
-      }
-    } else {
-      points_pip_kernel<T, false>
-        <<<points_grid(n), kPointsBlock, 0, s>>>(x, y, n, index.view(), lp, out, nullptr);
+  bool const grid = std::is_same<T, double>::value && points_use_grid(n, nv, filtered);
+  // filtered: the device chooses by the polygons' sizes, and the kernels of the other
+  // way return at once
+  T const bounds_share = grid && filtered ? T{kCellsPerPolygon / grid_side(n)} : T{0};
+  PolygonIndex<T> index(po, npo, ro, nro, vx, vy, nv, filtered, alloc, false, false, grid,
+                        bounds_share);
+  KernelTimer timer("points_pip", s);
+  if constexpr (std::is_same<T, double>::value)
+    if (grid)
+      bitmask_grid(x, y, n, index, npo - 1, bounds_share, alloc, out, refined.data());
+  uint32_t const lp = lanes_log2(npo - 1);
+  if (filtered) {
+    if constexpr (std::is_same<T, double>::value) {
+      points_pip_kernel<double, true><<<points_grid(n), kPointsBlock, 0, s>>>(
+        x, y, n, index.view(), bounds_share, lp, out, refined.data());
+      CSPT_CHECK_LAUNCH();
     }
+  } else if (!grid) {
+    points_pip_kernel<T, false>
+      <<<points_grid(n), kPointsBlock, 0, s>>>(x, y, n, index.view(), T{0}, lp, out, nullptr);
     CSPT_CHECK_LAUNCH();
   }
   *out_refined = filtered ? read_back(reinterpret_cast<uint64_t*>(refined.data()), s) : 0;

@@ -376,34 +376,60 @@ __global__ void __launch_bounds__(kIdxBlock)
   }
 }
 
-// The origin that edge bounds are relative to (origin[0], origin[1]), by one
-// warp: on each axis the median of the lower sides of 32 polygons spread over the
-// layer.  Float32 then resolves the layer wherever it lies, and a few polygons
-// that lie apart from the others (or without vertices) do not move it.  Relative
-// to (0, 0) instead, 31 polygons of 100 sides and 10M points at (10000, 20000)
-// took 14.1 ms (326 us there now, 325 at the origin), as the bounds told nothing.
+// The median of the warp's finite values (0 where there is none).
 template <typename T>
-__device__ inline void bounds_origin(T const* __restrict__ pminx, T const* __restrict__ pminy,
-                                     size_t np, T* origin)
+__device__ inline T warp_median(T v)
 {
-  int const lane = static_cast<int>(threadIdx.x & 31u);
-  T const* const low[2] = {pminx, pminy};
-#pragma unroll
-  for (int a = 0; a < 2; ++a) {
-    T const v            = np ? low[a][np * static_cast<size_t>(lane) / 32] : T{0};
-    bool const finite    = isfinite(v);
-    int const of         = __popc(__ballot_sync(0xFFFFFFFFu, finite));
-    int rank             = 0;  // among the finite ones
-    for (int l = 0; l < 32; ++l) {
-      T const o = __shfl_sync(0xFFFFFFFFu, v, l);
-      rank += isfinite(o) && (o < v || (o == v && l < lane)) ? 1 : 0;
-    }
-    if (of == 0 ? lane == 0 : finite && rank == (of - 1) / 2) origin[a] = of == 0 ? T{0} : v;
+  bool const finite    = isfinite(v);
+  unsigned const which = __ballot_sync(0xFFFFFFFFu, finite);
+  int const lane       = static_cast<int>(threadIdx.x & 31u);
+  int rank             = 0;  // among the finite ones
+  for (int l = 0; l < 32; ++l) {
+    T const o = __shfl_sync(0xFFFFFFFFu, v, l);
+    rank += ((which >> l) & 1u) && (o < v || (o == v && l < lane)) ? 1 : 0;
   }
+  unsigned const mid = __ballot_sync(0xFFFFFFFFu, finite && rank == (__popc(which) - 1) / 2);
+  T const m          = __shfl_sync(0xFFFFFFFFu, v, mid ? __ffs(mid) - 1 : 0);
+  return mid ? m : T{0};
+}
+
+// Where the layer lies, from 32 polygons spread over it, by one warp.
+// place[0], place[1]: the origin that edge bounds are relative to, the medians of
+// the polygons' lower sides.  Float32 then resolves the layer wherever it lies, and
+// a few polygons that lie apart from the others (or without vertices) do not move
+// it.  (Relative to (0, 0) 10M points x 31 polygons of 100 sides at (10000, 20000)
+// took 14.1 ms, as the bounds told nothing; 321 us this way.)
+// place[2] (median_share): the share of the polygons' common box that their median
+// box takes along an axis (the smaller one of the two axes).
+template <typename T>
+__device__ inline void layer_place(T const* __restrict__ pminx, T const* __restrict__ pminy,
+                                   T const* __restrict__ pmaxx, T const* __restrict__ pmaxy,
+                                   size_t np, T* place)
+{
+  uint32_t const lane  = threadIdx.x & 31u;
+  T const* const lo[2] = {pminx, pminy};
+  T const* const hi[2] = {pmaxx, pmaxy};
+  T share              = T{1};
+  for (int a = 0; a < 2; ++a) {
+    size_t const p = np * lane / 32;
+    T const l = np ? lo[a][p] : T{0}, h = np ? hi[a][p] : T{0};
+    T const origin = warp_median(l);
+    T const side   = warp_median(h - l);
+    T least = isfinite(l) ? l : origin, most = isfinite(h) ? h : origin;
+    for (int o = 16; o > 0; o >>= 1) {
+      T const b = __shfl_xor_sync(0xFFFFFFFFu, least, o), c = __shfl_xor_sync(0xFFFFFFFFu, most, o);
+      least     = b < least ? b : least;
+      most      = c > most ? c : most;
+    }
+    T const s = side / (most - least);
+    share     = s < share ? s : share;
+    if (lane == 0) place[a] = origin;
+  }
+  if (lane == 0) place[2] = share;
 }
 
 // The anchor grid: 2^(e-22) where 2^e bounds every finite polygon coordinate
-// (grid[0]), and the origin of the edge bounds (grid[1], grid[2]).
+// (grid[0]), and layer_place's three values (grid[1] on).
 // The largest magnitude is taken on the bit patterns (sign cleared,
 // non-finite skipped), which order as the magnitudes: integer work only, so
 // the FP64 pipe of the one SM this runs on stays out of the loop.
@@ -446,7 +472,7 @@ __device__ inline void anchor_grid(T const* __restrict__ pminx, T const* __restr
       *grid = ldexp(T{1}, e - 22);
     }
   } else if (threadIdx.x < 64) {
-    bounds_origin<T>(pminx, pminy, np, grid + 1);
+    layer_place<T>(pminx, pminy, pmaxx, pmaxy, np, grid + 1);
   }
 }
 template <typename T>
@@ -504,7 +530,7 @@ __global__ void __launch_bounds__(kIdxBlock)
                     T const* __restrict__ invh, uint32_t const* __restrict__ nslab,
                     uint32_t const* __restrict__ slab_base, uint32_t const* __restrict__ entry_base,
                     uint32_t const* __restrict__ vert_base, T const* __restrict__ grid,
-                    bool float32, bool bounds, T* anchor_x, T* anchor_y, long long* aix, long long* aiy,
+                    bool float32, bool bounds, T bounds_share, T* anchor_x, T* anchor_y, long long* aix, long long* aiy,
                     float4* box32, float* invh32, float* maxoff, uint32_t const* __restrict__ prev,
                     uint32_t const* __restrict__ spans, float4* edge32, uint32_t* slab_start,
                     uint32_t* slab_edges, float4* slab_e32, T* vert_x, float* vert_x32,
@@ -519,6 +545,10 @@ __global__ void __launch_bounds__(kIdxBlock)
   T const ginv = T{1} / g;  // g is a power of two: v * ginv == v / g while 1/g is finite
   bool const gi = isfinite(ginv);
   T const ox = grid[1], oy = grid[2];  // the bounds' origin
+  if (float32 && bounds) {
+    bounds  = has_bounds(grid[3], bounds_share);
+    float32 = !bounds;
+  }
   for (size_t p = blockIdx.x; p < np; p += gridDim.x) {
     uint32_t const r0 = po[p], r1 = po[p + 1];
     uint32_t const vb = ro[r0], ve = ro[r1];
@@ -824,6 +854,7 @@ struct PolygonIndex<T>::Sizing {
   T const *vx, *vy;
   size_t np, nslabs_total, nentries, nvertical;
   bool build_float32, order_slabs, edge_bounds;
+  T bounds_share;
   unsigned grd;
   Buffer<uint32_t> ebase, spans;
   Buffer<float> yslab;
@@ -834,10 +865,10 @@ template <typename T>
 PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro, size_t nro,
                               T const* vx, T const* vy, size_t nv, bool build_float32,
                               Allocator const& alloc, bool order_slabs, bool defer_fill,
-                              bool edge_bounds)
+                              bool edge_bounds, T bounds_share)
 {
   (void)nro;
-  CSPT_EXPECTS(!edge_bounds || (std::is_same<T, double>::value && !build_float32),
+  CSPT_EXPECTS(!edge_bounds || (std::is_same<T, double>::value && !order_slabs),
                "edge bounds belong to the float64 index");
   edge_bounds_         = edge_bounds;
   cudaStream_t const s = alloc.stream();
@@ -851,7 +882,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
   ax_        = Buffer<T>(alloc, np);
   ay_        = Buffer<T>(alloc, np);
   invh_      = Buffer<T>(alloc, np);
-  grid_      = Buffer<T>(alloc, 3);
+  grid_      = Buffer<T>(alloc, 4);
   maxoff_    = Buffer<float>(alloc, np);
   invh32_    = Buffer<float>(alloc, np);
   box32_     = Buffer<float4>(alloc, np);
@@ -936,7 +967,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
     nvertical    = tot[2];
   }
   sizing_.reset(new Sizing{po, ro, vx, vy, np, nslabs_total, nentries, nvertical, build_float32,
-                           order_slabs, edge_bounds, grd, std::move(ebase), std::move(spans),
+                           order_slabs, edge_bounds, bounds_share, grd, std::move(ebase), std::move(spans),
                            std::move(yslab), &alloc});
   if (!defer_fill) fill();
 }
@@ -970,7 +1001,7 @@ void PolygonIndex<T>::fill()
     index_fill_kernel<T><<<grd, kIdxBlock, 0, s>>>(
       po, ro, vx, vy, np, pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
       invh_.data(), nslab_.data(), slab_base_.data(), z->ebase.data(), vbeg_.data(), grid_.data(),
-      build_float32, z->edge_bounds, ax_.data(), ay_.data(), aix_.data(), aiy_.data(), box32_.data(),
+      build_float32, z->edge_bounds, z->bounds_share, ax_.data(), ay_.data(), aix_.data(), aiy_.data(), box32_.data(),
       invh32_.data(), maxoff_.data(), prev_.data(), z->spans.data(), edge32_.data(),
       slab_start_.data(),
       slab_edges_.data(), slab_e32_.data(), vert_x_.data(), vert_x32_.data(), vxy32.data(),

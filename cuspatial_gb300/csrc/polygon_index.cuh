@@ -85,6 +85,13 @@ __device__ inline float4 outward_box(float x0, float y0, float x1, float y1)
                      __fadd_ru(fmaxf(x0, x1), wx), __fadd_ru(fmaxf(y0, y1), wy));
 }
 
+// Whether an index that leaves the choice to the device carries edge bounds.
+template <typename T>
+__device__ inline bool has_bounds(T median_share, T bounds_share)
+{
+  return median_share >= bounds_share;
+}
+
 template <typename T>
 struct PolygonIndexView {
   // polygon topology (caller's arrays)
@@ -101,7 +108,7 @@ struct PolygonIndexView {
   T const* anchor_x;           // box centre rounded to the grid
   T const* anchor_y;
   T const* grid;               // device scalar: the anchor grid step
-  T const* origin;             // (x, y) that edge bounds are relative to
+  T const* origin;             // (x, y) that edge bounds are relative to, median_share
   long long const* anchor_ix;  // anchors in grid steps
   long long const* anchor_iy;
   float const* inv_slab_h32;   // inv_slab_h rounded to float
@@ -140,8 +147,11 @@ class PolygonIndex {
   // build the per-(slab, x-bin) windows.  It costs a pass over all slab
   // entries and pays off where the index is evaluated many times (batched
   // plans, resident polygon sets).
-  // edge_bounds (float64 index without float32 edges): slab entries carry
-  // their edge's box in float32, rounded outward (outward_box).
+  // edge_bounds (float64 index): slab entries carry their edge's box in float32,
+  // rounded outward (outward_box), in place of the float32 edges.  With
+  // build_float32 too, the device decides: bounds where median_share is at least
+  // bounds_share, else float32 edges; the kernels of both kinds are launched and ask
+  // has_bounds.
   // defer_fill: return once the per-polygon boxes, slab counts and the anchor
   // grid are enqueued (array sizes come from bounds on the host, so the call
   // does not wait for the device); fill() then writes the slab entries.  Work
@@ -150,7 +160,8 @@ class PolygonIndex {
   PolygonIndex(uint32_t const* poly_offsets, size_t num_poly_offsets,
                uint32_t const* ring_offsets, size_t num_ring_offsets, T const* vx, T const* vy,
                size_t num_vertices, bool build_float32, Allocator const& alloc,
-               bool order_slabs = false, bool defer_fill = false, bool edge_bounds = false);
+               bool order_slabs = false, bool defer_fill = false, bool edge_bounds = false,
+               T bounds_share = T{0});
   ~PolygonIndex();
   PolygonIndex(PolygonIndex const&)            = delete;
   PolygonIndex& operator=(PolygonIndex const&) = delete;

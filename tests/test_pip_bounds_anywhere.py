@@ -69,3 +69,44 @@ def test_small_polygons_over_a_large_extent(extent, outlier):
     got, want = join(x, y, P, *a, "exact"), join_oracle(x, y, P, *a)
     for c in ("polygon_index", "point_index"):
         np.testing.assert_array_equal(to_np(got[c]), want[c].astype(np.int32))
+
+
+@pytest.mark.parametrize("apart,n", [(0.0, 140_000), (60.0, 140_000), (60.0, 600_000),
+                                     (1e5, 131_072), (1e5, 400_000), (1e300, 140_000)])
+def test_filtered_bitmask_of_two_places(apart, n):
+    # cells of the common box that tell the polygons apart, and ones that do not:
+    # few candidates left to float64 either way
+    rng = np.random.default_rng(24)
+    P = layer(rng, 31, 1.0)
+    second = np.repeat(np.arange(31) % 2 == 1, np.diff(P.ring_offset))
+    P.x, P.y = P.x + apart * second, P.y + 0.3 * apart * second
+    x, y = points(rng, P, n, 1.0)
+    there = rng.random(n) < 0.5
+    x, y = np.where(there, x + apart, x), np.where(there, y + 0.3 * apart, y)
+    got = cs.point_in_polygon_bitmask(cs.GeoSeries.from_points(x, y), gpu_polygons(P),
+                                      "filtered")
+    want = O.point_in_polygon(x, y, P.part_offset, P.ring_offset, P.x, P.y)
+    np.testing.assert_array_equal(to_np(got).view(np.uint32), want.view(np.uint32))
+    assert last_refined_count() < n or apart > 1e6
+
+
+@pytest.mark.parametrize("sides", [2000, 30_000])
+def test_filtered_bitmask_with_more_vertices_than_half_the_points(sides):
+    rng = np.random.default_rng(sides)
+    count, n = 5, 140_000
+    a = np.linspace(0, 2 * np.pi, sides + 1)
+    r = 8 * rng.uniform(0.9, 1.0, (count, sides))
+    r = np.concatenate([r, r[:, :1]], 1)
+    c = rng.uniform(-4, 4, (2, count, 1))
+    x, y = (c[0] + r * np.cos(a)).ravel(), (c[1] + r * np.sin(a)).ravel()
+    from cuspatial_gb300.datasets import Polygons
+    i = np.arange(count + 1, dtype=np.int32)
+    P = Polygons(x, y, (i * (sides + 1)).astype(np.int32), i, i)
+    px, py = rng.uniform(-14, 14, (2, n))
+    got, exact = (to_np(cs.point_in_polygon_bitmask(cs.GeoSeries.from_points(px, py),
+                                                    gpu_polygons(P), m)).view(np.uint32)
+                  for m in ("filtered", "exact"))
+    np.testing.assert_array_equal(got, exact)
+    some = rng.integers(0, n, 3000)  # the oracle walks every edge
+    want = O.point_in_polygon(px[some], py[some], P.part_offset, P.ring_offset, P.x, P.y)
+    np.testing.assert_array_equal(got[some], want.view(np.uint32))
