@@ -940,11 +940,13 @@ void pairwise(T const* x, T const* y, size_t n, uint32_t const* po, uint32_t con
   size_t const fill       = n / (static_cast<size_t>(num_sms()) * 48u);
   uint32_t const per_warp = static_cast<uint32_t>(fill < 1 ? 1 : (fill > 32 ? 32 : fill));
   unsigned const grd      = grid_for((n + per_warp - 1) / per_warp * 32, kPointsBlock, sm_grid(64u));
-  // Float32 polygons of a few vertices: a lane walks one in fewer
-  // instructions than a run of 32 costs (1M pairs of 4..8 vertices: 43 us a
-  // call against 64).  Around 12 vertices the two meet; above, lanes wait for
-  // the largest polygon of their warp and read it uncoalesced.
-  bool const lanes = std::is_same<T, float>::value && nv < 12 * n;
+  // Exact polygons of a few vertices: a lane walks one in fewer instructions than a
+  // run of 32 costs (1M pairs of 4..8 float32 vertices: 43 us a call against 64;
+  // float64, 5 vertices: 10k pairs 43 us against 55, 1M 173 against 192).  Around 12
+  // vertices the two meet; above, lanes wait for the largest polygon of their warp
+  // and read it uncoalesced.  The filter's runs are faster from the start (1M pairs
+  // of 5 vertices: 108 us).
+  bool const lanes = !filtered && nv < 12 * n;
   {
     KernelTimer timer("pairwise_pip", s);
     if (lanes) {
