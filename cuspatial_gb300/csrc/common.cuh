@@ -11,9 +11,9 @@
 #include <string>
 #include <type_traits>
 #include <utility>
-#include <vector>
 
 #include "../../include/cuspatial_gb300.h"
+#include "slab_arena.h"
 
 namespace cspt {
 
@@ -160,89 +160,44 @@ class Allocator {
 
 // The scratch memory of one call.  A small join takes 60 to 150 buffers, most
 // of them a few kilobytes, and a caller's allocator is a callback (6 to 10 us
-// each from Python, a third of such a call); blocks of up to kMaxBlock bytes
-// are cut from slabs of the caller's memory instead, which go back when the
-// call ends.  Blocks are powers of two and are reused within the call in stream
-// order, as the allocator's own are.  Where the caller has no memory for a slab
-// the buffer is allocated as before.
+// each from Python, a third of such a call); blocks of up to 4 MiB are cut from
+// slabs of the caller's memory instead (slab_arena.h), which go back when the
+// call ends.  Blocks are reused within the call in stream order, as the allocator's
+// own are.  Where the caller has no memory for a slab the buffer is allocated as
+// before.
 class ScratchArena {
+  struct Upstream {
+    Allocator* a;
+    void* allocate(size_t bytes) const
+    {
+      try {
+        return a->allocate(bytes);
+      } catch (Error const&) {
+        return nullptr;
+      }
+    }
+    void deallocate(void* p, size_t bytes) const { a->deallocate(p, bytes); }
+  };
+
  public:
-  explicit ScratchArena(Allocator& a) : a_(a) { a_.arena_ = this; }
-  ~ScratchArena()
+  explicit ScratchArena(Allocator& a, size_t first_slab = size_t{2} << 20,
+                        size_t most = size_t{158} << 20)
+    : a_(a), slabs_(Upstream{&a}, first_slab, most)
   {
-    a_.arena_ = nullptr;
-    for (int i = 0; i < nslabs_; ++i) a_.deallocate(slabs_[i].p, slabs_[i].bytes);
+    a_.arena_ = this;
   }
+  ~ScratchArena() { a_.arena_ = nullptr; }
   ScratchArena(ScratchArena const&)            = delete;
   ScratchArena& operator=(ScratchArena const&) = delete;
 
-  void* take(size_t bytes)
-  {
-    if (bytes > kMaxBlock) return nullptr;
-    int const c  = size_class(bytes);
-    size_t const size = kMinBlock << c;
-    if (!free_[c].empty()) {
-      void* const p = free_[c].back();
-      free_[c].pop_back();
-      return p;
-    }
-    if (end_ - at_ < static_cast<ptrdiff_t>(size) && !grow(size)) return nullptr;
-    void* const p = at_;
-    at_ += size;
-    return p;
-  }
-  bool give(void* p, size_t bytes)
-  {
-    if (!owns(p)) return false;
-    free_[size_class(bytes)].push_back(p);
-    return true;
-  }
-  bool owns(void const* p) const
-  {
-    for (int i = 0; i < nslabs_; ++i) {
-      char const* const b = static_cast<char const*>(slabs_[i].p);
-      if (p >= b && p < b + slabs_[i].bytes) return true;
-    }
-    return false;
-  }
+  void* take(size_t bytes) { return slabs_.take(bytes); }
+  bool give(void* p, size_t bytes) { return slabs_.give(p, bytes); }
+  // gives back the slabs that hold no buffer in use
+  void trim() { slabs_.trim(); }
 
  private:
-  static constexpr size_t kMinBlock = 256, kMaxBlock = size_t{4} << 20;
-  static constexpr int kClasses = 15, kMaxSlabs = 8;
-  static constexpr size_t kFirstSlab = size_t{2} << 20, kLastSlab = size_t{32} << 20;
-  static_assert(kMinBlock << (kClasses - 1) == kMaxBlock && kLastSlab >= kMaxBlock, "sizes");
-  static int size_class(size_t bytes)
-  {
-    int c = 0;
-    while ((kMinBlock << c) < bytes) ++c;
-    return c;
-  }
-  bool grow(size_t least)
-  {
-    if (nslabs_ == kMaxSlabs) return false;
-    size_t const next = nslabs_ == 0 ? kFirstSlab : slabs_[nslabs_ - 1].bytes * 2;
-    size_t const want = next < least ? least : next;
-    size_t const size = want < kLastSlab ? want : kLastSlab;
-    void* p           = nullptr;
-    try {
-      p = a_.allocate(size);
-    } catch (Error const&) {
-      return false;
-    }
-    slabs_[nslabs_++] = Slab{p, size};
-    at_               = static_cast<char*>(p);
-    end_              = at_ + size;
-    return true;
-  }
-  struct Slab {
-    void* p;
-    size_t bytes;
-  };
   Allocator& a_;
-  Slab slabs_[kMaxSlabs];
-  int nslabs_ = 0;
-  char *at_ = nullptr, *end_ = nullptr;
-  std::vector<void*> free_[kClasses];
+  SlabArena<Upstream> slabs_;
 };
 
 inline void* Allocator::arena_take(size_t bytes) const { return arena_->take(bytes); }
