@@ -24,6 +24,6 @@ def test_small_plan_keeps_little():
         plan.run()
         offsets, polygon, point = (to_np(t).copy() for t in plan.rows())
         # a first slab of 1 MiB on each of its two streams and the rows
-        assert alloc.in_use <= (2 << 20) + 256 * KB
+        assert alloc.in_use <= (2 << 20) + (256 << 10)
     assert alloc.in_use == 0
     assert offsets[-1] == len(polygon) == len(point) > 0
