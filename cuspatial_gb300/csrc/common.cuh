@@ -112,7 +112,11 @@ cudaStream_t library_stream();
 
 class Allocator {
  public:
-  Allocator(cspt_allocator const* mr, cudaStream_t stream) : mr_(mr), stream_(stream) {}
+  // frugal: the call has run out of memory once (see with_scratch)
+  Allocator(cspt_allocator const* mr, cudaStream_t stream, bool frugal = false)
+    : mr_(mr), stream_(stream), frugal_(frugal)
+  {
+  }
   // scratch: the memory does not outlive the call (see ScratchArena)
   void* allocate(size_t bytes, bool scratch = false) const
   {
@@ -145,6 +149,8 @@ class Allocator {
   }
   cudaStream_t stream() const { return stream_; }
   cspt_allocator const* resource() const { return mr_; }
+  // whether to take the way that needs the least memory, not the fastest
+  bool frugal() const { return frugal_; }
   // before the first allocation
   void set_stream(cudaStream_t stream) { stream_ = stream; }
 
@@ -155,6 +161,7 @@ class Allocator {
 
   cspt_allocator const* mr_;
   cudaStream_t stream_;
+  bool frugal_;
   class ScratchArena* arena_ = nullptr;
 };
 
@@ -204,7 +211,8 @@ inline void* Allocator::arena_take(size_t bytes) const { return arena_->take(byt
 inline bool Allocator::arena_give(void* p, size_t bytes) const { return arena_->give(p, bytes); }
 
 // Runs body(alloc) with a scratch arena.  A call that runs out of memory so is
-// repeated without one: what fitted a caller's memory before still does.
+// repeated without one and by the ways that need the least memory: what fits a
+// caller's memory in some way is done.
 template <typename F>
 void with_scratch(cspt_allocator const* mr, cudaStream_t stream, F&& body)
 {
@@ -214,7 +222,7 @@ void with_scratch(cspt_allocator const* mr, cudaStream_t stream, F&& body)
     body(static_cast<Allocator const&>(alloc));
   } catch (Error const& e) {
     if (e.status != CSPT_OUT_OF_MEMORY) throw;
-    Allocator const alloc(mr, stream);
+    Allocator const alloc(mr, stream, true);
     body(alloc);
   }
 }

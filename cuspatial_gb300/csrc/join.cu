@@ -26,10 +26,12 @@ namespace {
 
 // Pairs the count pass may append (node + box, 8 bytes each): 64 per box, or, for
 // few boxes over a large tree, all there can be up to 4 Mi; at most 64 Mi.  A join
-// with more runs the write pass instead.
-inline size_t join_append_capacity(size_t nb, size_t nodes)
+// with more runs the write pass instead.  (frugal: 64 per box.)
+inline size_t join_append_capacity(size_t nb, size_t nodes, bool frugal)
 {
-  size_t const all = nodes < (size_t{4} << 20) / nb ? nodes * nb : size_t{4} << 20;
+  size_t const all = frugal                             ? 0
+                     : nodes < (size_t{4} << 20) / nb ? nodes * nb
+                                                        : size_t{4} << 20;
   size_t const c   = std::max(nb * 64, all);
   return c < (size_t{64} << 20) ? c : (size_t{64} << 20);
 }
@@ -124,7 +126,7 @@ void run(cspt_quadtree const* tree, T const* bminx, T const* bminy, T const* bma
   unsigned const blk = kJoinWarps * 32;
   unsigned const grd = grid_for(nb * 32, blk, sm_grid(16u));
   // the count pass also appends each (node, box) it finds while they fit
-  size_t const cap = join_append_capacity(nb, tree->num_nodes);
+  size_t const cap = join_append_capacity(nb, tree->num_nodes, alloc.frugal());
   Buffer<uint32_t> app_node(alloc, cap), app_box(alloc, cap);
   auto const count = [&](JoinSplit const& split) {
     KernelTimer timer("join_count", s);
@@ -190,9 +192,10 @@ void run(cspt_quadtree const* tree, T const* bminx, T const* bminy, T const* bma
     // both columns (0.52 ms for 43M pairs; a nearest-linestring call over 5M points and
     // 20k linestrings 10.95 -> 10.51 ms).  The table has an entry per point up to the
     // last leaf found; it is made for at most four entries per pair, so that its
-    // clearing costs less than the gather.
+    // clearing costs less than the gather.  With the table the write pass holds up to
+    // nine words a pair, without it eight, as a call short of memory does.
     size_t const entries = static_cast<size_t>(h.max_offset) + 1;
-    bool lookup          = entries <= 4 * k;
+    bool lookup          = entries <= 4 * k && !alloc.frugal();
     Buffer<uint32_t> at;
     if (lookup) {
       at = Buffer<uint32_t>(alloc, entries + 1);

@@ -107,7 +107,7 @@ constexpr int kSegChunk = 8;  // segments per pruning box
 // v0 / kSegChunk + l + c (v0 its first vertex): the ranges of successive
 // linestrings do not overlap, and no scan is needed to place them.
 struct LsBounds {
-  float4 const* ls;
+  float4 const* ls;  // null: nothing is pruned (a call short of memory)
   float4 const* chunk;
   uint32_t slots;  // chunk boxes; offsets that leave them are not pruned by chunk
   float2 const* vertex;  // the vertices to nearest float32 (exact method)
@@ -210,6 +210,12 @@ __device__ inline float box_lower(PointBounds const& p, float4 b)
   float const lb = __fadd_rd(__fmul_rd(dx, dx), __fmul_rd(dy, dy));
   float const D2 = __fadd_ru(__fmul_ru(fx, fx), __fmul_ru(fy, fy));
   return __fsub_rd(lb, __fmaf_ru(D2, k32u, 7.52316384526264e-37f));
+}
+
+template <typename T>
+__device__ inline float linestring_lower(PointBounds const& p, LsBounds const& b, uint32_t l)
+{
+  return b.ls ? box_lower<T>(p, b.ls[l]) : -INFINITY;
 }
 
 // An upper bound of the squared distance that the reference's expression gives
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(256)
       float bound = INFINITY;
       for (uint32_t k = k0; k < k1 && pb.finite; ++k) {
         uint32_t const lid = pair_ls[k];
-        if (lid >= nls || box_lower<T>(pb, bounds.ls[lid]) > bound) continue;
+        if (lid >= nls || linestring_lower<T>(pb, bounds, lid) > bound) continue;
         uint32_t const v0 = lso[lid], v1 = lso[lid + 1];
         for (uint32_t v = v0; v + 1 < v1 && v < bounds.nv; v += kSegChunk)
           bound = fminf(bound, vertex_upper(pb, bounds.vertex[v]));
@@ -368,7 +374,7 @@ __global__ void __launch_bounds__(256)
         for (uint32_t k = k0; k < k1; ++k) {
           uint32_t const lid = pair_ls[k];
           if (lid >= nls) continue;
-          if (pb.finite && box_lower<T>(pb, bounds.ls[lid]) > f.far) continue;
+          if (pb.finite && linestring_lower<T>(pb, bounds, lid) > f.far) continue;
           uint32_t const v0 = lso[lid];
           T const d = linestring_distance<T>(px, py, pb, lx, ly, v0, lso[lid + 1], bounds,
                                              v0 / kSegChunk + lid, f.far);
@@ -414,7 +420,7 @@ __device__ void fold_warp(FoldArgs<T> const& a, uint32_t k0, uint32_t k1, T px, 
   for (uint32_t kb = k0; kb < k1 && use_bound && pb.finite; kb += 32) {
     uint32_t const k   = kb + static_cast<uint32_t>(lane);
     uint32_t const lid = k < k1 ? a.pair_ls[k] : 0xFFFFFFFFu;
-    if (k < k1 && lid < a.nls && !(box_lower<T>(pb, a.bounds.ls[lid]) > bound)) {
+    if (k < k1 && lid < a.nls && !(linestring_lower<T>(pb, a.bounds, lid) > bound)) {
       uint32_t const v1 = a.lso[lid + 1];
       for (uint32_t v = a.lso[lid]; v + 1 < v1 && v < a.bounds.nv; v += kSegChunk)
         bound = fminf(bound, vertex_upper(pb, a.bounds.vertex[v]));
@@ -430,7 +436,7 @@ __device__ void fold_warp(FoldArgs<T> const& a, uint32_t k0, uint32_t k1, T px, 
       uint32_t const k   = kb + static_cast<uint32_t>(lane);
       uint32_t const lid = k < k1 ? a.pair_ls[k] : 0xFFFFFFFFu;
       bool const valid   = k < k1 && lid < a.nls;
-      float const lb     = valid && pb.finite ? box_lower<T>(pb, a.bounds.ls[lid]) : -INFINITY;
+      float const lb     = valid && pb.finite ? linestring_lower<T>(pb, a.bounds, lid) : -INFINITY;
       unsigned left      = __ballot_sync(kAll, valid);
       for (;;) {
         // the next in order that is not beyond the winner so far (which a zero
@@ -661,7 +667,7 @@ __global__ void __launch_bounds__(256)
         all.add(abs_box.b);
         if (cb + c < slots) {
           chunk_box[cb + c] = cbx;
-          abs_chunk[cb + c] = abs_box.b;
+          if (abs_chunk) abs_chunk[cb + c] = abs_box.b;
         }
       }
       float4 sbx = cbx;
@@ -683,7 +689,7 @@ __global__ void __launch_bounds__(256)
     all.b = make_float4(warp_min(all.b.x), warp_min(all.b.y), warp_max(all.b.z),
                         warp_max(all.b.w));
     if (lane == 0) {
-      abs_ls[l] = all.b;
+      if (abs_ls) abs_ls[l] = all.b;
       aix[l]    = static_cast<long long>(rx);
       aiy[l]    = static_cast<long long>(ry);
       maxoff[l] = m;
@@ -1309,21 +1315,26 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       Buffer<float> maxoff(alloc, nls);
       size_t const slots = chunk_slots(nv, nls);
       size_t const sslots = super_slots(nv, nls);
-      Buffer<float4> cbox(alloc, slots), seg32(alloc, nv), abs_ls(alloc, nls),
-        abs_chunk(alloc, slots), sbox(alloc, sslots);
-      Buffer<float2> vertex(alloc, nv);
+      // (short of memory: without the exact kernels' boxes)
+      size_t const bnls = alloc.frugal() ? 0 : nls, bslots = alloc.frugal() ? 0 : slots,
+                   bnv  = alloc.frugal() ? 0 : nv;
+      Buffer<float4> cbox(alloc, slots), seg32(alloc, nv), abs_ls(alloc, bnls),
+        abs_chunk(alloc, bslots), sbox(alloc, sslots);
+      Buffer<float2> vertex(alloc, bnv);
       Buffer<LsRec> lrec(alloc, nls);
       ls_fill_kernel<<<lgrd, 256, 0, s>>>(lso, nls, lx, ly, box.data(), grid.data(),
                                           lexact.data(), aix.data(), aiy.data(),
                                           maxoff.data(), cbox.data(), seg32.data(), lrec.data(),
                                           slots, abs_ls.data(), abs_chunk.data(), sslots, sbox.data(),
-                                          static_cast<uint32_t>(nv), vertex.data());
+                                          static_cast<uint32_t>(bnv), vertex.data());
       CSPT_CHECK_LAUNCH();
+      box.reset();
       double const g = read_back(grid.data(), s);
       index_timer.reset();
       // leaf frames of the groups
       Buffer<float2> u(alloc, npi);
-      Buffer<LeafFrame> frames(alloc, npairs);
+      size_t const most = alloc.frugal() ? read_back(gs + npairs, s) : npairs;  // groups
+      Buffer<LeafFrame> frames(alloc, most);
       std::unique_ptr<KernelTimer> frames_timer(new KernelTimer("leaf_frames", s));
       leaf_frame_kernel<<<grid_for(npairs * 32, 256, sm_grid(32u)), 256, 0, s>>>(
         gs, gs + npairs, pair_quad, tree->length, qoff, src, npi, grid.data(), u.data(),
@@ -1332,13 +1343,13 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       frames_timer.reset();
       LinestringIndexView liv{aix.data(),  aiy.data(),   maxoff.data(), cbox.data(),
                               sbox.data(), seg32.data(), lexact.data(), lrec.data()};
-      LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(slots),
-                            vertex.data(), static_cast<uint32_t>(nv)};
+      LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(bslots),
+                            vertex.data(), static_cast<uint32_t>(bnv)};
       // points folded whole, groups scanned, next group, float64 segment distances
       // (and the groups left, as 32 bits)
       Buffer<unsigned long long> fb(alloc, 5);
       CSPT_CUDA_TRY(cudaMemsetAsync(fb.data(), 0, 5 * sizeof(unsigned long long), s));
-      Buffer<uint32_t> left(alloc, npairs);
+      Buffer<uint32_t> left(alloc, most);
       uint32_t* const nleft = reinterpret_cast<uint32_t*>(fb.data() + 4);
       NearestArgs const na{gs,          gs + npairs,  npairs,     pair_ls,   pair_quad,
                            tree->length, qoff,        src,        npi,       lso,
@@ -1381,21 +1392,24 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
   if (nls)
     CSPT_CUDA_TRY(cudaMemcpyAsync(h + 1, lso + nls, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   CSPT_CUDA_TRY(cudaStreamSynchronize(s));
-  size_t const ng = h[0], slots = chunk_slots(h[1], nls);
-  Buffer<float4> ls_box(alloc, nls), chunk_box(alloc, slots);
-  Buffer<float2> vertex(alloc, h[1]);
-  ls_bounds_kernel<T><<<grid_for(nls * 32, 256, sm_grid(32u)), 256, 0, s>>>(
-    lso, nls, lx, ly, slots, ls_box.data(), chunk_box.data(), h[1], vertex.data());
-  CSPT_CHECK_LAUNCH();
+  bool const lean = alloc.frugal();  // without the boxes: every candidate is evaluated
+  size_t const ng = h[0], slots = lean ? 0 : chunk_slots(h[1], nls);
+  uint32_t const bnv = lean ? 0 : h[1];
+  Buffer<float4> ls_box(alloc, lean ? 0 : nls), chunk_box(alloc, slots);
+  Buffer<float2> vertex(alloc, bnv);
+  LsBounds const bounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots),
+                        vertex.data(), bnv};
+  if (!lean) {
+    ls_bounds_kernel<T><<<grid_for(nls * 32, 256, sm_grid(32u)), 256, 0, s>>>(
+      lso, nls, lx, ly, slots, ls_box.data(), chunk_box.data(), bnv, vertex.data());
+    CSPT_CHECK_LAUNCH();
+  }
   if (npi <= kWarpPoints) {
     KernelTimer timer("nearest", s);
     nearest_point_kernel<T><<<grid_for(npi * 32, 256, sm_grid(8u)), 256, 0, s>>>(
       nullptr, gs + npairs, gs, gs + npairs, npairs, kPointSplit, pair_quad, tree->length, qoff,
       src, npi,
-      FoldArgs<T>{pair_ls, lso, nls, lx, ly,
-                  LsBounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots),
-                           vertex.data(), h[1]}},
-      opt, ols, od);
+      FoldArgs<T>{pair_ls, lso, nls, lx, ly, bounds}, opt, ols, od);
     CSPT_CHECK_LAUNCH();
   } else {
     KernelTimer timer("nearest", s);
@@ -1405,9 +1419,8 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
     uint32_t const split = static_cast<uint32_t>(
       ng == 0 ? 1 : std::min<size_t>(kLaneSplit, std::max<size_t>(1, fill / ng)));
     nearest_kernel<T><<<grid_for(ng * split * 32, 256, sm_grid(32u)), 256, 0, s>>>(
-      nullptr, gs + npairs, gs, gs + npairs, npairs, split, pair_ls, pair_quad, tree->length, qoff, src, npi, lso, nls,
-      lx, ly, LsBounds{ls_box.data(), chunk_box.data(), static_cast<uint32_t>(slots), vertex.data(), h[1]},
-      opt, ols, od);
+      nullptr, gs + npairs, gs, gs + npairs, npairs, split, pair_ls, pair_quad, tree->length, qoff,
+      src, npi, lso, nls, lx, ly, bounds, opt, ols, od);
     CSPT_CHECK_LAUNCH();
   }
 }

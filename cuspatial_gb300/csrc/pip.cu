@@ -68,9 +68,10 @@ constexpr uint32_t kFreeScan = 1024;
 #endif
 constexpr size_t kBoundsPoints = CSPT_BOUNDS_POINTS;
 template <typename T>
-bool use_bounds(bool filtered, size_t points)
+bool use_bounds(bool filtered, size_t points, Allocator const& alloc)
 {
-  return !filtered && std::is_same<T, double>::value && points >= kBoundsPoints;
+  return !filtered && std::is_same<T, double>::value && points >= kBoundsPoints &&
+         !alloc.frugal();  // (the bounds take 8 bytes a point, 28 a pair and 22 a vertex more)
 }
 // Blocks of 256 threads per SM for the leaf frames (the index fill that runs
 // beside them takes what the frames leave; 2-8 measured within 1%).
@@ -949,7 +950,7 @@ void run(uint32_t const* pair_poly, uint32_t const* pair_quad, size_t npairs,
   Buffer<float2> u;
   Buffer<LeafFrame> frames;
   Buffer<QuadBounds> quads;
-  bool const bounded = prebuilt ? prebuilt->edge_bounds() : use_bounds<T>(filtered, npi);
+  bool const bounded = prebuilt ? prebuilt->edge_bounds() : use_bounds<T>(filtered, npi, alloc);
   if (filtered || bounded) {
     gstart       = Buffer<uint32_t>(alloc, npairs + 1);
     pgroup       = Buffer<uint32_t>(alloc, npairs);
@@ -1378,7 +1379,7 @@ void join_host(T const* hx, T const* hy, size_t n, double x_min, double x_max, d
     polygon_bounding_boxes(dpo.data(), npo, dro.data(), nro, dvx.data(), dvy.data(), nv, dtype,
                            0.0, bminx.data(), bminy.data(), bmaxx.data(), bmaxy.data(), palloc);
     index.reset(new PolygonIndex<T>(dpo.data(), npo, dro.data(), nro, dvx.data(), dvy.data(), nv,
-                                    filtered, palloc, false, false, use_bounds<T>(filtered, n)));
+                                    filtered, palloc, false, false, use_bounds<T>(filtered, n, palloc)));
   };
   uint32_t* pi_raw = nullptr;
   cspt_quadtree tree{nullptr, nullptr, nullptr, nullptr, nullptr, 0};

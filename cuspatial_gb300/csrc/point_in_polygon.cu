@@ -902,7 +902,8 @@ void bitmask(T const* x, T const* y, size_t n, uint32_t const* po, size_t npo, u
   cudaStream_t const s = alloc.stream();
   Buffer<unsigned long long> refined(alloc, 1);
   CSPT_CUDA_TRY(cudaMemsetAsync(refined.data(), 0, sizeof(unsigned long long), s));
-  bool const grid = std::is_same<T, double>::value && points_use_grid(n, nv, filtered);
+  bool const grid =
+    std::is_same<T, double>::value && points_use_grid(n, nv, filtered) && !alloc.frugal();
   // filtered: the device chooses by the polygons' sizes, and the kernels of the other
   // way return at once
   T const bounds_share = grid && filtered ? T{kCellsPerPolygon / grid_side(n)} : T{0};
