@@ -315,6 +315,26 @@ __device__ inline T linestring_distance(T px, T py, PointBounds const& pb, T con
   return sqrt(ds);
 }
 
+// Up to this many points take a warp each (exact method, and the groups the
+// filtered kernel leaves).  Whole calls, a warp per point against a lane: 1081
+// points x 3190 linestrings 585 and 1234 us, 2000 x 20k 4.7 and 19.4 ms, 1620 x 72
+// 459 and 541 us; 5000 x 1000 1081 to 1422 and 998 to 1067 us, 20k x 301 2003 and
+// 715 us.  What the filtered kernel leaves counts by its own points: 1M points x 3000
+// linestrings with 2000 (8000) more about one leaf 1230 us (1871), by the points of
+// the whole call 2299 (5683).
+constexpr size_t kWarpPoints = 4096;
+// warps that share a group: a warp per point, a lane per point
+constexpr uint32_t kPointSplit = 64, kLaneSplit = 8;
+
+// Whether the groups that the filtered kernel left are this kernel's: both kernels
+// are launched and the number of their points decides (count: [0] the groups,
+// [1] their points).
+template <bool Few>
+__device__ inline bool takes_left(uint32_t const* groups, uint32_t const* count)
+{
+  return !groups || (count[1] <= kWarpPoints) == Few;
+}
+
 // A lane per point; the candidates of its group in pair order.  `split` warps
 // share a group.  `groups`: those that the filtered kernel left (which may have
 // left its bound in place of the distance), or all where it is null.  Bound by the float64 pipe (two lanes a cycle and SM) and, on
@@ -334,6 +354,7 @@ __global__ void __launch_bounds__(256)
                  T const* __restrict__ ly, LsBounds const bounds, uint32_t* __restrict__ opt,
                  uint32_t* __restrict__ ols, T* __restrict__ od)
 {
+  if (!takes_left<false>(groups, count)) return;
   int const lane       = threadIdx.x & 31;
   size_t const warps   = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
   size_t const ngroups = *ngroups_p, n = *count;
@@ -484,6 +505,7 @@ __global__ void __launch_bounds__(256)
                        FoldArgs<T> const a, uint32_t* __restrict__ opt,
                        uint32_t* __restrict__ ols, T* __restrict__ od)
 {
+  if (!takes_left<true>(groups, count)) return;
   int const lane       = threadIdx.x & 31;
   size_t const warps   = (static_cast<size_t>(gridDim.x) * blockDim.x) >> 5;
   size_t const ngroups = *ngroups_p, n = *count;
@@ -788,7 +810,7 @@ struct NearestArgs {
   unsigned long long* stats;  // [0] points folded over every candidate, [1] groups scanned whole
   unsigned long long* next_group;
   uint32_t* left;   // groups that the listing cannot take
-  uint32_t* nleft;
+  uint32_t* nleft;  // [0] how many, [1] their points
 };
 
 // Folds the points of the lanes that ask for it, one after the other.
@@ -1149,7 +1171,10 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
     }
     if (!listed) {
       __syncwarp();
-      if (lane == 0) a.left[atomicAdd(a.nleft, 1u)] = static_cast<uint32_t>(gi);
+      if (lane == 0) {
+        a.left[atomicAdd(a.nleft, 1u)] = static_cast<uint32_t>(gi);
+        atomicAdd(a.nleft + 1, len);
+      }
       ++nscan;
       continue;
     }
@@ -1265,15 +1290,6 @@ __global__ void __launch_bounds__(kNearWarps * 32, 6)
   }
 }
 
-// Up to this many points take a warp each (exact method, and the groups the
-// filtered kernel leaves).  Whole calls, a warp per point against a lane: 1081
-// points x 3190 linestrings 585 and 1234 us, 2000 x 20k 4.7 and 19.4 ms, 1620 x 72
-// 459 and 541 us; 5000 x 1000 1081 to 1422 and 998 to 1067 us, 20k x 301 2003 and
-// 715 us.
-constexpr size_t kWarpPoints = 4096;
-// warps that share a group: a warp per point, a lane per point
-constexpr uint32_t kPointSplit = 64, kLaneSplit = 8;
-
 template <typename T>
 void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
          cspt_quadtree const* tree, uint32_t const* point_indices, size_t npi, T const* x,
@@ -1346,7 +1362,7 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
       LsBounds const bounds{abs_ls.data(), abs_chunk.data(), static_cast<uint32_t>(bslots),
                             vertex.data(), static_cast<uint32_t>(bnv)};
       // points folded whole, groups scanned, next group, float64 segment distances
-      // (and the groups left, as 32 bits)
+      // (and the groups left and their points, as 32 bits)
       Buffer<unsigned long long> fb(alloc, 5);
       CSPT_CUDA_TRY(cudaMemsetAsync(fb.data(), 0, 5 * sizeof(unsigned long long), s));
       Buffer<uint32_t> left(alloc, most);
@@ -1368,14 +1384,13 @@ void run(uint32_t const* pair_ls, uint32_t const* pair_quad, size_t npairs,
                                          sm_grid(static_cast<unsigned>(per_sm))),
                                 kNearWarps * 32, 0, s>>>(na);
       CSPT_CHECK_LAUNCH();
-      if (npi <= kWarpPoints)
-        nearest_point_kernel<double><<<sm_grid(4u), 256, 0, s>>>(
-          left.data(), nleft, gs, gs + npairs, npairs, kPointSplit, pair_quad, tree->length, qoff,
-          src, npi, FoldArgs<double>{pair_ls, lso, nls, lx, ly, bounds}, opt, ols, od);
-      else
-        nearest_kernel<double><<<sm_grid(8u), 256, 0, s>>>(
-          left.data(), nleft, gs, gs + npairs, npairs, kLaneSplit, pair_ls, pair_quad,
-          tree->length, qoff, src, npi, lso, nls, lx, ly, bounds, opt, ols, od);
+      nearest_point_kernel<double><<<sm_grid(4u), 256, 0, s>>>(
+        left.data(), nleft, gs, gs + npairs, npairs, kPointSplit, pair_quad, tree->length, qoff,
+        src, npi, FoldArgs<double>{pair_ls, lso, nls, lx, ly, bounds}, opt, ols, od);
+      CSPT_CHECK_LAUNCH();
+      nearest_kernel<double><<<sm_grid(8u), 256, 0, s>>>(
+        left.data(), nleft, gs, gs + npairs, npairs, kLaneSplit, pair_ls, pair_quad,
+        tree->length, qoff, src, npi, lso, nls, lx, ly, bounds, opt, ols, od);
       CSPT_CHECK_LAUNCH();
       unsigned long long st[4];
       CSPT_CUDA_TRY(cudaMemcpyAsync(st, fb.data(), sizeof(st), cudaMemcpyDeviceToHost, s));
