@@ -63,15 +63,12 @@ constexpr uint32_t kFreeScan = 1024;
 // (pip_bounds_kernel): at 1M points x 256 polygons the call takes 858 us with
 // the bounds, 940 without; at 1k points x 17 the bounds' launches cost what they
 // save (667 to 697 us with, 655 to 680 without).
-#ifndef CSPT_BOUNDS_POINTS
-#define CSPT_BOUNDS_POINTS 65536
-#endif
-constexpr size_t kBoundsPoints = CSPT_BOUNDS_POINTS;
+constexpr size_t kBoundsPoints = 65536;
 template <typename T>
 bool use_bounds(bool filtered, size_t points, Allocator const& alloc)
 {
   return !filtered && std::is_same<T, double>::value && points >= kBoundsPoints &&
-         !alloc.frugal();  // (the bounds take 8 bytes a point, 28 a pair and 22 a vertex more)
+         !alloc.frugal();  // (the bounds take 8 bytes a point, 28 a pair and 44 a vertex more)
 }
 // Blocks of 256 threads per SM for the leaf frames (the index fill that runs
 // beside them takes what the frames leave; 2-8 measured within 1%).

@@ -28,19 +28,19 @@ constexpr int kMaxSlabs = 4096;
 // set (build + evaluation): density 2 for the one-shot float32 index, whose
 // pair kernel classifies a quadrant's slab entries once (1: 12.90 ms,
 // 2: 12.51, 3: 12.71, 4: 13.29); 4 for the ordered index, whose per-point
-// windows gain from shorter slabs; 8 for the float64-only evaluation; 1 for the
-// edge bounds, whose entries cost a comparison (2M points x 10k polygons, whole
-// call: 1: 1.449 ms, 2: 1.534, 4: 1.588).
+// windows gain from shorter slabs; 8 for the float64-only evaluation; 2 for the
+// edge bounds, whose entries cost a comparison, and a float64 edge where the layer is
+// so wide that float32 does not tell them apart (2M points x 10k polygons, whole
+// call with 1 / 2 / 4 over an extent of 3162: 1180 / 1163 / 1156 us; with small
+// polygons over 1e6: 1219 / 1151 / 1148, over 1e7: 1615 / 1450 / 1412, 1500 without
+// bounds; the entries of 4 take twice the memory).
 #ifndef CSPT_SLAB_DENSITY32
 #define CSPT_SLAB_DENSITY32 2.0
 #endif
 constexpr double kSlabDensityFloat32 = CSPT_SLAB_DENSITY32;
 constexpr double kSlabDensityOrdered = 4.0;
 constexpr double kSlabDensityFloat64 = 8.0;
-#ifndef CSPT_SLAB_DENSITY_BOUNDS
-#define CSPT_SLAB_DENSITY_BOUNDS 1.0
-#endif
-constexpr double kSlabDensityBounds = CSPT_SLAB_DENSITY_BOUNDS;
+constexpr double kSlabDensityBounds  = 2.0;
 __device__ inline uint32_t choose_slabs(uint32_t nv, double height, double sum_rise,
                                         double density)
 {
