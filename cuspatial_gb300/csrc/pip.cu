@@ -15,7 +15,9 @@
 //
 // Per candidate test (see polygon_index.cuh for why it equals the reference):
 //   exact    : y-range reject, vertical-x lookup, then the reference's
-//              float64 edge test over the edges of the point's slab;
+//              float64 edge test over the edges of the point's slab; from
+//              kBoundsPoints float64 points on, float32 bounds and sides of lines
+//              decide what they certainly can before it (pip_bounds_kernel);
 //   filtered : the same edges in float32 on anchored coordinates with a
 //              forward error bound; any undecided edge sends the candidate
 //              to the exact test.
