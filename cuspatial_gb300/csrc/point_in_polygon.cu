@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kPointsBlock)
   points_cells_kernel(PolygonIndexView<double> ix, double bounds_share, uint32_t g,
                       uint32_t share, uint2* __restrict__ cells)
 {
-  if (!has_bounds(ix.origin[2], bounds_share)) return;
+  if (bounds_share > 0.0 && !has_bounds(ix.origin[2], bounds_share)) return;
   constexpr unsigned kAll = 0xFFFFFFFFu;
   __shared__ CellPoly s_poly[32];
   __shared__ CellGrid grid;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kPointsBlock)
                      uint2 const* __restrict__ cells, uint32_t sets, int32_t* __restrict__ out,
                      unsigned long long* __restrict__ refined)
 {
-  if (!has_bounds(ix.origin[2], bounds_share)) return;
+  if (bounds_share > 0.0 && !has_bounds(ix.origin[2], bounds_share)) return;
   constexpr unsigned kAll = 0xFFFFFFFFu;
   constexpr int kWarps = kPointsBlock / 32, kPts = 32 * kPointSets;
   __shared__ CellPoly s_poly[32];
