@@ -52,6 +52,17 @@ __device__ inline uint32_t choose_slabs(uint32_t nv, double height, double sum_r
   return static_cast<uint32_t>(s);
 }
 
+// Slab entries that a polygon of nv vertices may have; the arrays are made for the
+// sum of these (fill()).  The slab count keeps to them where sum_rise is the edges'
+// rise.  It is taken from truncated vertices, and where the polygon lies so far from
+// y = 0 that float32 has a few steps over its height, edges within a step count
+// nothing: such a polygon could have many times the entries, and the fill wrote
+// beyond the arrays.
+__device__ inline uint32_t max_entries(uint32_t nv, double density)
+{
+  return static_cast<uint32_t>((density + 2.0) * static_cast<double>(nv));
+}
+
 template <typename T>
 __device__ inline uint32_t slab_of(T y, T ymin, T inv_h, uint32_t ns)
 {
@@ -141,6 +152,7 @@ __device__ inline uint32_t block_scan_counts(uint32_t* cnt, uint32_t n, uint32_t
 // A vertex's edge (prev -> v), packed in 32 bits: slab range j0..j1 (12 bits
 // each), bit 24 degenerate (the reference skips it), bit 25 exactly vertical,
 // bit 26 degenerate by ULP but not equal (walk the reference loop instead).
+constexpr uint32_t kSpanSlabs = (1u << 24) - 1u;
 constexpr uint32_t kSpanSkip = 1u << 24, kSpanVertical = 1u << 25, kSpanTiny = 1u << 26;
 __device__ inline uint32_t span_j0(uint32_t s) { return s & 0xFFFu; }
 __device__ inline uint32_t span_j1(uint32_t s) { return (s >> 12) & 0xFFFu; }
@@ -361,13 +373,28 @@ __global__ void __launch_bounds__(kIdxBlock)
     local = block_sum(local, shU);
     verts = block_sum(verts, shU);
     bad   = block_sum(bad, shU);
+    uint32_t slabs = ns;
+    T per_unit     = ih;
+    if (local > max_entries(ve - vb, density)) {
+      // more than the arrays are made for: one slab, which holds every edge once
+      slabs    = 1;
+      per_unit = T{0};
+      local    = 0;
+      for (uint32_t v = vb + threadIdx.x; v < ve; v += kIdxBlock) {
+        uint32_t const sp = spans[v] & ~kSpanSlabs;
+        spans[v]          = sp;
+        yslab[v]          = 0.0f;
+        local += (sp & kSpanSkip) ? 0u : 1u;
+      }
+      local = block_sum(local, shU);
+    }
     if (threadIdx.x == 0) {
       pminx[p]    = mnx;
       pminy[p]    = mny;
       pmaxx[p]    = mxx;
       pmaxy[p]    = mxy;
-      invh[p]     = ih;
-      nslab[p]    = ns;
+      invh[p]     = per_unit;
+      nslab[p]    = slabs;
       nentries[p] = local;
       nvert[p]    = verts;
       exact[p]    = bad ? 1 : 0;
@@ -934,7 +961,8 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
   // r ns / H (1 + 2^-35) + 1 + 1/16 slabs (its range widened by 2^-36 of
   // itself plus 1/32 slab at each end, float32 slab coordinates within
   // 2^-12 slab), and the sum over edges of r ns / H is at most density V
-  // (with one slab every edge spans one).  So (density + 2) entries per
+  // (with one slab every edge spans one); a polygon whose rises float32 does not
+  // tell is counted again with one slab (max_entries).  So (density + 2) entries per
   // vertex, 1 + density / 2 slabs per polygon and one vertical edge per
   // vertex bound the arrays without reading the counts back: no host
   // synchronisation.  Only where those bounds reach 2^32 (the 32-bit
