@@ -92,8 +92,8 @@ class BatchedPip {
   {
     try {
       if (arenas) {
-        arena_.emplace(alloc_, kPlanFirst, kPlanMost);
-        parena_.emplace(palloc_, kPlanFirst, kPlanMost);
+        arena_.emplace(alloc_, kPlanFirst, kPlanMost, true);
+        parena_.emplace(palloc_, kPlanFirst, kPlanMost, true);
       }
       plan(h_pt_off, x, y, h_poly_off, po, npo, ro, nro, vx, vy, nv, params, method, ordered,
            block);

@@ -188,8 +188,8 @@ class ScratchArena {
 
  public:
   explicit ScratchArena(Allocator& a, size_t first_slab = size_t{2} << 20,
-                        size_t most = size_t{158} << 20)
-    : a_(a), slabs_(Upstream{&a}, first_slab, most)
+                        size_t most = size_t{158} << 20, bool fine = false)
+    : a_(a), slabs_(Upstream{&a}, first_slab, most, fine)
   {
     a_.arena_ = this;
   }

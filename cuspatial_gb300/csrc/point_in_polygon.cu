@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kPointsBlock)
                     int32_t* __restrict__ out, unsigned long long* __restrict__ refined)
 {
   // (bounds_share > 0: the index may carry bounds instead, for the grid of cells)
-  if (bounds_share > T{0} && has_bounds(ix.origin[2], bounds_share)) return;
+  if (bounds_share > T{0} && has_bounds(ix.origin, bounds_share)) return;
   int const lane       = threadIdx.x & 31;
   uint32_t const P     = 1u << lp;
   uint32_t const S     = 32u >> lp;
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kPointsBlock)
   points_cells_kernel(PolygonIndexView<double> ix, double bounds_share, uint32_t g,
                       uint32_t share, uint2* __restrict__ cells)
 {
-  if (bounds_share > 0.0 && !has_bounds(ix.origin[2], bounds_share)) return;
+  if (bounds_share > 0.0 && !has_bounds(ix.origin, bounds_share)) return;
   constexpr unsigned kAll = 0xFFFFFFFFu;
   __shared__ CellPoly s_poly[32];
   __shared__ CellGrid grid;
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kPointsBlock)
                      uint2 const* __restrict__ cells, uint32_t sets, int32_t* __restrict__ out,
                      unsigned long long* __restrict__ refined)
 {
-  if (bounds_share > 0.0 && !has_bounds(ix.origin[2], bounds_share)) return;
+  if (bounds_share > 0.0 && !has_bounds(ix.origin, bounds_share)) return;
   constexpr unsigned kAll = 0xFFFFFFFFu;
   constexpr int kWarps = kPointsBlock / 32, kPts = 32 * kPointSets;
   __shared__ CellPoly s_poly[32];

@@ -52,25 +52,15 @@ __device__ inline uint32_t choose_slabs(uint32_t nv, double height, double sum_r
   return static_cast<uint32_t>(s);
 }
 
-// Slab entries that a polygon of nv vertices may have; the arrays are made for the
-// sum of these (fill()).  The slab count keeps to them where sum_rise is the edges'
+// Slab entries that a polygon may have for each of its vertices; the arrays are made
+// for the sum of these (fill()).  The slab count keeps to them where sum_rise is the edges'
 // rise.  It is taken from truncated vertices, and where the polygon lies so far from
 // y = 0 that float32 has a few steps over its height, edges within a step count
 // nothing: such a polygon could have many times the entries, and the fill wrote
 // beyond the arrays.
-__device__ inline uint32_t max_entries(uint32_t nv, double density)
+__host__ __device__ inline uint32_t entries_per_vertex(double density)
 {
-  return static_cast<uint32_t>((density + 2.0) * static_cast<double>(nv));
-}
-
-template <typename T>
-__device__ inline uint32_t slab_of(T y, T ymin, T inv_h, uint32_t ns)
-{
-  T const f = (y - ymin) * inv_h;
-  if (!(f > T{0})) return 0;  // also NaN
-  if (f >= static_cast<T>(ns)) return ns - 1;
-  uint32_t const j = static_cast<uint32_t>(f);
-  return j < ns ? j : ns - 1;
+  return static_cast<uint32_t>(density + 2.0);
 }
 
 // Previous vertex of v within its ring (polygons have few rings).
@@ -276,7 +266,8 @@ __global__ void __launch_bounds__(kIdxBlock)
                      T const* __restrict__ vx, T const* __restrict__ vy, size_t np, T* pminx,
                      T* pminy, T* pmaxx, T* pmaxy, T* invh, uint32_t* nslab, uint32_t* nentries,
                      uint32_t* nvert, uint8_t* exact, uint32_t* __restrict__ prev_out,
-                     uint32_t* __restrict__ spans, float* __restrict__ yslab, double density)
+                     uint32_t* __restrict__ spans, float* __restrict__ yslab, double density,
+                     uint32_t per_vertex)
 {
   __shared__ uint32_t cnt[kMaxSlabs];
   __shared__ T shT[kIdxBlock / 32];
@@ -375,7 +366,7 @@ __global__ void __launch_bounds__(kIdxBlock)
     bad   = block_sum(bad, shU);
     uint32_t slabs = ns;
     T per_unit     = ih;
-    if (local > max_entries(ve - vb, density)) {
+    if (local > static_cast<uint64_t>(per_vertex) * (ve - vb)) {
       // more than the arrays are made for: one slab, which holds every edge once
       slabs    = 1;
       per_unit = T{0};
@@ -403,67 +394,63 @@ __global__ void __launch_bounds__(kIdxBlock)
   }
 }
 
-// The median of the warp's finite values (0 where there is none).
-template <typename T>
-__device__ inline T warp_median(T v)
+// The median of the warp's finite values (0 where there is none), ordered as
+// integers.
+__device__ inline double warp_median(double v)
 {
-  bool const finite    = isfinite(v);
+  long long const key  = order_key(v);
+  bool const finite    = is_finite_bits(v);
   unsigned const which = __ballot_sync(0xFFFFFFFFu, finite);
   int const lane       = static_cast<int>(threadIdx.x & 31u);
   int rank             = 0;  // among the finite ones
   for (int l = 0; l < 32; ++l) {
-    T const o = __shfl_sync(0xFFFFFFFFu, v, l);
-    rank += ((which >> l) & 1u) && (o < v || (o == v && l < lane)) ? 1 : 0;
+    long long const o = __shfl_sync(0xFFFFFFFFu, key, l);
+    rank += ((which >> l) & 1u) && (o < key || (o == key && l < lane)) ? 1 : 0;
   }
   unsigned const mid = __ballot_sync(0xFFFFFFFFu, finite && rank == (__popc(which) - 1) / 2);
-  T const m          = __shfl_sync(0xFFFFFFFFu, v, mid ? __ffs(mid) - 1 : 0);
-  return mid ? m : T{0};
+  double const m     = __shfl_sync(0xFFFFFFFFu, v, mid ? __ffs(mid) - 1 : 0);
+  return mid ? m : 0.0;
 }
 
-// Where the layer lies, from 32 polygons spread over it, by one warp.
-// place[0], place[1]: the origin that edge bounds are relative to, the medians of
-// the polygons' lower sides.  Float32 then resolves the layer wherever it lies, and
-// a few polygons that lie apart from the others (or without vertices) do not move
-// it.  (Relative to (0, 0) 10M points x 31 polygons of 100 sides at (10000, 20000)
-// took 14.1 ms, as the bounds told nothing; 321 us this way.)
-// place[2] (median_share): the share of the polygons' common box that their median
-// box takes along an axis (the smaller one of the two axes).
-template <typename T>
-__device__ inline void layer_place(T const* __restrict__ pminx, T const* __restrict__ pminy,
-                                   T const* __restrict__ pmaxx, T const* __restrict__ pmaxy,
-                                   size_t np, T* place)
+// Where the layer lies along an axis, from 32 polygons spread over it, by one warp
+// (lo, hi: their lower and upper sides).
+// place[0]: the origin that edge bounds are relative to, the median of the polygons'
+// lower sides.  Float32 then resolves the layer wherever it lies, and a few polygons
+// that lie apart from the others (or without vertices) do not move it.  (Relative to
+// 0 10M points x 31 polygons of 100 sides at (10000, 20000) took 14.1 ms, as the
+// bounds told nothing; 321 us this way.)
+// place[2]: the share of the polygons' common box that their median box takes.
+__device__ inline void layer_place(double const* __restrict__ lo, double const* __restrict__ hi,
+                                   size_t np, double* place)
 {
-  uint32_t const lane  = threadIdx.x & 31u;
-  T const* const lo[2] = {pminx, pminy};
-  T const* const hi[2] = {pmaxx, pmaxy};
-  T share              = T{1};
-  for (int a = 0; a < 2; ++a) {
-    size_t const p = np * lane / 32;
-    T const l = np ? lo[a][p] : T{0}, h = np ? hi[a][p] : T{0};
-    T const origin = warp_median(l);
-    T const side   = warp_median(h - l);
-    T least = isfinite(l) ? l : origin, most = isfinite(h) ? h : origin;
-    for (int o = 16; o > 0; o >>= 1) {
-      T const b = __shfl_xor_sync(0xFFFFFFFFu, least, o), c = __shfl_xor_sync(0xFFFFFFFFu, most, o);
-      least     = b < least ? b : least;
-      most      = c > most ? c : most;
-    }
-    T const s = side / (most - least);
-    share     = s < share ? s : share;
-    if (lane == 0) place[a] = origin;
+  uint32_t const lane = threadIdx.x & 31u;
+  size_t const p      = np * lane / 32;
+  double const l = np ? lo[p] : 0.0, h = np ? hi[p] : 0.0;
+  double const origin = warp_median(l);
+  double const side   = warp_median(h - l);
+  long long least = order_key(is_finite_bits(l) ? l : origin),
+            most  = order_key(is_finite_bits(h) ? h : origin);
+  for (int o = 16; o > 0; o >>= 1) {
+    long long const b = __shfl_xor_sync(0xFFFFFFFFu, least, o),
+                    c = __shfl_xor_sync(0xFFFFFFFFu, most, o);
+    least             = b < least ? b : least;
+    most              = c > most ? c : most;
   }
-  if (lane == 0) place[2] = share;
+  if (lane == 0) {
+    place[0] = origin;
+    place[2] = side / (from_order_key(most) - from_order_key(least));
+  }
 }
 
 // The anchor grid: 2^(e-22) where 2^e bounds every finite polygon coordinate
-// (grid[0]), and layer_place's three values (grid[1] on).
+// (grid[0]), and, if `place`, layer_place's values of x and y in turn (grid[1] on).
 // The largest magnitude is taken on the bit patterns (sign cleared,
 // non-finite skipped), which order as the magnitudes: integer work only, so
 // the FP64 pipe of the one SM this runs on stays out of the loop.
 template <typename T>
 __device__ inline void anchor_grid(T const* __restrict__ pminx, T const* __restrict__ pminy,
                                    T const* __restrict__ pmaxx, T const* __restrict__ pmaxy,
-                                   size_t np, T* grid)
+                                   size_t np, T* grid, bool place)
 {
   using U             = typename uint_of<T>::type;
   constexpr U kMag    = ~(U{1} << (8 * sizeof(U) - 1));
@@ -498,16 +485,22 @@ __device__ inline void anchor_grid(T const* __restrict__ pminx, T const* __restr
       frexp(mv > T{0} ? mv : T{1}, &e);  // mv < 2^e
       *grid = ldexp(T{1}, e - 22);
     }
-  } else if (threadIdx.x < 64) {
-    layer_place<T>(pminx, pminy, pmaxx, pmaxy, np, grid + 1);
+  } else if (threadIdx.x < 96) {
+    if constexpr (std::is_same<T, double>::value) {
+      if (place) {
+        bool const y = threadIdx.x >= 64;
+        layer_place(y ? pminy : pminx, y ? pmaxy : pmaxx, np, grid + (y ? 2 : 1));
+      }
+    }
   }
 }
 template <typename T>
 __global__ void __launch_bounds__(1024)
   grid_kernel(T const* __restrict__ pminx, T const* __restrict__ pminy,
-              T const* __restrict__ pmaxx, T const* __restrict__ pmaxy, size_t np, T* grid)
+              T const* __restrict__ pmaxx, T const* __restrict__ pmaxy, size_t np, T* grid,
+              bool place)
 {
-  anchor_grid<T>(pminx, pminy, pmaxx, pmaxy, np, grid);
+  anchor_grid<T>(pminx, pminy, pmaxx, pmaxy, np, grid, place);
 }
 
 // Few polygons: the anchor grid (as grid_kernel) and the three scans (slabs,
@@ -520,12 +513,12 @@ template <typename T>
 __global__ void __launch_bounds__(1024)
   few_polygons_kernel(T const* __restrict__ pminx, T const* __restrict__ pminy,
                       T const* __restrict__ pmaxx, T const* __restrict__ pmaxy, uint32_t np,
-                      T* grid, uint32_t const* __restrict__ nslab,
+                      T* grid, bool place, uint32_t const* __restrict__ nslab,
                       uint32_t const* __restrict__ nent, uint32_t const* __restrict__ nvert,
                       uint32_t* __restrict__ slab_base, uint32_t* __restrict__ ebase,
                       uint32_t* __restrict__ vbeg, uint32_t* __restrict__ vend)
 {
-  anchor_grid<T>(pminx, pminy, pmaxx, pmaxy, np, grid);
+  anchor_grid<T>(pminx, pminy, pmaxx, pmaxy, np, grid, place);
   __shared__ uint32_t total;
   uint32_t const* const in[3] = {nslab, nent, nvert};
   uint32_t* const out[3]      = {slab_base, ebase, vbeg};
@@ -548,7 +541,8 @@ __global__ void __launch_bounds__(1024)
 }
 
 // Pass 2: anchors, float32 edges, slab offsets and entries, vertical x.
-template <typename T>
+// Bounds: the entries carry edge bounds, or, with `float32` too, the device decides.
+template <typename T, bool Bounds>
 __global__ void __launch_bounds__(kIdxBlock)
   index_fill_kernel(uint32_t const* __restrict__ po, uint32_t const* __restrict__ ro,
                     T const* __restrict__ vx, T const* __restrict__ vy, size_t np,
@@ -557,7 +551,7 @@ __global__ void __launch_bounds__(kIdxBlock)
                     T const* __restrict__ invh, uint32_t const* __restrict__ nslab,
                     uint32_t const* __restrict__ slab_base, uint32_t const* __restrict__ entry_base,
                     uint32_t const* __restrict__ vert_base, T const* __restrict__ grid,
-                    bool float32, bool bounds, T bounds_share, T* anchor_x, T* anchor_y, long long* aix, long long* aiy,
+                    bool float32, T bounds_share, T* anchor_x, T* anchor_y, long long* aix, long long* aiy,
                     float4* box32, float* invh32, float* maxoff, uint32_t const* __restrict__ prev,
                     uint32_t const* __restrict__ spans, float4* edge32, uint32_t* slab_start,
                     uint32_t* slab_edges, float4* slab_e32, T* vert_x, float* vert_x32,
@@ -571,11 +565,9 @@ __global__ void __launch_bounds__(kIdxBlock)
   T const g    = *grid;
   T const ginv = T{1} / g;  // g is a power of two: v * ginv == v / g while 1/g is finite
   bool const gi = isfinite(ginv);
-  T const ox = grid[1], oy = grid[2];  // the bounds' origin
-  if (float32 && bounds) {
-    bounds  = has_bounds(grid[3], bounds_share);
-    float32 = !bounds;
-  }
+  bool const bounds = Bounds && (!float32 || has_bounds(grid + 1, bounds_share));
+  T const ox = Bounds ? grid[1] : T{0}, oy = Bounds ? grid[2] : T{0};  // the bounds' origin
+  if (bounds) float32 = false;
   for (size_t p = blockIdx.x; p < np; p += gridDim.x) {
     uint32_t const r0 = po[p], r1 = po[p + 1];
     uint32_t const vb = ro[r0], ve = ro[r1];
@@ -599,7 +591,7 @@ __global__ void __launch_bounds__(kIdxBlock)
       box32[p]    = make_float4(static_cast<float>(pminx[p] - cx), static_cast<float>(ymin - cy),
                                 static_cast<float>(pmaxx[p] - cx), static_cast<float>(pmaxy[p] - cy));
       invh32[p]   = static_cast<float>(invh[p]);
-      if constexpr (std::is_same<T, double>::value)
+      if constexpr (Bounds)
         if (bounds)
           box32[p] = outward_box(truncated_f32(pminx[p] - ox), truncated_f32(ymin - oy),
                                  truncated_f32(pmaxx[p] - ox), truncated_f32(pmaxy[p] - oy));
@@ -639,7 +631,7 @@ __global__ void __launch_bounds__(kIdxBlock)
                                            fmaxf(fabsf(ef.z), fabsf(ef.w))));
       }
       if (sp & kSpanSkip) continue;
-      if constexpr (std::is_same<T, double>::value) {
+      if constexpr (Bounds) {
         if (bounds) {
           ef        = make_float4(truncated_f32(vx[v] - ox), truncated_f32(vy[v] - oy),
                                   truncated_f32(vx[pv] - ox), truncated_f32(vy[pv] - oy));
@@ -909,7 +901,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
   ax_        = Buffer<T>(alloc, np);
   ay_        = Buffer<T>(alloc, np);
   invh_      = Buffer<T>(alloc, np);
-  grid_      = Buffer<T>(alloc, 4);
+  grid_      = Buffer<T>(alloc, 5);
   maxoff_    = Buffer<float>(alloc, np);
   invh32_    = Buffer<float>(alloc, np);
   box32_     = Buffer<float4>(alloc, np);
@@ -934,18 +926,19 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
     index_count_kernel<T><<<grd, kIdxBlock, 0, s>>>(
       po, ro, vx, vy, np, pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
       invh_.data(), nslab_.data(), nent.data(), nvert.data(), exact_.data(), prev_.data(),
-      spans.data(), yslab.data(), density);
+      spans.data(), yslab.data(), density, entries_per_vertex(density));
     CSPT_CHECK_LAUNCH();
   }
   if (np <= kFewPolygons) {
     few_polygons_kernel<T><<<1, 1024, 0, s>>>(
       pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(), static_cast<uint32_t>(np),
-      grid_.data(), nslab_.data(), nent.data(), nvert.data(), slab_base_.data(), ebase.data(),
+      grid_.data(), edge_bounds, nslab_.data(), nent.data(), nvert.data(), slab_base_.data(),
+      ebase.data(),
       vbeg_.data(), vend_.data());
     CSPT_CHECK_LAUNCH();
   } else {
     grid_kernel<T><<<1, 1024, 0, s>>>(pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
-                                      np, grid_.data());
+                                      np, grid_.data(), edge_bounds);
     CSPT_CHECK_LAUNCH();
     exclusive_scan<uint32_t>(nslab_.data(), slab_base_.data(), np, slab_base_.data() + np, alloc);
     exclusive_scan<uint32_t>(nent.data(), ebase.data(), np, ebase.data() + np, alloc);
@@ -962,7 +955,7 @@ PolygonIndex<T>::PolygonIndex(uint32_t const* po, size_t npo, uint32_t const* ro
   // itself plus 1/32 slab at each end, float32 slab coordinates within
   // 2^-12 slab), and the sum over edges of r ns / H is at most density V
   // (with one slab every edge spans one); a polygon whose rises float32 does not
-  // tell is counted again with one slab (max_entries).  So (density + 2) entries per
+  // tell is counted again with one slab (entries_per_vertex).  So (density + 2) entries per
   // vertex, 1 + density / 2 slabs per polygon and one vertical edge per
   // vertex bound the arrays without reading the counts back: no host
   // synchronisation.  Only where those bounds reach 2^32 (the 32-bit
@@ -1026,14 +1019,19 @@ void PolygonIndex<T>::fill()
   if (np == 0) CSPT_CUDA_TRY(cudaMemsetAsync(slab_start_.data(), 0, sizeof(uint32_t), s));
   Buffer<float2> vxy32(alloc, build_float32 ? nv : 0);
   if (np > 0) {
-    index_fill_kernel<T><<<grd, kIdxBlock, 0, s>>>(
-      po, ro, vx, vy, np, pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
-      invh_.data(), nslab_.data(), slab_base_.data(), z->ebase.data(), vbeg_.data(), grid_.data(),
-      build_float32, z->edge_bounds, z->bounds_share, ax_.data(), ay_.data(), aix_.data(), aiy_.data(), box32_.data(),
-      invh32_.data(), maxoff_.data(), prev_.data(), z->spans.data(), edge32_.data(),
-      slab_start_.data(),
-      slab_edges_.data(), slab_e32_.data(), vert_x_.data(), vert_x32_.data(), vxy32.data(),
-      z->yslab.data());
+    auto const launch = [&](auto kernel) {
+      kernel<<<grd, kIdxBlock, 0, s>>>(
+        po, ro, vx, vy, np, pminx_.data(), pminy_.data(), pmaxx_.data(), pmaxy_.data(),
+        invh_.data(), nslab_.data(), slab_base_.data(), z->ebase.data(), vbeg_.data(),
+        grid_.data(), build_float32, z->bounds_share, ax_.data(), ay_.data(), aix_.data(),
+        aiy_.data(), box32_.data(), invh32_.data(), maxoff_.data(), prev_.data(),
+        z->spans.data(), edge32_.data(), slab_start_.data(), slab_edges_.data(),
+        slab_e32_.data(), vert_x_.data(), vert_x32_.data(), vxy32.data(), z->yslab.data());
+    };
+    if constexpr (std::is_same<T, double>::value)
+      z->edge_bounds ? launch(index_fill_kernel<T, true>) : launch(index_fill_kernel<T, false>);
+    else
+      launch(index_fill_kernel<T, false>);
     CSPT_CHECK_LAUNCH();
   }
   vxy32.reset();

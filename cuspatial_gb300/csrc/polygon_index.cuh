@@ -85,11 +85,12 @@ __device__ inline float4 outward_box(float x0, float y0, float x1, float y1)
                      __fadd_ru(fmaxf(x0, x1), wx), __fadd_ru(fmaxf(y0, y1), wy));
 }
 
-// Whether an index that leaves the choice to the device carries edge bounds.
+// Whether an index that leaves the choice to the device carries edge bounds
+// (place: the view's origin).
 template <typename T>
-__device__ inline bool has_bounds(T median_share, T bounds_share)
+__device__ inline bool has_bounds(T const* place, T bounds_share)
 {
-  return median_share >= bounds_share;
+  return place[2] >= bounds_share && place[3] >= bounds_share;
 }
 
 template <typename T>
@@ -108,7 +109,8 @@ struct PolygonIndexView {
   T const* anchor_x;           // box centre rounded to the grid
   T const* anchor_y;
   T const* grid;               // device scalar: the anchor grid step
-  T const* origin;             // (x, y) that edge bounds are relative to, median_share
+  T const* origin;             // x and y that edge bounds are relative to, and the share
+                               // of the common box that the median polygon's takes
   long long const* anchor_ix;  // anchors in grid steps
   long long const* anchor_iy;
   float const* inv_slab_h32;   // inv_slab_h rounded to float
@@ -149,9 +151,9 @@ class PolygonIndex {
   // plans, resident polygon sets).
   // edge_bounds (float64 index): slab entries carry their edge's box in float32,
   // rounded outward (outward_box), in place of the float32 edges.  With
-  // build_float32 too, the device decides: bounds where median_share is at least
-  // bounds_share, else float32 edges; the kernels of both kinds are launched and ask
-  // has_bounds.
+  // build_float32 too, the device decides: bounds where the median polygon takes at
+  // least bounds_share of the common box along both axes, else float32 edges; the
+  // kernels of both kinds are launched and ask has_bounds.
   // defer_fill: return once the per-polygon boxes, slab counts and the anchor
   // grid are enqueued (array sizes come from bounds on the host, so the call
   // does not wait for the device); fill() then writes the slab entries.  Work

@@ -1,8 +1,9 @@
 // Small blocks cut from slabs of an upstream allocator.  Plain C++, so that the
 // host tests can check it.
 //
-// Blocks are multiples of 256 bytes, at most a quarter larger than asked for, and are
-// reused by size.  Slabs double from first_slab to kLastSlab; there are at most
+// Blocks are reused by size: powers of two, or, `fine`, multiples of 256 bytes at
+// most a quarter larger than asked for (what is kept wastes less, what is short-lived
+// is reused less).  Slabs double from first_slab to kLastSlab; there are at most
 // kMaxSlabs, `most` bytes in all.  take() returns null where a block is beyond
 // kMaxBlock or there is no memory for a slab: the caller then asks the upstream
 // itself.  give() allocates nothing: take() has made room for
@@ -22,8 +23,8 @@ class SlabArena {
   static constexpr size_t kLastSlab = size_t{32} << 20;
   static constexpr int kMaxSlabs = 8;
 
-  SlabArena(Upstream up, size_t first_slab, size_t most)
-    : up_(up), first_slab_(first_slab), next_slab_(first_slab), most_(most)
+  SlabArena(Upstream up, size_t first_slab, size_t most, bool fine)
+    : up_(up), first_slab_(first_slab), next_slab_(first_slab), most_(most), fine_(fine)
   {
   }
   ~SlabArena()
@@ -108,11 +109,17 @@ class SlabArena {
   // 1, 2, 3 and 4 units of kMinBlock, then four sizes an octave
   static constexpr int kClasses = 52;
   static_assert(kMinBlock << 14 == kMaxBlock && kLastSlab >= kMaxBlock, "sizes");
-  static int size_class(size_t bytes, size_t& size)
+  int size_class(size_t bytes, size_t& size) const
   {
     size_t const units = (bytes + kMinBlock - 1) / kMinBlock;
     int octave         = 2;  // 2^octave < units <= 2^(octave + 1)
     while ((size_t{2} << octave) < units) ++octave;
+    if (!fine_) {
+      size = kMinBlock;
+      while (size < bytes) size *= 2;
+      if (units > 4) return 4 * octave - 1;
+      return units == 3 ? 3 : static_cast<int>(units) - 1;
+    }
     size_t const step = units <= 4 ? 1 : size_t{1} << (octave - 2);
     size_t const k    = (units + step - 1) / step;  // 5 to 8 beyond 4 units
     size              = k * step * kMinBlock;
@@ -140,6 +147,7 @@ class SlabArena {
 
   Upstream up_;
   size_t first_slab_, next_slab_, most_;
+  bool fine_;
   Slab slabs_[kMaxSlabs];
   int nslabs_ = 0;
   char *at_ = nullptr, *end_ = nullptr;  // the rest of the last slab

@@ -1,6 +1,6 @@
 """The slabs that small device blocks are cut from (csrc/slab_arena.h), on the host:
-random takes and gives against a model (no overlap, alignment, at most a quarter
-more than asked for beyond 4 units, reuse, the limits), slabs given back by trim()
+random takes and gives against a model (no overlap, alignment, sizes at most twice
+or a quarter beyond what is asked for, reuse, the limits), slabs given back by trim()
 and at the end, no allocation by give(), and an upstream without memory."""
 
 import shutil
@@ -66,13 +66,14 @@ struct Up {
 };
 using Arena = cspt::SlabArena<Up>;
 
-static void walk(unsigned seed, std::size_t first, std::size_t most, std::size_t limit)
+static void walk(unsigned seed, std::size_t first, std::size_t most, std::size_t limit,
+                 bool fine)
 {
   State st;
   st.limit = limit;
   std::mt19937 rng(seed);
   {
-    Arena a(Up{&st}, first, most);
+    Arena a(Up{&st}, first, most, fine);
     std::map<char*, std::pair<std::size_t, std::size_t>> live;  // asked, room up to the next block
     for (int step = 0; step < 4000; ++step) {
       bool const shrink = (step / 500) %% 2;
@@ -129,20 +130,23 @@ static void walk(unsigned seed, std::size_t first, std::size_t most, std::size_t
 int main()
 {
   for (unsigned s = 0; s < 6; ++s) {
-    walk(s, std::size_t{2} << 20, std::size_t{158} << 20, SIZE_MAX);
-    walk(s, std::size_t{1} << 20, std::size_t{31} << 20, SIZE_MAX);
-    walk(s, std::size_t{2} << 20, std::size_t{158} << 20, std::size_t{7} << 20);
-    walk(s, std::size_t{2} << 20, std::size_t{158} << 20, 0);
+    walk(s, std::size_t{2} << 20, std::size_t{158} << 20, SIZE_MAX, false);
+    walk(s, std::size_t{1} << 20, std::size_t{31} << 20, SIZE_MAX, true);
+    walk(s, std::size_t{2} << 20, std::size_t{158} << 20, std::size_t{7} << 20, s %% 2 == 0);
+    walk(s, std::size_t{2} << 20, std::size_t{158} << 20, 0, true);
   }
   // the size of a block: what two of them of one slab lie apart
-  State st;
-  Arena a(Up{&st}, std::size_t{32} << 20, std::size_t{32} << 20);
-  for (std::size_t n = 1; n <= Arena::kMaxBlock / 4; n += 1 + n / 7) {
-    char* const p = static_cast<char*>(a.take(n));
-    char* const q = static_cast<char*>(a.take(n));
-    if (!p || !q) break;
-    std::size_t const size = q - p;
-    CHECK(size >= n && size %% 256 == 0 && (size <= n + n / 4 || size < n + 256));
+  for (bool fine : {false, true}) {
+    State st;
+    Arena a(Up{&st}, std::size_t{32} << 20, std::size_t{32} << 20, fine);
+    for (std::size_t n = 1; n <= Arena::kMaxBlock / 4; n += 1 + n / 7) {
+      char* const p = static_cast<char*>(a.take(n));
+      char* const q = static_cast<char*>(a.take(n));
+      if (!p || !q) break;
+      std::size_t const size = q - p;
+      CHECK(size >= n && size %% 256 == 0 &&
+            (size <= (fine ? n + n / 4 : 2 * n) || size < n + 256));
+    }
   }
   std::puts("ok");
 }
