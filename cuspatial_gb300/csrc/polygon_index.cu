@@ -53,11 +53,11 @@ __device__ inline uint32_t choose_slabs(uint32_t nv, double height, double sum_r
 }
 
 // Slab entries that a polygon may have for each of its vertices; the arrays are made
-// for the sum of these (fill()).  The slab count keeps to them where sum_rise is the edges'
-// rise.  It is taken from truncated vertices, and where the polygon lies so far from
-// y = 0 that float32 has a few steps over its height, edges within a step count
-// nothing: such a polygon could have many times the entries, and the fill wrote
-// beyond the arrays.
+// for the sum of these (fill()).  The slab count keeps to them where sum_rise is the
+// edges' rise.  That is a float32 sum, of truncated vertices where the polygon is many
+// float32 steps high: a polygon that has more entries all the same is counted again
+// with one slab.  (With truncated vertices for all, edges within a step counted
+// nothing, and the fill of a polygon few steps high wrote far beyond the arrays.)
 __host__ __device__ inline uint32_t entries_per_vertex(double density)
 {
   return static_cast<uint32_t>(density + 2.0);
@@ -310,6 +310,14 @@ __global__ void __launch_bounds__(kIdxBlock)
       mny      = from_order_key(block_min_ll(ky0, shL));
       mxx      = from_order_key(block_max_ll(kx1, shL));
       mxy      = from_order_key(block_max_ll(ky1, shL));
+      // Up to 64 float32 steps of y high (a polygon of 30 units at y = 1e7), its edges
+      // lose too much to the truncation: their rises are taken in float64.
+      float const fy0 = truncated_f32(mny), fy1 = truncated_f32(mxy);
+      if ((fy1 - fy0) * 131072.0f <= fmaxf(fabsf(fy0), fabsf(fy1))) {
+        rise = 0.0f;
+        for (uint32_t v = vb + threadIdx.x; v < ve; v += kIdxBlock)
+          rise += fabsf(truncated_f32(vy[prev_out[v]] - vy[v]));
+      }
       sum_rise = static_cast<double>(block_sum(rise, shF));
     } else {
       mnx = INFINITY;
