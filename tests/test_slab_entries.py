@@ -47,7 +47,7 @@ def test_truncated_rises_would_exceed_the_arrays(top, vertices):
             s = density * nv * height / np.abs(np.diff(step)).sum()
             slabs = int(max(1.0, min(s, 0.5 * density * nv, 4096)))
             entries += np.abs(np.diff(y)).sum() * slabs / height
-        assert entries > 4 * (density + 2) * len(P.y)
+        assert entries > 2 * (density + 2) * len(P.y)
 
 
 @pytest.mark.gpu
