@@ -223,6 +223,7 @@ constexpr int kPointSets        = 4;   // rounds of 32 points a warp takes toget
 // 300k points of 1000 sides - / 181 / 195)
 constexpr size_t kPointsPerCell = 16;
 constexpr uint32_t kGridMin = 32, kGridMax = 1024;  // cells along an axis
+constexpr uint32_t kRowEntries = 512;  // entries of a polygon that any row streams
 
 struct CellPoly {
   float4 box;  // outward
@@ -374,8 +375,14 @@ __global__ void __launch_bounds__(kPointsBlock)
                        jc = slab_lookup(cy, f.y0, f.invh, f.ns);
         uint32_t const E0 = ix.slab_start[f.slab0 + j0], E1 = ix.slab_start[f.slab0 + j1 + 1];
         uint32_t const C0 = ix.slab_start[f.slab0 + jc], C1 = ix.slab_start[f.slab0 + jc + 1];
+        uint32_t const all = ix.slab_start[f.slab0 + f.ns] - ix.slab_start[f.slab0];
+        // (a row that holds much of a large polygon decides little: 31 polygons of 1000
+        // sides one cell wide, 200k points, exact: 948 us with its entries streamed, 313
+        // without, 663 without the grid)
+        bool const many = E1 - E0 > kRowEntries && E1 - E0 > all / 8u;
+        if (many) meets = true;
 #pragma unroll 4
-        for (uint32_t k = E0; k < E1; ++k) {
+        for (uint32_t k = many ? E1 : E0; k < E1; ++k) {
           float4 const e = ix.slab_e32[k];
           bool const near = !(xl > e.z || xu < e.x || yl > e.w || yu < e.y);
           // (beyond the cell's box the centre sees it left, right, above or below)
@@ -855,8 +862,7 @@ bool points_use_grid(size_t n, size_t nv, bool filtered)
 // of 31 polygons of 1000 sides 100 radii off, 2M points around the others (5 cells a
 // polygon): 1069 us and 639, 10M points (10 cells): 2536 and 2610.  (Where few
 // polygons overlap fewer cells would do: 31 of 1000 sides spread over 20 radii, 140k
-// points, 6 cells: 458 us and 1021.)  The exact method gains in all of these but at
-// small sizes in the second (200k points, 1 cell: 790 us and 663).
+// points, 6 cells: 458 us and 1021.)  The exact method gains in all of these.
 constexpr double kCellsPerPolygon = 8.0;
 
 // Cells along an axis: one cell for every kPointsPerCell points.
