@@ -116,9 +116,10 @@ static_assert(kSortBlock == 256, "the scatter assigns one thread per digit");
 // Stable scatter of one tile: items are ranked per warp with
 // __match_any_sync (rounds in input order), placed in shared memory in the
 // tile's digit order, then written out in that order, so the global writes
-// of each digit's run are contiguous.  Bound by the shared-memory pipe and the
-// waits of few blocks: 50M pairs, four passes: 1657 us with keys and values
-// apart and 61 registers (four blocks an SM), 1423 us as here with six.
+// of each digit's run are contiguous.  Bound by its waits for shared memory (17 of
+// them per issued instruction, the pipe 45% busy; 20M keys) and too few blocks to
+// cover them: 50M pairs, four passes: 1657 us with keys and values apart and 61
+// registers (four blocks an SM), 1423 us as here with six.
 template <typename K, typename Tiles>
 __global__ void __launch_bounds__(kSortBlock, 6)
   radix_scatter_kernel(K const* keys_in, uint32_t const* vals_in, K* keys_out, uint32_t* vals_out,
@@ -127,8 +128,7 @@ __global__ void __launch_bounds__(kSortBlock, 6)
 {
   __shared__ uint32_t wcount[kSortWarps][256];
   __shared__ uint32_t global_base[256];  // the digit's output start minus its tile start
-  // (32-bit keys beside their values: one 64-bit access for both; the shared
-  // memory pipe bounds the kernel)
+  // (32-bit keys beside their values: one 64-bit access for both)
   constexpr bool kPacked = sizeof(K) == 4;
   __shared__ K skey[kPacked ? 1 : kSortTile];
   __shared__ uint32_t sval[kPacked ? 1 : kSortTile];
