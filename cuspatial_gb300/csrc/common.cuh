@@ -13,7 +13,7 @@
 #include <utility>
 
 #include "../../include/cuspatial_gb300.h"
-#include "slab_arena.h"
+#include "slab_arena.cuh"
 
 namespace cspt {
 
@@ -168,7 +168,7 @@ class Allocator {
 // The scratch memory of one call.  A small join takes 60 to 150 buffers, most
 // of them a few kilobytes, and a caller's allocator is a callback (6 to 10 us
 // each from Python, a third of such a call); blocks of up to 4 MiB are cut from
-// slabs of the caller's memory instead (slab_arena.h), which go back when the
+// slabs of the caller's memory instead (slab_arena.cuh), which go back when the
 // call ends.  Blocks are reused within the call in stream order, as the allocator's
 // own are.  Where the caller has no memory for a slab the buffer is allocated as
 // before.

@@ -1,4 +1,4 @@
-"""The slabs that small device blocks are cut from (csrc/slab_arena.h), on the host:
+"""The slabs that small device blocks are cut from (csrc/slab_arena.cuh), on the host:
 random takes and gives against a model (no overlap, alignment, sizes at most twice
 or a quarter beyond what is asked for, reuse, the limits), slabs given back by trim()
 and at the end, no allocation by give(), and an upstream without memory."""
@@ -157,7 +157,7 @@ def test_slab_arena(tmp_path):
     gxx = shutil.which("g++")
     if gxx is None:
         pytest.skip("g++ not available")
-    header = Path(__file__).resolve().parent.parent / "cuspatial_gb300" / "csrc" / "slab_arena.h"
+    header = Path(__file__).resolve().parent.parent / "cuspatial_gb300" / "csrc" / "slab_arena.cuh"
     src, exe = tmp_path / "arena.cpp", tmp_path / "arena"
     src.write_text(SOURCE % header)
     subprocess.run([gxx, "-O1", "-std=c++17", str(src), "-o", str(exe)],
